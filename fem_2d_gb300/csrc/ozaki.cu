@@ -30,8 +30,14 @@
 // an error flag, waits once more (bounded) for its MMAs in flight, frees its TMEM and returns.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <functional>
 #include <mutex>
+#include <numeric>
+#include <queue>
+#include <utility>
+#include <vector>
 
 #include "device.h"
 #include "ozaki.h"
@@ -1243,28 +1249,48 @@ void TcSpmm::build(Ctx& c, int64_t n, const std::vector<int32_t>& grp_h, const s
   plane_units = pcur;
   exp_count = ecur;
   nzero = (int)zr.size();
-  // the product kernel's order: CTA b takes the runs b, b + grid, ... (two CTAs per SM)
+  // The product kernel's order (two CTAs per SM): runs by falling cost, each to the CTA with the least
+  // work so far, every CTA's runs then in pattern order (neighbouring runs gather the same rows of X).
+  // An item costs about the same whatever its rows, since the gather, the MMAs and the waits are per item,
+  // so its weight grows slowly with R. Dealing the runs out in turn instead left the busiest CTA with
+  // 53 items against a mean of 36 at 83k DoFs, and that CTA sets the kernel's time.
   grid = std::max(1, std::min(std::max(nruns, 1), 2 * c.num_sms));
-  std::vector<TcSpmmItem> ci;
-  std::vector<int32_t> cp;
-  ci.reserve(it.size());
-  for (int b = 0; b < grid; b++) {
-    cp.push_back((int32_t)ci.size());
-    for (int g = b; g < nruns; g += grid)
-      for (int q = run_first[g]; q < run_first[g + 1]; q++) {
-        const int4 w = it[q];
-        TcSpmmItem m;
-        m.cbase = row_ptr[grp_h[g]] + w.y;
-        m.poff = po[q];
-        m.eoff = (int32_t)eo[q];
-        m.r0 = grp_h[g];
-        m.R = (int16_t)w.z;
-        m.Lc = (int16_t)w.w;
-        m.last = q + 1 == run_first[g + 1] ? 1 : 0;
-        ci.push_back(m);
-      }
+  auto cost = [&](int g) {
+    return (int64_t)(run_first[g + 1] - run_first[g]) * (64 + grp_h[g + 1] - grp_h[g]);
+  };
+  std::vector<int32_t> by_cost(nruns), owner(nruns, 0);
+  std::iota(by_cost.begin(), by_cost.end(), 0);
+  std::stable_sort(by_cost.begin(), by_cost.end(), [&](int32_t x, int32_t y) { return cost(x) > cost(y); });
+  {
+    typedef std::pair<int64_t, int> Load;   // work so far, CTA
+    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
+    for (int b = 0; b < grid; b++) least.push({0, b});
+    for (int32_t g : by_cost) {
+      Load l = least.top();
+      least.pop();
+      owner[g] = l.second;
+      l.first += cost(g);
+      least.push(l);
+    }
   }
-  cp.push_back((int32_t)ci.size());
+  std::vector<TcSpmmItem> ci(it.size());
+  std::vector<int32_t> cp(grid + 1, 0);
+  for (int g = 0; g < nruns; g++) cp[owner[g] + 1] += run_first[g + 1] - run_first[g];
+  for (int b = 0; b < grid; b++) cp[b + 1] += cp[b];
+  std::vector<int32_t> fill(cp.begin(), cp.end() - 1);
+  for (int g = 0; g < nruns; g++)
+    for (int q = run_first[g]; q < run_first[g + 1]; q++) {
+      const int4 w = it[q];
+      TcSpmmItem m;
+      m.cbase = row_ptr[grp_h[g]] + w.y;
+      m.poff = po[q];
+      m.eoff = (int32_t)eo[q];
+      m.r0 = grp_h[g];
+      m.R = (int16_t)w.z;
+      m.Lc = (int16_t)w.w;
+      m.last = q + 1 == run_first[g + 1] ? 1 : 0;
+      ci[fill[owner[g]]++] = m;
+    }
   items.upload(it, c.stream);
   poff.upload(po, c.stream);
   eoff.upload(eo, c.stream);
