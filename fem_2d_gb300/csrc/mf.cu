@@ -25,13 +25,17 @@ namespace {
 
 constexpr int PANEL = 32;
 
+// the solve workspace holds one row of kLdW values per front row (row-major, one right-hand side per
+// column), so a row that a parent gathers from a child is one contiguous read
+constexpr int kLdW = 32;
+
 constexpr int MAXKIDS = 4;   // binary dissection nodes; Elem nodes have 2 (U/V) or 4 (T) children
 
 struct FrontDesc {   // device copy of the per-front scalars
   int32_t f, p, parent;
   int32_t kid[MAXKIDS];
   int64_t off, dptr, aptr, aend, eptr;
-  int64_t prow;   // tiled fronts: offset of the front's f + 1 pull-list row pointers
+  int64_t prow;   // tiled fronts: the front's first pull record (one per row)
   int64_t aux;    // tiled fronts with p > kSmallP: offset of the p x p scratch copy of the LU square
 };
 
@@ -296,7 +300,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
   for (int q = r; q < nchunk; q += CL)
     for (int t = threadIdx.x; t < 32 * nb; t += blockDim.x) {
       const int i = q * 32 + (t & 31), c = t >> 5;
-      if (i < f) v[(int64_t)c * f + i] = i < p ? B[(int64_t)D[pm[i]] * ldb + c] : 0.0;
+      if (i < f) v[(int64_t)i * kLdW + c] = i < p ? B[(int64_t)D[pm[i]] * ldb + c] : 0.0;
     }
   __syncthreads();
   for (int slot = 0; slot < MAXKIDS; slot++) {
@@ -309,7 +313,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
     for (int t = threadIdx.x; t < s * nb; t += blockDim.x) {
       const int i = t % s, c = t / s;
       const int row = m[i] < p ? ipm[m[i]] : m[i];   // pivot rows are stored permuted
-      if (((row >> 5) % CL) == r) v[(int64_t)c * f + row] += cw[(int64_t)c * cd.f + cd.p + i];
+      if (((row >> 5) % CL) == r) v[(int64_t)row * kLdW + c] += cw[(int64_t)(cd.p + i) * kLdW + c];
     }
     __syncthreads();
   }
@@ -320,7 +324,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
     const int bw = min(32, p - jb);
     for (int t = threadIdx.x; t < 32 * nb; t += blockDim.x) {
       const int u = t & 31, c = t >> 5;
-      ys[u][c] = u < bw ? v[(int64_t)c * f + jb + u] : 0.0;
+      ys[u][c] = u < bw ? v[(int64_t)(jb + u) * kLdW + c] : 0.0;
     }
     for (int t = threadIdx.x; t < 32 * 32; t += blockDim.x) {
       const int u = t & 31, k = t >> 5;   // row jb+u, col jb+k
@@ -345,7 +349,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
         if (i < first || i >= f) continue;
         double acc = 0.0;
         for (int u = 0; u < bw; u++) acc += F[d.off + (int64_t)(jb + u) * f + i] * ys[u][c];
-        v[(int64_t)c * f + i] -= acc;
+        v[(int64_t)i * kLdW + c] -= acc;
       }
     }
     cluster.sync();
@@ -353,7 +357,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
     if (((jb >> 5) % CL) == r)
       for (int t = threadIdx.x; t < 32 * nb; t += blockDim.x) {
         const int u = t & 31, c = t >> 5;
-        if (u < bw) v[(int64_t)c * f + jb + u] = ys[u][c];
+        if (u < bw) v[(int64_t)(jb + u) * kLdW + c] = ys[u][c];
       }
     __syncthreads();
   }
@@ -378,9 +382,9 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
     for (int t = threadIdx.x; t < 32 * nb; t += blockDim.x) {
       const int i = q * 32 + (t & 31), c = t >> 5;
       if (i >= p) continue;
-      double s = v[(int64_t)c * f + i];
+      double s = v[(int64_t)i * kLdW + c];
       for (int j = p; j < f; j++) s -= F[d.off + (int64_t)j * f + i] * X[(int64_t)D[j] * ldx + c];
-      v[(int64_t)c * f + i] = s;
+      v[(int64_t)i * kLdW + c] = s;
     }
   cluster.sync();
   __shared__ double xs[32][33];
@@ -390,7 +394,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
     const int bw = min(32, p - jb);
     for (int t = threadIdx.x; t < 32 * nb; t += blockDim.x) {
       const int u = t & 31, c = t >> 5;
-      xs[u][c] = u < bw ? v[(int64_t)c * f + jb + u] : 0.0;
+      xs[u][c] = u < bw ? v[(int64_t)(jb + u) * kLdW + c] : 0.0;
     }
     for (int t = threadIdx.x; t < 32 * 32; t += blockDim.x) {
       const int u = t & 31, k = t >> 5;
@@ -412,7 +416,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
         if (i >= jb) continue;
         double acc = 0.0;
         for (int u = 0; u < bw; u++) acc += F[d.off + (int64_t)(jb + u) * f + i] * xs[u][c];
-        v[(int64_t)c * f + i] -= acc;
+        v[(int64_t)i * kLdW + c] -= acc;
       }
     if (((jb >> 5) % CL) == r)
       for (int t = threadIdx.x; t < 32 * nb; t += blockDim.x) {
@@ -493,247 +497,140 @@ struct SolveArgs {
   double* X;
   int64_t ldx;
   int nb;
+  int per;   // right-hand sides per CTA: blockIdx.y takes the columns from blockIdx.y * per on
 };
 
-// the front's gathered right-hand side v[c * f + i] (pivot rows permuted): the pivot rows' entries of
+// One CTA solves a front for `per` right-hand sides. The kernels are bound by the FP64 pipe (under two
+// FMA per clock and SM) where a level fills the chip, and by what is left idle around it elsewhere:
+//   - global rows (B, X, the workspace) are read and written with the right-hand sides along the lanes, so
+//     a row is one contiguous access; the dot products take the rows along the lanes and read the factor
+//     contiguously. Shared columns have odd length, so both orders are free of bank conflicts.
+//   - a level with few fronts per SM splits the right-hand sides over CTAs (blockIdx.y): the SMs then
+//     finish together, and one CTA's gathers overlap another's dot products.
+// At 83k DoFs (1,179 leaf fronts, 24 right-hand sides) the leaf level took 348 / 315 us forward / backward
+// with column-major rows and one CTA per front; a whole solve went from 0.99 to 0.70 ms there, from 0.48 to
+// 0.31 ms at 29k DoFs and from 5.95 to 4.93 ms at 1M (13 right-hand sides on average), upper levels included.
+
+// the front's gathered right-hand side v[c * ld + i] (pivot rows permuted): the pivot rows' entries of
 // B, then each child's update vector added in slot order (rows are distinct within one child, so no
 // atomics are needed, and the fixed order makes the sums, and the whole solve, reproducible bit for bit)
 __device__ __forceinline__ void gather_front_rhs(const FrontDesc& d, const FrontDesc* __restrict__ fd,
                                                  const int32_t* __restrict__ emap, const int32_t* __restrict__ ipm,
                                                  const double* __restrict__ W, const int64_t* __restrict__ woff,
                                                  const double* __restrict__ B, int64_t ldb,
-                                                 const int32_t* __restrict__ D, const int32_t* __restrict__ pm, int nb,
-                                                 double* v) {
+                                                 const int32_t* __restrict__ D, const int32_t* __restrict__ pm, int c0,
+                                                 int w, int ld, double* v) {
   const int f = d.f, p = d.p;
-  for (int t = threadIdx.x; t < f * nb; t += blockDim.x) {
-    const int i = t % f, c = t / f;
-    v[t] = i < p ? B[(int64_t)D[pm[i]] * ldb + c] : 0.0;
+  for (int t = threadIdx.x; t < f * w; t += blockDim.x) {
+    const int i = t / w, c = t - i * w;
+    v[c * ld + i] = i < p ? B[(int64_t)D[pm[i]] * ldb + c0 + c] : 0.0;
   }
   for (int slot = 0; slot < MAXKIDS; slot++) {
     const int ch = d.kid[slot];
     if (ch < 0) continue;   // uniform across the CTA
     const FrontDesc cd = fd[ch];
     const int sz = cd.f - cd.p;
-    const double* cw = W + woff[ch];
+    const double* cw = W + woff[ch] + (int64_t)cd.p * kLdW + c0;
     const int32_t* m = emap + cd.eptr;
     __syncthreads();
-    for (int t = threadIdx.x; t < sz * nb; t += blockDim.x) {
-      const int i = t % sz, c = t / sz;
+    for (int t = threadIdx.x; t < sz * w; t += blockDim.x) {
+      const int i = t / w, c = t - i * w;
       const int mi = m[i];
       const int row = mi < p ? ipm[mi] : mi;   // pivot rows are stored permuted
-      v[c * f + row] += cw[(int64_t)c * cd.f + cd.p + i];
+      v[c * ld + row] += cw[(int64_t)i * kLdW + c];
     }
   }
   __syncthreads();
 }
 
-// forward solve of one small front by the calling CTA (sm: (f + p) * nb doubles)
-__device__ __forceinline__ void forward_small_front(int fr, const SolveArgs& a, double* sm) {
-  const FrontDesc* __restrict__ fd = a.fd;
-  const int32_t* __restrict__ dofs = a.dofs;
-  const int32_t* __restrict__ emap = a.emap;
-  const int32_t* __restrict__ perm = a.perm;
-  const int32_t* __restrict__ iperm = a.iperm;
-  const int64_t* __restrict__ piv_off = a.piv_off;
-  const int64_t* __restrict__ woff = a.woff;
-  const double* __restrict__ F = a.F;
-  const double* __restrict__ B = a.B;
-  const int64_t ldb = a.ldb;
-  const int nb = a.nb;
-  double* __restrict__ W = a.W;
-  const FrontDesc d = fd[fr];
-  const int f = d.f, p = d.p;
-  double* v = sm;            // v[c * f + i]
-  double* y = sm + f * nb;   // y[c * p + i]
-  const int32_t* D = dofs + d.dptr;
-  const int32_t* pm = perm + piv_off[fr];
-  const int32_t* ipm = iperm + piv_off[fr];
-  const double* A = F + d.off;
-  gather_front_rhs(d, fd, emap, ipm, W, woff, B, ldb, D, pm, nb, v);
-  // the unit lower triangle: row i is a dot product of length i, so a thread takes the rows q and
-  // p - 1 - q (p - 1 terms together) and the lanes of a warp run equally long
-  const int hp = (p + 1) >> 1;
-  for (int t = threadIdx.x; t < hp * nb; t += blockDim.x) {
-    const int q = t % hp, c = t / hp;
-    const double* vc = v + c * f;
-    y[c * p + q] = vc[q] + col_dot(A + q, f, vc, 0, q);
-    const int i2 = p - 1 - q;
-    if (i2 != q) y[c * p + i2] = vc[i2] + col_dot(A + i2, f, vc, 0, i2);
-  }
-  __syncthreads();
-  double* out = W + woff[fr];
-  const int s = f - p;
-  for (int t = threadIdx.x; t < s * nb; t += blockDim.x) {
-    const int i = p + t % s, c = t / s;
-    const double* yc = y + c * p;
-    out[(int64_t)c * f + i] = v[c * f + i] - col_dot(A + i, f, yc, 0, p);
-  }
-  for (int t = threadIdx.x; t < p * nb; t += blockDim.x) {
-    const int i = t % p, c = t / p;
-    out[(int64_t)c * f + i] = y[c * p + i];
-  }
-}
+// shared memory of the two kernels in doubles per right-hand side
+__host__ __device__ constexpr int forward_cols(int f, int p) { return (f | 1) + (p | 1); }
+__host__ __device__ constexpr int backward_cols(int f, int p) { return (p | 1) + ((f - p > p ? f - p : p) | 1); }
 
-// NT threads per front: 256 for wide levels, 1024 for the narrow upper levels of the tree, where a
-// few fronts occupy the GPU and each front's dependent dot products set the level's latency
+// NT threads per front: 256 for wide levels, up to 1024 for narrow ones, where a few fronts occupy the
+// GPU and each front's dependent dot products set the level's latency
 template <int NT>
 __global__ void __launch_bounds__(NT) mf_forward_small_kernel(const int32_t* __restrict__ lf, SolveArgs a) {
   extern __shared__ double sm[];
-  forward_small_front(lf[blockIdx.x], a, sm);
-}
-
-// backward solve of one small front by the calling CTA (sm: f * nb doubles)
-__device__ __forceinline__ void backward_small_front(int fr, const SolveArgs& a, double* sm) {
-  const FrontDesc* __restrict__ fd = a.fd;
-  const int32_t* __restrict__ dofs = a.dofs;
-  const int64_t* __restrict__ woff = a.woff;
-  const double* __restrict__ F = a.F;
-  const double* __restrict__ W = a.W;
-  const int nb = a.nb;
-  double* __restrict__ X = a.X;
-  const int64_t ldx = a.ldx;
-  const FrontDesc d = fd[fr];
-  const int f = d.f, p = d.p;
-  if (p == 0) return;
-  const int s = f - p;
-  double* xs = sm;            // xs[c * s + j]: solved struct unknowns
-  double* z = sm + s * nb;    // z[c * p + i]
-  const int32_t* D = dofs + d.dptr;
-  const double* A = F + d.off;
-  const double* v = W + woff[fr];
-  for (int t = threadIdx.x; t < s * nb; t += blockDim.x) {
-    const int j = t % s, c = t / s;
-    xs[t] = X[(int64_t)D[p + j] * ldx + c];
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < p * nb; t += blockDim.x) {
-    const int i = t % p, c = t / p;
-    const double* xc = xs + c * s;
-    z[c * p + i] = v[(int64_t)c * f + i] - col_dot(A + (int64_t)p * f + i, f, xc, 0, s);
-  }
-  __syncthreads();
-  // the upper triangle: row i is a dot product of length p - i; rows q and p - 1 - q share a thread
+  const int fr = lf[blockIdx.x];
+  const int c0 = blockIdx.y * a.per, w = min(a.per, a.nb - c0);
+  const FrontDesc d = a.fd[fr];
+  const int f = d.f, p = d.p, lv = f | 1, ly = p | 1;
+  double* v = sm;            // v[c * lv + i]
+  double* y = sm + lv * w;   // y[c * ly + i]
+  const double* A = a.F + d.off;
+  gather_front_rhs(d, a.fd, a.emap, a.iperm + a.piv_off[fr], a.W, a.woff, a.B, a.ldb, a.dofs + d.dptr,
+                   a.perm + a.piv_off[fr], c0, w, lv, v);
+  // the unit lower triangle: row i is a dot product of length i, so a thread takes the rows q and
+  // p - 1 - q (p - 1 terms together) and the lanes of a warp run equally long
   const int hp = (p + 1) >> 1;
-  for (int t = threadIdx.x; t < hp * nb; t += blockDim.x) {
-    const int q = t % hp, c = t / hp;
-    const double* zc = z + c * p;
-    X[(int64_t)D[q] * ldx + c] = col_dot(A + q, f, zc, q, p);
+  for (int t = threadIdx.x; t < hp * w; t += blockDim.x) {
+    const int c = t / hp, q = t - c * hp;
+    const double* vc = v + c * lv;
+    y[c * ly + q] = vc[q] + col_dot(A + q, f, vc, 0, q);
     const int i2 = p - 1 - q;
-    if (i2 != q) X[(int64_t)D[i2] * ldx + c] = col_dot(A + i2, f, zc, i2, p);
+    if (i2 != q) y[c * ly + i2] = vc[i2] + col_dot(A + i2, f, vc, 0, i2);
+  }
+  __syncthreads();
+  const int s = f - p;
+  for (int t = threadIdx.x; t < s * w; t += blockDim.x) {
+    const int c = t / s, i = p + t - c * s;
+    v[c * lv + i] -= col_dot(A + i, f, y + c * ly, 0, p);
+  }
+  __syncthreads();
+  double* out = a.W + a.woff[fr] + c0;
+  for (int t = threadIdx.x; t < f * w; t += blockDim.x) {
+    const int i = t / w, c = t - i * w;
+    out[(int64_t)i * kLdW + c] = i < p ? y[c * ly + i] : v[c * lv + i];
   }
 }
 
 template <int NT>
 __global__ void __launch_bounds__(NT) mf_backward_small_kernel(const int32_t* __restrict__ lf, SolveArgs a) {
   extern __shared__ double sm[];
-  backward_small_front(lf[blockIdx.x], a, sm);
-}
-
-// The narrow upper levels of the tree hold a few fronts each, and GB300's FP64 rate per SM (about two
-// FMA per clock) makes one CTA per front the bottleneck there: these variants spread one front over a
-// cluster of CL CTAs (CL SMs). Every CTA gathers the front's right-hand side (cheap) and owns a
-// contiguous slice of its rows; the block that all rows need (y of the forward pass, z of the backward
-// pass) is exchanged through the front's workspace in global memory across one cluster barrier (cluster
-// scope orders the global writes before the reads).
-__device__ __forceinline__ void row_slice(int rows, int r, int& r0, int& r1) {
-  const int per = (rows + CL - 1) / CL;
-  r0 = min(rows, r * per);
-  r1 = min(rows, r0 + per);
-}
-
-__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
-    mf_forward_small_cluster_kernel(const int32_t* __restrict__ lf, SolveArgs a) {
-  extern __shared__ double sm[];
-  cg::cluster_group cluster = cg::this_cluster();
-  const int r = (int)cluster.block_rank();
-  const int fr = lf[blockIdx.x / CL];
-  const FrontDesc* __restrict__ fd = a.fd;
-  const int32_t* __restrict__ emap = a.emap;
-  const int32_t* __restrict__ ipm = a.iperm + a.piv_off[fr];
-  const int32_t* __restrict__ pm = a.perm + a.piv_off[fr];
-  const int nb = a.nb;
-  const FrontDesc d = fd[fr];
-  const int f = d.f, p = d.p, s = f - p;
-  double* v = sm;            // v[c * f + i]: the whole gathered right-hand side
-  double* y = sm + f * nb;   // y[c * p + i]: the whole pivot block after the exchange
-  const int32_t* D = a.dofs + d.dptr;
-  const double* A = a.F + d.off;
-  double* out = a.W + a.woff[fr];
-  gather_front_rhs(d, fd, emap, ipm, a.W, a.woff, a.B, a.ldb, D, pm, nb, v);
-  // y = L11^-1 v[0:p] for this CTA's slice of pivot rows, straight into the workspace
-  int r0, r1;
-  row_slice(p, r, r0, r1);
-  const int pr = r1 - r0;
-  for (int t = threadIdx.x; t < pr * nb; t += blockDim.x) {
-    const int i = r0 + t % pr, c = t / pr;
-    const double* vc = v + c * f;
-    out[(int64_t)c * f + i] = vc[i] + col_dot(A + i, f, vc, 0, i);
-  }
-  cluster.sync();
-  for (int t = threadIdx.x; t < p * nb; t += blockDim.x) {
-    const int i = t % p, c = t / p;
-    y[c * p + i] = out[(int64_t)c * f + i];
-  }
-  __syncthreads();
-  // out[p:f] = v[p:f] - L21 y for this CTA's slice of the remaining rows
-  row_slice(s, r, r0, r1);
-  const int sr = r1 - r0;
-  for (int t = threadIdx.x; t < sr * nb; t += blockDim.x) {
-    const int i = p + r0 + t % sr, c = t / sr;
-    const double* yc = y + c * p;
-    out[(int64_t)c * f + i] = v[c * f + i] - col_dot(A + i, f, yc, 0, p);
-  }
-}
-
-__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
-    mf_backward_small_cluster_kernel(const int32_t* __restrict__ lf, SolveArgs a) {
-  extern __shared__ double sm[];
-  cg::cluster_group cluster = cg::this_cluster();
-  const int r = (int)cluster.block_rank();
-  const int fr = lf[blockIdx.x / CL];
-  const int nb = a.nb;
+  const int fr = lf[blockIdx.x];
+  const int c0 = blockIdx.y * a.per, w = min(a.per, a.nb - c0);
   const FrontDesc d = a.fd[fr];
   const int f = d.f, p = d.p;
-  if (p == 0) return;   // uniform over the cluster: every CTA of it leaves before any barrier
-  const int s = f - p;
-  double* xs = sm;            // xs[c * s + j]: solved struct unknowns
-  double* z = sm + s * nb;    // z[c * p + i]: the whole pivot block after the exchange
+  if (p == 0) return;
+  const int s = f - p, lz = p | 1, lx = (s > p ? s : p) | 1;
+  double* z = sm;             // z[c * lz + i]
+  double* xs = sm + lz * w;   // xs[c * lx + j]: solved struct unknowns, then the front's own
   const int32_t* D = a.dofs + d.dptr;
   const double* A = a.F + d.off;
-  double* v = a.W + a.woff[fr];
-  for (int t = threadIdx.x; t < s * nb; t += blockDim.x) {
-    const int j = t % s, c = t / s;
-    xs[t] = a.X[(int64_t)D[p + j] * a.ldx + c];
+  const double* v = a.W + a.woff[fr] + c0;
+  double* X = a.X + c0;
+  for (int t = threadIdx.x; t < f * w; t += blockDim.x) {
+    const int i = t / w, c = t - i * w;
+    if (i < p) z[c * lz + i] = v[(int64_t)i * kLdW + c];
+    else xs[c * lx + i - p] = X[(int64_t)D[i] * a.ldx + c];
   }
   __syncthreads();
-  // z = y - U12 xs for this CTA's slice of pivot rows, in place over y in the workspace (each row is
-  // read and written by its owner only before the barrier)
-  int r0, r1;
-  row_slice(p, r, r0, r1);
-  const int pr = r1 - r0;
-  for (int t = threadIdx.x; t < pr * nb; t += blockDim.x) {
-    const int i = r0 + t % pr, c = t / pr;
-    const double* xc = xs + c * s;
-    v[(int64_t)c * f + i] = v[(int64_t)c * f + i] - col_dot(A + (int64_t)p * f + i, f, xc, 0, s);
-  }
-  cluster.sync();
-  for (int t = threadIdx.x; t < p * nb; t += blockDim.x) {
-    const int i = t % p, c = t / p;
-    z[c * p + i] = v[(int64_t)c * f + i];
+  for (int t = threadIdx.x; t < p * w; t += blockDim.x) {
+    const int c = t / p, i = t - c * p;
+    z[c * lz + i] -= col_dot(A + (int64_t)p * f + i, f, xs + c * lx, 0, s);
   }
   __syncthreads();
-  // x = U11^-1 z for the same slice
-  for (int t = threadIdx.x; t < pr * nb; t += blockDim.x) {
-    const int i = r0 + t % pr, c = t / pr;
-    const double* zc = z + c * p;
-    a.X[(int64_t)D[i] * a.ldx + c] = col_dot(A + i, f, zc, i, p);
+  // the upper triangle: row i is a dot product of length p - i; rows q and p - 1 - q share a thread
+  const int hp = (p + 1) >> 1;
+  for (int t = threadIdx.x; t < hp * w; t += blockDim.x) {
+    const int c = t / hp, q = t - c * hp;
+    const double* zc = z + c * lz;
+    xs[c * lx + q] = col_dot(A + q, f, zc, q, p);
+    const int i2 = p - 1 - q;
+    if (i2 != q) xs[c * lx + i2] = col_dot(A + i2, f, zc, i2, p);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < p * w; t += blockDim.x) {
+    const int i = t / w, c = t - i * w;
+    X[(int64_t)D[i] * a.ldx + c] = xs[c * lx + i];
   }
 }
 
 // ------------------------------------------------------------------ tiled solves (partitioned inverse)
-// The narrow upper levels of the tree hold a few fronts each, some far too large for one CTA, and
-// GB300's FP64 rate per SM (under two FMA per clock) makes any solve confined to a few SMs the
-// bottleneck. After the factorization, every front of such a level is turned into its partitioned
+// The upper levels of the tree hold few or small fronts, some far too large for one CTA, and GB300's
+// FP64 rate per SM (under two FMA per clock) makes any solve confined to a few SMs the bottleneck. After
+// the factorization, every front of such a level is turned into its partitioned
 // inverse:
 //   diagonal square: unit lower L11^-1 and upper U11^-1      (mf_invdiag_kernel / _wide_kernel)
 //   L21 -> L21' = -L21 L11^-1,  U12 -> U12' = -U11^-1 U12    (mf_partinv_kernel)
@@ -741,13 +638,21 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
 //   forward:  out[r] = v[r] + sum_{k < min(r, p)} F(r, k) v[k]            every row r < f
 //   backward: x[r]   = sum_{k = r}^{f - 1} F(r, k) z[k],  z = [y; x_s]    every pivot row r < p
 // (v: the gathered right-hand side in pivot order; out[0:p] = y, out[p:f] the update for the parent).
-// A level's rows are cut into tiles of kTileRows (one warp per row, lane c owns right-hand side c),
-// so a level of a few large fronts spreads over hundreds of CTAs. v is pulled without atomics from
-// the B rows and the children's update vectors through a per-front source list, chunk by chunk, into
-// shared memory by every CTA of the front.
+// A level's rows are cut into tiles of kTileRows = 8 rows x 8 NT right-hand sides, one CTA of four warps
+// each, so a level of a few fronts spreads over the whole chip. The products run as FP64 MMAs
+// (mma.sync m8n8k4, the same rate as the FP64 FMAs on this chip but one instruction per 256 of them, with
+// operands shared across the warp); the four warps split the inner dimension, since an 8 x 8 tile of a
+// 200-row front keeps one quarter of an SM busy for 15 us and four quarters for 4 us. v is pulled without
+// atomics from the B rows and the children's update vectors through a per-front source list, chunk by
+// chunk, into shared memory; sums have one fixed order, so solves are reproducible bit for bit.
+// With one row per warp and DFMAs a level of 4 to 64 fronts took 18 to 37 us per direction at 83k DoFs
+// (24 right-hand sides), a level of 54 to 213 fronts on one CTA per front 27 to 35 us; now 8 to 14 us.
 constexpr int kTileRows = 8;
 constexpr int kChunkK = 128;
 constexpr int kTiledMaxP = 768;   // the wide inversion keeps one column per thread in shared memory
+constexpr int kTileThreads = 128;
+constexpr int kTiledLeaves = 304;
+constexpr int kTileSteps = kChunkK / 16;   // MMA steps (4 columns of the front) per warp and chunk
 
 struct TiledArgs {
   const FrontDesc* fd;
@@ -755,9 +660,7 @@ struct TiledArgs {
   const int32_t* perm;
   const int64_t* piv_off;
   const int64_t* woff;
-  const int64_t* prow;      // per tiled front (at FrontDesc::prow): f + 1 offsets into the sources
-  const int64_t* src_off;   // source: W[src_off + c * src_str] (a child's update row)
-  const int32_t* src_str;
+  const int4* pull;   // per row of a tiled front (from FrontDesc::prow on), two int4: see pull_row
   const double* F;
   const double* B;
   int64_t ldb;
@@ -765,86 +668,131 @@ struct TiledArgs {
   double* X;
   int64_t ldx;
   int nb;
+  int chunk;   // rows of v in shared memory (see tile_product)
 };
 
-// row k (pivot order) of front d's gathered right-hand side, column c
-__device__ __forceinline__ double pull_row(const TiledArgs& a, const FrontDesc& d, const int32_t* D, const int32_t* pm,
-                                           int k, int c) {
+// row k (pivot order) of front d's gathered right-hand side, column c: the row's record holds its DoF (the
+// row of B, -1 past the pivots), then up to MAXKIDS workspace rows of the children, in slot order, -1 past
+// the last
+__device__ __forceinline__ double pull_row(const TiledArgs& a, const FrontDesc& d, const int32_t* pm, int k, int c) {
   const int u = k < d.p ? pm[k] : k;
-  double s = k < d.p ? a.B[(int64_t)D[u] * a.ldb + c] : 0.0;
-  const int64_t* pr = a.prow + d.prow;
-  const int64_t q1 = pr[u + 1];
-  for (int64_t q = pr[u]; q < q1; q++) s += a.W[a.src_off[q] + (int64_t)c * a.src_str[q]];
+  const int4* rec = a.pull + 2 * (d.prow + u);
+  const int4 q = __ldg(rec);
+  double s = q.x >= 0 ? a.B[(int64_t)q.x * a.ldb + c] : 0.0;
+  if (q.y >= 0) s += a.W[(int64_t)q.y * kLdW + c];
+  if (q.z >= 0) s += a.W[(int64_t)q.z * kLdW + c];
+  if (q.w >= 0) {
+    s += a.W[(int64_t)q.w * kLdW + c];
+    const int last = __ldg(&rec[1].x);
+    if (last >= 0) s += a.W[(int64_t)last * kLdW + c];
+  }
   return s;
 }
 
-// items: (front, first row) pairs
-__global__ void __launch_bounds__(256) mf_forward_tiled_kernel(const int2* __restrict__ items, TiledArgs a) {
-  __shared__ double vs[kChunkK * 33];   // vs[kk * 33 + c]: row k0 + kk of v
-  const int2 it = items[blockIdx.x];
-  const FrontDesc d = a.fd[it.x];
-  const int f = d.f, p = d.p, nb = a.nb;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = it.y + warp;
-  const bool live = r < f && lane < nb;
-  const int32_t* D = a.dofs + d.dptr;
-  const int32_t* pm = a.perm + a.piv_off[it.x];
-  const double* Ar = a.F + d.off + r;
-  const int kend = min(p, it.y + kTileRows);   // rows r < p need k < r, rows r >= p need k < p
-  const int klim = min(r, p);
-  double acc0 = 0.0, acc1 = 0.0;
-  for (int k0 = 0; k0 < kend; k0 += kChunkK) {
-    const int kc = min(kChunkK, kend - k0);
-    __syncthreads();
-    for (int t = threadIdx.x; t < kc * nb; t += blockDim.x) {
-      const int kk = t % kc, c = t / kc;
-      vs[kk * 33 + c] = pull_row(a, d, D, pm, k0 + kk, c);
-    }
-    __syncthreads();
-    if (live) {
-      const int k1 = min(k0 + kc, klim);
-      int k = k0;
-      for (; k + 2 <= k1; k += 2) {
-        acc0 += Ar[(int64_t)k * f] * vs[(k - k0) * 33 + lane];
-        acc1 += Ar[(int64_t)(k + 1) * f] * vs[(k + 1 - k0) * 33 + lane];
-      }
-      if (k < k1) acc0 += Ar[(int64_t)k * f] * vs[(k - k0) * 33 + lane];
-    }
-  }
-  if (live) a.W[a.woff[it.x] + (int64_t)lane * f + r] = pull_row(a, d, D, pm, r, lane) + (acc0 + acc1);
+// c += a b on an 8 x 8 tile, inner dimension 4: lane l holds a[l / 4][l % 4], b[l % 4][l / 4] and
+// c[l / 4][2 (l % 4) + {0, 1}]
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
 }
 
-__global__ void __launch_bounds__(256) mf_backward_tiled_kernel(const int2* __restrict__ items, TiledArgs a) {
-  __shared__ double zs[kChunkK * 33];   // zs[kk * 33 + c]: row k0 + kk of z = [y; x_s]
-  const int2 it = items[blockIdx.x];
-  const FrontDesc d = a.fd[it.x];
-  const int f = d.f, p = d.p, nb = a.nb;
+// One tile: rows r0 .. r0 + 7, columns c0 .. c0 + 8 NT - 1: init(r, c) + sum over kbeg <= k < kend of
+// F(r, k) v[k], F taken only where use(r, k). load(k, c) gives v[k][c0 + c]; done(r, c, sum) gets each row
+// below rlim. vs holds `chunk` rows of v (a multiple of 16, as many as the level's longest sum needs, so
+// that short sums leave room for more CTAs per SM; never 0).
+template <int NT, class Use, class Load, class Init, class Done>
+__device__ __forceinline__ void tile_product(const double* __restrict__ A, int f, int r0, int rlim, int kbeg, int kend,
+                                             int ncol, int chunk, const Use& use, const Load& load, const Init& init,
+                                             const Done& done) {
+  constexpr int LD = 8 * NT + 4;   // rows 4 banks apart: the B fragments read without conflicts
+  extern __shared__ double vs[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = it.y + warp;
-  const bool live = r < p && lane < nb;
-  const int32_t* D = a.dofs + d.dptr;
-  const double* Ar = a.F + d.off + r;
-  const double* y = a.W + a.woff[it.x];
-  double acc0 = 0.0, acc1 = 0.0;
-  for (int k0 = it.y; k0 < f; k0 += kChunkK) {
-    const int kc = min(kChunkK, f - k0);
-    __syncthreads();
-    for (int t = threadIdx.x; t < kc * nb; t += blockDim.x) {
-      const int kk = t % kc, c = t / kc, k = k0 + kk;
-      zs[kk * 33 + c] = k < p ? y[(int64_t)c * f + k] : a.X[(int64_t)D[k] * a.ldx + c];
+  const int row = r0 + (lane >> 2), kl = lane & 3;
+  constexpr int OWN = (64 * NT + kTileThreads - 1) / kTileThreads;
+  double own[OWN];
+  double acc[NT][2];
+#pragma unroll
+  for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = 0.0;
+#pragma unroll
+  for (int i = 0; i < OWN; i++) {   // the tile's own rows
+    const int t = threadIdx.x + i * kTileThreads, r = t / (8 * NT), c = t - r * (8 * NT);
+    own[i] = (t < 64 * NT && r0 + r < rlim && c < ncol) ? init(r0 + r, c) : 0.0;
+  }
+  for (int k0 = kbeg; k0 < kend; k0 += chunk) {
+    const int kc = min(chunk, kend - k0), kc4 = (kc + 3) & ~3;
+    double af[kTileSteps];   // this warp's steps warp, warp + 4, ... of the chunk
+#pragma unroll
+    for (int i = 0; i < kTileSteps; i++) {
+      const int k = k0 + 4 * (warp + 4 * i) + kl;
+      af[i] = (4 * (warp + 4 * i) < kc && k < kend && row < rlim && use(row, k)) ? __ldg(A + (int64_t)k * f + row) : 0.0;
+    }
+    if (k0 > kbeg) __syncthreads();
+    for (int t = threadIdx.x; t < kc4 * 8 * NT; t += kTileThreads) {
+      const int kk = t / (8 * NT), c = t - kk * (8 * NT);
+      vs[kk * LD + c] = (kk < kc && c < ncol) ? load(k0 + kk, c) : 0.0;
     }
     __syncthreads();
-    if (live) {
-      const int k1 = k0 + kc;
-      int k = max(k0, r);
-      for (; k + 2 <= k1; k += 2) {
-        acc0 += Ar[(int64_t)k * f] * zs[(k - k0) * 33 + lane];
-        acc1 += Ar[(int64_t)(k + 1) * f] * zs[(k + 1 - k0) * 33 + lane];
+#pragma unroll
+    for (int i = 0; i < kTileSteps; i++) {
+      const int st = warp + 4 * i;
+      if (4 * st < kc4) {
+        const double* vb = vs + (4 * st + kl) * LD + (lane >> 2);
+#pragma unroll
+        for (int n = 0; n < NT; n++) dmma(acc[n], af[i], vb[8 * n]);
       }
-      if (k < k1) acc0 += Ar[(int64_t)k * f] * zs[(k - k0) * 33 + lane];
     }
   }
-  if (live) a.X[(int64_t)D[r] * a.ldx + lane] = acc0 + acc1;
+  __syncthreads();
+  // the four warps' partial sums, added in warp order
+#pragma unroll
+  for (int n = 0; n < NT; n++) {
+    double* o = vs + (warp * 8 + (lane >> 2)) * (8 * NT) + 8 * n + 2 * kl;
+    o[0] = acc[n][0];
+    o[1] = acc[n][1];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < OWN; i++) {
+    const int t = threadIdx.x + i * kTileThreads, r = t / (8 * NT), c = t - r * (8 * NT);
+    if (t < 64 * NT && r0 + r < rlim && c < ncol)
+      done(r0 + r, c, own[i] + ((vs[t] + vs[64 * NT + t]) + (vs[128 * NT + t] + vs[192 * NT + t])));
+  }
+}
+
+// dynamic shared memory of a tile with `chunk` rows of v: those rows, later the four partial sums
+constexpr size_t tile_smem(int nt, int chunk) {
+  return sizeof(double) * (size_t)(chunk * (8 * nt + 4) > 256 * nt ? chunk * (8 * nt + 4) : 256 * nt);
+}
+
+// items: (front, first row) pairs; blockIdx.y: the columns from 8 NT blockIdx.y on
+template <int NT>
+__global__ void __launch_bounds__(kTileThreads) mf_forward_tiled_kernel(const int2* __restrict__ items, TiledArgs a) {
+  const int2 it = items[blockIdx.x];
+  const FrontDesc d = a.fd[it.x];
+  const int p = d.p, c0 = blockIdx.y * 8 * NT;
+  const int32_t* pm = a.perm + a.piv_off[it.x];
+  double* out = a.W + a.woff[it.x] + c0;
+  // rows r < p need k < r, rows r >= p need k < p
+  auto pull = [&](int k, int c) { return pull_row(a, d, pm, k, c0 + c); };
+  tile_product<NT>(
+      a.F + d.off, d.f, it.y, d.f, 0, min(p, it.y + kTileRows), min(8 * NT, a.nb - c0), a.chunk,
+      [p](int r, int k) { return k < r || r >= p; }, pull, pull,
+      [&](int r, int c, double s) { out[(int64_t)r * kLdW + c] = s; });
+}
+
+template <int NT>
+__global__ void __launch_bounds__(kTileThreads) mf_backward_tiled_kernel(const int2* __restrict__ items, TiledArgs a) {
+  const int2 it = items[blockIdx.x];
+  const FrontDesc d = a.fd[it.x];
+  const int p = d.p, c0 = blockIdx.y * 8 * NT;
+  const int32_t* D = a.dofs + d.dptr;
+  const double* y = a.W + a.woff[it.x] + c0;
+  double* X = a.X + c0;
+  tile_product<NT>(
+      a.F + d.off, d.f, it.y, p, it.y, d.f, min(8 * NT, a.nb - c0), a.chunk, [](int r, int k) { return k >= r; },
+      [&](int k, int c) { return k < p ? y[(int64_t)k * kLdW + c] : X[(int64_t)D[k] * a.ldx + c]; },
+      [](int, int) { return 0.0; }, [&](int r, int c, double s) { X[(int64_t)D[r] * a.ldx + c] = s; });
 }
 
 // the p x p LU square of each listed front, copied (column-major) to scratch at FrontDesc::aux
@@ -1061,6 +1009,7 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   level_ptr = s.level_ptr;
   max_f = s.max_f;
   max_p = s.max_p;
+  if (nb_max > kLdW) fail(FEM2D_E_INVALID_ARG, "solve block wider than the workspace rows");
   nb_cap = nb_max;
   factor_flops = s.flops;
   // fronts laid out level by level so each level's storage is contiguous
@@ -1086,7 +1035,7 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
       poff[f] = po;
       po += s.p[f];
       woff_h[f] = wo;
-      wo += (int64_t)s.f[f] * nb_max;
+      wo += (int64_t)s.f[f] * kLdW;
     }
   }
   level_off[nlevels] = o;
@@ -1105,14 +1054,22 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
     x.eptr = s.ea_ptr[f];
   }
   for (FrontDesc& x : fdh) x.prow = x.aux = 0;
-  // Tiled levels: the narrow upper levels (at most 2 * num_sms / CL small fronts, or any front too
-  // large for one CTA) whose fronts all have p <= kTiledMaxP. Their fronts get pull lists (for each
-  // front row, the children's update rows that add into it) and factor-time work items.
+  // Tiled levels: every level above the leaves, and leaf levels of at most kTiledLeaves fronts (or with a
+  // front too large for one CTA), if all their fronts have p <= kTiledMaxP. Their fronts get pull records
+  // (for each front row, the children's update rows that add into it) and factor-time work items. Upper
+  // levels gain at every width, since one CTA per front leaves its threads idle on the few pivots that
+  // such fronts have (5,487 fronts of 10 pivots at 1M DoFs; all levels: 5.8 -> 4.9 ms per solve of 20
+  // right-hand sides). Leaf fronts have most of their rows as pivots and fill a CTA: at 414 leaves the tiled
+  // form took 0.34 instead of 0.31 ms per solve and 12% more factorization time, at 125 leaves both took
+  // 0.14 ms.
   level_tiled.assign(nlevels, 0);
+  level_kmax.assign(nlevels, 0);
+  level_pmax.assign(nlevels, 0);
+  if (wo / kLdW > INT32_MAX) fail(FEM2D_E_TOO_LARGE, "solve workspace rows exceed 32 bits");
   tf_ptr.assign(nlevels + 1, 0);
   tb_ptr.assign(nlevels + 1, 0);
-  std::vector<int32_t> tf_h, tb_h, mid_h, wide_h, wi_h, pi_h, sstr_h;
-  std::vector<int64_t> prow_h, soff_h;
+  std::vector<int32_t> tf_h, tb_h, mid_h, wide_h, wi_h, pi_h;
+  std::vector<int32_t> pull_h;   // 8 per row: DoF, children's workspace rows (see pull_row)
   nmid = nwide = npinv = 0;
   max_mid_p = max_wide_p = max_tiled_p = 0;
   int64_t sq_total = 0;
@@ -1128,7 +1085,7 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
       else nl++;
       if (s.p[fr] > kTiledMaxP) fits = false;
     }
-    if (single_dense || !fits || !(nl > 0 || ns * CL <= 2 * c.num_sms)) continue;
+    if (single_dense || !fits || !(nl > 0 || l > 0 || ns <= kTiledLeaves)) continue;
     level_tiled[l] = 1;
     for (int k = s.level_ptr[l]; k < s.level_ptr[l + 1]; k++) {
       const int fr = s.level_fronts[k];
@@ -1150,8 +1107,11 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
       }
       if (P > 0)
         for (int t0 = 0; t0 < F - P; t0 += kTileRows) pi_h.insert(pi_h.end(), {fr, 0, t0, 0, fr, 1, t0, 0});
-      // pull lists: row u of the front (before pivoting) receives row i of child ch's update block
-      std::vector<std::vector<std::pair<int64_t, int32_t>>> rows(F);
+      // pull records: row u of the front (before pivoting) receives row i of child ch's update block
+      fdh[fr].prow = (int64_t)pull_h.size() / 8;
+      pull_h.resize(pull_h.size() + (size_t)8 * F, -1);
+      int32_t* rec = pull_h.data() + 8 * fdh[fr].prow;
+      for (int u = 0; u < P; u++) rec[8 * u] = s.dofs[s.dof_ptr[fr] + u];
       for (int slot = 0; slot < MAXKIDS; slot++) {
         const int ch = kids[fr][slot];
         if (ch < 0) continue;
@@ -1159,18 +1119,14 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
         for (int i = 0; i < sc; i++) {
           const int u = s.ea_map[s.ea_ptr[ch] + i];
           if (u < 0 || u >= F) fail(FEM2D_E_INVALID_ARG, "extend-add map outside the parent front");
-          rows[u].push_back({woff_h[ch] + s.p[ch] + i, s.f[ch]});
+          int q = 1;
+          while (q <= MAXKIDS && rec[8 * u + q] >= 0) q++;
+          if (q > MAXKIDS) fail(FEM2D_E_INVALID_ARG, "a child adds to one row twice");
+          rec[8 * u + q] = (int32_t)(woff_h[ch] / kLdW + s.p[ch] + i);
         }
       }
-      fdh[fr].prow = (int64_t)prow_h.size();
-      for (int u = 0; u < F; u++) {
-        prow_h.push_back((int64_t)soff_h.size());
-        for (const auto& e : rows[u]) {
-          soff_h.push_back(e.first);
-          sstr_h.push_back(e.second);
-        }
-      }
-      prow_h.push_back((int64_t)soff_h.size());
+      level_kmax[l] = std::max(level_kmax[l], std::max(F, P));
+      level_pmax[l] = std::max(level_pmax[l], P);
     }
   }
   tf_ptr[nlevels] = (int32_t)(tf_h.size() / 2);
@@ -1181,9 +1137,7 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   npinv = (int)(pi_h.size() / 4);
   tf_items.upload(tf_h, st);
   tb_items.upload(tb_h, st);
-  prow.upload(prow_h, st);
-  src_off.upload(soff_h, st);
-  src_str.upload(sstr_h, st);
+  pull.upload(pull_h, st);
   lmid.upload(mid_h, st);
   lwide.upload(wide_h, st);
   wide_items.upload(wi_h, st);
@@ -1217,8 +1171,8 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   std::vector<int32_t> ls, ll;
   small_ptr.assign(nlevels + 1, 0);
   large_ptr.assign(nlevels + 1, 0);
-  level_small_f.assign(nlevels, 0);
-  level_small_p.assign(nlevels, 0);
+  level_fwd_cols.assign(nlevels, 0);
+  level_bwd_cols.assign(nlevels, 0);
   max_small_p = 0;
   for (int l = 0; l < nlevels; l++) {
     small_ptr[l] = (int32_t)ls.size();
@@ -1227,8 +1181,8 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
       const int fr = s.level_fronts[k];
       if (s.p[fr] <= kSmallP && s.f[fr] <= kSmallF) {
         ls.push_back(fr);
-        level_small_f[l] = std::max(level_small_f[l], s.f[fr]);
-        level_small_p[l] = std::max(level_small_p[l], s.p[fr]);
+        level_fwd_cols[l] = std::max(level_fwd_cols[l], forward_cols(s.f[fr], s.p[fr]));
+        level_bwd_cols[l] = std::max(level_bwd_cols[l], backward_cols(s.f[fr], s.p[fr]));
         max_small_p = std::max(max_small_p, s.p[fr]);
       } else {
         ll.push_back(fr);
@@ -1245,24 +1199,15 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   static bool attr_done[256] = {};
   std::lock_guard<std::mutex> lk(attr_mu);
   if (c.device >= 0 && c.device < 256 && !attr_done[c.device]) {
+    const int smem = (kSmallF + kSmallP + 2) * kLdW * (int)sizeof(double);
     FEM2D_CUDA(cudaFuncSetAttribute(mf_invdiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     kSmallP * kSmallP * (int)sizeof(double)));
-    FEM2D_CUDA(cudaFuncSetAttribute(mf_forward_small_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (kSmallF + kSmallP) * 32 * (int)sizeof(double)));
-    FEM2D_CUDA(cudaFuncSetAttribute(mf_forward_small_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (kSmallF + kSmallP) * 32 * (int)sizeof(double)));
-    FEM2D_CUDA(cudaFuncSetAttribute(mf_forward_small_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (kSmallF + kSmallP) * 32 * (int)sizeof(double)));
-    FEM2D_CUDA(cudaFuncSetAttribute(mf_backward_small_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kSmallF * 32 * (int)sizeof(double)));
-    FEM2D_CUDA(cudaFuncSetAttribute(mf_backward_small_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kSmallF * 32 * (int)sizeof(double)));
-    FEM2D_CUDA(cudaFuncSetAttribute(mf_backward_small_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kSmallF * 32 * (int)sizeof(double)));
-    FEM2D_CUDA(cudaFuncSetAttribute(mf_forward_small_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (kSmallF + kSmallP) * 32 * (int)sizeof(double)));
-    FEM2D_CUDA(cudaFuncSetAttribute(mf_backward_small_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kSmallF * 32 * (int)sizeof(double)));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_forward_small_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_forward_small_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_forward_small_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_backward_small_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_backward_small_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_backward_small_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     FEM2D_CUDA(cudaFuncSetAttribute(mf_invdiag_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     kTiledMaxP * 32 * (int)sizeof(double)));
     FEM2D_CUDA(cudaFuncSetAttribute(mf_partinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1377,14 +1322,35 @@ void MFDevice::factor(Ctx& c, const double* va, const double* vb, double ca, dou
   }
 }
 
-// Threads per front for a level of ns small fronts solved one CTA per front: a level that fits one
-// front per SM takes 1024 threads (one CTA per SM at 40 registers a thread), one that fits two fronts per
-// SM takes 512 (two CTAs per SM when their shared memory fits twice), wider levels 256. Narrow levels are
-// latency-bound within each front, so the threads a front gets set their time.
-static int small_threads(int ns, size_t smem, int num_sms) {
-  if (ns <= num_sms) return 1024;
-  if (ns <= 2 * num_sms && smem <= 100 * 1024) return 512;
-  return 256;
+// The leaf level of a tree with fewer than kSplitFronts fronts per SM splits its right-hand sides over two
+// CTAs: 1,179 fronts and 24 right-hand sides took 0.75 ms per solve instead of 0.81 (three CTAs: 0.74), while
+// at 18,502 fronts, where the level fills the chip many times over, splitting cost 3 to 10%.
+constexpr int kSplitFronts = 16;
+
+// How a level of ns small fronts with `cols` doubles of shared memory per right-hand side is solved, one CTA
+// per front and `per` right-hand sides.
+struct SmallShape {
+  int per, threads;
+};
+
+static SmallShape small_shape(int ns, int cols, int nb, int num_sms) {
+  const int split = ns < kSplitFronts * num_sms && nb > 8 ? 2 : 1;
+  SmallShape s;
+  s.per = (nb + split - 1) / split;
+  const size_t smem = (size_t)cols * s.per * sizeof(double);
+  const int ctas = ns * ((nb + s.per - 1) / s.per);
+  s.threads = ctas <= num_sms ? 1024 : (ctas <= 2 * num_sms && smem <= 100 * 1024) ? 512 : 256;
+  return s;
+}
+
+// Right-hand sides (in groups of 8) per tile of a tiled level with `items` row tiles: narrow tiles while the
+// level leaves SMs idle, wide ones once it fills the chip and what counts is gathering each row once (the
+// line between 4 and 32 CTAs per SM made no difference beyond 2% at 29k to 1M DoFs).
+constexpr int kTileFill = 8;
+static int tile_groups(int items, int nb, int num_sms) {
+  const int groups = (nb + 7) / 8;
+  int nt = items * groups <= kTileFill * num_sms ? 1 : (items * ((groups + 1) / 2) <= kTileFill * num_sms ? 2 : groups);
+  return std::min(nt, groups);
 }
 
 void MFDevice::solve(Ctx& c, const MFFactor& fac, const double* B, int64_t ldb, double* X, int64_t ldx, int nb) {
@@ -1405,34 +1371,54 @@ void MFDevice::solve(Ctx& c, const MFFactor& fac, const double* B, int64_t ldb, 
   for (double b : level_factor_bytes) fbytes += b;
   // the whole solve is one profiled region: per-level events would dominate the short level launches
   ProfScope ps(c, "mf_solve", 2.0 * fbytes, 2.0 * 2.0 * (fbytes / 8.0) * nb);
-  SolveArgs a{fd, dofs.p, ea_map.p, fac.perm.p, fac.iperm.p, piv_off.p, woff.p, Fbuf.p, B, ldb, work.p, X, ldx, nb};
-  TiledArgs ta{fd,     dofs.p, fac.perm.p, piv_off.p, woff.p, prow.p, src_off.p, src_str.p,
-               Fbuf.p, B,      ldb,        work.p,    X,      ldx,    nb};
+  SolveArgs a{fd, dofs.p, ea_map.p, fac.perm.p, fac.iperm.p, piv_off.p, woff.p, Fbuf.p, B, ldb, work.p, X, ldx, nb, nb};
+  TiledArgs ta{fd, dofs.p, fac.perm.p, piv_off.p, woff.p, reinterpret_cast<const int4*>(pull.p), Fbuf.p, B, ldb, work.p, X, ldx, nb, 0};
+  auto tiled = [&](bool fwd, int l, const int2* items, int ni) {
+    const int nt = tile_groups(ni, nb, c.num_sms);
+    ta.chunk = std::max(16, std::min(kChunkK, ((fwd ? level_pmax[l] : level_kmax[l]) + 15) & ~15));
+    const size_t smem = tile_smem(nt, ta.chunk);
+    const dim3 grid(ni, (nb + 8 * nt - 1) / (8 * nt));
+    if (fwd) {
+      if (nt == 1) mf_forward_tiled_kernel<1><<<grid, kTileThreads, smem, st>>>(items, ta);
+      else if (nt == 2) mf_forward_tiled_kernel<2><<<grid, kTileThreads, smem, st>>>(items, ta);
+      else if (nt == 3) mf_forward_tiled_kernel<3><<<grid, kTileThreads, smem, st>>>(items, ta);
+      else mf_forward_tiled_kernel<4><<<grid, kTileThreads, smem, st>>>(items, ta);
+    } else {
+      if (nt == 1) mf_backward_tiled_kernel<1><<<grid, kTileThreads, smem, st>>>(items, ta);
+      else if (nt == 2) mf_backward_tiled_kernel<2><<<grid, kTileThreads, smem, st>>>(items, ta);
+      else if (nt == 3) mf_backward_tiled_kernel<3><<<grid, kTileThreads, smem, st>>>(items, ta);
+      else mf_backward_tiled_kernel<4><<<grid, kTileThreads, smem, st>>>(items, ta);
+    }
+    c.launches++;
+  };
+  auto small = [&](bool fwd, int l, int ns) {
+    const int cols = fwd ? level_fwd_cols[l] : level_bwd_cols[l];
+    const SmallShape s = small_shape(ns, cols, nb, c.num_sms);
+    a.per = s.per;
+    const dim3 grid(ns, (nb + s.per - 1) / s.per);
+    const size_t smem = (size_t)cols * s.per * sizeof(double);
+    const int32_t* lf = lsmall.p + small_ptr[l];
+    if (fwd) {
+      if (s.threads == 1024) mf_forward_small_kernel<1024><<<grid, 1024, smem, st>>>(lf, a);
+      else if (s.threads == 512) mf_forward_small_kernel<512><<<grid, 512, smem, st>>>(lf, a);
+      else mf_forward_small_kernel<256><<<grid, 256, smem, st>>>(lf, a);
+    } else {
+      if (s.threads == 1024) mf_backward_small_kernel<1024><<<grid, 1024, smem, st>>>(lf, a);
+      else if (s.threads == 512) mf_backward_small_kernel<512><<<grid, 512, smem, st>>>(lf, a);
+      else mf_backward_small_kernel<256><<<grid, 256, smem, st>>>(lf, a);
+    }
+    c.launches++;
+  };
   const int2* tfi = reinterpret_cast<const int2*>(tf_items.p);
   const int2* tbi = reinterpret_cast<const int2*>(tb_items.p);
   for (int l = 0; l < nlevels; l++) {
     if (level_tiled[l]) {
       const int ni = tf_ptr[l + 1] - tf_ptr[l];
-      if (ni > 0) {
-        mf_forward_tiled_kernel<<<ni, 256, 0, st>>>(tfi + tf_ptr[l], ta);
-        c.launches++;
-      }
+      if (ni > 0) tiled(true, l, tfi + tf_ptr[l], ni);
       continue;
     }
     const int ns = small_ptr[l + 1] - small_ptr[l], nl = large_ptr[l + 1] - large_ptr[l];
-    if (ns > 0) {
-      const size_t smem = (size_t)(level_small_f[l] + level_small_p[l]) * nb * sizeof(double);
-      const int nt = small_threads(ns, smem, c.num_sms);
-      if (ns * CL <= 2 * c.num_sms)
-        mf_forward_small_cluster_kernel<<<ns * CL, 256, smem, st>>>(lsmall.p + small_ptr[l], a);
-      else if (nt == 1024)
-        mf_forward_small_kernel<1024><<<ns, 1024, smem, st>>>(lsmall.p + small_ptr[l], a);
-      else if (nt == 512)
-        mf_forward_small_kernel<512><<<ns, 512, smem, st>>>(lsmall.p + small_ptr[l], a);
-      else
-        mf_forward_small_kernel<256><<<ns, 256, smem, st>>>(lsmall.p + small_ptr[l], a);
-      c.launches++;
-    }
+    if (ns > 0) small(true, l, ns);
     if (nl > 0) {
       mf_forward_cluster_kernel<<<nl * CL, 256, 0, st>>>(llarge.p + large_ptr[l], fd, dofs.p, ea_map.p, fac.perm.p,
                                                          fac.iperm.p, piv_off.p, woff.p, Fbuf.p, B, ldb, nb,
@@ -1443,26 +1429,11 @@ void MFDevice::solve(Ctx& c, const MFFactor& fac, const double* B, int64_t ldb, 
   for (int l = nlevels - 1; l >= 0; l--) {
     if (level_tiled[l]) {
       const int ni = tb_ptr[l + 1] - tb_ptr[l];
-      if (ni > 0) {
-        mf_backward_tiled_kernel<<<ni, 256, 0, st>>>(tbi + tb_ptr[l], ta);
-        c.launches++;
-      }
+      if (ni > 0) tiled(false, l, tbi + tb_ptr[l], ni);
       continue;
     }
     const int ns = small_ptr[l + 1] - small_ptr[l], nl = large_ptr[l + 1] - large_ptr[l];
-    if (ns > 0) {
-      const size_t smem = (size_t)level_small_f[l] * nb * sizeof(double);
-      const int nt = small_threads(ns, smem, c.num_sms);
-      if (ns * CL <= 2 * c.num_sms)
-        mf_backward_small_cluster_kernel<<<ns * CL, 256, smem, st>>>(lsmall.p + small_ptr[l], a);
-      else if (nt == 1024)
-        mf_backward_small_kernel<1024><<<ns, 1024, smem, st>>>(lsmall.p + small_ptr[l], a);
-      else if (nt == 512)
-        mf_backward_small_kernel<512><<<ns, 512, smem, st>>>(lsmall.p + small_ptr[l], a);
-      else
-        mf_backward_small_kernel<256><<<ns, 256, smem, st>>>(lsmall.p + small_ptr[l], a);
-      c.launches++;
-    }
+    if (ns > 0) small(false, l, ns);
     if (nl > 0) {
       mf_backward_cluster_kernel<<<nl * CL, 256, 0, st>>>(llarge.p + large_ptr[l], fd, dofs.p, woff.p, Fbuf.p,
                                                           work.p, nb, X, ldx);

@@ -42,7 +42,7 @@ struct MFDevice {
   DBuf<int> weak_count;
   // per level, the fronts solved by one CTA each (inverted diagonal blocks) and the rest (clusters)
   std::vector<int32_t> small_ptr, large_ptr;   // nlevels + 1 offsets into lsmall / llarge
-  std::vector<int32_t> level_small_f, level_small_p;
+  std::vector<int32_t> level_fwd_cols, level_bwd_cols;   // shared doubles per right-hand side of their kernels
   DBuf<int32_t> lsmall, llarge;
   int nsmall = 0, max_small_p = 0;
   // tiled levels (narrow upper levels solved through the fronts' partitioned inverses, rows spread over
@@ -50,8 +50,8 @@ struct MFDevice {
   std::vector<uint8_t> level_tiled;
   std::vector<int32_t> tf_ptr, tb_ptr;
   DBuf<int32_t> tf_items, tb_items;
-  DBuf<int64_t> prow, src_off;   // pull lists of the tiled fronts' right-hand sides
-  DBuf<int32_t> src_str;
+  DBuf<int32_t> pull;   // pull records of the tiled fronts' right-hand sides (8 per row)
+  std::vector<int32_t> level_pmax, level_kmax;   // tiled levels: longest sums of the two directions
   // factor-time work of the tiled fronts: diagonal inversion of those outside lsmall (p <= kSmallP:
   // lmid; larger: lwide, 32-column items, scratch squares sq), then the partitioned-inverse items
   DBuf<int32_t> lmid, lwide, wide_items, pinv_items;

@@ -63,3 +63,32 @@ def test_shifted_solve_wide_fronts(ctx, ca, cb, spd):
     bwd = np.max(np.abs(K @ X - R), axis=0) / (knorm * np.max(np.abs(X), axis=0) + np.max(np.abs(R), axis=0))
     assert np.all(np.isfinite(X))
     assert np.max(bwd) < 1e-13, bwd
+
+
+@pytest.mark.parametrize("columns", [1, 7, 8, 9, 16, 23, 32, 33])
+@pytest.mark.parametrize("mesh", ["empty_level", "uneven", "leaves"])
+def test_shifted_solve_columns(kat, ctx, mesh, columns):
+    """Right-hand side counts around the tiles of 8 and the column splits, on trees with a level of fronts
+    without pivots (kat_b), with fronts of many sizes on eleven levels, and with more leaf fronts than the
+    tiled solve takes: the normwise backward error stays at the FP64 level (450 units of rounding)."""
+    if mesh == "empty_level":
+        pm = fg.Mesh.from_json(kat["mesh_b"])
+        configs.apply_ops(pm, [("pref", 3, 3, None), ("href", 0, None, -1), ("href", 0, [6, 9, 12], -1)])
+    elif mesh == "uneven":
+        pm = configs.build_mesh(configs.full_scale(seed=5, nx=9, ny=5, rounds=3, fraction=0.4, pmin=2, pmax=7))
+    else:
+        pm = configs.build_mesh(configs.full_scale(seed=6, nx=23, ny=17, rounds=1, fraction=0.2, pmin=2, pmax=4))
+    dom = fg.Domain.from_mesh(pm)
+    fronts = fg.factor_plan(dom)["fronts"]
+    levels = [fronts[fronts[:, 1] == k] for k in range(fronts[:, 1].max() + 1)]
+    assert {"empty_level": min(q[:, 3].max() for q in levels) == 0, "uneven": len(levels) >= 8,
+            "leaves": len(levels[0]) > 304}[mesh]
+    gep = fg.galerkin_sample_gep_hcurl(fg.KOLeg, fg.CurlCurl, fg.L2Inner, dom, [10, 10], ctx=ctx)
+    A, B = gep.scipy()
+    for ca, cb, spd in ((1.0, -10.0, False), (1.0, 10.0, True)):
+        K = (ca * A + cb * B).tocsr()
+        R = np.random.default_rng(columns).standard_normal((gep.dimension, columns))
+        X = gep.shifted_solve(ca, cb, R, spd=spd)
+        knorm = np.max(np.asarray(abs(K).sum(axis=1)).ravel())
+        bwd = np.max(np.abs(K @ X - R), axis=0) / (knorm * np.max(np.abs(X), axis=0) + np.max(np.abs(R), axis=0))
+        assert np.max(bwd) < 1e-13, bwd
