@@ -23,8 +23,6 @@ namespace fem2d {
 
 namespace {
 
-constexpr int PANEL = 32;
-
 // the solve workspace holds one row of kLdW values per front row (row-major, one right-hand side per
 // column), so a row that a parent gathers from a child is one contiguous read
 constexpr int kLdW = 32;
@@ -36,7 +34,7 @@ struct FrontDesc {   // device copy of the per-front scalars
   int32_t kid[MAXKIDS];
   int64_t off, dptr, aptr, aend, eptr;
   int64_t prow;   // tiled fronts: the front's first pull record (one per row)
-  int64_t aux;    // tiled fronts with p > kSmallP: offset of the p x p scratch copy of the LU square
+  int64_t aux;    // fronts factored in global memory: offset of the p x p scratch square of their inverses
 };
 
 __global__ void mf_assemble_kernel(const int32_t* __restrict__ lf, const FrontDesc* __restrict__ fd,
@@ -51,203 +49,673 @@ __global__ void mf_assemble_kernel(const int32_t* __restrict__ lf, const FrontDe
   }
 }
 
-// add the child's trailing block (rows/cols >= p_child) into the parent at mapped positions
-__global__ void mf_extend_add_kernel(const int32_t* __restrict__ lf, const FrontDesc* __restrict__ fd, int slot,
-                                     const int32_t* __restrict__ emap, double* __restrict__ F) {
+// add the children's trailing blocks (rows/cols >= p_child) into the parent at mapped positions, in slot
+// order; a CTA owns kExtendCols columns of the parent and takes the child columns that map there
+constexpr int kExtendCols = 16;
+__global__ void __launch_bounds__(256) mf_extend_add_kernel(const int32_t* __restrict__ lf,
+                                                            const FrontDesc* __restrict__ fd,
+                                                            const int32_t* __restrict__ emap, double* __restrict__ F) {
   const FrontDesc par = fd[lf[blockIdx.y]];
-  const int32_t ch = par.kid[slot];
-  if (ch < 0) return;
-  const FrontDesc c = fd[ch];
-  const int s = c.f - c.p;
-  const int64_t total = (int64_t)s * s;
-  const int32_t* m = emap + c.eptr;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(t % s), j = (int)(t / s);   // child (row p+i, col p+j), column-major
-    const double v = F[c.off + (int64_t)(c.p + j) * c.f + (c.p + i)];
-    F[par.off + (int64_t)m[j] * par.f + m[i]] += v;
+  const int j0 = blockIdx.x * kExtendCols;
+  if (j0 >= par.f) return;
+  __shared__ int from[kExtendCols], count;   // child column of each parent column (-1: none), any at all
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int slot = 0; slot < MAXKIDS; slot++) {
+    const int32_t ch = par.kid[slot];
+    if (ch < 0) continue;   // uniform across the CTA
+    const FrontDesc c = fd[ch];
+    const int s = c.f - c.p;
+    const int32_t* m = emap + c.eptr;
+    __syncthreads();   // one child after the other: the sums keep their order
+    if (threadIdx.x < kExtendCols) from[threadIdx.x] = -1;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    for (int j = threadIdx.x; j < s; j += 256) {
+      const int to = m[j] - j0;
+      if (to >= 0 && to < kExtendCols) {
+        from[to] = j;
+        count = 1;
+      }
+    }
+    __syncthreads();
+    if (count == 0) continue;
+    for (int q = warp; q < kExtendCols; q += 8) {
+      const int j = from[q];
+      if (j < 0) continue;
+      const double* src = F + c.off + (int64_t)(c.p + j) * c.f + c.p;
+      double* dst = F + par.off + (int64_t)(j0 + q) * par.f;
+#pragma unroll 4
+      for (int i = lane; i < s; i += 32) dst[m[i]] += src[i];
+    }
   }
 }
 
-// columns k0 .. k0+w-1 of every front with p > k0: pivot, swap full rows, scale, update the panel
+// c += a b on an 8 x 8 tile, inner dimension 4: lane l holds a[l / 4][l % 4], b[l % 4][l / 4] and
+// c[l / 4][2 (l % 4) + {0, 1}]
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+// ------------------------------------------------------------------ fronts in shared memory
+// A front of up to kFusedF rows is factored by one CTA in one pass (mf_front_kernel): assembled from the
+// CSR values and the children's Schur complements into shared memory, factored there, its inverted
+// diagonal blocks (and, where the solves want them, L21' and U12') formed there, and written once. What
+// bounds it is the FP64 pipe: updates and inverses run as FP64 MMAs on 8 x 8 tiles, a pivot column costs
+// one or two barriers, and pivots are compared as integers (a double comparison takes a slot of the FP64
+// pipe). Passing each front through global memory seven times per 32 columns (assembly, extend-adds, panel,
+// triangular solve, update, inverse, with 20 to 400 us per panel whatever its size) took 0.59 ms per
+// factorization at 832 DoFs, 3.7 at 29k, 7.0 at 83k and 59 at 1M; now 0.24, 2.6, 4.7 and 37.
+// Larger fronts, and those above kFusedNarrowF rows of levels that would leave SMs idle, stay in global
+// memory and are factored by many CTAs each (mf_strip_kernel): a front of 160 rows keeps one SM's FP64 pipe
+// busy for half a millisecond. (Lines at 32 to 128 rows were within 10% of each other at 5k to 83k DoFs;
+// at 832 DoFs 32 rows cost a third more.)
+constexpr int kFusedF = 164;
+constexpr int kFusedNarrowF = 64;   // on levels of at most one front per SM
+constexpr int kFusedSmallF = 64;   // fronts up to here: 128 threads
+
+// fronts that the solves may give one CTA (see there)
+constexpr int kSmallP = 160;
+constexpr int kSmallF = 512;
+
+constexpr int strip_smem(int rows) { return (int)sizeof(double) * 8 * (rows | 1); }
+
+struct FactorArgs {
+  const FrontDesc* fd;
+  const int64_t *apos, *acsr;
+  const double *va, *vb;
+  double ca, cb;
+  const int32_t *emap, *dofs;
+  const int64_t* piv_off;
+  double* F;
+  int32_t *piv, *perm, *iperm;
+  int* flags;
+  int32_t* weak;
+  int* nweak;
+  int weak_cap;
+  int pivoting;
+};
+
 // A column whose largest fully-summed entry is below kWeakPivot times its largest entry in the rows of
 // the front's other (not yet summed) DoFs has no stable pivot here: its DoF is recorded, and the solver
 // moves its elimination to the parent front and refactors (delayed pivoting).
 constexpr double kWeakPivot = 1e-3;
 
-__global__ void __launch_bounds__(256) mf_panel_kernel(const int32_t* __restrict__ lf,
-                                                       const FrontDesc* __restrict__ fd, int k0, int pivoting,
-                                                       double* __restrict__ F, int32_t* __restrict__ piv,
-                                                       const int64_t* __restrict__ piv_off, int* __restrict__ flags,
-                                                       const int32_t* __restrict__ dofs,
-                                                       int32_t* __restrict__ weak, int* __restrict__ nweak,
-                                                       int weak_cap) {
-  const int fr = lf[blockIdx.x];
-  const FrontDesc d = fd[fr];
-  if (d.p <= k0) return;
-  const int w = min(PANEL, d.p - k0);
-  const int f = d.f;
-  double* A = F + d.off;
-  __shared__ double sval[256];
-  __shared__ int sidx[256];
-  __shared__ int s_piv;
-  __shared__ double s_d;
-  for (int k = k0; k < k0 + w; k++) {
-    double* colk = A + (int64_t)k * f;
+// |a| as an integer that orders like |a| (0 for NaN)
+__device__ __forceinline__ unsigned long long mag_key(double a) {
+  const unsigned long long k = (unsigned long long)__double_as_longlong(a) & 0x7FFFFFFFFFFFFFFFull;
+  return k > 0x7FF0000000000000ull ? 0ull : k;
+}
+
+template <int NT>
+struct LuScratch {   // double-buffered by column parity, so that a column costs one barrier
+  unsigned long long key[2][NT / 32], other[2][NT / 32];   // per warp: largest candidate, largest other entry
+  int row[2][NT / 32];
+  double cand[2][NT / 32][8];   // the candidates' rows of the micro-panel
+  double top[2][8];             // row k
+  double inv[2];
+};
+
+// largest key of the warp and, among equal keys, the smallest row
+__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long key) {
+  const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32));
+  const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32) == hi ? (unsigned)key : 0u);
+  return ((unsigned long long)hi << 32) | lo;
+}
+
+// A micro-panel: w <= 8 pivot columns k0 .. of the nr-row block, carried in registers (thread: the rows
+// k0 + tid + NT m) with `nc` >= w columns, so that columns past the pivots are solved and updated with them.
+// Rows below pr are pivot candidates; A points at column k0, pv[k] gets the row swapped with row k. Bound by
+// its chain per column: a warp reduction, one barrier, a division (some 700 clocks on this FP64 pipe) and
+// the row update.
+template <int NT, int RPT>
+__device__ __forceinline__ void micro_panel(double* A, int ld, int k0, int nr, int nc, int w, int pr,
+                                            const FactorArgs& a, const int32_t* col_dof, bool has_parent, int32_t* pv,
+                                            LuScratch<NT>& sc) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool pivoting = a.pivoting != 0;
+  const bool one_divides = nr - k0 > 128;   // else every warp with rows does, without a second barrier
+  double x[RPT][8];
+#pragma unroll
+  for (int m = 0; m < RPT; m++) {
+    const int i = k0 + tid + NT * m;
+#pragma unroll
+    for (int c = 0; c < 8; c++) x[m][c] = (i < nr && c < nc) ? A[c * ld + i] : 0.0;
+  }
+#pragma unroll
+  for (int jj = 0; jj < 8; jj++) {
+    if (jj >= w) break;   // uniform
+    const int k = k0 + jj, par = jj & 1;
+    if (pivoting) {
+      unsigned long long bk = 0, ok = 0;
+      int bi = INT32_MAX;
+#pragma unroll
+      for (int m = 0; m < RPT; m++) {
+        const int i = k0 + tid + NT * m;
+        if (i < k || i >= nr) continue;
+        const unsigned long long q = mag_key(x[m][jj]);
+        if (i >= pr) ok = max(ok, q);
+        else if (bi == INT32_MAX || q > bk) {
+          bk = q;
+          bi = i;
+        }
+      }
+      const unsigned long long best = warp_max_key(bk);
+      const int row = __reduce_min_sync(0xffffffffu, bk == best ? bi : INT32_MAX);
+      ok = warp_max_key(ok);
+      if (lane == 0) {
+        sc.key[par][warp] = best;
+        sc.row[par][warp] = row;
+        sc.other[par][warp] = ok;
+      }
+#pragma unroll
+      for (int m = 0; m < RPT; m++)
+        if (k0 + tid + NT * m == row) {
+#pragma unroll
+          for (int c = 0; c < 8; c++) sc.cand[par][warp][c] = x[m][c];
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < RPT; m++)
+      if (k0 + tid + NT * m == k) {
+#pragma unroll
+        for (int c = 0; c < 8; c++) sc.top[par][c] = x[m][c];
+      }
+    __syncthreads();
+    int best = k;
+    const double* ur = sc.top[par];
+    if (pivoting) {
+      unsigned long long bk = 0, ok = 0;
+      int bw = 0;
+      best = INT32_MAX;
+#pragma unroll
+      for (int q = 0; q < NT / 32; q++) {
+        const unsigned long long kq = sc.key[par][q];
+        const int rq = sc.row[par][q];
+        ok = max(ok, sc.other[par][q]);
+        if (kq > bk || (kq == bk && rq < best)) {
+          bk = kq;
+          best = rq;
+          bw = q;
+        }
+      }
+      ur = sc.cand[par][bw];
+      if (tid == 0 && has_parent && bk < ok &&   // (the factor is below 1)
+          __longlong_as_double((long long)bk) < kWeakPivot * __longlong_as_double((long long)ok)) {
+        const int slot = atomicAdd(a.nweak, 1);
+        if (slot < a.weak_cap) a.weak[slot] = col_dof[k];
+      }
+    }
+    double u[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++) u[c] = ur[c];
+    const long long ub = __double_as_longlong(u[jj]);
+    const unsigned long long uk = mag_key(u[jj]);   // 0: zero or NaN
+    if (uk == 0 || (!pivoting && ub < 0)) {
+      if (tid == 0) atomicOr(a.flags, pivoting ? 1 : 2);   // 1: zero pivot (perturbed), 2: not positive definite
+      if ((ub & 0x7FFFFFFFFFFFFFFFll) == 0) u[jj] = 1e-300;
+    }
+    if (tid == 0) pv[k] = best;
+    double inv = 0.0;
+    if (one_divides) {
+      if (warp == 0) {
+        inv = 1.0 / u[jj];
+        if (lane == 0) sc.inv[par] = inv;
+      }
+      __syncthreads();
+      inv = sc.inv[par];
+    } else if (k0 + 32 * warp < nr) {
+      inv = 1.0 / u[jj];
+    }
+#pragma unroll
+    for (int m = 0; m < RPT; m++) {
+      const int i = k0 + tid + NT * m;
+      if (i == k) {
+#pragma unroll
+        for (int c = 0; c < 8; c++) x[m][c] = u[c];
+      } else if (i > k && i < nr) {
+        if (i == best) {
+#pragma unroll
+          for (int c = 0; c < 8; c++) x[m][c] = sc.top[par][c];
+        }
+        const double l = x[m][jj] * inv;
+        x[m][jj] = l;
+#pragma unroll
+        for (int c = jj + 1; c < 8; c++) x[m][c] -= l * u[c];
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < RPT; m++) {
+    const int i = k0 + tid + NT * m;
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+      if (i < nr && c < nc) A[c * ld + i] = x[m][c];
+  }
+}
+
+// The same on rows left in memory, any number of them (fronts of more than 2048 rows, which no mesh measured
+// here has)
+__device__ __forceinline__ void micro_panel_memory(double* A, int64_t ld, int k0, int nr, int nc, int w, int pr,
+                                                   const FactorArgs& a, const int32_t* col_dof, bool has_parent,
+                                                   int32_t* pv, LuScratch<256>& sc) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool pivoting = a.pivoting != 0;
+  for (int jj = 0; jj < w; jj++) {
+    const int k = k0 + jj;
+    double* ck = A + jj * ld;
+    __syncthreads();
     int best = k;
     if (pivoting) {
-      double bv = -1.0;
-      int bi = k;
-      for (int i = k + threadIdx.x; i < d.p; i += blockDim.x) {
-        const double a = fabs(colk[i]);
-        if (a > bv) { bv = a; bi = i; }
+      unsigned long long bk = 0, ok = 0;
+      int bi = INT32_MAX;
+      for (int i = k + tid; i < nr; i += 256) {
+        const unsigned long long q = mag_key(ck[i]);
+        if (i >= pr) ok = max(ok, q);
+        else if (bi == INT32_MAX || q > bk) {
+          bk = q;
+          bi = i;
+        }
       }
-      sval[threadIdx.x] = bv;
-      sidx[threadIdx.x] = bi;
+      const unsigned long long wk = warp_max_key(bk);
+      const int row = __reduce_min_sync(0xffffffffu, bk == wk ? bi : INT32_MAX);
+      ok = warp_max_key(ok);
+      if (lane == 0) {
+        sc.key[0][warp] = wk;
+        sc.row[0][warp] = row;
+        sc.other[0][warp] = ok;
+      }
       __syncthreads();
-      for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-        if (threadIdx.x < st) {
-          const double o = sval[threadIdx.x + st];
-          const int oi = sidx[threadIdx.x + st];
-          if (o > sval[threadIdx.x] || (o == sval[threadIdx.x] && oi < sidx[threadIdx.x])) {
-            sval[threadIdx.x] = o;
-            sidx[threadIdx.x] = oi;
+      bk = 0;
+      best = INT32_MAX;
+      for (int q = 0; q < 8; q++) {
+        ok = max(ok, sc.other[0][q]);
+        if (sc.key[0][q] > bk || (sc.key[0][q] == bk && sc.row[0][q] < best)) {
+          bk = sc.key[0][q];
+          best = sc.row[0][q];
+        }
+      }
+      if (tid == 0 && has_parent &&
+          __longlong_as_double((long long)bk) < kWeakPivot * __longlong_as_double((long long)ok)) {
+        const int slot = atomicAdd(a.nweak, 1);
+        if (slot < a.weak_cap) a.weak[slot] = col_dof[k];
+      }
+      __syncthreads();
+    }
+    if (tid < nc && best != k) {
+      const double x = A[tid * ld + k];
+      A[tid * ld + k] = A[tid * ld + best];
+      A[tid * ld + best] = x;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      pv[k] = best;
+      double dk = ck[k];
+      if (!(fabs(dk) > 0.0) || (!pivoting && !(dk > 0.0))) {
+        atomicOr(a.flags, pivoting ? 1 : 2);
+        if (dk == 0.0) ck[k] = dk = 1e-300;
+      }
+      sc.inv[0] = 1.0 / dk;
+    }
+    __syncthreads();
+    const double inv = sc.inv[0];
+    for (int i = k + 1 + tid; i < nr; i += 256) {
+      const double l = ck[i] * inv;
+      ck[i] = l;
+      for (int c = jj + 1; c < nc; c++) A[c * ld + i] -= l * A[c * ld + k];
+    }
+  }
+  __syncthreads();
+}
+
+// U12 = L11^-1 A12 for one column c (rows k0 ..) after the micro-panel's row swaps; L11 unit lower, at A
+__device__ __forceinline__ void swap_solve8(double* c, const double* A, int64_t ld, int k0, int w, const int32_t* pv,
+                                            bool solve) {
+  for (int k = k0; k < k0 + w; k++) {
+    const int r = pv[k];
+    if (r != k) {
+      const double x = c[k];
+      c[k] = c[r];
+      c[r] = x;
+    }
+  }
+  if (!solve) return;
+  double x[8];
+#pragma unroll
+  for (int r = 0; r < 8; r++) x[r] = r < w ? c[k0 + r] : 0.0;
+#pragma unroll
+  for (int q = 0; q < 7; q++)
+#pragma unroll
+    for (int r = q + 1; r < 8; r++)
+      if (r < w) x[r] -= A[q * ld + k0 + r] * x[q];
+#pragma unroll
+  for (int r = 0; r < 8; r++)
+    if (r < w) c[k0 + r] = x[r];
+}
+
+// LU of the first np columns of the f x f column-major block A in shared memory (leading dimension ld)
+template <int NT>
+__device__ __forceinline__ void lu_shared(double* A, int ld, int f, int np, const FactorArgs& a,
+                                          const int32_t* col_dof, bool has_parent, int32_t* pv, LuScratch<NT>& sc) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int k0 = 0; k0 < np; k0 += 8) {
+    const int w = min(8, np - k0);
+    micro_panel<NT, 1>(A + k0 * ld, ld, k0, f, w, w, np, a, col_dof, has_parent, pv, sc);
+    __syncthreads();
+    for (int j = tid; j < f; j += NT)
+      if (j < k0 || j >= k0 + w) swap_solve8(A + j * ld, A + k0 * ld, ld, k0, w, pv, j > k0);
+    __syncthreads();
+    // A22 -= L21 U12
+    const int b0 = k0 + w, tr = (f - b0 + 7) >> 3;
+    const int g = lane >> 2, kl = lane & 3;
+    for (int q = warp; q < tr * tr; q += NT / 32) {
+      const int rt = q % tr, ct = q / tr;
+      const int i = b0 + 8 * rt + g, j = b0 + 8 * ct + g;
+      const bool ri = i < f, cj = j < f;
+      const double a0 = (ri && kl < w) ? -A[(k0 + kl) * ld + i] : 0.0;
+      const double a1 = (ri && 4 + kl < w) ? -A[(k0 + 4 + kl) * ld + i] : 0.0;
+      const double u0 = (cj && kl < w) ? A[j * ld + k0 + kl] : 0.0;
+      const double u1 = (cj && 4 + kl < w) ? A[j * ld + k0 + 4 + kl] : 0.0;
+      const int jc = b0 + 8 * ct + 2 * kl;
+      double* o = A + jc * ld + i;
+      double c[2] = {(ri && jc < f) ? o[0] : 0.0, (ri && jc + 1 < f) ? o[ld] : 0.0};
+      dmma(c, a0, u0);
+      if (w > 4) dmma(c, a1, u1);
+      if (ri && jc < f) o[0] = c[0];
+      if (ri && jc + 1 < f) o[ld] = c[1];
+    }
+    __syncthreads();
+  }
+}
+
+// element (r, c) of the unit lower / upper triangular factor in the LU square of order p, 0 outside
+__device__ __forceinline__ double lower_at(const double* A, int ld, int p, int r, int c) {
+  return (r >= p || c > r) ? 0.0 : (c == r ? 1.0 : A[c * ld + r]);
+}
+__device__ __forceinline__ double upper_at(const double* A, int ld, int p, int r, int c) {
+  return (c >= p || c < r) ? 0.0 : A[c * ld + r];
+}
+
+// The LU square of order p (the first p rows and columns of A) overwritten by (unit lower L11^-1, U11^-1):
+// the 8 x 8 diagonal blocks by substitution, then block row by block row
+//   X_ij = -L_ii^-1 sum_{j <= k < i} L_ik X_kj        (and the same for U, from the last block row up).
+// scr: 64 doubles per warp; p <= MAXP.
+template <int NT, int MAXP>
+__device__ __forceinline__ void invert_square(double* A, int ld, int p, double* scr) {
+  constexpr int NW = NT / 32, MAXT = (2 * ((MAXP + 7) / 8 - 1) + NW - 1) / NW;   // tiles per warp and step
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, kl = lane & 3;
+  const int nb = (p + 7) >> 3;
+  for (int t0 = 0; t0 < 16 * nb; t0 += NT) {   // one column of one diagonal block's inverse per thread
+    const int t = t0 + tid, blk = t >> 4, c = t & 7, d0 = 8 * blk, w = min(8, p - d0);
+    const bool up = (t & 8) != 0, on = t < 16 * nb && c < w;
+    double x[8];
+#pragma unroll
+    for (int r = 0; r < 8; r++) x[r] = 0.0;
+    if (on) {
+      if (!up) {
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+          double s = r == c ? 1.0 : 0.0;
+#pragma unroll
+          for (int k = 0; k < r; k++)
+            if (k >= c && r < w) s -= A[(d0 + k) * ld + d0 + r] * x[k];
+          x[r] = r >= c ? s : 0.0;
+        }
+      } else {
+#pragma unroll
+        for (int r = 7; r >= 0; r--) {
+          if (r > c || r >= w) continue;
+          double s = r == c ? 1.0 : 0.0;
+#pragma unroll
+          for (int k = r + 1; k < 8; k++)
+            if (k <= c) s -= A[(d0 + k) * ld + d0 + r] * x[k];
+          x[r] = s / A[(d0 + r) * ld + d0 + r];
+        }
+      }
+    }
+    __syncthreads();   // a block's columns are read by its own 16 threads only, all in this pass
+    if (on) {
+#pragma unroll
+      for (int r = 0; r < 8; r++)
+        if (r < w && (up ? r <= c : r > c)) A[(d0 + c) * ld + d0 + r] = x[r];
+    }
+  }
+  __syncthreads();
+  double* ws = scr + 64 * warp;
+  for (int st = 1; st < nb; st++) {
+    // block row st of L^-1 (tiles j < st) and block row nb - 1 - st of U^-1 (tiles j > nb - 1 - st)
+    const int iu = nb - 1 - st;
+    double out[MAXT][2];
+#pragma unroll
+    for (int m = 0; m < MAXT; m++) {
+      const int q = warp + m * NW;   // tiles 0 .. st - 1 of L, then st tiles of U
+      out[m][0] = out[m][1] = 0.0;
+      if (q >= 2 * st) continue;   // uniform per warp
+      const bool up = q >= st;
+      const int j = up ? iu + 1 + (q - st) : q, i = up ? iu : st;
+      double s[2] = {0.0, 0.0};
+      if (!up) {
+        for (int k = j; k < i; k++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int kk = 8 * k + 4 * h + kl;
+            const int r = 8 * i + g;
+            dmma(s, r < p ? A[kk * ld + r] : 0.0, lower_at(A, ld, p, kk, 8 * j + g));
+          }
+      } else {
+        for (int k = i + 1; k <= j; k++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int kk = 8 * k + 4 * h + kl, c = 8 * j + g;
+            dmma(s, kk < p ? A[kk * ld + 8 * i + g] : 0.0, kk < p ? upper_at(A, ld, p, kk, c) : 0.0);
+          }
+      }
+      ws[(2 * kl) * 8 + g] = s[0];   // column-major 8 x 8
+      ws[(2 * kl + 1) * 8 + g] = s[1];
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int kk = 4 * h + kl;
+        const double x = up ? upper_at(A, ld, p, 8 * i + g, 8 * i + kk) : lower_at(A, ld, p, 8 * i + g, 8 * i + kk);
+        dmma(out[m], -x, ws[g * 8 + kk]);
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < MAXT; m++) {
+      const int q = warp + m * NW;
+      if (q >= 2 * st) continue;
+      const bool up = q >= st;
+      const int j = up ? iu + 1 + (q - st) : q, i = up ? iu : st;
+      const int r = 8 * i + g, c = 8 * j + 2 * kl;
+      if (r < p && c < p) A[c * ld + r] = out[m][0];
+      if (r < p && c + 1 < p) A[(c + 1) * ld + r] = out[m][1];
+    }
+    __syncthreads();
+  }
+}
+
+// L21 -> -L21 L11^-1 (8-row strips, tiles left to right: a tile needs the strip's columns from its own on)
+// and U12 -> -U11^-1 U12 (8-column strips, tiles downwards), in place, one warp per strip
+template <int NT>
+__device__ __forceinline__ void partinv_shared(double* A, int ld, int f, int p) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, kl = lane & 3;
+  const int nb = (p + 7) >> 3, ns = (f - p + 7) >> 3;
+  for (int q = warp; q < 2 * ns; q += NT / 32) {
+    const bool up = q >= ns;
+    const int s0 = p + 8 * (up ? q - ns : q);
+    for (int t = 0; t < nb; t++) {
+      double s[2] = {0.0, 0.0};
+      for (int k = t; k < nb; k++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int kk = 8 * k + 4 * h + kl;
+          if (!up) {
+            const double b = (kk < p && s0 + g < f) ? A[kk * ld + s0 + g] : 0.0;
+            dmma(s, b, lower_at(A, ld, p, kk, 8 * t + g));
+          } else {
+            const double b = (kk < p && s0 + g < f) ? A[(s0 + g) * ld + kk] : 0.0;
+            dmma(s, 8 * t + g < p ? upper_at(A, ld, p, 8 * t + g, kk) : 0.0, b);
           }
         }
-        __syncthreads();
+      __syncwarp();
+      if (!up) {
+        const int r = s0 + g, c = 8 * t + 2 * kl;
+        if (r < f && c < p) A[c * ld + r] = -s[0];
+        if (r < f && c + 1 < p) A[(c + 1) * ld + r] = -s[1];
+      } else {
+        const int r = 8 * t + g, c = s0 + 2 * kl;
+        if (r < p && c < f) A[c * ld + r] = -s[0];
+        if (r < p && c + 1 < f) A[(c + 1) * ld + r] = -s[1];
       }
-      best = sidx[0];
-      const double fully = sval[0];
-      __syncthreads();
-      // largest entry of column k in the rows of the not-yet-summed DoFs
-      double sm = 0.0;
-      for (int i = d.p + threadIdx.x; i < f; i += blockDim.x) sm = fmax(sm, fabs(colk[i]));
-      sval[threadIdx.x] = sm;
-      __syncthreads();
-      for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-        if (threadIdx.x < st) sval[threadIdx.x] = fmax(sval[threadIdx.x], sval[threadIdx.x + st]);
-        __syncthreads();
-      }
-      if (threadIdx.x == 0 && fully < kWeakPivot * sval[0] && d.parent >= 0) {
-        const int slot = atomicAdd(nweak, 1);
-        if (slot < weak_cap) weak[slot] = dofs[d.dptr + k];
-      }
+      __syncwarp();
     }
-    if (threadIdx.x == 0) {
-      s_piv = best;
-      piv[piv_off[fr] + k] = best;
-    }
-    __syncthreads();
-    const int pr = s_piv;
-    if (pr != k)
-      for (int j = threadIdx.x; j < f; j += blockDim.x) {
-        const double t = A[(int64_t)j * f + k];
-        A[(int64_t)j * f + k] = A[(int64_t)j * f + pr];
-        A[(int64_t)j * f + pr] = t;
-      }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double dk = colk[k];
-      if (!(fabs(dk) > 0.0) || (!pivoting && !(dk > 0.0))) {
-        atomicOr(flags, pivoting ? 1 : 2);   // 1: zero pivot (perturbed), 2: not positive definite
-        dk = dk == 0.0 ? 1e-300 : dk;
-        colk[k] = dk;
-      }
-      s_d = 1.0 / dk;
-    }
-    __syncthreads();
-    const double inv = s_d;
-    for (int i = k + 1 + threadIdx.x; i < f; i += blockDim.x) colk[i] *= inv;
-    __syncthreads();
-    // rank-1 update of the remaining panel columns
-    const int ncols = k0 + w - (k + 1);
-    const int nrows = f - (k + 1);
-    for (int64_t t = threadIdx.x; t < (int64_t)ncols * nrows; t += blockDim.x) {
-      const int jj = k + 1 + (int)(t / nrows);
-      const int ii = k + 1 + (int)(t % nrows);
-      A[(int64_t)jj * f + ii] -= colk[ii] * A[(int64_t)jj * f + k];
-    }
-    __syncthreads();
   }
 }
 
-// U12 = L11^-1 A12 for rows k0..k0+w-1 and columns k0+w..f-1 (unit lower L11)
-__global__ void __launch_bounds__(128) mf_trsm_kernel(const int32_t* __restrict__ lf, const FrontDesc* __restrict__ fd,
-                                                      int k0, double* __restrict__ F) {
-  const FrontDesc d = fd[lf[blockIdx.y]];
-  if (d.p <= k0) return;
-  const int w = min(PANEL, d.p - k0);
-  const int f = d.f;
-  const int j = k0 + w + blockIdx.x * blockDim.x + threadIdx.x;
-  __shared__ double L[PANEL][PANEL + 1];
-  double* A = F + d.off;
-  if (k0 + w + blockIdx.x * blockDim.x >= f) return;
-  for (int t = threadIdx.x; t < w * w; t += blockDim.x) {
-    const int r = t % w, c = t / w;
-    L[r][c] = A[(int64_t)(k0 + c) * f + (k0 + r)];
-  }
-  __syncthreads();
-  if (j >= f) return;
-  double x[PANEL];
-  double* col = A + (int64_t)j * f + k0;
-#pragma unroll
-  for (int r = 0; r < PANEL; r++)
-    if (r < w) x[r] = col[r];
-#pragma unroll
-  for (int r = 0; r < PANEL; r++) {
-    if (r >= w) break;
-    double s = x[r];
-#pragma unroll
-    for (int c = 0; c < PANEL; c++)
-      if (c < r) s -= L[r][c] * x[c];
-    x[r] = s;
-  }
-#pragma unroll
-  for (int r = 0; r < PANEL; r++)
-    if (r < w) col[r] = x[r];
+__host__ __device__ constexpr size_t fused_smem(int f, int nt) {
+  return sizeof(double) * ((size_t)f * (f | 1) + 2 * nt);
 }
 
-// trailing update: A22 -= L21 * U12, rows/cols k0+w .. f-1; 64x64 tile per CTA, K = w
-__global__ void __launch_bounds__(256) mf_gemm_kernel(const int32_t* __restrict__ lf, const FrontDesc* __restrict__ fd,
-                                                      int k0, double* __restrict__ F) {
-  const FrontDesc d = fd[lf[blockIdx.z]];
-  if (d.p <= k0) return;
-  const int w = min(PANEL, d.p - k0);
-  const int f = d.f;
-  const int base = k0 + w;
-  const int r0 = base + blockIdx.x * 64, c0 = base + blockIdx.y * 64;
-  if (r0 >= f || c0 >= f) return;
-  double* A = F + d.off;
-  __shared__ double Ls[PANEL][64];
-  __shared__ double Us[PANEL][64 + 1];
-  for (int t = threadIdx.x; t < PANEL * 64; t += blockDim.x) {
-    const int r = t % 64, c = t / 64;
-    Ls[c][r] = (c < w && r0 + r < f) ? A[(int64_t)(k0 + c) * f + r0 + r] : 0.0;
-    const int uc = t / PANEL, ur = t % PANEL;   // U tile: PANEL rows x 64 cols, coalesced along rows
-    Us[ur][uc] = (ur < w && c0 + uc < f) ? A[(int64_t)(c0 + uc) * f + k0 + ur] : 0.0;
+// one front (f <= MAXF) per CTA: see above. partinv: the solves use L21' and U12' too.
+template <int NT, int MAXF>
+__global__ void __launch_bounds__(NT, 768 / NT) mf_front_kernel(const int32_t* __restrict__ lf, FactorArgs a, int partinv) {
+  extern __shared__ double A[];
+  __shared__ int32_t pv[kFusedF], pm[kFusedF];
+  __shared__ LuScratch<NT> sc;
+  const int fr = lf[blockIdx.x], tid = threadIdx.x;
+  const FrontDesc d = a.fd[fr];
+  const int f = d.f, p = d.p, ld = f | 1;
+  double* scr = A + f * ld;
+  for (int t = tid; t < f * ld; t += NT) A[t] = 0.0;
+  __syncthreads();
+#pragma unroll 4
+  for (int64_t k = d.aptr + tid; k < d.aend; k += NT) {
+    const int pos = (int)__ldg(a.apos + k), j = pos / f;
+    const int64_t c = __ldg(a.acsr + k);
+    A[j * ld + (pos - j * f)] = a.ca * __ldg(a.va + c) + a.cb * __ldg(a.vb + c);
+  }
+  for (int slot = 0; slot < MAXKIDS; slot++) {
+    const int ch = d.kid[slot];
+    if (ch < 0) continue;   // uniform across the CTA
+    const FrontDesc cd = a.fd[ch];
+    const int s = cd.f - cd.p;
+    const int32_t* m = a.emap + cd.eptr;
+    const double* C = a.F + cd.off + (int64_t)cd.p * cd.f + cd.p;
+    __syncthreads();
+    for (int t0 = tid; t0 < s * s; t0 += 4 * NT) {   // four entries (distinct targets) in flight per thread
+      double v[4];
+      int to[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int t = t0 + q * NT, j = t / s, i = t - j * s;
+        to[q] = t < s * s ? __ldg(m + j) * ld + __ldg(m + i) : -1;
+        v[q] = t < s * s ? C[(int64_t)j * cd.f + i] : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (to[q] >= 0) A[to[q]] += v[q];
+    }
   }
   __syncthreads();
-  const int tr = threadIdx.x % 16, tc = threadIdx.x / 16;
-  double acc[4][4] = {};
-  for (int t = 0; t < w; t++) {
-    double a[4], b[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      a[q] = Ls[t][tr + 16 * q];
-      b[q] = Us[t][tc + 16 * q];
+  lu_shared<NT>(A, ld, f, p, a, a.dofs + d.dptr, d.parent >= 0, pv, sc);
+  if (tid == 0) {   // the row swaps as a gather permutation
+    for (int i = 0; i < p; i++) pm[i] = i;
+    for (int k = 0; k < p; k++) {
+      const int r = pv[k], x = pm[k];
+      pm[k] = pm[r];
+      pm[r] = x;
     }
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-#pragma unroll
-      for (int s = 0; s < 4; s++) acc[q][s] += a[q] * b[s];
   }
-#pragma unroll
-  for (int s = 0; s < 4; s++) {
-    const int c = c0 + tc + 16 * s;
-    if (c >= f) continue;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int r = r0 + tr + 16 * q;
-      if (r < f) A[(int64_t)c * f + r] -= acc[q][s];
+  __syncthreads();
+  invert_square<NT, MAXF>(A, ld, p, scr);
+  if (partinv) partinv_shared<NT>(A, ld, f, p);
+  __syncthreads();
+  double* out = a.F + d.off;
+  for (int t = tid; t < f * f; t += NT) {
+    const int j = t / f;
+    out[t] = A[j * ld + (t - j * f)];
+  }
+  const int64_t po = a.piv_off[fr];
+  for (int i = tid; i < p; i += NT) {
+    a.piv[po + i] = pv[i];
+    a.perm[po + i] = pm[i];
+    a.iperm[po + pm[i]] = i;
+  }
+}
+
+// Fronts factored in global memory advance eight columns per launch, one CTA per 8-column strip (blockIdx.x)
+// and front (blockIdx.y): step s applies the micro-panel 8 (s - 1) to the strip -- its row swaps, U12, and the
+// update of the rows below -- and the CTA of strip s then factors that strip, the next micro-panel, while the
+// other strips are still being updated. A strip of f rows costs a few microseconds, so a narrow level of
+// large fronts is spread over the chip instead of being bound by one SM's FP64 rate per front; 32-column
+// panels by one CTA, whose own update is nearly all of it on one SM's FP64 pipe, took 85 to 170 us each at 1M DoFs, a strip step 20 to 80.
+// RPT: rows of the strip per thread in the micro-panel; 0: the front has more rows than fit, the strip stays
+// in global memory.
+template <int NT, int RPT>
+__global__ void __launch_bounds__(NT) mf_strip_kernel(const int32_t* __restrict__ lf, FactorArgs a, int s) {
+  extern __shared__ double S[];
+  __shared__ int32_t pv[16];
+  __shared__ LuScratch<NT> sc;
+  const int fr = lf[blockIdx.y], tid = threadIdx.x;
+  const FrontDesc d = a.fd[fr];
+  const int f = d.f, p = d.p, q = blockIdx.x, kp = 8 * (s - 1), j0 = 8 * q;
+  if (j0 >= f || kp >= p || (s > 0 ? q == s - 1 : q != 0)) return;
+  double* G = a.F + d.off;
+  const int nc = min(8, f - j0);
+  const int w = s > 0 ? min(8, p - kp) : 0;
+  const int rb = s > 0 ? kp : 0, nr = f - rb, ld = RPT > 0 ? (nr | 1) : f;   // rows from rb on
+  double* C = RPT > 0 ? S : G + (int64_t)j0 * f + rb;
+  int32_t* piv = a.piv + a.piv_off[fr];
+  if (tid < w) pv[tid] = piv[kp + tid] - rb;
+  if (s > 0 && q < s - 1) {   // left of the micro-panel: row swaps only
+    __syncthreads();
+    if (tid < nc) swap_solve8(G + (int64_t)(j0 + tid) * f + rb, nullptr, 0, 0, w, pv, false);
+    return;
+  }
+  if (RPT > 0) {
+    for (int t = tid; t < nr * nc; t += NT) {
+      const int c = t / nr, i = t - c * nr;
+      S[c * ld + i] = G[(int64_t)(j0 + c) * f + rb + i];
+    }
+  }
+  __syncthreads();
+  if (s > 0) {
+    const double* P = G + (int64_t)kp * f + rb;   // the micro-panel's columns, rows from rb on
+    if (tid < nc) swap_solve8(C + (int64_t)tid * ld, P, f, 0, w, pv, true);
+    __syncthreads();
+    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, kl = lane & 3;
+    const double u0 = (g < nc && kl < w) ? C[(int64_t)g * ld + kl] : 0.0;
+    const double u1 = (g < nc && 4 + kl < w) ? C[(int64_t)g * ld + 4 + kl] : 0.0;
+    for (int i0 = w + 8 * warp; i0 < nr; i0 += NT / 4) {
+      const int i = i0 + g;
+      const bool ri = i < nr;
+      const double a0 = (ri && kl < w) ? -P[(int64_t)kl * f + i] : 0.0;
+      const double a1 = (ri && 4 + kl < w) ? -P[(int64_t)(4 + kl) * f + i] : 0.0;
+      double* o = C + (int64_t)(2 * kl) * ld + i;
+      double c[2] = {(ri && 2 * kl < nc) ? o[0] : 0.0, (ri && 2 * kl + 1 < nc) ? o[ld] : 0.0};
+      dmma(c, a0, u0);
+      dmma(c, a1, u1);
+      if (ri && 2 * kl < nc) o[0] = c[0];
+      if (ri && 2 * kl + 1 < nc) o[ld] = c[1];
+    }
+    __syncthreads();
+  }
+  if (q == s && j0 < p) {   // the next micro-panel (its columns past the pivots are solved with it)
+    const int k0 = j0 - rb, wn = min(8, p - j0);
+    if constexpr (RPT > 0)
+      micro_panel<NT, RPT>(C, ld, k0, nr, nc, wn, p - rb, a, a.dofs + d.dptr + rb, d.parent >= 0, pv, sc);
+    else
+      micro_panel_memory(C, ld, k0, nr, nc, wn, p - rb, a, a.dofs + d.dptr + rb, d.parent >= 0, pv, sc);
+    __syncthreads();
+    if (tid < wn) piv[j0 + tid] = pv[k0 + tid] + rb;
+  }
+  if (RPT > 0) {
+    for (int t = tid; t < nr * nc; t += NT) {
+      const int c = t / nr, i = t - c * nr;
+      G[(int64_t)(j0 + c) * f + rb + i] = S[c * ld + i];
     }
   }
 }
@@ -261,11 +729,12 @@ __global__ void __launch_bounds__(256) mf_gemm_kernel(const int32_t* __restrict_
 constexpr int CL = 8;
 
 // sequential LAPACK-style row swaps -> gather permutation (v'[i] = v[perm[i]])
-__global__ void mf_perm_kernel(int nf, const FrontDesc* __restrict__ fd, const int32_t* __restrict__ piv,
-                               const int64_t* __restrict__ piv_off, int32_t* __restrict__ perm,
+__global__ void mf_perm_kernel(int nl, const int32_t* __restrict__ lf, const FrontDesc* __restrict__ fd,
+                               const int32_t* __restrict__ piv, const int64_t* __restrict__ piv_off, int32_t* __restrict__ perm,
                                int32_t* __restrict__ iperm) {
-  const int fr = blockIdx.x * blockDim.x + threadIdx.x;
-  if (fr >= nf) return;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= nl) return;
+  const int fr = lf[q];
   const int p = fd[fr].p;
   const int32_t* pv = piv + piv_off[fr];
   int32_t* pm = perm + piv_off[fr];
@@ -436,38 +905,153 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
 // fully parallel products:
 //   forward:  y = L11^-1 P b_p,  b_s -= L21 y          (b_s goes to the parent)
 //   backward: x_p = U11^-1 (y - U12 x_s)
-constexpr int kSmallP = 160;
-constexpr int kSmallF = 512;
 
-// column j of L11^-1 and of U11^-1 per thread, from a shared-memory copy of the LU square
-__global__ void __launch_bounds__(256) mf_invdiag_kernel(const int32_t* __restrict__ lf,
-                                                         const FrontDesc* __restrict__ fd, double* __restrict__ F) {
-  const FrontDesc d = fd[lf[blockIdx.x]];
-  const int f = d.f, p = d.p;
-  extern __shared__ double S[];   // S[k * p + i] = LU(i, k)
-  double* A = F + d.off;
-  for (int t = threadIdx.x; t < p * p; t += blockDim.x) {
-    const int i = t % p, k = t / p;
-    S[t] = A[(int64_t)k * f + i];
+// One 8-column strip of L11^-1 (kind 0) or U11^-1 (kind 1) of a front factored in global memory, per CTA:
+//   X_i = -L_ii^-1 sum_{j <= k < i} L_ik X_k   down from the strip's diagonal block (up from it for U),
+// the strip in shared memory, the sums over k split over the four warps. Results go to the scratch square
+// (FrontDesc::aux), since the other strips of the front still read the factors.
+__global__ void __launch_bounds__(128) mf_inverse_kernel(const int4* __restrict__ items,
+                                                         const FrontDesc* __restrict__ fd,
+                                                         const double* __restrict__ F, double* __restrict__ sq) {
+  extern __shared__ double X[];   // X[n * ldx + row]: column n of the strip
+  __shared__ double part[4][64];
+  const int4 it = items[blockIdx.x];
+  const FrontDesc d = fd[it.x];
+  const int p = d.p, f = d.f, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, kl = lane & 3;
+  const bool up = it.y != 0;
+  const int j = it.z, nb = (p + 7) >> 3, ldx = (8 * nb) | 4;
+  const double* A = F + d.off;
+  auto at = [&](int r, int c) -> double {   // the triangular factor
+    if (r >= p || c >= p) return 0.0;
+    if (r == c) return up ? A[(int64_t)c * f + r] : 1.0;
+    return (up ? r < c : r > c) ? A[(int64_t)c * f + r] : 0.0;
+  };
+  for (int t = tid; t < 8 * ldx; t += 128) X[t] = 0.0;
+  // the inverses of the diagonal blocks that the strip passes, one column per thread
+  const int steps = up ? j + 1 : nb - j, i_lo = up ? 0 : j;
+  double* dg = X + 8 * ldx;   // 64 per block, column-major
+  for (int t = tid; t < 8 * steps; t += 128) {
+    const int c = t & 7, d0 = 8 * (i_lo + (t >> 3));
+    double x[8];
+#pragma unroll
+    for (int r = 0; r < 8; r++) x[r] = 0.0;
+    if (d0 + c < p) {
+      if (!up) {
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+          double s = r == c ? 1.0 : 0.0;
+#pragma unroll
+          for (int k = 0; k < r; k++) s -= at(d0 + r, d0 + k) * x[k];
+          x[r] = r >= c ? s : 0.0;
+        }
+      } else {
+#pragma unroll
+        for (int r = 7; r >= 0; r--) {
+          if (r > c) continue;
+          double s = r == c ? 1.0 : 0.0;
+#pragma unroll
+          for (int k = r + 1; k < 8; k++) s -= at(d0 + r, d0 + k) * x[k];
+          x[r] = s / A[(int64_t)(d0 + r) * f + d0 + r];
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 8; r++) dg[8 * t + r] = x[r];
   }
   __syncthreads();
-  for (int j = threadIdx.x; j < p; j += blockDim.x) {
-    double* out = A + (int64_t)j * f;   // column j; only this thread writes it
-    // L11 x = e_j (unit diagonal): x_j = 1, x_i = -sum_{k=j}^{i-1} L(i,k) x_k
-    for (int i = j + 1; i < p; i++) {
-      double acc = -S[j * p + i];
-      for (int k = j + 1; k < i; k++) acc -= S[k * p + i] * out[k];
-      out[i] = acc;
+  for (int st = 0; st < steps; st++) {
+    const int i = up ? j - st : j + st;
+    // S = sum over the block columns between i and j, the strip's rows known so far
+    double s[2] = {0.0, 0.0};
+    const int klo = up ? i + 1 : j, khi = up ? j + 1 : i;
+    for (int k = klo + warp; k < khi; k += 4)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int kk = 8 * k + 4 * h + kl;
+        const int r = 8 * i + g;
+        dmma(s, (r < p && kk < p) ? A[(int64_t)kk * f + r] : 0.0, X[g * ldx + kk]);
+      }
+    part[warp][(2 * kl) * 8 + g] = s[0];
+    part[warp][(2 * kl + 1) * 8 + g] = s[1];
+    __syncthreads();
+    if (warp == 0) {
+      double o[2] = {0.0, 0.0};
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int kk = 4 * h + kl, e = g * 8 + kk;   // S[kk][g]
+        const double sv = i == j ? (kk == g ? -1.0 : 0.0) : (part[0][e] + part[1][e]) + (part[2][e] + part[3][e]);
+        dmma(o, -dg[64 * (i - i_lo) + kk * 8 + g], sv);
+      }
+      X[(2 * kl) * ldx + 8 * i + g] = o[0];
+      X[(2 * kl + 1) * ldx + 8 * i + g] = o[1];
     }
-    // U11 y = e_j: y_j = 1 / U(j,j), y_i = -(sum_{k=i+1}^{j} U(i,k) y_k) / U(i,i)
-    out[j] = 1.0 / S[j * p + j];
-    for (int i = j - 1; i >= 0; i--) {
-      double acc = 0.0;
-      for (int k = i + 1; k <= j; k++) acc += S[k * p + i] * out[k];
-      out[i] = -acc / S[i * p + i];
+    __syncthreads();
+  }
+  double* out = sq + d.aux;
+  const int r_lo = up ? 0 : 8 * j, r_hi = up ? min(p, 8 * j + 8) : p;
+  for (int t = tid; t < 8 * (r_hi - r_lo); t += 128) {
+    const int n = t / (r_hi - r_lo), r = r_lo + t - n * (r_hi - r_lo), c = 8 * j + n;
+    if (c < p && (up ? r <= c : r > c)) out[(int64_t)c * p + r] = X[n * ldx + r];
+  }
+}
+
+// the scratch squares back into their fronts
+__global__ void mf_square_copy_kernel(const int32_t* __restrict__ lf, const FrontDesc* __restrict__ fd,
+                                      const double* __restrict__ S, double* __restrict__ F) {
+  const FrontDesc d = fd[lf[blockIdx.y]];
+  const int64_t pp = (int64_t)d.p * d.p;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < pp; t += (int64_t)gridDim.x * blockDim.x) {
+    const int i = (int)(t % d.p), k = (int)(t / d.p);
+    F[d.off + (int64_t)k * d.f + i] = S[d.aux + t];
+  }
+}
+
+// One 8-row strip of L21' = -L21 L11^-1 (kind 0) or 8-column strip of U12' = -U11^-1 U12 (kind 1) of a front
+// factored in global memory, per CTA: the strip in shared memory, its 8 x 8 tiles dealt to four warps; items
+// are (front, kind, first row / column past the pivots).
+__global__ void __launch_bounds__(128) mf_partinv_kernel(const int4* __restrict__ items,
+                                                         const FrontDesc* __restrict__ fd, double* __restrict__ F) {
+  extern __shared__ double X[];   // X[n * ldx + k]: pivot row / column k of the strip's n-th column / row
+  const int4 it = items[blockIdx.x];
+  const FrontDesc d = fd[it.x];
+  const int p = d.p, f = d.f, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, kl = lane & 3;
+  const bool up = it.y != 0;
+  const int s0 = p + it.z, nb = (p + 7) >> 3, ldx = (8 * nb) | 4;
+  double* A = F + d.off;
+  for (int t = tid; t < 8 * ldx; t += 128) X[t] = 0.0;
+  __syncthreads();
+  for (int t = tid; t < 8 * p; t += 128) {
+    const int n = up ? t / p : t & 7, k = up ? t - n * p : t >> 3;
+    if (s0 + n < f) X[n * ldx + k] = up ? A[(int64_t)(s0 + n) * f + k] : A[(int64_t)k * f + s0 + n];
+  }
+  __syncthreads();
+  for (int q = warp; q < nb; q += 4) {
+    double s[2] = {0.0, 0.0};
+    for (int k = q; k < nb; k++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int kk = 8 * k + 4 * h + kl, e = 8 * q + g;
+        if (!up) {
+          const double l = (kk >= p || e > kk) ? 0.0 : (e == kk ? 1.0 : A[(int64_t)e * f + kk]);   // L11^-1(kk, e)
+          dmma(s, X[g * ldx + kk], l);
+        } else {
+          const double u = (kk >= p || kk < e) ? 0.0 : A[(int64_t)kk * f + e];   // U11^-1(e, kk)
+          dmma(s, u, X[g * ldx + kk]);
+        }
+      }
+    if (!up) {
+      const int r = s0 + g, c = 8 * q + 2 * kl;
+      if (r < f && c < p) A[(int64_t)c * f + r] = -s[0];
+      if (r < f && c + 1 < p) A[(int64_t)(c + 1) * f + r] = -s[1];
+    } else {
+      const int r = 8 * q + g, c = s0 + 2 * kl;
+      if (r < p && c < f) A[(int64_t)c * f + r] = -s[0];
+      if (r < p && c + 1 < f) A[(int64_t)(c + 1) * f + r] = -s[1];
     }
   }
 }
+
+constexpr size_t inverse_smem(int p) { return sizeof(double) * 8 * (size_t)((((p + 7) / 8 * 8) | 4) + (p + 7) / 8 * 8); }
 
 // sum_{k = k0}^{k1 - 1} A[k * f] * v[k] with four independent accumulators (eight loads in flight per
 // thread): the solve loops are latency-bound on the factor reads, not FP64-bound
@@ -689,14 +1273,6 @@ __device__ __forceinline__ double pull_row(const TiledArgs& a, const FrontDesc& 
   return s;
 }
 
-// c += a b on an 8 x 8 tile, inner dimension 4: lane l holds a[l / 4][l % 4], b[l % 4][l / 4] and
-// c[l / 4][2 (l % 4) + {0, 1}]
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(c[0]), "+d"(c[1])
-      : "d"(a), "d"(b));
-}
-
 // One tile: rows r0 .. r0 + 7, columns c0 .. c0 + 8 NT - 1: init(r, c) + sum over kbeg <= k < kend of
 // F(r, k) v[k], F taken only where use(r, k). load(k, c) gives v[k][c0 + c]; done(r, c, sum) gets each row
 // below rlim. vs holds `chunk` rows of v (a multiple of 16, as many as the level's longest sum needs, so
@@ -793,97 +1369,6 @@ __global__ void __launch_bounds__(kTileThreads) mf_backward_tiled_kernel(const i
       a.F + d.off, d.f, it.y, p, it.y, d.f, min(8 * NT, a.nb - c0), a.chunk, [](int r, int k) { return k >= r; },
       [&](int k, int c) { return k < p ? y[(int64_t)k * kLdW + c] : X[(int64_t)D[k] * a.ldx + c]; },
       [](int, int) { return 0.0; }, [&](int r, int c, double s) { X[(int64_t)D[r] * a.ldx + c] = s; });
-}
-
-// the p x p LU square of each listed front, copied (column-major) to scratch at FrontDesc::aux
-__global__ void mf_square_copy_kernel(const int32_t* __restrict__ lf, const FrontDesc* __restrict__ fd,
-                                      const double* __restrict__ F, double* __restrict__ S) {
-  const FrontDesc d = fd[lf[blockIdx.y]];
-  const int64_t pp = (int64_t)d.p * d.p;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < pp; t += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(t % d.p), k = (int)(t / d.p);
-    S[d.aux + t] = F[d.off + (int64_t)k * d.f + i];
-  }
-}
-
-// columns j0 .. j0 + 31 of (L11^-1, U11^-1) of a front with p > kSmallP, one thread per column, from
-// the scratch copy of its LU square; the column being built stays in shared memory (o[i * 32])
-__global__ void __launch_bounds__(32) mf_invdiag_wide_kernel(const int2* __restrict__ items,
-                                                             const FrontDesc* __restrict__ fd,
-                                                             const double* __restrict__ S, double* __restrict__ F) {
-  extern __shared__ double ob[];
-  const int2 it = items[blockIdx.x];
-  const FrontDesc d = fd[it.x];
-  const int p = d.p, f = d.f;
-  const int lane = threadIdx.x, j = it.y + lane;
-  if (j >= p) return;
-  const double* Sp = S + d.aux;   // Sp[k * p + i] = LU(i, k)
-  double* o = ob + lane;
-  // L11 x = e_j (unit diagonal): x_i = -L(i, j) - sum_{k = j+1}^{i-1} L(i, k) x_k for i > j
-  for (int i = j + 1; i < p; i++) {
-    double a0 = -Sp[(int64_t)j * p + i], a1 = 0.0;
-    int k = j + 1;
-    for (; k + 2 <= i; k += 2) {
-      a0 -= Sp[(int64_t)k * p + i] * o[k * 32];
-      a1 -= Sp[(int64_t)(k + 1) * p + i] * o[(k + 1) * 32];
-    }
-    if (k < i) a0 -= Sp[(int64_t)k * p + i] * o[k * 32];
-    o[i * 32] = a0 + a1;
-  }
-  // U11 y = e_j: y_j = 1 / U(j, j), y_i = -(sum_{k = i+1}^{j} U(i, k) y_k) / U(i, i) for i < j
-  o[j * 32] = 1.0 / Sp[(int64_t)j * p + j];
-  for (int i = j - 1; i >= 0; i--) {
-    double a0 = 0.0, a1 = 0.0;
-    int k = i + 1;
-    for (; k + 2 <= j + 1; k += 2) {
-      a0 += Sp[(int64_t)k * p + i] * o[k * 32];
-      a1 += Sp[(int64_t)(k + 1) * p + i] * o[(k + 1) * 32];
-    }
-    if (k <= j) a0 += Sp[(int64_t)k * p + i] * o[k * 32];
-    o[i * 32] = -(a0 + a1) / Sp[(int64_t)i * p + i];
-  }
-  double* out = F + d.off + (int64_t)j * f;
-  for (int i = 0; i < p; i++) out[i] = o[i * 32];
-}
-
-// L21' = -L21 L11^-1 (kind 0: rows t0 .. t0 + 7 of L21) and U12' = -U11^-1 U12 (kind 1: columns
-// t0 .. t0 + 7 of U12), one warp per row / column, from the inverted diagonal square; items are
-// (front, kind, t0, 0). Each warp reads only the square and writes only its own row / column.
-__global__ void __launch_bounds__(256) mf_partinv_kernel(const int4* __restrict__ items,
-                                                         const FrontDesc* __restrict__ fd, double* __restrict__ F) {
-  extern __shared__ double pb[];   // kTileRows x p: the warp's original row / column
-  const int4 it = items[blockIdx.x];
-  const FrontDesc d = fd[it.x];
-  const int f = d.f, p = d.p;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q = p + it.z + warp;   // row (kind 0) or column (kind 1) of the front
-  double* A = F + d.off;
-  double* b = pb + (size_t)warp * p;
-  if (q >= f) return;   // no block-wide barrier below
-  if (it.y == 0) {
-    for (int i = lane; i < p; i += 32) b[i] = A[(int64_t)i * f + q];
-    __syncwarp();
-    for (int k = 0; k < p; k++) {
-      double s = 0.0;
-      for (int i = k + 1 + lane; i < p; i += 32) s += b[i] * A[(int64_t)k * f + i];
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-      if (lane == 0) A[(int64_t)k * f + q] = -(b[k] + s);
-    }
-  } else {
-    for (int k = lane; k < p; k += 32) b[k] = A[(int64_t)q * f + k];
-    __syncwarp();
-    for (int i = lane; i < p; i += 32) {
-      double s0 = 0.0, s1 = 0.0;
-      int k = i;
-      for (; k + 2 <= p; k += 2) {
-        s0 += A[(int64_t)k * f + i] * b[k];
-        s1 += A[(int64_t)(k + 1) * f + i] * b[k + 1];
-      }
-      if (k < p) s0 += A[(int64_t)k * f + i] * b[k];
-      A[(int64_t)q * f + i] = -(s0 + s1);
-    }
-  }
 }
 
 // X = Kinv B for a dense inverse (n x n, row-major): one warp per row, lane c owns right-hand side c;
@@ -1026,16 +1511,29 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   }
   int64_t o = 0, po = 0, wo = 0;
   level_off.assign(nlevels + 1, 0);
+  std::vector<uint8_t> fused(nf, 0);
+  for (int l = 0; l < nlevels; l++) {
+    const int n = s.level_ptr[l + 1] - s.level_ptr[l];
+    for (int k = s.level_ptr[l]; k < s.level_ptr[l + 1]; k++) {
+      const int f = s.level_fronts[k];
+      fused[f] = s.p[f] <= kSmallP && s.f[f] <= (n <= c.num_sms ? kFusedNarrowF : kFusedF);
+    }
+  }
+  level_big_end.assign(nlevels, 0);
   for (int l = 0; l < nlevels; l++) {
     level_off[l] = o;
-    for (int k = s.level_ptr[l]; k < s.level_ptr[l + 1]; k++) {
-      int f = s.level_fronts[k];
-      off[f] = o;
-      o += (int64_t)s.f[f] * s.f[f];
-      poff[f] = po;
-      po += s.p[f];
-      woff_h[f] = wo;
-      wo += (int64_t)s.f[f] * kLdW;
+    for (int pass = 0; pass < 2; pass++) {   // the fronts factored in global memory first: their range is zeroed
+      for (int k = s.level_ptr[l]; k < s.level_ptr[l + 1]; k++) {
+        int f = s.level_fronts[k];
+        if (fused[f] != (pass == 1)) continue;
+        off[f] = o;
+        o += (int64_t)s.f[f] * s.f[f];
+        poff[f] = po;
+        po += s.p[f];
+        woff_h[f] = wo;
+        wo += (int64_t)s.f[f] * kLdW;
+      }
+      if (pass == 0) level_big_end[l] = o;
     }
   }
   level_off[nlevels] = o;
@@ -1068,10 +1566,9 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   if (wo / kLdW > INT32_MAX) fail(FEM2D_E_TOO_LARGE, "solve workspace rows exceed 32 bits");
   tf_ptr.assign(nlevels + 1, 0);
   tb_ptr.assign(nlevels + 1, 0);
-  std::vector<int32_t> tf_h, tb_h, mid_h, wide_h, wi_h, pi_h;
+  std::vector<int32_t> tf_h, tb_h, inv_h, ii_h, pi_h;
   std::vector<int32_t> pull_h;   // 8 per row: DoF, children's workspace rows (see pull_row)
-  nmid = nwide = npinv = 0;
-  max_mid_p = max_wide_p = max_tiled_p = 0;
+  max_inv_p = 0;
   int64_t sq_total = 0;
   const bool single_dense = nf == 1 && max_p == max_f && max_f <= 4096;   // factor() inverts it whole
   for (int l = 0; l < nlevels; l++) {
@@ -1090,23 +1587,8 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
     for (int k = s.level_ptr[l]; k < s.level_ptr[l + 1]; k++) {
       const int fr = s.level_fronts[k];
       const int F = s.f[fr], P = s.p[fr];
-      max_tiled_p = std::max(max_tiled_p, P);
       for (int r0 = 0; r0 < F; r0 += kTileRows) tf_h.insert(tf_h.end(), {fr, r0});
       for (int r0 = 0; r0 < P; r0 += kTileRows) tb_h.insert(tb_h.end(), {fr, r0});
-      const bool small = P <= kSmallP && F <= kSmallF;
-      if (!small && P > 0 && P <= kSmallP) {
-        mid_h.push_back(fr);
-        max_mid_p = std::max(max_mid_p, P);
-      }
-      if (P > kSmallP) {
-        wide_h.push_back(fr);
-        fdh[fr].aux = sq_total;
-        sq_total += (int64_t)P * P;
-        max_wide_p = std::max(max_wide_p, P);
-        for (int j0 = 0; j0 < P; j0 += 32) wi_h.insert(wi_h.end(), {fr, j0});
-      }
-      if (P > 0)
-        for (int t0 = 0; t0 < F - P; t0 += kTileRows) pi_h.insert(pi_h.end(), {fr, 0, t0, 0, fr, 1, t0, 0});
       // pull records: row u of the front (before pivoting) receives row i of child ch's update block
       fdh[fr].prow = (int64_t)pull_h.size() / 8;
       pull_h.resize(pull_h.size() + (size_t)8 * F, -1);
@@ -1129,18 +1611,60 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
       level_pmax[l] = std::max(level_pmax[l], P);
     }
   }
+  // factorization work: per level the fronts factored in global memory, and groups of the others (wide
+  // levels by size class, so that small fronts share an SM; within a group the largest first)
+  std::vector<int32_t> big_h, fused_h;
+  big_ptr.assign(nlevels + 1, 0);
+  fused_groups.clear();
+  level_big_f.assign(nlevels, 0);
+  level_big_p.assign(nlevels, 0);
+  for (int l = 0; l < nlevels; l++) {
+    big_ptr[l] = (int32_t)big_h.size();
+    std::vector<int32_t> q;
+    for (int k = s.level_ptr[l]; k < s.level_ptr[l + 1]; k++) {
+      const int fr = s.level_fronts[k], F = s.f[fr], P = s.p[fr];
+      if (fused[fr]) {
+        q.push_back(fr);
+        continue;
+      }
+      big_h.push_back(fr);
+      level_big_f[l] = std::max(level_big_f[l], F);
+      level_big_p[l] = std::max(level_big_p[l], P);
+      if (P == 0 || !(level_tiled[l] || (P <= kSmallP && F <= kSmallF))) continue;
+      inv_h.push_back(fr);
+      max_inv_p = std::max(max_inv_p, P);
+      fdh[fr].aux = sq_total;
+      sq_total += (int64_t)P * P;
+      for (int j = 0; j < (P + 7) / 8; j++) ii_h.insert(ii_h.end(), {fr, 0, j, 0, fr, 1, j, 0});
+      if (level_tiled[l])
+        for (int t0 = 0; t0 < F - P; t0 += 8) pi_h.insert(pi_h.end(), {fr, 0, t0, 0, fr, 1, t0, 0});
+    }
+    std::stable_sort(q.begin(), q.end(), [&](int32_t x, int32_t y) { return s.f[x] > s.f[y]; });
+    const int classes[] = {kFusedF, 116, 95, 82, kFusedSmallF, 48, 32};   // 1, 2, 3, 4, 6, ... CTAs per SM
+    const int ncl = (int)q.size() <= 2 * c.num_sms ? 1 : 7;
+    size_t k0 = 0;
+    for (int cl = 0; cl < ncl && k0 < q.size(); cl++) {
+      size_t k1 = k0;
+      while (k1 < q.size() && (cl + 1 == ncl || s.f[q[k1]] > classes[cl + 1])) k1++;
+      if (k1 == k0) continue;
+      fused_groups.push_back({l, (int)fused_h.size(), (int)(k1 - k0), s.f[q[k0]]});
+      fused_h.insert(fused_h.end(), q.begin() + k0, q.begin() + k1);
+      k0 = k1;
+    }
+  }
+  big_ptr[nlevels] = (int32_t)big_h.size();
+  lbig.upload(big_h, st);
+  lfused.upload(fused_h, st);
   tf_ptr[nlevels] = (int32_t)(tf_h.size() / 2);
   tb_ptr[nlevels] = (int32_t)(tb_h.size() / 2);
-  nmid = (int)mid_h.size();
-  nwide = (int)wide_h.size();
-  nwide_items = (int)(wi_h.size() / 2);
+  ninv = (int)inv_h.size();
+  ninv_items = (int)(ii_h.size() / 4);
   npinv = (int)(pi_h.size() / 4);
   tf_items.upload(tf_h, st);
   tb_items.upload(tb_h, st);
   pull.upload(pull_h, st);
-  lmid.upload(mid_h, st);
-  lwide.upload(wide_h, st);
-  wide_items.upload(wi_h, st);
+  linv.upload(inv_h, st);
+  inv_items.upload(ii_h, st);
   pinv_items.upload(pi_h, st);
   sq.alloc(std::max<int64_t>(sq_total, 1));
   std::vector<uint8_t> raw(fdh.size() * sizeof(FrontDesc));
@@ -1158,14 +1682,10 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   flags.alloc(1);
   weak_list.alloc(std::max<int64_t>(s.n, 1));
   weak_count.alloc(1);
-  level_max_f.assign(nlevels, 0);
-  level_max_p.assign(nlevels, 0);
   level_factor_bytes.assign(nlevels, 0.0);
   for (int l = 0; l < nlevels; l++)
     for (int k = s.level_ptr[l]; k < s.level_ptr[l + 1]; k++) {
       const double F = s.f[s.level_fronts[k]], P = s.p[s.level_fronts[k]];
-      level_max_f[l] = std::max(level_max_f[l], s.f[s.level_fronts[k]]);
-      level_max_p[l] = std::max(level_max_p[l], s.p[s.level_fronts[k]]);
       level_factor_bytes[l] += 8.0 * (0.5 * P * P + P * (F - P));
     }
   std::vector<int32_t> ls, ll;
@@ -1173,7 +1693,6 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   large_ptr.assign(nlevels + 1, 0);
   level_fwd_cols.assign(nlevels, 0);
   level_bwd_cols.assign(nlevels, 0);
-  max_small_p = 0;
   for (int l = 0; l < nlevels; l++) {
     small_ptr[l] = (int32_t)ls.size();
     large_ptr[l] = (int32_t)ll.size();
@@ -1183,7 +1702,6 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
         ls.push_back(fr);
         level_fwd_cols[l] = std::max(level_fwd_cols[l], forward_cols(s.f[fr], s.p[fr]));
         level_bwd_cols[l] = std::max(level_bwd_cols[l], backward_cols(s.f[fr], s.p[fr]));
-        max_small_p = std::max(max_small_p, s.p[fr]);
       } else {
         ll.push_back(fr);
       }
@@ -1191,7 +1709,6 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   }
   small_ptr[nlevels] = (int32_t)ls.size();
   large_ptr[nlevels] = (int32_t)ll.size();
-  nsmall = (int)ls.size();
   lsmall.upload(ls, st);
   llarge.upload(ll, st);
   // dynamic shared memory limits are set once per device (a function attribute of the device's context)
@@ -1200,18 +1717,23 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   std::lock_guard<std::mutex> lk(attr_mu);
   if (c.device >= 0 && c.device < 256 && !attr_done[c.device]) {
     const int smem = (kSmallF + kSmallP + 2) * kLdW * (int)sizeof(double);
-    FEM2D_CUDA(cudaFuncSetAttribute(mf_invdiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kSmallP * kSmallP * (int)sizeof(double)));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_front_kernel<256, kFusedF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)fused_smem(kFusedF, 256)));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_front_kernel<128, kFusedSmallF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)fused_smem(kFusedSmallF, 128)));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_strip_kernel<256, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, strip_smem(256)));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_strip_kernel<512, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, strip_smem(1024)));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_strip_kernel<512, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, strip_smem(2048)));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)inverse_smem(kTiledMaxP)));
+    FEM2D_CUDA(cudaFuncSetAttribute(mf_partinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)inverse_smem(kTiledMaxP)));
     FEM2D_CUDA(cudaFuncSetAttribute(mf_forward_small_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     FEM2D_CUDA(cudaFuncSetAttribute(mf_forward_small_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     FEM2D_CUDA(cudaFuncSetAttribute(mf_forward_small_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     FEM2D_CUDA(cudaFuncSetAttribute(mf_backward_small_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     FEM2D_CUDA(cudaFuncSetAttribute(mf_backward_small_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     FEM2D_CUDA(cudaFuncSetAttribute(mf_backward_small_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    FEM2D_CUDA(cudaFuncSetAttribute(mf_invdiag_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kTiledMaxP * 32 * (int)sizeof(double)));
-    FEM2D_CUDA(cudaFuncSetAttribute(mf_partinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kTileRows * kTiledMaxP * (int)sizeof(double)));
     attr_done[c.device] = true;
   }
 }
@@ -1254,56 +1776,58 @@ void MFDevice::factor(Ctx& c, const double* va, const double* vb, double ca, dou
     out.flags = read_flags(c);
     return;
   }
+  if (out.perm.n != out.piv.n) out.perm.alloc_on(out.piv.n, st);
+  if (out.iperm.n != out.piv.n) out.iperm.alloc_on(out.piv.n, st);
+  const FactorArgs fa{fd,     asm_pos.p,  asm_csr.p,  va,        vb,      ca,          cb,           ea_map.p,
+                      dofs.p, piv_off.p,  Fbuf.p,     out.piv.p, out.perm.p, out.iperm.p, flags.p,  weak_list.p,
+                      weak_count.p, (int)weak_list.n, cholesky ? 0 : 1};
+  size_t group = 0;
   for (int l = 0; l < nlevels; l++) {
-    const int nfl = level_ptr[l + 1] - level_ptr[l];
-    const int32_t* lf = lfronts.p + level_ptr[l];
-    FEM2D_CUDA(cudaMemsetAsync(Fbuf.p + level_off[l], 0, (level_off[l + 1] - level_off[l]) * sizeof(double), st));
-    mf_assemble_kernel<<<dim3(8, nfl), 256, 0, st>>>(lf, fd, asm_pos.p, asm_csr.p, va, vb, ca, cb, Fbuf.p);
-    c.launches++;
-    if (l > 0) {
-      for (int slot = 0; slot < MAXKIDS; slot++) {
-        mf_extend_add_kernel<<<dim3(16, nfl), 256, 0, st>>>(lf, fd, slot, ea_map.p, Fbuf.p);
-        c.launches++;
-      }
+    for (; group < fused_groups.size() && fused_groups[group].level == l; group++) {
+      const FusedGroup& g = fused_groups[group];
+      const int32_t* lf = lfused.p + g.first;
+      if (g.max_f <= kFusedSmallF)
+        mf_front_kernel<128, kFusedSmallF><<<g.count, 128, fused_smem(g.max_f, 128), st>>>(lf, fa, level_tiled[l]);
+      else
+        mf_front_kernel<256, kFusedF><<<g.count, 256, fused_smem(g.max_f, 256), st>>>(lf, fa, level_tiled[l]);
+      c.launches++;
     }
-    const int mf = level_max_f[l], mp = level_max_p[l];
-    for (int k0 = 0; k0 < mp; k0 += PANEL) {
-      mf_panel_kernel<<<nfl, 256, 0, st>>>(lf, fd, k0, cholesky ? 0 : 1, Fbuf.p, out.piv.p, piv_off.p, flags.p,
-                                           dofs.p, weak_list.p, weak_count.p, (int)weak_list.n);
-      const int rest = mf - k0;   // upper bound of remaining columns
-      if (rest > 0) {
-        dim3 gt((rest + 127) / 128, nfl);
-        mf_trsm_kernel<<<gt, 128, 0, st>>>(lf, fd, k0, Fbuf.p);
-        dim3 gg((rest + 63) / 64, (rest + 63) / 64, nfl);
-        mf_gemm_kernel<<<gg, 256, 0, st>>>(lf, fd, k0, Fbuf.p);
-        c.launches += 2;
-      }
+    const int nbig = big_ptr[l + 1] - big_ptr[l];
+    if (nbig == 0) continue;
+    const int32_t* lf = lbig.p + big_ptr[l];
+    FEM2D_CUDA(cudaMemsetAsync(Fbuf.p + level_off[l], 0, (level_big_end[l] - level_off[l]) * sizeof(double), st));
+    mf_assemble_kernel<<<dim3(8, nbig), 256, 0, st>>>(lf, fd, asm_pos.p, asm_csr.p, va, vb, ca, cb, Fbuf.p);
+    c.launches++;
+    const int mf = level_big_f[l], mp = level_big_p[l], strips = (mf + 7) / 8;
+    if (l > 0) {
+      mf_extend_add_kernel<<<dim3((mf + kExtendCols - 1) / kExtendCols, nbig), 256, 0, st>>>(lf, fd, ea_map.p, Fbuf.p);
+      c.launches++;
+    }
+    for (int s = 0; mp > 0 && s <= (mp + 7) / 8; s++) {
+      const dim3 grid(s == 0 ? 1 : strips, nbig);
+      const int rows = mf - std::max(0, 8 * (s - 1));   // upper bound of the strips' rows
+      if (rows <= 256) mf_strip_kernel<256, 1><<<grid, 256, strip_smem(rows), st>>>(lf, fa, s);
+      else if (rows <= 1024) mf_strip_kernel<512, 2><<<grid, 512, strip_smem(rows), st>>>(lf, fa, s);
+      else if (rows <= 2048) mf_strip_kernel<512, 4><<<grid, 512, strip_smem(rows), st>>>(lf, fa, s);
+      else mf_strip_kernel<256, 0><<<grid, 256, 0, st>>>(lf, fa, s);
       c.launches++;
     }
   }
-  if (out.perm.n != out.piv.n) out.perm.alloc_on(out.piv.n, st);
-  if (out.iperm.n != out.piv.n) out.iperm.alloc_on(out.piv.n, st);
-  mf_perm_kernel<<<(nf + 127) / 128, 128, 0, st>>>(nf, fd, out.piv.p, piv_off.p, out.perm.p, out.iperm.p);
-  c.launches++;
-  if (nsmall > 0) {
-    mf_invdiag_kernel<<<nsmall, 256, (size_t)max_small_p * max_small_p * sizeof(double), st>>>(lsmall.p, fd,
-                                                                                              Fbuf.p);
+  const int nbig = big_ptr[nlevels];
+  if (nbig > 0) {
+    mf_perm_kernel<<<(nbig + 31) / 32, 32, 0, st>>>(nbig, lbig.p, fd, out.piv.p, piv_off.p, out.perm.p, out.iperm.p);
     c.launches++;
   }
-  // the tiled levels' fronts: inverted diagonal squares, then L21' = -L21 L11^-1 and U12' = -U11^-1 U12
-  if (nmid > 0) {
-    mf_invdiag_kernel<<<nmid, 256, (size_t)max_mid_p * max_mid_p * sizeof(double), st>>>(lmid.p, fd, Fbuf.p);
-    c.launches++;
-  }
-  if (nwide > 0) {
-    mf_square_copy_kernel<<<dim3(64, nwide), 256, 0, st>>>(lwide.p, fd, Fbuf.p, sq.p);
-    mf_invdiag_wide_kernel<<<nwide_items, 32, (size_t)max_wide_p * 32 * sizeof(double), st>>>(
-        reinterpret_cast<const int2*>(wide_items.p), fd, sq.p, Fbuf.p);
+  // their inverted diagonal squares, then L21' = -L21 L11^-1 and U12' = -U11^-1 U12
+  if (ninv > 0) {
+    mf_inverse_kernel<<<ninv_items, 128, inverse_smem(max_inv_p), st>>>(reinterpret_cast<const int4*>(inv_items.p), fd,
+                                                                        Fbuf.p, sq.p);
+    mf_square_copy_kernel<<<dim3(8, ninv), 256, 0, st>>>(linv.p, fd, sq.p, Fbuf.p);
     c.launches += 2;
   }
   if (npinv > 0) {
-    mf_partinv_kernel<<<npinv, 256, (size_t)kTileRows * max_tiled_p * sizeof(double), st>>>(
-        reinterpret_cast<const int4*>(pinv_items.p), fd, Fbuf.p);
+    mf_partinv_kernel<<<npinv, 128, inverse_smem(max_inv_p), st>>>(reinterpret_cast<const int4*>(pinv_items.p), fd,
+                                                                   Fbuf.p);
     c.launches++;
   }
 

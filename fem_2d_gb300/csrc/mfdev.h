@@ -31,7 +31,7 @@ struct MFDevice {
   double factor_flops = 0;   // LU flops of all fronts, 2/3 (f^3 - (f - p)^3) each (half for Cholesky)
   std::vector<int32_t> level_ptr;
   std::vector<int64_t> level_off;
-  std::vector<int32_t> level_max_f, level_max_p;
+  std::vector<int64_t> level_big_end;   // end of the storage of a level's fronts factored in global memory
   std::vector<double> level_factor_bytes;   // L (forward) or U (backward) bytes read per level
   DBuf<uint8_t> desc;
   DBuf<int32_t> lfronts, dofs, ea_map;
@@ -44,7 +44,14 @@ struct MFDevice {
   std::vector<int32_t> small_ptr, large_ptr;   // nlevels + 1 offsets into lsmall / llarge
   std::vector<int32_t> level_fwd_cols, level_bwd_cols;   // shared doubles per right-hand side of their kernels
   DBuf<int32_t> lsmall, llarge;
-  int nsmall = 0, max_small_p = 0;
+  // factorization: per level the fronts factored in global memory (lbig), and the groups of fronts factored
+  // by one CTA each in shared memory (lfused)
+  struct FusedGroup {
+    int level, first, count, max_f;
+  };
+  std::vector<FusedGroup> fused_groups;
+  std::vector<int32_t> big_ptr, level_big_f, level_big_p;
+  DBuf<int32_t> lbig, lfused;
   // tiled levels (narrow upper levels solved through the fronts' partitioned inverses, rows spread over
   // many CTAs): per level a flag and offsets into the (front, first row) items of each direction
   std::vector<uint8_t> level_tiled;
@@ -52,11 +59,11 @@ struct MFDevice {
   DBuf<int32_t> tf_items, tb_items;
   DBuf<int32_t> pull;   // pull records of the tiled fronts' right-hand sides (8 per row)
   std::vector<int32_t> level_pmax, level_kmax;   // tiled levels: longest sums of the two directions
-  // factor-time work of the tiled fronts: diagonal inversion of those outside lsmall (p <= kSmallP:
-  // lmid; larger: lwide, 32-column items, scratch squares sq), then the partitioned-inverse items
-  DBuf<int32_t> lmid, lwide, wide_items, pinv_items;
+  // inverses of the fronts factored in global memory: the fronts, their (front, L or U, column strip) items and
+  // scratch squares, then the partitioned-inverse items of those on tiled levels
+  DBuf<int32_t> linv, inv_items, pinv_items;
   DBuf<double> sq;
-  int nmid = 0, max_mid_p = 0, nwide = 0, nwide_items = 0, max_wide_p = 0, npinv = 0, max_tiled_p = 0;
+  int ninv = 0, ninv_items = 0, max_inv_p = 0, npinv = 0;
 
   void setup(Ctx& c, const MFSymbolic& s, int nb_max);
   // factor c_a*A + c_b*B (values in full-CSR order); Cholesky mode skips pivoting (SPD shifts)

@@ -92,3 +92,27 @@ def test_shifted_solve_columns(kat, ctx, mesh, columns):
         knorm = np.max(np.asarray(abs(K).sum(axis=1)).ravel())
         bwd = np.max(np.abs(K @ X - R), axis=0) / (knorm * np.max(np.abs(X), axis=0) + np.max(np.abs(R), axis=0))
         assert np.max(bwd) < 1e-13, bwd
+
+
+@pytest.mark.parametrize("orders", [(1, 2), (3, 3), (5, 4), (8, 7), (9, 9), (12, 10)])
+@pytest.mark.parametrize("copies", [1, 90])
+def test_factor_front_sizes(ctx, orders, copies):
+    """Factorizations whose leaf fronts run from a few rows to more than a CTA's shared memory holds (two to
+    several hundred rows, pivot counts that are and are not multiples of 8, up to p > 160), on levels
+    narrower and wider than the chip: normwise backward errors at the FP64 level (450 units of rounding)."""
+    nx, ny = (3, 2) if copies == 1 else (16, 12)
+    if copies > 1 and orders[0] * orders[1] > 60:
+        nx, ny = 13, 12
+    pm = configs.build_mesh(configs.full_scale(seed=3, nx=nx, ny=ny, rounds=1, fraction=0.15, pmin=1, pmax=1))
+    leaves = [int(e) for e in np.nonzero(pm.elem_info()[:, 0] == 1)[0]]
+    pm.set_expansion_on_elems(leaves[::2], fg.Orders(*orders))
+    pm.set_expansion_on_elems(leaves[1::2], fg.Orders(orders[0], max(1, orders[1] - 1)))
+    gep = fg.galerkin_sample_gep_hcurl(fg.KOLeg, fg.CurlCurl, fg.L2Inner, fg.Domain.from_mesh(pm), [14, 14], ctx=ctx)
+    A, B = gep.scipy()
+    for ca, cb, spd in ((1.0, -10.0, False), (1.0, 10.0, True)):
+        K = (ca * A + cb * B).tocsr()
+        R = np.random.default_rng(7).standard_normal((gep.dimension, 3))
+        X = gep.shifted_solve(ca, cb, R, spd=spd)
+        knorm = np.max(np.asarray(abs(K).sum(axis=1)).ravel())
+        bwd = np.max(np.abs(K @ X - R), axis=0) / (knorm * np.max(np.abs(X), axis=0) + np.max(np.abs(R), axis=0))
+        assert np.max(bwd) < 1e-13, bwd
