@@ -62,30 +62,30 @@ std::vector<int32_t> row_runs(const HostGEP& g) {
 
 void device_upload(Ctx& c, const HostGEP& g, DeviceGEP& d) {
   cudaStream_t s = c.stream;
-  d.row_ptr.upload(g.row_ptr, s);
-  d.col.upload(g.col, s);
-  d.vptr.upload(g.vptr, s);
-  d.fsrc.upload(g.fsrc, s);
-  d.codes.upload(g.codes, s);
-  d.blocks.upload(g.blocks, s);
-  d.specs.upload(g.specs, s);
+  d.arena.add(d.row_ptr, g.row_ptr);
+  d.arena.add(d.col, g.col);
+  d.arena.add(d.vptr, g.vptr);
+  d.arena.add(d.fsrc, g.fsrc);
+  d.arena.add(d.codes, g.codes);
+  d.arena.add(d.blocks, g.blocks);
+  d.arena.add(d.specs, g.specs);
   std::vector<double> iv(2 * g.ivl_s.size());
   for (size_t k = 0; k < g.ivl_s.size(); k++) {
     iv[2 * k] = g.ivl_s[k];
     iv[2 * k + 1] = g.ivl_o[k];
   }
-  d.ivl.upload(iv, s);
+  d.arena.add(d.ivl, iv);
   d.nivl = (int)g.ivl_s.size();
   std::vector<double> q;
   q.insert(q.end(), g.glq_u_x.begin(), g.glq_u_x.end());
   q.insert(q.end(), g.glq_u_w.begin(), g.glq_u_w.end());
   q.insert(q.end(), g.glq_v_x.begin(), g.glq_v_x.end());
   q.insert(q.end(), g.glq_v_w.begin(), g.glq_v_w.end());
-  d.glq.upload(q, s);
+  d.arena.add(d.glq, q);
   const int P = g.pmax + 1;
-  d.tables.alloc((size_t)2 * d.nivl * 5 * P * P);
-  d.a.alloc(g.nnz_full);
-  d.b.alloc(g.nnz_full);
+  d.arena.reserve(d.tables, (size_t)2 * d.nivl * 5 * P * P);
+  d.arena.reserve(d.a, g.nnz_full);
+  d.arena.reserve(d.b, g.nnz_full);
   // rows of one Elem's interior functions share their column list; the operator products stage each
   // run's gathered X rows once (eigen.cu spmm_group_kernel, ozaki.cu spmm_tc_kernel)
   std::vector<int32_t> grp = row_runs(g);
@@ -94,9 +94,10 @@ void device_upload(Ctx& c, const HostGEP& g, DeviceGEP& d) {
     const int64_t len = g.row_ptr[grp[q] + 1] - g.row_ptr[grp[q]];
     for (int64_t c0 = 0; c0 < std::max<int64_t>(len, 1); c0 += 256) work.push_back(make_int2((int)q, (int)c0));
   }
-  d.grp.upload(grp, s);
+  d.arena.add(d.grp, grp);
   d.grp_h = grp;
-  d.gwork.upload(work, s);
+  d.arena.add(d.gwork, work);
+  d.arena.commit(s);
   d.ngrp = (int)grp.size() - 1;
   d.nwork = (int)work.size();
   d.h2d_bytes = (int64_t)(grp.size() * 4 + work.size() * 8 + g.row_ptr.size() * 8 + g.col.size() * 4 + g.vptr.size() * 8 + g.fsrc.size() * 4 + g.codes.size() * 8 +

@@ -2,8 +2,11 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <chrono>
 #include <cstdint>
+#include <cstring>
+#include <functional>
 #include <map>
 #include <string>
 #include <vector>
@@ -95,18 +98,20 @@ struct DBuf {
   T* p = nullptr;
   size_t n = 0;
   cudaStream_t st = nullptr;   // set when the buffer came from the stream-ordered allocator
+  bool owned = true;           // false: a piece of a DArena, which frees it
   DBuf() = default;
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
   ~DBuf() { release(); }
   void release() {
-    if (p) {
+    if (p && owned) {
       if (st) cudaFreeAsync(p, st);
       else cudaFree(p);
     }
     p = nullptr;
     n = 0;
     st = nullptr;
+    owned = true;
   }
   void alloc(size_t count) {
     release();
@@ -133,7 +138,62 @@ struct DBuf {
   }
 };
 
+// Buffers that are made together and live as long as one object, in one allocation: each cudaMalloc and
+// cudaFree costs some 10 us and more, and a cudaFree waits for the whole device, so the twenty buffers of a
+// plan held up the solves of every other stream. Collect with add (uploaded) and reserve (left as it is),
+// then commit once; the vectors must live until then. Small sets go up as one copy.
+struct DArena {
+  DBuf<uint8_t> mem;
+  struct Piece {
+    size_t off, bytes;
+    const void* src;
+  };
+  std::vector<Piece> pieces;
+  std::vector<std::function<void(uint8_t*)>> views;
+  size_t total = 0;
+  static constexpr size_t kAlign = 256, kOneCopy = 1 << 20;
+
+  template <class T, class Alloc>
+  void add(DBuf<T>& b, const std::vector<T, Alloc>& v) {
+    place(b, v.size(), v.data());
+  }
+  template <class T>
+  void reserve(DBuf<T>& b, size_t count) {
+    place(b, count, nullptr);
+  }
+  void commit(cudaStream_t s) {
+    mem.alloc(std::max<size_t>(total, 1));
+    for (auto& v : views) v(mem.p);
+    if (total <= kOneCopy) {
+      std::vector<uint8_t> all(total);
+      for (const Piece& q : pieces)
+        if (q.src && q.bytes) std::memcpy(all.data() + q.off, q.src, q.bytes);
+      if (total) FEM2D_CUDA(cudaMemcpyAsync(mem.p, all.data(), total, cudaMemcpyHostToDevice, s));
+    } else {
+      for (const Piece& q : pieces)
+        if (q.src && q.bytes) FEM2D_CUDA(cudaMemcpyAsync(mem.p + q.off, q.src, q.bytes, cudaMemcpyHostToDevice, s));
+    }
+    pieces.clear();
+    views.clear();
+  }
+
+ private:
+  template <class T>
+  void place(DBuf<T>& b, size_t count, const void* src) {
+    b.release();
+    const size_t off = total, bytes = count * sizeof(T);
+    pieces.push_back({off, bytes, src});
+    views.push_back([&b, off, count](uint8_t* base) {
+      b.p = count ? reinterpret_cast<T*>(base + off) : nullptr;
+      b.n = count;
+      b.owned = false;
+    });
+    total += (bytes + kAlign - 1) / kAlign * kAlign;
+  }
+};
+
 struct DeviceGEP {
+  DArena arena;   // holds all of the buffers below
   DBuf<int64_t> row_ptr, vptr;
   DBuf<int32_t> col, fsrc;
   DBuf<uint64_t> codes;

@@ -34,6 +34,7 @@
 #include <memory>
 
 #include "eigen.h"
+#include "host_pool.h"
 #include "ozaki.h"
 #include "precond.h"
 #include "mf.h"
@@ -443,6 +444,23 @@ __global__ void densify_kernel(int64_t n, const int64_t* __restrict__ rp, const 
 }
 
 // ---------------------------------------------------------------- host helpers
+// C (m x n, row-major, zeroed) += A B with A(i, k) at a[i * ai + k * ak] and B k x n row-major: rows of C in
+// parallel, each summed over k in order along rows of B
+void host_gemm(int m, int n, int k, const double* a, int64_t ai, int64_t ak, const double* b, double* c) {
+  parallel_for(
+      m,
+      [=](int64_t i0, int64_t i1) {
+        for (int64_t i = i0; i < i1; i++)
+          for (int q = 0; q < k; q++) {
+            const double x = a[i * ai + q * ak];
+            const double* bq = b + (size_t)q * n;
+            double* ci = c + (size_t)i * n;
+            for (int j = 0; j < n; j++) ci[j] += x * bq[j];
+          }
+      },
+      64);
+}
+
 void setup_gemm_smem(int device);
 
 struct Dev {
@@ -861,7 +879,7 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
   V.alloc_on((size_t)n * mmax, c.stream);
   AV.alloc_on((size_t)n * mmax, c.stream);
   BV.alloc_on((size_t)n * mmax, c.stream);
-  for (DBuf<double>* buf : {&X, &AX, &BX, &G0, &W1, &W2, &W3}) buf->alloc((size_t)n * 32);
+  for (DBuf<double>* buf : {&X, &AX, &BX, &G0, &W1, &W2, &W3}) buf->alloc_on((size_t)n * 32, c.stream);
   int64_t spmv = 0, napply = 0;
 
   // x = K^-1 rhs for K = ka A + kb B (factored as fac) followed by nref steps of iterative refinement
@@ -1201,27 +1219,12 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
     for (int i = 0; i < ma; i++)
       for (int q = 0; q < m2; q++) Wh[(size_t)i * m2 + q] = zb[(size_t)i * ma + kb[q]] / std::sqrt(wb[kb[q]]);
     std::vector<double> S((size_t)m2 * m2, 0.0), tmp((size_t)ma * m2, 0.0);
-    for (int i = 0; i < ma; i++)
-      for (int q = 0; q < m2; q++) {
-        double acc = 0.0;
-        for (int k2 = 0; k2 < ma; k2++) acc += GA[(size_t)i * ma + k2] * Wh[(size_t)k2 * m2 + q];
-        tmp[(size_t)i * m2 + q] = acc;
-      }
-    for (int p2 = 0; p2 < m2; p2++)
-      for (int q = 0; q < m2; q++) {
-        double acc = 0.0;
-        for (int i = 0; i < ma; i++) acc += Wh[(size_t)i * m2 + p2] * tmp[(size_t)i * m2 + q];
-        S[(size_t)p2 * m2 + q] = acc;
-      }
+    host_gemm(ma, m2, ma, GA.data(), ma, 1, Wh.data(), tmp.data());
+    host_gemm(m2, m2, ma, Wh.data(), 1, m2, tmp.data(), S.data());   // Wh^T (GA Wh)
     std::vector<double> th, Z;
     if (!symeig(m2, S, th, Z)) fail(FEM2D_E_NOT_CONVERGED, "Rayleigh-Ritz eigen-decomposition failed");
     std::vector<double> Y((size_t)ma * m2, 0.0);
-    for (int i = 0; i < ma; i++)
-      for (int q = 0; q < m2; q++) {
-        double acc = 0.0;
-        for (int k2 = 0; k2 < m2; k2++) acc += Wh[(size_t)i * m2 + k2] * Z[(size_t)k2 * m2 + q];
-        Y[(size_t)i * m2 + q] = acc;
-      }
+    host_gemm(ma, m2, m2, Wh.data(), m2, 1, Z.data(), Y.data());
     // Ritz residuals AV*y - BV*y*theta of the non-spurious pairs nearest sigma only (twice the block):
     // the selection never reaches further, and the products scale with the number of columns
     std::vector<int> order;

@@ -13,47 +13,13 @@
 #include <cstring>
 #include <map>
 #include <memory>
-#include <thread>
 
 #include "common.h"
 #include "domain.h"
 #include "gep.h"
+#include "host_pool.h"
 
 namespace fem2d {
-
-int num_host_threads() {
-  unsigned h = std::thread::hardware_concurrency();
-  return h == 0 ? 4 : (int)std::min(h, 64u);
-}
-
-template <class F>
-static void parallel_for(int64_t n, F f) {
-  int nt = num_host_threads();
-  if (n < 4096 || nt <= 1) {
-    f(0, n);
-    return;
-  }
-  std::vector<std::thread> th;
-  int64_t chunk = (n + nt - 1) / nt;
-  for (int t = 0; t < nt; t++) {
-    int64_t a = t * chunk, b = std::min(n, a + chunk);
-    if (a >= b) break;
-    th.emplace_back([=]() { f(a, b); });
-  }
-  for (auto& x : th) x.join();
-}
-
-// f(t) on nt threads (t = 0..nt-1), inline when nt == 1
-template <class F>
-static void run_threads(int nt, F f) {
-  if (nt <= 1) {
-    f(0);
-    return;
-  }
-  std::vector<std::thread> th;
-  for (int t = 0; t < nt; t++) th.emplace_back([=]() { f(t); });
-  for (auto& x : th) x.join();
-}
 
 // out[0] = 0, out[r + 1] = out[r] + term(r) for r < n: the terms in parallel, then a two-pass prefix
 // sum over contiguous chunks (the same integers as the serial loop)

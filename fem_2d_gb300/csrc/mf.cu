@@ -1653,35 +1653,35 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
     }
   }
   big_ptr[nlevels] = (int32_t)big_h.size();
-  lbig.upload(big_h, st);
-  lfused.upload(fused_h, st);
+  arena.add(lbig, big_h);
+  arena.add(lfused, fused_h);
   tf_ptr[nlevels] = (int32_t)(tf_h.size() / 2);
   tb_ptr[nlevels] = (int32_t)(tb_h.size() / 2);
   ninv = (int)inv_h.size();
   ninv_items = (int)(ii_h.size() / 4);
   npinv = (int)(pi_h.size() / 4);
-  tf_items.upload(tf_h, st);
-  tb_items.upload(tb_h, st);
-  pull.upload(pull_h, st);
-  linv.upload(inv_h, st);
-  inv_items.upload(ii_h, st);
-  pinv_items.upload(pi_h, st);
-  sq.alloc(std::max<int64_t>(sq_total, 1));
+  arena.add(tf_items, tf_h);
+  arena.add(tb_items, tb_h);
+  arena.add(pull, pull_h);
+  arena.add(linv, inv_h);
+  arena.add(inv_items, ii_h);
+  arena.add(pinv_items, pi_h);
+  arena.reserve(sq, std::max<int64_t>(sq_total, 1));
   std::vector<uint8_t> raw(fdh.size() * sizeof(FrontDesc));
   std::memcpy(raw.data(), fdh.data(), raw.size());
-  desc.upload(raw, st);
-  lfronts.upload(s.level_fronts, st);
-  dofs.upload(s.dofs, st);
-  asm_pos.upload(s.asm_pos, st);
-  asm_csr.upload(s.asm_csr, st);
-  ea_map.upload(s.ea_map, st);
-  piv_off.upload(poff, st);
-  woff.upload(woff_h, st);
+  arena.add(desc, raw);
+  arena.add(lfronts, s.level_fronts);
+  arena.add(dofs, s.dofs);
+  arena.add(asm_pos, s.asm_pos);
+  arena.add(asm_csr, s.asm_csr);
+  arena.add(ea_map, s.ea_map);
+  arena.add(piv_off, poff);
+  arena.add(woff, woff_h);
   piv_total = po;
-  work.alloc(std::max<int64_t>(wo, 1));
-  flags.alloc(1);
-  weak_list.alloc(std::max<int64_t>(s.n, 1));
-  weak_count.alloc(1);
+  arena.reserve(work, std::max<int64_t>(wo, 1));
+  arena.reserve(flags, 1);
+  arena.reserve(weak_list, std::max<int64_t>(s.n, 1));
+  arena.reserve(weak_count, 1);
   level_factor_bytes.assign(nlevels, 0.0);
   for (int l = 0; l < nlevels; l++)
     for (int k = s.level_ptr[l]; k < s.level_ptr[l + 1]; k++) {
@@ -1709,8 +1709,9 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   }
   small_ptr[nlevels] = (int32_t)ls.size();
   large_ptr[nlevels] = (int32_t)ll.size();
-  lsmall.upload(ls, st);
-  llarge.upload(ll, st);
+  arena.add(lsmall, ls);
+  arena.add(llarge, ll);
+  arena.commit(st);
   // dynamic shared memory limits are set once per device (a function attribute of the device's context)
   static std::mutex attr_mu;
   static bool attr_done[256] = {};

@@ -12,16 +12,14 @@
 #include <functional>
 
 #include <atomic>
-#include <thread>
 
 #include "common.h"
 #include "domain.h"
 #include "gep.h"
+#include "host_pool.h"
 #include "mf.h"
 
 namespace fem2d {
-
-int num_host_threads();
 
 namespace {
 // f(t, i0, i1) on up to nt threads over [0, n) in contiguous chunks (inline for small n)
@@ -32,14 +30,8 @@ void chunked(int64_t n, F f) {
     f(0, (int64_t)0, n);
     return;
   }
-  std::vector<std::thread> th;
   const int64_t chunk = (n + nt - 1) / nt;
-  for (int t = 0; t < nt; t++) {
-    const int64_t a = t * chunk, b = std::min(n, a + chunk);
-    if (a >= b) break;
-    th.emplace_back([=]() { f(t, a, b); });
-  }
-  for (auto& x : th) x.join();
+  run_threads((int)((n + chunk - 1) / chunk), [&](int t) { f(t, t * chunk, std::min(n, (t + 1) * chunk)); });
 }
 }  // namespace
 

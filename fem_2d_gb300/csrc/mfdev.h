@@ -33,6 +33,7 @@ struct MFDevice {
   std::vector<int64_t> level_off;
   std::vector<int64_t> level_big_end;   // end of the storage of a level's fronts factored in global memory
   std::vector<double> level_factor_bytes;   // L (forward) or U (backward) bytes read per level
+  DArena arena;   // holds all of the buffers below
   DBuf<uint8_t> desc;
   DBuf<int32_t> lfronts, dofs, ea_map;
   DBuf<int64_t> asm_pos, asm_csr, piv_off, woff;

@@ -33,20 +33,27 @@ bool symeig(int n, const std::vector<double>& a, std::vector<double>& w, std::ve
         e[i] = scale * g;
         h -= f * g;
         at(i, l) = f - g;
+        // e = V at(i, .) / h over the leading l + 1 rows: both triangles are kept, so row k serves every
+        // sum, and all loops run along rows
+        double* vi = &V[(size_t)i * n];
+        for (int j = 0; j <= l; j++) e[j] = 0.0;
+        for (int k = 0; k <= l; k++) {
+          const double* vk = &V[(size_t)k * n];
+          const double x = vi[k];
+          for (int j = 0; j <= l; j++) e[j] += vk[j] * x;
+        }
         f = 0.0;
         for (int j = 0; j <= l; j++) {
-          at(j, i) = at(i, j) / h;
-          g = 0.0;
-          for (int k = 0; k <= j; k++) g += at(j, k) * at(i, k);
-          for (int k = j + 1; k <= l; k++) g += at(k, j) * at(i, k);
-          e[j] = g / h;
-          f += e[j] * at(i, j);
+          at(j, i) = vi[j] / h;
+          e[j] /= h;
+          f += e[j] * vi[j];
         }
         double hh = f / (h + h);
+        for (int j = 0; j <= l; j++) e[j] -= hh * vi[j];
         for (int j = 0; j <= l; j++) {
-          f = at(i, j);
-          e[j] = g = e[j] - hh * f;
-          for (int k = 0; k <= j; k++) at(j, k) -= (f * e[k] + g * at(i, k));
+          double* vj = &V[(size_t)j * n];
+          const double fj = vi[j], gj = e[j];
+          for (int k = 0; k <= l; k++) vj[k] -= fj * e[k] + gj * vi[k];
         }
       }
     } else {
@@ -57,20 +64,29 @@ bool symeig(int n, const std::vector<double>& a, std::vector<double>& w, std::ve
   d[0] = 0.0;
   e[0] = 0.0;
   // accumulate the transforms
+  std::vector<double> g;
   for (int i = 0; i < n; i++) {
     int l = i - 1;
     if (d[i] != 0.0) {
-      for (int j = 0; j <= l; j++) {
-        double g = 0.0;
-        for (int k = 0; k <= l; k++) g += at(i, k) * at(k, j);
-        for (int k = 0; k <= l; k++) at(k, j) -= g * at(k, i);
+      g.assign(l + 1, 0.0);
+      for (int k = 0; k <= l; k++) {
+        const double* vk = &V[(size_t)k * n];
+        const double x = at(i, k);
+        for (int j = 0; j <= l; j++) g[j] += x * vk[j];
+      }
+      for (int k = 0; k <= l; k++) {
+        double* vk = &V[(size_t)k * n];
+        const double x = at(k, i);
+        for (int j = 0; j <= l; j++) vk[j] -= g[j] * x;
       }
     }
     d[i] = at(i, i);
     at(i, i) = 1.0;
     for (int j = 0; j <= l; j++) at(j, i) = at(i, j) = 0.0;
   }
-  // implicit QL with shifts on (d, e)
+  // implicit QL with shifts on (d, e); the rotations mix two vectors, kept as rows (transposed) here
+  for (int i = 0; i < n; i++)
+    for (int j = 0; j < i; j++) std::swap(at(i, j), at(j, i));
   for (int i = 1; i < n; i++) e[i - 1] = e[i];
   e[n - 1] = 0.0;
   for (int l = 0; l < n; l++) {
@@ -103,10 +119,11 @@ bool symeig(int n, const std::vector<double>& a, std::vector<double>& w, std::ve
           p = s * r;
           d[i + 1] = g + p;
           g = c * r - b;
+          double *v0 = &V[(size_t)i * n], *v1 = v0 + n;
           for (int k = 0; k < n; k++) {
-            f = at(k, i + 1);
-            at(k, i + 1) = s * at(k, i) + c * f;
-            at(k, i) = c * at(k, i) - s * f;
+            const double x = v1[k], y = v0[k];
+            v1[k] = s * y + c * x;
+            v0[k] = c * y - s * x;
           }
         }
         if (r == 0.0 && i >= l) continue;
@@ -121,7 +138,7 @@ bool symeig(int n, const std::vector<double>& a, std::vector<double>& w, std::ve
   std::sort(idx.begin(), idx.end(), [&](int x, int y) { return d[x] < d[y]; });
   for (int k = 0; k < n; k++) {
     w[k] = d[idx[k]];
-    for (int i = 0; i < n; i++) z[(size_t)i * n + k] = at(i, idx[k]);
+    for (int i = 0; i < n; i++) z[(size_t)i * n + k] = at(idx[k], i);
   }
   return true;
 }
