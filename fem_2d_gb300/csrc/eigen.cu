@@ -33,6 +33,7 @@
 #include "blockscale.h"
 #include <memory>
 
+#include "dmma.h"
 #include "eigen.h"
 #include "host_pool.h"
 #include "ozaki.h"
@@ -178,50 +179,87 @@ __global__ void __launch_bounds__(256) spmm_group_kernel(int nwork, const int2* 
   }
 }
 
-__global__ void __launch_bounds__(256) gram_partial_kernel(int64_t n, const double* __restrict__ X, int64_t ldx, int a,
-                                                           const double* __restrict__ Y, int64_t ldy, int b,
-                                                           int64_t rows_per_block, int e0, double* __restrict__ P) {
-  extern __shared__ double sm[];
-  double* xs = sm;               // 32 x a
-  double* ys = sm + 32 * a;      // 32 x b
-  const int64_t r0 = blockIdx.x * rows_per_block;
-  const int64_t r1 = min(n, r0 + rows_per_block);
-  const int ab = a * b;
-  double acc[8];
-  for (int q = 0; q < 8; q++) acc[q] = 0.0;
-  for (int64_t rt = r0; rt < r1; rt += 32) {
-    const int nr = (int)min((int64_t)32, r1 - rt);
-    __syncthreads();
-    for (int t = threadIdx.x; t < 32 * a; t += blockDim.x) {
-      const int r = t / a, i = t % a;
-      xs[t] = r < nr ? X[(rt + r) * ldx + i] : 0.0;
-    }
-    for (int t = threadIdx.x; t < 32 * b; t += blockDim.x) {
-      const int r = t / b, j = t % b;
-      ys[t] = r < nr ? Y[(rt + r) * ldy + j] : 0.0;
-    }
-    __syncthreads();
-    for (int q = 0; q < 8; q++) {
-      const int e = e0 + threadIdx.x + q * blockDim.x;
-      if (e >= ab) break;
-      const int i = e / b, j = e % b;
-      double s = acc[q];
-      for (int r = 0; r < nr; r++) s += xs[r * a + i] * ys[r * b + j];
-      acc[q] = s;
+// Gram products in FP64 MMAs (mma.sync m8n8k4): the same rate as FP64 FMAs, but operands come straight from
+// global memory into the fragments and one instruction does 256 FMAs, so the kernel runs at the FP64 pipe's
+// rate (1.05 TFLOP/s) or, at a few thousand rows, at load latency. One FMA per two shared-memory reads took
+// 170 us for 5,403 x 72 x 24 (now 32) and 369 us for 28,686 x 120 x 24 (now 167). The block update below gains
+// nothing from it: its reads are broadcasts, and one output per thread spreads short blocks further.
+
+// partial C = X^T Y: CTA (x, y, z): a slice of the rows, 8 NTL columns of Y, up to 128 columns of X. Its
+// eight warps own 32 columns of X each; with fewer than 128 columns, the warps left split the rows again.
+constexpr int kGramMT = 4;   // 8-column tiles of X per warp
+template <int NTL>
+__global__ void __launch_bounds__(256) dgram_kernel(int64_t n, const double* __restrict__ X, int64_t ldx, int a,
+                                                    const double* __restrict__ Y, int64_t ldy, int b, int64_t rows,
+                                                    double* __restrict__ P) {
+  extern __shared__ double sm[];   // one 32 x 8 NTL tile per warp
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, kl = lane & 3;
+  const int a0 = blockIdx.z * 128, b0 = blockIdx.y * 8 * NTL;
+  const int groups = min(4, (a - a0 + 31) / 32), slices = 8 / groups;
+  const int grp = warp % groups, slice = warp / groups;
+  const int64_t r0 = blockIdx.x * rows, r1 = min(n, r0 + rows);
+  double acc[kGramMT][NTL][2];
+#pragma unroll
+  for (int m = 0; m < kGramMT; m++)
+#pragma unroll
+    for (int q = 0; q < NTL; q++) acc[m][q][0] = acc[m][q][1] = 0.0;
+  if (slice < slices) {
+    const int am = a0 + 32 * grp + g, bn = b0 + g;
+    const double* xp = X + am;
+    const double* yp = Y + bn;
+#pragma unroll 2
+    for (int64_t r = r0 + 4 * slice; r < r1; r += 4 * slices) {
+      const int64_t row = r + kl;
+      const bool ok = row < r1;
+      double xf[kGramMT], yf[NTL];
+#pragma unroll
+      for (int m = 0; m < kGramMT; m++) xf[m] = (ok && am + 8 * m < a) ? __ldg(xp + row * ldx + 8 * m) : 0.0;
+#pragma unroll
+      for (int q = 0; q < NTL; q++) yf[q] = (ok && bn + 8 * q < b) ? __ldg(yp + row * ldy + 8 * q) : 0.0;
+#pragma unroll
+      for (int m = 0; m < kGramMT; m++)
+        if (a0 + 32 * grp + 8 * m < a)   // uniform across the warp
+#pragma unroll
+          for (int q = 0; q < NTL; q++) dmma(acc[m][q], xf[m], yf[q]);
     }
   }
-  for (int q = 0; q < 8; q++) {
-    const int e = e0 + threadIdx.x + q * blockDim.x;
-    if (e < ab) P[(int64_t)blockIdx.x * ab + e] = acc[q];
+  constexpr int W = 8 * NTL;
+  double* mine = sm + warp * 32 * W;
+#pragma unroll
+  for (int m = 0; m < kGramMT; m++)
+#pragma unroll
+    for (int q = 0; q < NTL; q++) {
+      mine[(8 * m + g) * W + 8 * q + 2 * kl] = acc[m][q][0];
+      mine[(8 * m + g) * W + 8 * q + 2 * kl + 1] = acc[m][q][1];
+    }
+  __syncthreads();
+  double* out = P + (int64_t)blockIdx.x * a * b;
+  for (int t = threadIdx.x; t < groups * 32 * W; t += 256) {
+    const int i = t / W, j = t - i * W;
+    if (a0 + i >= a || b0 + j >= b) continue;
+    double s = 0.0;
+    for (int q = 0; q < slices; q++) s += sm[((q * groups + (i >> 5)) * 32 + (i & 31)) * W + j];
+    out[(int64_t)(a0 + i) * b + b0 + j] = s;
   }
 }
 
-__global__ void reduce_partials_kernel(const double* __restrict__ P, int nblk, int ab, double* __restrict__ C) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ab) return;
+// C[e] = sum of the nblk partials, in a fixed order: 32 entries per CTA, eight threads each
+__global__ void __launch_bounds__(256) reduce_partials_kernel(const double* __restrict__ P, int nblk, int ab,
+                                                              double* __restrict__ C) {
+  __shared__ double part[8][32];
+  const int e = blockIdx.x * 32 + (threadIdx.x & 31), w = threadIdx.x >> 5;
   double s = 0.0;
-  for (int k = 0; k < nblk; k++) s += P[(int64_t)k * ab + e];
-  C[e] = s;
+  if (e < ab) {
+#pragma unroll 4
+    for (int k = w; k < nblk; k += 8) s += P[(int64_t)k * ab + e];
+  }
+  part[w][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (w == 0 && e < ab) {
+#pragma unroll
+    for (int q = 1; q < 8; q++) s += part[q][threadIdx.x];
+    C[e] = s;
+  }
 }
 
 // Z = beta*Z + X * C; X n x a (ldx), C a x b row-major (device), Z n x b (ldz)
@@ -549,6 +587,27 @@ struct Dev {
       c.launches++;
     }
   }
+  // C (device, a x b) = X^T Y on the FP64 pipe
+  void fp64_gram(const double* X, int64_t ldx, int a, const double* Y, int64_t ldy, int b, double* Cd) {
+    ProfScope ps(c, "dense_block", 8.0 * h.n * (a + b), 2.0 * h.n * a * b);
+    const int ab = a * b, ntl = std::min(4, (b + 7) / 8);
+    const int ny = (b + 8 * ntl - 1) / (8 * ntl), nz = (a + 127) / 128;
+    // rows per CTA: all SMs busy, but at least one MMA step of four rows for each of its row slices
+    const int groups = std::min(4, (a + 31) / 32), step = 4 * (8 / groups);
+    const int64_t want = std::max<int64_t>(1, 2 * c.num_sms / (ny * nz));
+    const int64_t rows = std::max<int64_t>(step, ((h.n + want - 1) / want + step - 1) / step * step);
+    const int nblk = (int)std::max<int64_t>(1, (h.n + rows - 1) / rows);
+    if (part.n < (size_t)nblk * ab) part.alloc_on((size_t)nblk * ab, c.stream);
+    const dim3 grid(nblk, ny, nz);
+    const size_t smem = sizeof(double) * 8 * 32 * 8 * ntl;
+    auto launch = [&](auto k) { k<<<grid, 256, smem, c.stream>>>(h.n, X, ldx, a, Y, ldy, b, rows, part.p); };
+    if (ntl == 1) launch(dgram_kernel<1>);
+    else if (ntl == 2) launch(dgram_kernel<2>);
+    else if (ntl == 3) launch(dgram_kernel<3>);
+    else launch(dgram_kernel<4>);
+    reduce_partials_kernel<<<(ab + 31) / 32, 256, 0, c.stream>>>(part.p, nblk, ab, Cd);
+    c.launches += 2;
+  }
   // C (a x b, host row-major) = X^T Y
   void gram(const double* X, int64_t ldx, int a, const double* Y, int64_t ldy, int b, std::vector<double>& C) {
     const int ab = a * b;
@@ -559,19 +618,7 @@ struct Dev {
       check_tensor();
       return;
     }
-    ProfScope ps(c, "dense_block", 8.0 * h.n * (a + b), 2.0 * h.n * a * b);
-    const int nblk = std::min<int64_t>(grid_rows(), std::max<int64_t>(1, (h.n + 255) / 256));
-    const int64_t rpb = (h.n + nblk - 1) / nblk;
-
-    if (part.n < (size_t)nblk * ab) part.alloc_on((size_t)nblk * ab, c.stream);
-    if (small.n < (size_t)ab) small.alloc_on(std::max<size_t>(ab, 16384), c.stream);
-    const size_t smem = (size_t)32 * (a + b) * sizeof(double);
-    for (int e0 = 0; e0 < ab; e0 += 8 * 256) {
-      gram_partial_kernel<<<nblk, 256, smem, c.stream>>>(h.n, X, ldx, a, Y, ldy, b, rpb, e0, part.p);
-      c.launches++;
-    }
-    reduce_partials_kernel<<<(ab + 255) / 256, 256, 0, c.stream>>>(part.p, nblk, ab, small.p);
-    c.launches++;
+    fp64_gram(X, ldx, a, Y, ldy, b, small.p);
     C.resize(ab);
     FEM2D_CUDA(cudaMemcpyAsync(C.data(), small.p, ab * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     FEM2D_CUDA(cudaStreamSynchronize(c.stream));
@@ -620,19 +667,7 @@ struct Dev {
   }
   // C (a x b, device, row-major) = X^T Y without leaving the device
   void gram_dev(const double* X, int64_t ldx, int a, const double* Y, int64_t ldy, int b, double* Cd) {
-    if (tensor_gram(X, ldx, a, Y, ldy, b, Cd)) return;
-    ProfScope ps(c, "dense_block", 8.0 * h.n * (a + b), 2.0 * h.n * a * b);
-    const int nblk = std::min<int64_t>(grid_rows(), std::max<int64_t>(1, (h.n + 255) / 256));
-    const int64_t rpb = (h.n + nblk - 1) / nblk;
-    const int ab = a * b;
-    if (part.n < (size_t)nblk * ab) part.alloc_on((size_t)nblk * ab, c.stream);
-    const size_t smem = (size_t)32 * (a + b) * sizeof(double);
-    for (int e0 = 0; e0 < ab; e0 += 8 * 256) {
-      gram_partial_kernel<<<nblk, 256, smem, c.stream>>>(h.n, X, ldx, a, Y, ldy, b, rpb, e0, part.p);
-      c.launches++;
-    }
-    reduce_partials_kernel<<<(ab + 255) / 256, 256, 0, c.stream>>>(part.p, nblk, ab, Cd);
-    c.launches++;
+    if (!tensor_gram(X, ldx, a, Y, ldy, b, Cd)) fp64_gram(X, ldx, a, Y, ldy, b, Cd);
   }
   // Z = beta Z + alpha X C with C (a x b) already on the device (a * b * 8 bytes fit the kernel's smem)
   void gemm_dev(const double* X, int64_t ldx, int a, const double* Cd, int b, double alpha, double beta, double* Z,
@@ -661,8 +696,12 @@ void setup_gemm_smem(int device) {
   static bool done[256] = {};
   std::lock_guard<std::mutex> lk(mu);
   if (device < 0 || device >= 256 || done[device]) return;
-  FEM2D_CUDA(cudaFuncSetAttribute(gemm_nn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-  FEM2D_CUDA(cudaFuncSetAttribute(gram_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+  auto allow = [](auto k, size_t bytes) {
+    FEM2D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  };
+  allow(dgram_kernel<3>, 8 * 32 * 24 * sizeof(double));
+  allow(dgram_kernel<4>, 8 * 32 * 32 * sizeof(double));
+  allow(gemm_nn_kernel, 96 * 1024);
   done[device] = true;
 }
 

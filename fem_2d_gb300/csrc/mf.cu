@@ -17,6 +17,7 @@
 
 namespace cg = cooperative_groups;
 
+#include "dmma.h"
 #include "mfdev.h"
 
 namespace fem2d {
@@ -88,14 +89,6 @@ __global__ void __launch_bounds__(256) mf_extend_add_kernel(const int32_t* __res
       for (int i = lane; i < s; i += 32) dst[m[i]] += src[i];
     }
   }
-}
-
-// c += a b on an 8 x 8 tile, inner dimension 4: lane l holds a[l / 4][l % 4], b[l % 4][l / 4] and
-// c[l / 4][2 (l % 4) + {0, 1}]
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(c[0]), "+d"(c[1])
-      : "d"(a), "d"(b));
 }
 
 // ------------------------------------------------------------------ fronts in shared memory

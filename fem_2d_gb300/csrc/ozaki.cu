@@ -193,24 +193,37 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 // byte offset of core matrix (row group rg, k group kg) in a K-major tile with kSub columns
 __device__ __forceinline__ int core_off(int rg, int kg) { return (rg * (kSub / 8) + kg) * 128; }
 
-// E[c * a + j] = biased exponent of max |X[r][j]| over the 128-row chunk c (one pass, coalesced)
-__global__ void __launch_bounds__(128) chunk_exp_kernel(int64_t n, const double* __restrict__ X, int64_t ldx, int a,
-                                                         int* __restrict__ E) {
-  const int64_t c0 = (int64_t)blockIdx.x * kChunk;
-  const int col = blockIdx.y * 128 + threadIdx.x;
-  if (col >= a) return;
-  const int rows = (int)min((int64_t)kChunk, n - c0);
-  const double* xp = X + c0 * ldx + col;
-  int e = 0, r = 0;
-  for (; r + 16 <= rows; r += 16) {
+// E[c * a + j] = biased exponent of max |X[r][j]| over the 128-row chunk c, for X and, past its column groups
+// (blockIdx.y), for Y: 32 columns x 8 row groups of 16 per CTA, all 16 loads of a thread in flight (one thread
+// per column took 12 us at any size, twice per product)
+__global__ void __launch_bounds__(256) chunk_exp_kernel(int64_t n, const double* __restrict__ X, int64_t ldx, int a,
+                                                         int* __restrict__ EX, const double* __restrict__ Y,
+                                                         int64_t ldy, int b, int* __restrict__ EY) {
+  __shared__ int part[8][32];
+  const int ga = (a + 31) / 32;
+  const bool first = (int)blockIdx.y < ga;
+  const double* V = first ? X : Y;
+  const int64_t ld = first ? ldx : ldy;
+  const int w = first ? a : b, lane = threadIdx.x & 31, part_id = threadIdx.x >> 5;
+  const int col = (first ? blockIdx.y : blockIdx.y - ga) * 32 + lane;
+  const int64_t c0 = (int64_t)blockIdx.x * kChunk + 16 * part_id;
+  const int rows = (int)max((int64_t)0, min((int64_t)16, n - c0));
+  const double* p = V + c0 * ld + col;
+  int e = 0;
+  if (col < w) {
     double v[16];
 #pragma unroll
-    for (int q = 0; q < 16; q++) v[q] = __ldg(xp + (int64_t)(r + q) * ldx);
+    for (int q = 0; q < 16; q++) v[q] = q < rows ? __ldg(p + q * ld) : 0.0;
 #pragma unroll
     for (int q = 0; q < 16; q++) e = max(e, biased_exp(v[q]));
   }
-  for (; r < rows; r++) e = max(e, biased_exp(__ldg(xp + (int64_t)r * ldx)));
-  E[(int64_t)blockIdx.x * a + col] = e;
+  part[part_id][lane] = e;
+  __syncthreads();
+  if (part_id == 0 && col < w) {
+#pragma unroll
+    for (int q = 1; q < 8; q++) e = max(e, part[q][lane]);
+    (first ? EX : EY)[(int64_t)blockIdx.x * w + col] = e;
+  }
 }
 
 // 8 warps per CTA: thread t owns row t % 128 of the C tile (the TMEM lane) and column half t / 128
@@ -427,15 +440,23 @@ __global__ void __launch_bounds__(kGramThreads, 2)
 }
 
 // C[i * b + j] (row-major a x b) = sum over the CTAs of row range of the partial tiles
-__global__ void ozaki_reduce_kernel(const double* __restrict__ P, int nrb, int ny, int a, int b, double* __restrict__ C) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= a * b) return;
-  const int i = e / b, j = e % b;
-  const int mz = i / kM, nyi = j / kN;
-  const int64_t base = (((int64_t)mz * ny + nyi) * nrb) * (kM * kN) + (int64_t)(i % kM) * kN + (j % kN);
+// C = the sum of the partial tiles over the CTA row ranges, in a fixed order: 32 entries of one row of a tile
+// per CTA, eight threads each (one thread per entry took 42 us for 304 row ranges)
+__global__ void __launch_bounds__(256) ozaki_reduce_kernel(const double* __restrict__ P, int nrb, int ny, int a, int b,
+                                                           double* __restrict__ C) {
+  __shared__ double part[8][32];
+  const int i = blockIdx.x, nyi = blockIdx.y, jj = threadIdx.x & 31, w = threadIdx.x >> 5, j = nyi * kN + jj;
+  const double* p = P + (((int64_t)(i / kM) * ny + nyi) * nrb) * (kM * kN) + (int64_t)(i % kM) * kN + jj;
   double s = 0.0;
-  for (int k = 0; k < nrb; k++) s += P[base + (int64_t)k * (kM * kN)];
-  C[e] = s;
+#pragma unroll 4
+  for (int k = w; k < nrb; k += 8) s += p[(int64_t)k * (kM * kN)];
+  part[w][jj] = s;
+  __syncthreads();
+  if (w == 0 && j < b) {
+#pragma unroll
+    for (int q = 1; q < 8; q++) s += part[q][jj];
+    C[(int64_t)i * b + j] = s;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -1375,17 +1396,17 @@ void ozaki_gram(Ctx& c, int64_t n, const double* X, int64_t ldx, int a, const do
   int* EX = reinterpret_cast<int*>(work + (size_t)nrb * mz * ny * kM * kN);
   int* EY = EX + chunks * a;
   if (n > 0) {
-    chunk_exp_kernel<<<dim3((unsigned)chunks, (a + 127) / 128), 128, 0, c.stream>>>(n, X, ldx, a, EX);
-    chunk_exp_kernel<<<dim3((unsigned)chunks, (b + 127) / 128), 128, 0, c.stream>>>(n, Y, ldy, b, EY);
+    chunk_exp_kernel<<<dim3((unsigned)chunks, (a + 31) / 32 + (b + 31) / 32), 256, 0, c.stream>>>(n, X, ldx, a, EX, Y,
+                                                                                                   ldy, b, EY);
     FEM2D_CUDA(cudaGetLastError());
-    c.launches += 2;
+    c.launches++;
   }
   int64_t rpc = (std::max<int64_t>(n, 1) + nrb - 1) / nrb;
   rpc = (rpc + kChunk - 1) / kChunk * kChunk;
   dim3 grid(nrb, ny, mz);
   ozaki_gram_kernel<<<grid, kGramThreads, kSmemBytes, c.stream>>>(n, X, ldx, a, Y, ldy, b, rpc, EX, EY, work, err);
   FEM2D_CUDA(cudaGetLastError());
-  ozaki_reduce_kernel<<<(a * b + 255) / 256, 256, 0, c.stream>>>(work, nrb, ny, a, b, C);
+  ozaki_reduce_kernel<<<dim3(a, ny), 256, 0, c.stream>>>(work, nrb, ny, a, b, C);
   FEM2D_CUDA(cudaGetLastError());
   c.launches += 2;
 }

@@ -147,3 +147,25 @@ def test_mma_issue_cost(ctx):
     assert (256 / c[256]) >= 2.0 * (32 / c[32])
     with pytest.raises(fg.Fem2dError):
         ctx.mma_ns(24)
+
+
+@pytest.mark.parametrize("n", [1, 3, 31, 127, 129, 5403])
+@pytest.mark.parametrize("a,b", [(1, 1), (8, 8), (9, 7), (33, 16), (40, 33), (97, 24), (129, 32), (160, 65)])
+def test_block_gram_shapes(ctx, n, a, b):
+    """Gram products around the tiles of 8, 32 and 128 columns and the row slices, on padded blocks, with both
+    kernels: each sum of n products within n + 8 roundings (FP64), or 128 roundings of the chunk maxima per
+    128 rows (digit slices), of the sum of magnitudes."""
+    import torch
+
+    rng = np.random.default_rng(1000 * n + a + b)
+    x, y = rng.standard_normal((n, a + 3)), rng.standard_normal((n, b + 5))
+    xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    c = torch.full((a, b), float("nan"), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ref = x[:, :a].T @ y[:, :b]
+    mag = np.abs(x[:, :a]).T @ np.abs(y[:, :b])
+    top = np.max(np.abs(x[:, :a]), axis=0)[:, None] * np.max(np.abs(y[:, :b]), axis=0)[None, :]
+    for method in (fg.GRAM_FP64, fg.GRAM_TENSOR):
+        fg.block_gram_device(ctx, method, n, xd.data_ptr(), a + 3, a, yd.data_ptr(), b + 5, b, c.data_ptr())
+        bound = 2.0 ** -53 * ((n + 8) * mag if method == fg.GRAM_FP64 else 2 * (n + 8) * mag + 2 * n * top)
+        assert np.all(np.abs(c.cpu().numpy() - ref) <= 2 * bound), method
