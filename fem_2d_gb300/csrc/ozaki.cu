@@ -120,36 +120,39 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
   for (int q = 0; q < 8; q++) v[q] = __uint_as_float(r[q]);
 }
 
-// the eight digits of v relative to the biased exponent E of its column's largest magnitude
-__device__ __forceinline__ void digits8(double v, int E, float (&d)[kDigits]) {
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
-  const int ex = (int)((bits >> 52) & 0x7FF);
-  const int shift = E - ex;
-  const unsigned long long mant = (bits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-  const unsigned long long A = (ex == 0 || shift > 55) ? 0ull : ((mant << 3) >> shift);
-  const bool neg = (bits >> 63) != 0;
-#pragma unroll
-  for (int s = 0; s < kDigits; s++) {
-    const int dg = (int)((A >> (49 - 7 * s)) & 0x7F);
-    d[s] = (float)(neg ? -dg : dg);
-  }
+// The eight digits of va and vb relative to E, the biased exponent of the largest magnitude of their column
+// (or row), packed as BF16 pairs with va's in the low half: digit s is bits 49 - 7 s .. 55 - 7 s of the
+// mantissa shifted to E, with the value's sign. The kernels are bound by this integer work, so a pair of digits goes through each
+// step at once: a 28-bit half of the mantissa holds two 14-bit fields, one byte permute lays the same field of
+// both values side by side, and the BF16 number 128 + d is the bit pattern 0x4300 | d, from which one packed
+// FMA, (128 + d) sign - 128 sign, makes the signed digit. Some 26 instructions a value instead of 40.
+__device__ __forceinline__ uint32_t signed_digits(uint32_t d, uint32_t sign, uint32_t off) {
+  uint32_t r;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"((d & 0x007F007Fu) | 0x43004300u), "r"(sign), "r"(off));
+  return r;
 }
 
-// digits8 with integer digit extraction on 32-bit halves and a float conversion by the 2^23 offset
-// (no integer-to-float conversions); the same eight values as digits8
-__device__ __forceinline__ void digits8_fast(double v, int E, float (&d)[kDigits]) {
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
-  const int ex = (int)((bits >> 52) & 0x7FF);
-  const int shift = E - ex;
-  const unsigned long long mant = (bits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-  const unsigned long long A = (ex == 0 || shift > 55) ? 0ull : ((mant << 3) >> shift);
-  const uint32_t hi = (uint32_t)(A >> 32), lo = (uint32_t)A;
-  const float sg = (bits >> 63) ? -1.0f : 1.0f, off = -8388608.0f * sg;
-  const uint32_t dg[kDigits] = {(hi >> 17) & 0x7Fu, (hi >> 10) & 0x7Fu, (hi >> 3) & 0x7Fu,
-                                __funnelshift_r(lo, hi, 28) & 0x7Fu, (lo >> 21) & 0x7Fu, (lo >> 14) & 0x7Fu,
-                                (lo >> 7) & 0x7Fu, lo & 0x7Fu};
+__device__ __forceinline__ void digits8_pair(double va, double vb, int E, uint32_t (&pk)[kDigits]) {
+  const unsigned long long ba = (unsigned long long)__double_as_longlong(va);
+  const unsigned long long bb = (unsigned long long)__double_as_longlong(vb);
+  auto align = [E](unsigned long long bits) {   // the 56 bits of the digits
+    const int ex = (int)((bits >> 52) & 0x7FF);
+    const unsigned long long mant = ex == 0 ? 0ull : ((bits & 0xFFFFFFFFFFFFFull) | (1ull << 52));
+    return (mant << 3) >> min(E - ex, 63);
+  };
+  const unsigned long long A = align(ba), B = align(bb);
+  const uint32_t signs = __byte_perm((uint32_t)(ba >> 32), (uint32_t)(bb >> 32), 0x7632) & 0x80008000u;
+  const uint32_t sign = signs | 0x3F803F80u, off = signs ^ 0xC300C300u;   // +-1 and -+128
 #pragma unroll
-  for (int s = 0; s < kDigits; s++) d[s] = fmaf(__uint_as_float(0x4B000000u | dg[s]), sg, off);
+  for (int h = 0; h < 2; h++) {
+    const uint32_t a = h == 0 ? __funnelshift_r((uint32_t)A, (uint32_t)(A >> 32), 28) : (uint32_t)A;
+    const uint32_t b = h == 0 ? __funnelshift_r((uint32_t)B, (uint32_t)(B >> 32), 28) : (uint32_t)B;
+    const uint32_t top = __byte_perm(a << 2, b << 2, 0x7632), low = __byte_perm(a, b, 0x5410);
+    pk[4 * h] = signed_digits(top >> 7, sign, off);
+    pk[4 * h + 1] = signed_digits(top, sign, off);
+    pk[4 * h + 2] = signed_digits(low >> 7, sign, off);
+    pk[4 * h + 3] = signed_digits(low, sign, off);
+  }
 }
 
 __device__ __forceinline__ int biased_exp(double v) {
@@ -183,11 +186,6 @@ __device__ __forceinline__ double scale_pow2(double a, int k) {
   const int e = (int)((bits >> 52) & 0x7FF);
   if (e != 0 && e + k >= 1 && e + k <= 2046) return __longlong_as_double(bits + ((long long)k << 52));
   return a * pow2(k);
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&h);
 }
 
 // byte offset of core matrix (row group rg, k group kg) in a K-major tile with kSub columns
@@ -321,11 +319,10 @@ __global__ void __launch_bounds__(kGramThreads, 2)
         uint32_t pk[kDigits][4];
 #pragma unroll
         for (int r8 = 0; r8 < 8; r8 += 2) {
-          float d0[kDigits], d1[kDigits];
-          digits8_fast(xv[kh * 8 + r8], Ex, d0);
-          digits8_fast(xv[kh * 8 + r8 + 1], Ex, d1);
+          uint32_t d[kDigits];
+          digits8_pair(xv[kh * 8 + r8], xv[kh * 8 + r8 + 1], Ex, d);
 #pragma unroll
-          for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = pack_bf16(d0[s2], d1[s2]);
+          for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = d[s2];
         }
         const int off = core_off(row >> 3, kg) + (row & 7) * 16;
 #pragma unroll
@@ -336,11 +333,10 @@ __global__ void __launch_bounds__(kGramThreads, 2)
         uint32_t pk[kDigits][4];
 #pragma unroll
         for (int r8 = 0; r8 < 8; r8 += 2) {
-          float d0[kDigits], d1[kDigits];
-          digits8_fast(yv[r8], Ey, d0);
-          digits8_fast(yv[r8 + 1], Ey, d1);
+          uint32_t d[kDigits];
+          digits8_pair(yv[r8], yv[r8 + 1], Ey, d);
 #pragma unroll
-          for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = pack_bf16(d0[s2], d1[s2]);
+          for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = d[s2];
         }
         const int off = core_off(yj >> 3, ykg) + (yj & 7) * 16;
 #pragma unroll
@@ -572,12 +568,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     uint32_t pk[kDigits][4];
 #pragma unroll
     for (int r8 = 0; r8 < 8; r8 += 2) {
-      float d0[kDigits], d1[kDigits];
+      uint32_t d[kDigits];
       const int k0 = kg * 8 + r8;
-      digits8((j < b && k0 < a) ? C[(int64_t)k0 * b + j] : 0.0, eC[j], d0);
-      digits8((j < b && k0 + 1 < a) ? C[(int64_t)(k0 + 1) * b + j] : 0.0, eC[j], d1);
+      digits8_pair((j < b && k0 < a) ? C[(int64_t)k0 * b + j] : 0.0,
+                   (j < b && k0 + 1 < a) ? C[(int64_t)(k0 + 1) * b + j] : 0.0, eC[j], d);
 #pragma unroll
-      for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = pack_bf16(d0[s2], d1[s2]);
+      for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = d[s2];
     }
     const int off = core_off_k(j >> 3, kg, kc) + (j & 7) * 16;
 #pragma unroll
@@ -640,11 +636,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         uint32_t pk[kDigits][4];
 #pragma unroll
         for (int r8 = 0; r8 < 8; r8 += 2) {
-          float d0[kDigits], d1[kDigits];
-          digits8_fast(xv[kh * 8 + r8], Ex, d0);
-          digits8_fast(xv[kh * 8 + r8 + 1], Ex, d1);
+          uint32_t d[kDigits];
+          digits8_pair(xv[kh * 8 + r8], xv[kh * 8 + r8 + 1], Ex, d);
 #pragma unroll
-          for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = pack_bf16(d0[s2], d1[s2]);
+          for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = d[s2];
         }
         const int off = core_off(rl >> 3, kg) + (rl & 7) * 16;
 #pragma unroll
@@ -743,7 +738,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 //
 // Rows of one Elem's interior functions share a column list (a run of R <= 64 rows); an item is one
 // run and 64 consecutive columns of its list. M's values are sliced once per solve (spmm_slice_kernel)
-// into the eight 7-bit digit planes of digits8 (one exponent per item row), in the K-major
+// into the eight 7-bit digit planes of digits8_pair (one exponent per item row), in the K-major
 // core-matrix layout the MMA reads. The product kernel gathers the item's 64 rows of X and slices them
 // the same way (one exponent per column) into a sequence of digit planes of X, 16 or 32 rows (one per
 // column) each, preceded by zero planes. The MMA's 128 rows are (digit-sum group g, column of X) and
@@ -818,11 +813,10 @@ __global__ void __launch_bounds__(256) spmm_slice_kernel(int nitems, const int4*
 #pragma unroll
       for (int r8 = 0; r8 < 8; r8 += 2) {
         const int q = kg8 * 8 + r8;
-        float d0[kDigits], d1[kDigits];
-        digits8((k0 >= 0 && q < Lc) ? val(k0 + q) : 0.0, E, d0);
-        digits8((k0 >= 0 && q + 1 < Lc) ? val(k0 + q + 1) : 0.0, E, d1);
+        uint32_t d[kDigits];
+        digits8_pair((k0 >= 0 && q < Lc) ? val(k0 + q) : 0.0, (k0 >= 0 && q + 1 < Lc) ? val(k0 + q + 1) : 0.0, E, d);
 #pragma unroll
-        for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = pack_bf16(d0[s2], d1[s2]);
+        for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = d[s2];
       }
       const int64_t cm = (int64_t)((r >> 3) * 4 + kg) * 8 + (r & 7);   // uint4 index within a plane
 #pragma unroll
@@ -862,11 +856,10 @@ __device__ __forceinline__ void sp_stage_x(const int* cq, const double* __restri
     uint32_t pk[kDigits][4];
 #pragma unroll
     for (int r = 0; r < 8; r += 2) {
-      float d0[kDigits], d1[kDigits];
-      digits8_fast(xv[r], E, d0);
-      digits8_fast(xv[r + 1], E, d1);
+      uint32_t d[kDigits];
+      digits8_pair(xv[r], xv[r + 1], E, d);
 #pragma unroll
-      for (int s = 0; s < kDigits; s++) pk[s][r >> 1] = pack_bf16(d0[s], d1[s]);
+      for (int s = 0; s < kDigits; s++) pk[s][r >> 1] = d[s];
     }
     // digit s: plane 3 + s, row j
 #pragma unroll
@@ -891,11 +884,10 @@ __device__ __forceinline__ void sp_stage_x(const int* cq, const double* __restri
     uint32_t pk[kDigits][2];
 #pragma unroll
     for (int r = 0; r < 4; r += 2) {
-      float d0[kDigits], d1[kDigits];
-      digits8_fast(xv[r], E, d0);
-      digits8_fast(xv[r + 1], E, d1);
+      uint32_t d[kDigits];
+      digits8_pair(xv[r], xv[r + 1], E, d);
 #pragma unroll
-      for (int s = 0; s < kDigits; s++) pk[s][r >> 1] = pack_bf16(d0[s], d1[s]);
+      for (int s = 0; s < kDigits; s++) pk[s][r >> 1] = d[s];
     }
     // digit s: plane 7 + s, row j
 #pragma unroll
