@@ -458,8 +458,9 @@ __global__ void __launch_bounds__(256) ozaki_reduce_kernel(const double* __restr
 // ---------------------------------------------------------------------------------------------------
 // Z = beta Z + alpha X C for a tall X (n x a, a <= 256) and a small C (a x b, b <= 32): the block
 // updates of the B-orthogonalisation and the Ritz-vector products. Each CTA owns 128-row tiles of X
-// and Z (TMEM lane = row; 8 warps, two threads per row, each slicing 16 of a sub-block's 32 columns of
-// X and owning 16 of the 32 columns of Z). X is sliced with one exponent per row (over its a entries)
+// and Z (TMEM lane = row; 16 warps, four threads per row, each slicing 8 of a sub-block's 32 columns of
+// X and owning 8 of the 32 columns of Z: with two threads per row one CTA of 8 warps, all that fits an SM,
+// issued on 28% of its cycles and waited on loads and barriers for the rest). X is sliced with one exponent per row (over its a entries)
 // and C with one per column (over its a entries), so every K sub-block's digit sums share one scale:
 // they are read from TMEM after each 128 columns of K (the exact-accumulation limit) and summed exactly
 // in int64, fused into one integer (fuse_digit_sums) and converted to FP64 once per output element, with
@@ -469,7 +470,8 @@ __global__ void __launch_bounds__(256) ozaki_reduce_kernel(const double* __restr
 // buffer, one sub-block ahead of its slicing when two staging buffers fit. The row exponents come from
 // a coalesced pre-pass (row_exp_kernel).
 constexpr int kGemmKMax = 256;
-constexpr int kGemmThreads = 256;
+constexpr int kGemmThreads = 512;
+constexpr int kGemmCols = kN / 4;                // columns of Z per thread
 constexpr int kGemmPlanes = kDigits * kPlaneA;   // digit planes of one 128 x 32 sub-block of X (64 KB)
 constexpr int kGemmRow = kSub + 1;               // staged doubles per row (padded: no bank conflicts)
 constexpr int kGemmStage = kM * kGemmRow * 8;    // one staged 128 x 32 sub-block of X (33 KB)
@@ -539,7 +541,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   uint64_t* bar = reinterpret_cast<uint64_t*>(eC + kN);       // MMAs committed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int rl = tid & (kM - 1), half = tid >> 7;  // row of the tile (TMEM lane), column half
+  const int rl = tid & (kM - 1), part = tid >> 7;  // row of the tile (TMEM lane), column quarter
   const int64_t ntiles = (n + kM - 1) / kM;
   const int nsub = kc / kSub;
 
@@ -556,11 +558,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   // the first sub-block's copies, then C's column exponents and digit planes (row j of the B operand =
   // column j of C)
   if (blockIdx.x < ntiles) gemm_stage(X, n, ldx, a, blockIdx.x, 0, sX);
-  if (tid < kN) {
+  if (tid < kN) eC[tid] = 0;
+  __syncthreads();
+  {
+    const int j = tid % kN;
     int e = 0;
-    if (tid < b)
-      for (int k = 0; k < a; k++) e = max(e, biased_exp(C[(int64_t)k * b + tid]));
-    eC[tid] = e;
+    if (j < b)
+      for (int k = tid / kN; k < a; k += kGemmThreads / kN) e = max(e, biased_exp(C[(int64_t)k * b + j]));
+    atomicMax(&eC[j], e);
   }
   __syncthreads();
   for (int t = tid; t < kN * (kc / 8); t += kGemmThreads) {
@@ -597,9 +602,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const int64_t row = tile * kM + rl;
     const bool row_ok = row < n;
     const int Ex = row_ok ? EXr[row] : 0;
-    long long Th[kN / 2], Tl[kN / 2];
+    long long Th[kGemmCols], Tl[kGemmCols];
 #pragma unroll
-    for (int j = 0; j < kN / 2; j++) Th[j] = Tl[j] = 0;
+    for (int j = 0; j < kGemmCols; j++) Th[j] = Tl[j] = 0;
+    double zv[kGemmCols];
     for (int sb = 0; sb < nsub && !failed; sb++, sbc++) {
       const int k0 = sb * kSub;
       const double* sx = sX + (stages == 2 ? (sbc & 1) : 0) * (kGemmStage / 8);
@@ -618,9 +624,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
       __syncthreads();   // every thread's copies of this sub-block have landed
-      double xv[kSub / 2];
+      double xv[8];
 #pragma unroll
-      for (int q = 0; q < kSub / 2; q++) xv[q] = sx[rl * kGemmRow + half * (kSub / 2) + q];
+      for (int q = 0; q < 8; q++) xv[q] = sx[rl * kGemmRow + part * 8 + q];
       if (pending) {   // the digit planes are free once the previous MMAs completed
         if (mbar_wait(smem_addr(bar), ph)) {
           ph ^= 1u;
@@ -630,18 +636,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       }
-#pragma unroll
-      for (int kh = 0; kh < 2; kh++) {
-        const int kg = half * 2 + kh;
+      {
         uint32_t pk[kDigits][4];
 #pragma unroll
         for (int r8 = 0; r8 < 8; r8 += 2) {
           uint32_t d[kDigits];
-          digits8_pair(xv[kh * 8 + r8], xv[kh * 8 + r8 + 1], Ex, d);
+          digits8_pair(xv[r8], xv[r8 + 1], Ex, d);
 #pragma unroll
           for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = d[s2];
         }
-        const int off = core_off(rl >> 3, kg) + (rl & 7) * 16;
+        const int off = core_off(rl >> 3, part) + (rl & 7) * 16;
 #pragma unroll
         for (int s2 = 0; s2 < kDigits; s2++)
           *reinterpret_cast<uint4*>(sA + s2 * kPlaneA + off) = make_uint4(pk[s2][0], pk[s2][1], pk[s2][2], pk[s2][3]);
@@ -672,7 +676,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
       pending = true;
       const bool last = (k0 + kSub) % kChunk == 0 || k0 + kSub >= kc;
-      if (last) {   // the accumulators are read back: wait for these MMAs now
+      if (last) {   // the accumulators are read back: wait for these MMAs now (the old Z in flight meanwhile)
+        if (beta != 0.0 && k0 + kSub >= kc && row_ok) {
+          const double* zr = Z + row * ldz + part * kGemmCols;
+#pragma unroll
+          for (int q = 0; q < kGemmCols; q++) zv[q] = part * kGemmCols + q < b ? zr[q] : 0.0;
+        }
         if (mbar_wait(smem_addr(bar), ph)) {
           ph ^= 1u;
           pending = false;
@@ -686,18 +695,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         }
         // exact digit sums of these (at most 128) columns of K into the int64 accumulators
 #pragma unroll
-        for (int cb = 0; cb < kN / 2; cb += 8) {
-          float v[kDigits][8];
+        for (int g0 = 0; g0 < kDigits; g0 += 4) {
+          float v[4][8];
 #pragma unroll
-          for (int g = 0; g < kDigits; g++) tmem_ld8(lane_base + (uint32_t)(g * kN + half * (kN / 2) + cb), v[g]);
+          for (int g = 0; g < 4; g++) tmem_ld8(lane_base + (uint32_t)((g0 + g) * kN + part * kGemmCols), v[g]);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int g = 0; g < kDigits; g++)
+          for (int g = 0; g < 4; g++)
 #pragma unroll
             for (int q = 0; q < 8; q++) {
-              const long long iv = (long long)__float2int_rn(v[g][q]);
-              if (g < 4) Th[cb + q] += iv << (7 * (3 - g));
-              else Tl[cb + q] += iv << (7 * (7 - g));
+              const long long iv = (long long)__float2int_rn(v[g][q]) << (7 * (3 - g));
+              if (g0 == 0) Th[q] += iv;
+              else Tl[q] += iv;
             }
         }
         // every thread's reads of the accumulators precede the next MMAs
@@ -710,14 +719,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     if (row_ok) {
       // one conversion and one multiply (or FMA) per output: alpha and the power-of-two scale are
       // combined exactly in the exponent field
-      double* zr = Z + row * ldz + half * (kN / 2);
+      double* zr = Z + row * ldz + part * kGemmCols;
 #pragma unroll
-      for (int q = 0; q < kN / 2; q++) {
-        const int j = half * (kN / 2) + q;
+      for (int q = 0; q < kGemmCols; q++) {
+        const int j = part * kGemmCols + q;
         if (j >= b) break;
         const double t = (double)fuse_digit_sums<kFuseGemm>(Th[q], Tl[q]);
         const double m = scale_pow2(alpha, Ex + eC[j] - 2044 - 35 - kFuseGemm);
-        zr[q] = beta == 0.0 ? t * m : fma(t, m, beta == 1.0 ? zr[q] : beta * zr[q]);
+        zr[q] = beta == 0.0 ? t * m : fma(t, m, beta == 1.0 ? zv[q] : beta * zv[q]);
       }
     }
   }
