@@ -8,9 +8,10 @@
 // space is generated with
 //     T = (A - sigma B)^-1 A (A + c B)^-1 B
 // with c = |sigma|: eigenvalue lambda / ((lambda - sigma)(lambda + c)), close to the plain
-// shift-invert 1 / (lambda - sigma) for the physical modes, zero on the null space (A kills it
-// whatever the accuracy of the SPD solve; rounding smears it to small lambda, damped by
-// lambda / (lambda + c)) and small for high-frequency modes; exact multifrontal solves (mf.cu). Each
+// shift-invert 1 / (lambda - sigma) for the physical modes, zero on the null space (to rounding, which
+// smears it to small lambda, damped by lambda / (lambda + c)) and small for high-frequency modes; exact
+// multifrontal solves (mf.cu), for targets above zero in partial fractions, as two solves of one right-hand
+// side (see apply_T). Each
 // cycle builds a block Krylov basis [XL, X, TX, ..., T^s X] (s = 4 by default; XL the locked converged
 // pairs, X the active Ritz vectors), B-orthonormalised by CGS2 in FP64, then a Rayleigh-Ritz step on
 // the pencil (A, B) itself (FP64) over the active columns; Ritz pairs with a relative residual above 1
@@ -1035,26 +1036,41 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
   }
   if (o.refine > 0) nref_p = nref_m = std::min(o.refine, 3);
   if (o.refine < 0) nref_p = nref_m = 0;
-  // Out (ld lo) = T In (ld li), nb columns; In and Out may not alias W1..W3
-  auto apply_T = [&](const double* In, int64_t li, double* Out, int64_t lo, int nb) {
-    D.spmm(0.0, 1.0, In, li, nb, W1.p, 32);
-    if (iterative) {
+  // T by partial fractions: (c + sigma) A = c (A - sigma B) + sigma (A + c B), so
+  //     T = (A - sigma B)^-1 A (A + c B)^-1 B = (c (A + c B)^-1 B + sigma (A - sigma B)^-1 B) / (c + sigma):
+  // two solves of the same right-hand side, which go through the levels of the tree together, and no product
+  // with A between them. The null space cancels to the rounding of the two solves, and the errors of the
+  // first solve are not multiplied by ||A|| any more: the pencils that took 4 to 5 cycles at 160k and 1M DoFs
+  // take 3 to 4, and HierPoly pencils at 1M DoFs on which the product form ran out of cycles converge. A
+  // target below zero keeps the product form: c + sigma may vanish there.
+  const bool fractions = !iterative && sigma > 0.0;
+  // Out (ld lo) = T x for the nb columns x with B x given (BIn, ld lb); BIn and Out may not alias W1..W3
+  auto apply_T = [&](const double* BIn, int64_t lb, double* Out, int64_t lo, int nb) {
+    if (fractions) {
+      if (nref_p == 0 && nref_m == 0) {
+        M->solve_pair(c, fp, fm, BIn, lb, W2.p, 32, Out, lo, nb);
+      } else {
+        solve_ref(fp, 1.0, cshift, BIn, lb, W2.p, 32, nb, nref_p);
+        solve_ref(fm, 1.0, -sigma, BIn, lb, Out, lo, nb, nref_m);
+      }
+      D.axpby(cshift / (cshift + sigma), W2.p, 32, nb, sigma / (cshift + sigma), Out, lo);
+    } else if (iterative) {
       PCGStats s1, s2;
-      pcg->cg_device(W1.p, 32, W2.p, 32, nb, inner_tol, max_inner, &s1);
+      pcg->cg_device(BIn, lb, W2.p, 32, nb, inner_tol, max_inner, &s1);
       D.spmm(1.0, 0.0, W2.p, 32, nb, W3.p, 32);
       // the learned coarse space is trained on, and corrects, the SPD system's errors: the MINRES solves
       // of the indefinite system keep the additive-Schwarz preconditioner alone
       pcg->minres_device(1.0, -sigma, W3.p, 32, Out, lo, nb, inner_tol, max_inner, &s2, false);
       cg_iters += s1.iters;
       minres_iters += s2.iters;
-      spmv += (int64_t)nb * (s1.iters + s2.iters);
+      spmv += (int64_t)nb * (1 + s1.iters + s2.iters);
       inner_worst = std::max(inner_worst, std::max(s1.relres, s2.relres));
     } else {
-      solve_ref(fp, 1.0, cshift, W1.p, 32, W2.p, 32, nb, nref_p);
+      solve_ref(fp, 1.0, cshift, BIn, lb, W2.p, 32, nb, nref_p);
       D.spmm(1.0, 0.0, W2.p, 32, nb, W3.p, 32);
       solve_ref(fm, 1.0, -sigma, W3.p, 32, Out, lo, nb, nref_m);
+      spmv += nb;
     }
-    spmv += 2 * nb;
     napply += nb;
   };
   // W = V[:, m0:m0+r]: B-orthogonalise against V[:, :m0] (CGS2 with the stored B V), form B W once,
@@ -1153,7 +1169,9 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
     DBuf<double> R;
     R.alloc_on((size_t)n * b, c.stream);
     random_block_device(c, n, b, 12345, R.p, b);
-    apply_T(R.p, b, X.p, 32, b);
+    D.spmm(0.0, 1.0, R.p, b, b, W1.p, 32);
+    spmv += b;
+    apply_T(W1.p, 32, X.p, 32, b);
   }
   // A pair is converged when its relative residual is below tol or its normwise backward error
   // ||A x - theta B x|| / ((||A|| + |theta| ||B||) ||x||) is below kBackward: the pair is then exact for
@@ -1215,14 +1233,14 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
       if (m + bx > mmax) fail(FEM2D_E_NOT_CONVERGED, "gpu_solve_gep: basis capacity exceeded");
       // expand with T applied to the active Ritz vectors: T kills their null-space part and damps
       // high-frequency content, which also pushes spurious Ritz vectors out of the basis
-      apply_T(X.p, 32, V.p + m, mmax, bx);
+      apply_T(BX.p, 32, V.p + m, mmax, bx);   // the basis carries the exact products: no product with B here
       const int r = borth_new(m, bx);
       last0 = m;
       lastn = r;
       m += r;
     }
     for (int st2 = (cycles == 0 ? 0 : 1); st2 < steps && lastn > 0 && m + lastn <= mmax; st2++) {
-      apply_T(V.p + last0, mmax, V.p + m, mmax, lastn);
+      apply_T(BV.p + last0, mmax, V.p + m, mmax, lastn);
       int r = borth_new(m, lastn);
       if (r == 0) break;
       last0 = m;

@@ -1063,16 +1063,23 @@ __device__ __forceinline__ double col_dot(const double* __restrict__ A, int f, c
   return (a0 + a1) + (a2 + a3);
 }
 
-struct SolveArgs {
-  const FrontDesc* fd;
-  const int32_t *dofs, *emap, *perm, *iperm;
-  const int64_t *piv_off, *woff;
+// One factorization of the plan and what a solve with it writes. A launch serves one or two of them
+// (blockIdx.z): the solves of one right-hand side with both shifted matrices go level by level together.
+struct SolveSet {
+  const int32_t *perm, *iperm;
   const double* F;
-  const double* B;
-  int64_t ldb;
   double* W;
   double* X;
   int64_t ldx;
+};
+
+struct SolveArgs {
+  const FrontDesc* fd;
+  const int32_t *dofs, *emap;
+  const int64_t *piv_off, *woff;
+  const double* B;
+  int64_t ldb;
+  SolveSet set[2];
   int nb;
   int per;   // right-hand sides per CTA: blockIdx.y takes the columns from blockIdx.y * per on
 };
@@ -1130,14 +1137,15 @@ template <int NT>
 __global__ void __launch_bounds__(NT) mf_forward_small_kernel(const int32_t* __restrict__ lf, SolveArgs a) {
   extern __shared__ double sm[];
   const int fr = lf[blockIdx.x];
+  const SolveSet set = a.set[blockIdx.z];
   const int c0 = blockIdx.y * a.per, w = min(a.per, a.nb - c0);
   const FrontDesc d = a.fd[fr];
   const int f = d.f, p = d.p, lv = f | 1, ly = p | 1;
   double* v = sm;            // v[c * lv + i]
   double* y = sm + lv * w;   // y[c * ly + i]
-  const double* A = a.F + d.off;
-  gather_front_rhs(d, a.fd, a.emap, a.iperm + a.piv_off[fr], a.W, a.woff, a.B, a.ldb, a.dofs + d.dptr,
-                   a.perm + a.piv_off[fr], c0, w, lv, v);
+  const double* A = set.F + d.off;
+  gather_front_rhs(d, a.fd, a.emap, set.iperm + a.piv_off[fr], set.W, a.woff, a.B, a.ldb, a.dofs + d.dptr,
+                   set.perm + a.piv_off[fr], c0, w, lv, v);
   // the unit lower triangle: row i is a dot product of length i, so a thread takes the rows q and
   // p - 1 - q (p - 1 terms together) and the lanes of a warp run equally long
   const int hp = (p + 1) >> 1;
@@ -1155,7 +1163,7 @@ __global__ void __launch_bounds__(NT) mf_forward_small_kernel(const int32_t* __r
     v[c * lv + i] -= col_dot(A + i, f, y + c * ly, 0, p);
   }
   __syncthreads();
-  double* out = a.W + a.woff[fr] + c0;
+  double* out = set.W + a.woff[fr] + c0;
   for (int t = threadIdx.x; t < f * w; t += blockDim.x) {
     const int i = t / w, c = t - i * w;
     out[(int64_t)i * kLdW + c] = i < p ? y[c * ly + i] : v[c * lv + i];
@@ -1166,6 +1174,7 @@ template <int NT>
 __global__ void __launch_bounds__(NT) mf_backward_small_kernel(const int32_t* __restrict__ lf, SolveArgs a) {
   extern __shared__ double sm[];
   const int fr = lf[blockIdx.x];
+  const SolveSet set = a.set[blockIdx.z];
   const int c0 = blockIdx.y * a.per, w = min(a.per, a.nb - c0);
   const FrontDesc d = a.fd[fr];
   const int f = d.f, p = d.p;
@@ -1174,13 +1183,13 @@ __global__ void __launch_bounds__(NT) mf_backward_small_kernel(const int32_t* __
   double* z = sm;             // z[c * lz + i]
   double* xs = sm + lz * w;   // xs[c * lx + j]: solved struct unknowns, then the front's own
   const int32_t* D = a.dofs + d.dptr;
-  const double* A = a.F + d.off;
-  const double* v = a.W + a.woff[fr] + c0;
-  double* X = a.X + c0;
+  const double* A = set.F + d.off;
+  const double* v = set.W + a.woff[fr] + c0;
+  double* X = set.X + c0;
   for (int t = threadIdx.x; t < f * w; t += blockDim.x) {
     const int i = t / w, c = t - i * w;
     if (i < p) z[c * lz + i] = v[(int64_t)i * kLdW + c];
-    else xs[c * lx + i - p] = X[(int64_t)D[i] * a.ldx + c];
+    else xs[c * lx + i - p] = X[(int64_t)D[i] * set.ldx + c];
   }
   __syncthreads();
   for (int t = threadIdx.x; t < p * w; t += blockDim.x) {
@@ -1200,7 +1209,7 @@ __global__ void __launch_bounds__(NT) mf_backward_small_kernel(const int32_t* __
   __syncthreads();
   for (int t = threadIdx.x; t < p * w; t += blockDim.x) {
     const int i = t / w, c = t - i * w;
-    X[(int64_t)D[i] * a.ldx + c] = xs[c * lx + i];
+    X[(int64_t)D[i] * set.ldx + c] = xs[c * lx + i];
   }
 }
 
@@ -1234,16 +1243,12 @@ constexpr int kTileSteps = kChunkK / 16;   // MMA steps (4 columns of the front)
 struct TiledArgs {
   const FrontDesc* fd;
   const int32_t* dofs;
-  const int32_t* perm;
   const int64_t* piv_off;
   const int64_t* woff;
   const int4* pull;   // per row of a tiled front (from FrontDesc::prow on), two int4: see pull_row
-  const double* F;
   const double* B;
   int64_t ldb;
-  double* W;
-  double* X;
-  int64_t ldx;
+  SolveSet set[2];
   int nb;
   int chunk;   // rows of v in shared memory (see tile_product)
 };
@@ -1251,17 +1256,18 @@ struct TiledArgs {
 // row k (pivot order) of front d's gathered right-hand side, column c: the row's record holds its DoF (the
 // row of B, -1 past the pivots), then up to MAXKIDS workspace rows of the children, in slot order, -1 past
 // the last
-__device__ __forceinline__ double pull_row(const TiledArgs& a, const FrontDesc& d, const int32_t* pm, int k, int c) {
+__device__ __forceinline__ double pull_row(const TiledArgs& a, const FrontDesc& d, const double* W, const int32_t* pm, int k,
+                                           int c) {
   const int u = k < d.p ? pm[k] : k;
   const int4* rec = a.pull + 2 * (d.prow + u);
   const int4 q = __ldg(rec);
   double s = q.x >= 0 ? a.B[(int64_t)q.x * a.ldb + c] : 0.0;
-  if (q.y >= 0) s += a.W[(int64_t)q.y * kLdW + c];
-  if (q.z >= 0) s += a.W[(int64_t)q.z * kLdW + c];
+  if (q.y >= 0) s += W[(int64_t)q.y * kLdW + c];
+  if (q.z >= 0) s += W[(int64_t)q.z * kLdW + c];
   if (q.w >= 0) {
-    s += a.W[(int64_t)q.w * kLdW + c];
+    s += W[(int64_t)q.w * kLdW + c];
     const int last = __ldg(&rec[1].x);
-    if (last >= 0) s += a.W[(int64_t)last * kLdW + c];
+    if (last >= 0) s += W[(int64_t)last * kLdW + c];
   }
   return s;
 }
@@ -1338,14 +1344,15 @@ constexpr size_t tile_smem(int nt, int chunk) {
 template <int NT>
 __global__ void __launch_bounds__(kTileThreads) mf_forward_tiled_kernel(const int2* __restrict__ items, TiledArgs a) {
   const int2 it = items[blockIdx.x];
+  const SolveSet set = a.set[blockIdx.z];
   const FrontDesc d = a.fd[it.x];
   const int p = d.p, c0 = blockIdx.y * 8 * NT;
-  const int32_t* pm = a.perm + a.piv_off[it.x];
-  double* out = a.W + a.woff[it.x] + c0;
+  const int32_t* pm = set.perm + a.piv_off[it.x];
+  double* out = set.W + a.woff[it.x] + c0;
   // rows r < p need k < r, rows r >= p need k < p
-  auto pull = [&](int k, int c) { return pull_row(a, d, pm, k, c0 + c); };
+  auto pull = [&](int k, int c) { return pull_row(a, d, set.W, pm, k, c0 + c); };
   tile_product<NT>(
-      a.F + d.off, d.f, it.y, d.f, 0, min(p, it.y + kTileRows), min(8 * NT, a.nb - c0), a.chunk,
+      set.F + d.off, d.f, it.y, d.f, 0, min(p, it.y + kTileRows), min(8 * NT, a.nb - c0), a.chunk,
       [p](int r, int k) { return k < r || r >= p; }, pull, pull,
       [&](int r, int c, double s) { out[(int64_t)r * kLdW + c] = s; });
 }
@@ -1353,15 +1360,16 @@ __global__ void __launch_bounds__(kTileThreads) mf_forward_tiled_kernel(const in
 template <int NT>
 __global__ void __launch_bounds__(kTileThreads) mf_backward_tiled_kernel(const int2* __restrict__ items, TiledArgs a) {
   const int2 it = items[blockIdx.x];
+  const SolveSet set = a.set[blockIdx.z];
   const FrontDesc d = a.fd[it.x];
   const int p = d.p, c0 = blockIdx.y * 8 * NT;
   const int32_t* D = a.dofs + d.dptr;
-  const double* y = a.W + a.woff[it.x] + c0;
-  double* X = a.X + c0;
+  const double* y = set.W + a.woff[it.x] + c0;
+  double* X = set.X + c0;
   tile_product<NT>(
-      a.F + d.off, d.f, it.y, p, it.y, d.f, min(8 * NT, a.nb - c0), a.chunk, [](int r, int k) { return k >= r; },
-      [&](int k, int c) { return k < p ? y[(int64_t)k * kLdW + c] : X[(int64_t)D[k] * a.ldx + c]; },
-      [](int, int) { return 0.0; }, [&](int r, int c, double s) { X[(int64_t)D[r] * a.ldx + c] = s; });
+      set.F + d.off, d.f, it.y, p, it.y, d.f, min(8 * NT, a.nb - c0), a.chunk, [](int r, int k) { return k >= r; },
+      [&](int k, int c) { return k < p ? y[(int64_t)k * kLdW + c] : X[(int64_t)D[k] * set.ldx + c]; },
+      [](int, int) { return 0.0; }, [&](int r, int c, double s) { X[(int64_t)D[r] * set.ldx + c] = s; });
 }
 
 // X = Kinv B for a dense inverse (n x n, row-major): one warp per row, lane c owns right-hand side c;
@@ -1672,6 +1680,7 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   arena.add(woff, woff_h);
   piv_total = po;
   arena.reserve(work, std::max<int64_t>(wo, 1));
+  arena.reserve(work2, std::max<int64_t>(wo, 1));
   arena.reserve(flags, 1);
   arena.reserve(weak_list, std::max<int64_t>(s.n, 1));
   arena.reserve(weak_count, 1);
@@ -1872,30 +1881,47 @@ static int tile_groups(int items, int nb, int num_sms) {
 }
 
 void MFDevice::solve(Ctx& c, const MFFactor& fac, const double* B, int64_t ldb, double* X, int64_t ldx, int nb) {
-  const DBuf<double>& Fbuf = fac.F;
-  cudaStream_t st = c.stream;
   if (nb > nb_cap) fail(FEM2D_E_INVALID_ARG, "solve block wider than the workspace");
   if (fac.inv_n > 0) {
     ProfScope ps(c, "mf_solve", 8.0 * fac.inv_n * fac.inv_n, 2.0 * fac.inv_n * fac.inv_n * nb);
     const int64_t blocks = std::min<int64_t>((fac.inv_n * 32 + 255) / 256, (int64_t)c.num_sms * 8);
-    dense_inverse_apply_kernel<<<(int)std::max<int64_t>(blocks, 1), 256, 0, st>>>(fac.inv_n, Fbuf.p, B, ldb, nb, X,
+    dense_inverse_apply_kernel<<<(int)std::max<int64_t>(blocks, 1), 256, 0, c.stream>>>(fac.inv_n, fac.F.p, B, ldb, nb, X,
                                                                                  ldx);
     c.launches++;
     FEM2D_CUDA(cudaGetLastError());
     return;
   }
+  solve_sets(c, 1, &fac, nullptr, B, ldb, X, ldx, nullptr, 0, nb);
+}
+
+void MFDevice::solve_pair(Ctx& c, const MFFactor& f1, const MFFactor& f2, const double* B, int64_t ldb, double* X1,
+                          int64_t ldx1, double* X2, int64_t ldx2, int nb) {
+  if (f1.inv_n > 0 || f2.inv_n > 0) {
+    solve(c, f1, B, ldb, X1, ldx1, nb);
+    solve(c, f2, B, ldb, X2, ldx2, nb);
+    return;
+  }
+  if (nb > nb_cap) fail(FEM2D_E_INVALID_ARG, "solve block wider than the workspace");
+  solve_sets(c, 2, &f1, &f2, B, ldb, X1, ldx1, X2, ldx2, nb);
+}
+
+void MFDevice::solve_sets(Ctx& c, int sets, const MFFactor* f1, const MFFactor* f2, const double* B, int64_t ldb,
+                          double* X1, int64_t ldx1, double* X2, int64_t ldx2, int nb) {
+  cudaStream_t st = c.stream;
   const FrontDesc* fd = reinterpret_cast<const FrontDesc*>(desc.p);
   double fbytes = 0.0;
   for (double b : level_factor_bytes) fbytes += b;
   // the whole solve is one profiled region: per-level events would dominate the short level launches
-  ProfScope ps(c, "mf_solve", 2.0 * fbytes, 2.0 * 2.0 * (fbytes / 8.0) * nb);
-  SolveArgs a{fd, dofs.p, ea_map.p, fac.perm.p, fac.iperm.p, piv_off.p, woff.p, Fbuf.p, B, ldb, work.p, X, ldx, nb, nb};
-  TiledArgs ta{fd, dofs.p, fac.perm.p, piv_off.p, woff.p, reinterpret_cast<const int4*>(pull.p), Fbuf.p, B, ldb, work.p, X, ldx, nb, 0};
+  ProfScope ps(c, "mf_solve", sets * 2.0 * fbytes, sets * 2.0 * 2.0 * (fbytes / 8.0) * nb);
+  const SolveSet s1{f1->perm.p, f1->iperm.p, f1->F.p, work.p, X1, ldx1};
+  const SolveSet s2 = sets == 2 ? SolveSet{f2->perm.p, f2->iperm.p, f2->F.p, work2.p, X2, ldx2} : s1;
+  SolveArgs a{fd, dofs.p, ea_map.p, piv_off.p, woff.p, B, ldb, {s1, s2}, nb, nb};
+  TiledArgs ta{fd, dofs.p, piv_off.p, woff.p, reinterpret_cast<const int4*>(pull.p), B, ldb, {s1, s2}, nb, 0};
   auto tiled = [&](bool fwd, int l, const int2* items, int ni) {
-    const int nt = tile_groups(ni, nb, c.num_sms);
+    const int nt = tile_groups(sets * ni, nb, c.num_sms);
     ta.chunk = std::max(16, std::min(kChunkK, ((fwd ? level_pmax[l] : level_kmax[l]) + 15) & ~15));
     const size_t smem = tile_smem(nt, ta.chunk);
-    const dim3 grid(ni, (nb + 8 * nt - 1) / (8 * nt));
+    const dim3 grid(ni, (nb + 8 * nt - 1) / (8 * nt), sets);
     if (fwd) {
       if (nt == 1) mf_forward_tiled_kernel<1><<<grid, kTileThreads, smem, st>>>(items, ta);
       else if (nt == 2) mf_forward_tiled_kernel<2><<<grid, kTileThreads, smem, st>>>(items, ta);
@@ -1911,9 +1937,9 @@ void MFDevice::solve(Ctx& c, const MFFactor& fac, const double* B, int64_t ldb, 
   };
   auto small = [&](bool fwd, int l, int ns) {
     const int cols = fwd ? level_fwd_cols[l] : level_bwd_cols[l];
-    const SmallShape s = small_shape(ns, cols, nb, c.num_sms);
+    const SmallShape s = small_shape(sets * ns, cols, nb, c.num_sms);
     a.per = s.per;
-    const dim3 grid(ns, (nb + s.per - 1) / s.per);
+    const dim3 grid(ns, (nb + s.per - 1) / s.per, sets);
     const size_t smem = (size_t)cols * s.per * sizeof(double);
     const int32_t* lf = lsmall.p + small_ptr[l];
     if (fwd) {
@@ -1938,10 +1964,12 @@ void MFDevice::solve(Ctx& c, const MFFactor& fac, const double* B, int64_t ldb, 
     const int ns = small_ptr[l + 1] - small_ptr[l], nl = large_ptr[l + 1] - large_ptr[l];
     if (ns > 0) small(true, l, ns);
     if (nl > 0) {
-      mf_forward_cluster_kernel<<<nl * CL, 256, 0, st>>>(llarge.p + large_ptr[l], fd, dofs.p, ea_map.p, fac.perm.p,
-                                                         fac.iperm.p, piv_off.p, woff.p, Fbuf.p, B, ldb, nb,
-                                                         work.p);
-      c.launches++;
+      for (int q = 0; q < sets; q++) {
+        const SolveSet& s = a.set[q];
+        mf_forward_cluster_kernel<<<nl * CL, 256, 0, st>>>(llarge.p + large_ptr[l], fd, dofs.p, ea_map.p, s.perm, s.iperm,
+                                                           piv_off.p, woff.p, s.F, B, ldb, nb, s.W);
+        c.launches++;
+      }
     }
   }
   for (int l = nlevels - 1; l >= 0; l--) {
@@ -1953,9 +1981,12 @@ void MFDevice::solve(Ctx& c, const MFFactor& fac, const double* B, int64_t ldb, 
     const int ns = small_ptr[l + 1] - small_ptr[l], nl = large_ptr[l + 1] - large_ptr[l];
     if (ns > 0) small(false, l, ns);
     if (nl > 0) {
-      mf_backward_cluster_kernel<<<nl * CL, 256, 0, st>>>(llarge.p + large_ptr[l], fd, dofs.p, woff.p, Fbuf.p,
-                                                          work.p, nb, X, ldx);
-      c.launches++;
+      for (int q = 0; q < sets; q++) {
+        const SolveSet& s = a.set[q];
+        mf_backward_cluster_kernel<<<nl * CL, 256, 0, st>>>(llarge.p + large_ptr[l], fd, dofs.p, woff.p, s.F, s.W, nb, s.X,
+                                                            s.ldx);
+        c.launches++;
+      }
     }
   }
   FEM2D_CUDA(cudaGetLastError());

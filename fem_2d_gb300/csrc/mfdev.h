@@ -37,7 +37,7 @@ struct MFDevice {
   DBuf<uint8_t> desc;
   DBuf<int32_t> lfronts, dofs, ea_map;
   DBuf<int64_t> asm_pos, asm_csr, piv_off, woff;
-  DBuf<double> work;
+  DBuf<double> work, work2;   // a workspace per factorization of a pair of solves
   DBuf<int> flags;
   DBuf<int32_t> weak_list;   // capacity n: weak-pivot DoFs recorded by the panel kernel
   DBuf<int> weak_count;
@@ -71,7 +71,14 @@ struct MFDevice {
   void factor(Ctx& c, const double* va, const double* vb, double ca, double cb, bool cholesky, MFFactor& out);
   // X = K^-1 B for an n x nb row-major block (nb <= nb_cap); B and X must not alias
   void solve(Ctx& c, const MFFactor& fac, const double* B, int64_t ldb, double* X, int64_t ldx, int nb);
+  // X1 = K1^-1 B and X2 = K2^-1 B in one pass over the levels (B may alias neither)
+  void solve_pair(Ctx& c, const MFFactor& f1, const MFFactor& f2, const double* B, int64_t ldb, double* X1, int64_t ldx1,
+                  double* X2, int64_t ldx2, int nb);
   int read_flags(Ctx& c);
+
+ private:
+  void solve_sets(Ctx& c, int sets, const MFFactor* f1, const MFFactor* f2, const double* B, int64_t ldb, double* X1,
+                  int64_t ldx1, double* X2, int64_t ldx2, int nb);
 };
 
 // The factorization plan of one GEP: the host symbolic phase and its device copy depend on the

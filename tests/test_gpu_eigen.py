@@ -110,3 +110,19 @@ def test_gpu_solve_precision_config(oracle_lib, ctx):
     ws, _, rs = ref.sparse_nearest_physical(A, B, w.target, w.n_pairs)
     assert np.max(np.abs(res.values - ws) / np.abs(ws)) <= EIG_TOL
     assert np.max(res.residuals) < 1e-9
+
+
+@pytest.mark.parametrize("target,k", [(10.0, 6), (2.6, 1), (30.0, 4), (-3.0, 3)])
+@pytest.mark.parametrize("opts", [{}, {"refine": 2}, {"damping": 0.05}, {"damping": 1.0}, {"damping": 4.0, "refine": -1}])
+def test_targets_and_dampings(oracle_lib, ctx, target, k, opts):
+    """The search operator in both forms: partial fractions (targets above zero), with and without
+    refinement and with dampings around |target|, and the product form (below zero, where with a damping of
+    one the two shifted matrices coincide)."""
+    w = configs.full_scale(seed=4, nx=5, ny=3, rounds=2, fraction=0.4, pmin=3, pmax=5, basis=1)
+    w.mesh_json = configs.grid_mesh_json(5, 3, 0.0, 1.87, 0.0, 1.0)
+    gep = _gep(w.mesh_json, w.ops, 1, w.glq, ctx)
+    A, B = gep.scipy()
+    ref, _ = oracle_lib.dense_nearest_physical(A, B, target, k)
+    r = fg.gpu_solve_gep_n(gep, target, k, **opts)
+    assert np.max(np.abs(r.values - ref) / np.abs(ref)) <= EIG_TOL
+    assert np.all(np.abs(np.einsum("ij,ij->i", r.vectors, (B @ r.vectors.T).T) - 1.0) < 1e-9)
