@@ -23,7 +23,7 @@ def sources():
 def _compile(src):
     obj = os.path.join(BUILD, src + ".o")
     path = os.path.join(CSRC, src)
-    deps = [path] + [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith(".h")]
+    deps = [path] + [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith((".h", ".cuh"))]
     deps.append(os.path.join(HERE, "..", "include", "fem2d_gb300.h"))
     if os.path.exists(obj) and os.path.getmtime(obj) >= max(os.path.getmtime(d) for d in deps):
         return obj

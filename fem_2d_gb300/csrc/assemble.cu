@@ -113,7 +113,7 @@ void device_assemble(Ctx& c, const HostGEP& g, DeviceGEP& d, float* ms_tables, f
   const int P = g.pmax + 1;
   FEM2D_CUDA(cudaEventRecord(e0, s));
   dim3 grid1(d.nivl, 2, 5);
-  fem2d_contract1d_kernel<<<grid1, 128, 0, s>>>(g.basis, P, d.nivl, d.ivl.p, d.glq.p, g.nq_u, g.nq_v, d.tables.p);
+  fem2d_contract1d_kernel<<<grid1, kTabThreads, 0, s>>>(g.basis, P, d.nivl, d.ivl.p, d.glq.p, g.nq_u, g.nq_v, d.tables.p);
   FEM2D_CUDA(cudaGetLastError());
   c.launches++;
   FEM2D_CUDA(cudaEventRecord(e1, s));
@@ -194,7 +194,7 @@ void device_values_noalloc(Ctx& c, const HostGEP& g, const DeviceGEP& d, double*
   // every table entry the values kernel reads is written by the contraction kernel first, so the
   // previous call's contents never leak into this one
   dim3 grid1(d.nivl, 2, 5);
-  fem2d_contract1d_kernel<<<grid1, 128, 0, c.stream>>>(g.basis, P, d.nivl, d.ivl.p, d.glq.p, g.nq_u, g.nq_v, tables);
+  fem2d_contract1d_kernel<<<grid1, kTabThreads, 0, c.stream>>>(g.basis, P, d.nivl, d.ivl.p, d.glq.p, g.nq_u, g.nq_v, tables);
   FEM2D_CUDA(cudaGetLastError());
   c.launches++;
   if (g.nnz_full > 0) {

@@ -150,7 +150,7 @@ void batch_assemble(Ctx& c, const std::vector<BatchMember>& members, bool autotu
   FEM2D_CUDA(cudaEventCreate(&e2));
   FEM2D_CUDA(cudaEventRecord(e0, c.stream));
   if (total_ivl > 0) {
-    fem2d_contract1d_batch_kernel<<<dim3((unsigned)total_ivl, 2, 5), 128, 0, c.stream>>>(di, ip.p, count);
+    fem2d_contract1d_batch_kernel<<<dim3((unsigned)total_ivl, 2, 5), kTabThreads, 0, c.stream>>>(di, ip.p, count);
     c.launches++;
     FEM2D_CUDA(cudaGetLastError());
   }

@@ -23,33 +23,72 @@ __device__ __forceinline__ int2 kind_families(int kind) {
 
 // One (interval, axis, kind) table of 1-D contractions, P x P entries, strided over the block's threads:
 //   G[a][b] = sum_m w_m X_a(s x_m + o) Y_b(x_m)            (glq.rs:19-32 restricted to one axis)
+// The shape functions are tabulated per chunk of points first (up to kTabP of them; evaluating two of them
+// per term, each a recurrence of FP64 operations, took 254 us for KOLeg tables of order 7 and 418 us for
+// order 8, against 0.2 and 2.6 ms of the values themselves).
+constexpr int kTabP = 24, kTabPts = 16, kTabThreads = 128;
 __device__ __forceinline__ void contract1d_table(int basis, int P, int nivl, int iv, int axis, int kind,
                                                  const double* __restrict__ ivl, const double* __restrict__ glq,
                                                  int nq_u, int nq_v, double* __restrict__ tables) {
+  __shared__ double tx[kTabPts][kTabP], ty[kTabPts][kTabP];
   const int nq = axis == 0 ? nq_u : nq_v;
   const double* xs = axis == 0 ? glq : glq + 2 * nq_u;
   const double* ws = xs + nq;
   const double s = ivl[2 * iv], o = ivl[2 * iv + 1];
   const int2 fam = kind_families(kind);
   double* out = tables + (((size_t)axis * nivl + iv) * 5 + kind) * P * P;
-  for (int t = threadIdx.x; t < P * P; t += blockDim.x) {
-    const int a = t / P, b = t % P;
-    double acc = 0.0;
-    for (int m = 0; m < nq; m++) {
-      const double x = xs[m];
-      acc += ws[m] * shape(basis, fam.x, a, s * x + o) * shape(basis, fam.y, b, x);
+  if (P > kTabP) {   // uniform
+    for (int t = threadIdx.x; t < P * P; t += blockDim.x) {
+      const int a = t / P, b = t % P;
+      double acc = 0.0;
+      for (int m = 0; m < nq; m++) {
+        const double x = xs[m];
+        acc += ws[m] * shape(basis, fam.x, a, s * x + o) * shape(basis, fam.y, b, x);
+      }
+      out[t] = acc;
     }
-    out[t] = acc;
+    return;
+  }
+  constexpr int kOut = (kTabP * kTabP + kTabThreads - 1) / kTabThreads;   // entries per thread (kTabThreads of them)
+  double acc[kOut];
+#pragma unroll
+  for (int i = 0; i < kOut; i++) acc[i] = 0.0;
+  for (int m0 = 0; m0 < nq; m0 += kTabPts) {
+    const int mc = min(kTabPts, nq - m0);
+    if (m0 > 0) __syncthreads();
+    for (int t = threadIdx.x; t < 2 * mc * P; t += blockDim.x) {
+      const bool second = t >= mc * P;
+      const int r = second ? t - mc * P : t, m = r / P, a = r - m * P;
+      const double x = xs[m0 + m];
+      if (second) ty[m][a] = shape(basis, fam.y, a, x);
+      else tx[m][a] = shape(basis, fam.x, a, s * x + o);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kOut; i++) {
+      const int t = threadIdx.x + i * kTabThreads;
+      if (t >= P * P) break;
+      const int a = t / P, b = t % P;
+      for (int m = 0; m < mc; m++) acc[i] += ws[m0 + m] * tx[m][a] * ty[m][b];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kOut; i++) {
+    const int t = threadIdx.x + i * kTabThreads;
+    if (t < P * P) out[t] = acc[i];
   }
 }
 
-// The value of one full CSR entry of A and B: the sum of its visits k0..k1-1, each the product
-// C * Gu * Gv that equals the reference's 2-D Gauss sum (integrals.rs:26-92, 292-354).
+// The value of one CSR entry of A and B: the sum of its visits k0..k1-1, each the product C * Gu * Gv that
+// equals the reference's 2-D Gauss sum (integrals.rs:26-92, 292-354). The FP64 pipe bounds the kernels that
+// call this (79% busy): the four direction pairs share one sequence of products, with the tables chosen by
+// index, since a warp of mixed pairs would run each branch's products, and the first visit is not added to
+// zero (nearly every entry has one visit).
 __device__ __forceinline__ void entry_values(int64_t k0, int64_t k1, const uint64_t* __restrict__ codes,
                                              const GBlock* __restrict__ blocks, const uint32_t* __restrict__ specs,
                                              const double* __restrict__ tables, int P, int nivl, double& out_a,
                                              double& out_b) {
-  const size_t PP = (size_t)P * P;
+  const int PP = P * P;
   const size_t axis_stride = (size_t)nivl * 5 * PP;
   double sa = 0.0, sb = 0.0;
   for (int64_t k = k0; k < k1; k++) {
@@ -61,26 +100,23 @@ __device__ __forceinline__ void entry_values(int64_t k0, int64_t k1, const uint6
     const uint32_t q = __ldg(specs + sp.y + (int)(code & 0xffff));
     const int pi = p & 0xff, pj = (p >> 8) & 0xff, pd = (p >> 16) & 0xff;
     const int qi = q & 0xff, qj = (q >> 8) & 0xff, qd = (q >> 16) & 0xff;
-    const double* gu = tables + (size_t)iv.x * 5 * PP + (size_t)pi * P + qi;
-    const double* gv = tables + axis_stride + (size_t)iv.y * 5 * PP + (size_t)pj * P + qj;
+    const double* gu = tables + (size_t)iv.x * 5 * PP + pi * P + qi;
+    const double* gv = tables + axis_stride + (size_t)iv.y * 5 * PP + pj * P + qj;
     const int dd = pd * 2 + qd;   // 0 UU, 1 UV, 2 VU, 3 VV
-    const double ca = __ldg(bl->ca + dd);
-    double va, vb = 0.0;
-    if (dd == 0) {
-      const double nn = __ldg(gu + G_NN * PP);
-      va = ca * nn * __ldg(gv + G_DD * PP);
-      vb = __ldg(bl->cb) * nn * __ldg(gv + G_TT * PP);
-    } else if (dd == 3) {
-      const double nn = __ldg(gv + G_NN * PP);
-      va = ca * __ldg(gu + G_DD * PP) * nn;
-      vb = __ldg(bl->cb + 1) * __ldg(gu + G_TT * PP) * nn;
-    } else if (dd == 1) {
-      va = ca * __ldg(gu + G_ND * PP) * __ldg(gv + G_DN * PP);
+    // curl-curl: UU (NN, DD), UV (ND, DN), VU (DN, ND), VV (DD, NN); mass: UU (NN, TT), VV (TT, NN)
+    const int ku = dd == 0 ? G_NN : dd == 1 ? G_ND : dd == 2 ? G_DN : G_DD;
+    const int kv = dd == 0 ? G_DD : dd == 1 ? G_DN : dd == 2 ? G_ND : G_NN;
+    const double va = __ldg(bl->ca + dd) * __ldg(gu + ku * PP) * __ldg(gv + kv * PP);
+    double vb = 0.0;
+    if (pd == qd)
+      vb = __ldg(bl->cb + pd) * __ldg(gu + (pd ? G_TT : G_NN) * PP) * __ldg(gv + (pd ? G_NN : G_TT) * PP);
+    if (k == k0) {
+      sa = va;
+      sb = vb;
     } else {
-      va = ca * __ldg(gu + G_DN * PP) * __ldg(gv + G_ND * PP);
+      sa += va;
+      sb += vb;
     }
-    sa += va;
-    sb += vb;
   }
   out_a = sa;
   out_b = sb;
