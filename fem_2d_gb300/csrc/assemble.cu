@@ -3,8 +3,8 @@
 // K1 fem2d_contract1d_kernel: the 1-D quadrature contractions (basis x quad-point x basis) between
 //    the shape-function families of an outer Elem sampled over a dyadic sub-interval and of the inner
 //    Elem (glq.rs:19-32 restricted to one axis; shape functions hierarchical_basis_fns.rs).
-// K2 fem2d_values_kernel: one thread per entry of the full symmetric CSR; sums its visits, each the
-//    product C * Gu * Gv that equals the reference's 2-D sum (integrals.rs:26-92, 292-354) for affine
+// K2 fem2d_values_kernel: one thread per upper-triangle entry; sums its visits into both full CSR entries,
+//    each visit the product C * Gu * Gv that equals the reference's 2-D sum (integrals.rs:26-92, 292-354) for affine
 //    Elems. FP64 throughout, deterministic (fixed summation order, no atomics). HBM-bound: the
 //    traffic is the contribution list read and the two FP64 value arrays written.
 #include <cuda_runtime.h>
@@ -27,19 +27,20 @@ __global__ void fem2d_contract1d_kernel(int basis, int P, int nivl, const double
   contract1d_table(basis, P, nivl, blockIdx.x, blockIdx.y, blockIdx.z, ivl, glq, nq_u, nq_v, tables);
 }
 
-__global__ void __launch_bounds__(256) fem2d_values_kernel(int64_t nnz, const int32_t* __restrict__ fsrc,
+// one thread per upper entry: its value goes to both full entries. The mirrored stores are scattered, but the
+// rows of one run fill the same lines one after the other while those are in L2; computing each full entry by
+// itself ran the FP64 products and the random reads of codes twice (120M entries: 1.88 ms)
+__global__ void __launch_bounds__(256) fem2d_values_kernel(int64_t nnz_upper, const EntryPos* __restrict__ upos,
                                                            const int64_t* __restrict__ vptr,
                                                            const uint64_t* __restrict__ codes,
                                                            const GBlock* __restrict__ blocks,
                                                            const uint32_t* __restrict__ specs,
                                                            const double* __restrict__ tables, int P, int nivl,
                                                            double* __restrict__ A, double* __restrict__ B) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < nnz_upper; u += (int64_t)gridDim.x * blockDim.x) {
     double sa, sb;
-    const int64_t u = __ldg(fsrc + e);   // the upper entry whose visits this entry sums
     entry_values(__ldg(vptr + u), __ldg(vptr + u + 1), codes, blocks, specs, tables, P, nivl, sa, sb);
-    A[e] = sa;
-    B[e] = sb;
+    store_entry(upos[u], sa, sb, A, B);
   }
 }
 
@@ -65,7 +66,7 @@ void device_upload(Ctx& c, const HostGEP& g, DeviceGEP& d) {
   d.arena.add(d.row_ptr, g.row_ptr);
   d.arena.add(d.col, g.col);
   d.arena.add(d.vptr, g.vptr);
-  d.arena.add(d.fsrc, g.fsrc);
+  d.arena.add(d.upos, g.upos);
   d.arena.add(d.codes, g.codes);
   d.arena.add(d.blocks, g.blocks);
   d.arena.add(d.specs, g.specs);
@@ -100,7 +101,7 @@ void device_upload(Ctx& c, const HostGEP& g, DeviceGEP& d) {
   d.arena.commit(s);
   d.ngrp = (int)grp.size() - 1;
   d.nwork = (int)work.size();
-  d.h2d_bytes = (int64_t)(grp.size() * 4 + work.size() * 8 + g.row_ptr.size() * 8 + g.col.size() * 4 + g.vptr.size() * 8 + g.fsrc.size() * 4 + g.codes.size() * 8 +
+  d.h2d_bytes = (int64_t)(grp.size() * 4 + work.size() * 8 + g.row_ptr.size() * 8 + g.col.size() * 4 + g.vptr.size() * 8 + g.upos.size() * 8 + g.codes.size() * 8 +
                           g.blocks.size() * sizeof(GBlock) + g.specs.size() * 4 + iv.size() * 8 + q.size() * 8);
 }
 
@@ -118,12 +119,12 @@ void device_assemble(Ctx& c, const HostGEP& g, DeviceGEP& d, float* ms_tables, f
   c.launches++;
   FEM2D_CUDA(cudaEventRecord(e1, s));
   if (g.nnz_full > 0) {
-    ProfScope ps(c, "assembly_values", 20.0 * g.nnz_full + 8.0 * (g.nnz_upper + 1) + 8.0 * g.codes.size());
+    ProfScope ps(c, "assembly_values", 16.0 * g.nnz_full + 16.0 * (g.nnz_upper + 1) + 8.0 * g.codes.size());
     const int threads = 256;
-    int64_t want = (g.nnz_full + threads - 1) / threads;
+    int64_t want = (g.nnz_upper + threads - 1) / threads;
     int64_t cap = (int64_t)c.num_sms * 8 * 4;   // persistent-ish grid: 8 blocks/SM x 4 waves
     int grid = (int)std::max<int64_t>(1, std::min(want, cap));
-    fem2d_values_kernel<<<grid, threads, 0, s>>>(g.nnz_full, d.fsrc.p, d.vptr.p, d.codes.p, d.blocks.p, d.specs.p,
+    fem2d_values_kernel<<<grid, threads, 0, s>>>(g.nnz_upper, d.upos.p, d.vptr.p, d.codes.p, d.blocks.p, d.specs.p,
                                                  d.tables.p, P, d.nivl, d.a.p, d.b.p);
     FEM2D_CUDA(cudaGetLastError());
     c.launches++;
@@ -199,10 +200,10 @@ void device_values_noalloc(Ctx& c, const HostGEP& g, const DeviceGEP& d, double*
   c.launches++;
   if (g.nnz_full > 0) {
     const int threads = 256;
-    int64_t want = (g.nnz_full + threads - 1) / threads;
+    int64_t want = (g.nnz_upper + threads - 1) / threads;
     int64_t cap = (int64_t)c.num_sms * 8 * 4;
     int grid = (int)std::max<int64_t>(1, std::min(want, cap));
-    fem2d_values_kernel<<<grid, threads, 0, c.stream>>>(g.nnz_full, d.fsrc.p, d.vptr.p, d.codes.p, d.blocks.p,
+    fem2d_values_kernel<<<grid, threads, 0, c.stream>>>(g.nnz_upper, d.upos.p, d.vptr.p, d.codes.p, d.blocks.p,
                                                         d.specs.p, tables, P, d.nivl, out_a, out_b);
     FEM2D_CUDA(cudaGetLastError());
     c.launches++;

@@ -29,7 +29,7 @@ namespace fem2d {
 namespace {
 
 struct BatchItem {
-  const int32_t* fsrc;
+  const EntryPos* upos;
   const int64_t* vptr;
   const uint64_t* codes;
   const GBlock* blocks;
@@ -66,12 +66,10 @@ __global__ void fem2d_values_batch_kernel(const BatchItem* __restrict__ items, c
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int it = find_item(nnz_pref, count, e);
     const BatchItem& b = items[it];
-    const int64_t local = e - __ldg(nnz_pref + it);
-    const int64_t u = __ldg(b.fsrc + local);
+    const int64_t u = e - __ldg(nnz_pref + it);
     double sa, sb;
     entry_values(__ldg(b.vptr + u), __ldg(b.vptr + u + 1), b.codes, b.blocks, b.specs, b.tables, b.P, b.nivl, sa, sb);
-    b.A[local] = sa;
-    b.B[local] = sb;
+    store_entry(b.upos[u], sa, sb, b.A, b.B);
   }
 }
 
@@ -107,11 +105,12 @@ void batch_assemble(Ctx& c, const std::vector<BatchMember>& members, bool autotu
   std::vector<BatchItem> items(count);
   std::vector<int64_t> nnz_pref(count + 1, 0), ivl_pref(count + 1, 0);
   int Pmax = 0;
+  int64_t total_full = 0;   // entries of the full CSRs: the size class of the autotuner's key
   for (int i = 0; i < count; i++) {
     const HostGEP& h = *members[i].h;
     DeviceGEP& d = *members[i].d;
     BatchItem& b = items[i];
-    b.fsrc = d.fsrc.p;
+    b.upos = d.upos.p;
     b.vptr = d.vptr.p;
     b.codes = d.codes.p;
     b.blocks = d.blocks.p;
@@ -127,7 +126,8 @@ void batch_assemble(Ctx& c, const std::vector<BatchMember>& members, bool autotu
     b.nq_u = h.nq_u;
     b.nq_v = h.nq_v;
     b.pad = 0;
-    nnz_pref[i + 1] = nnz_pref[i] + h.nnz_full;
+    nnz_pref[i + 1] = nnz_pref[i] + h.nnz_upper;
+    total_full += h.nnz_full;
     ivl_pref[i + 1] = ivl_pref[i] + d.nivl;
     Pmax = std::max(Pmax, b.P);
   }
@@ -158,7 +158,7 @@ void batch_assemble(Ctx& c, const std::vector<BatchMember>& members, bool autotu
 
   LaunchShape shape{256, 8};
   bool tuned = false;
-  const std::string key = tune_key(c.device, Pmax, total);
+  const std::string key = tune_key(c.device, Pmax, total_full);
   if (autotune && total > 0) {
     {
       std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -213,7 +213,7 @@ void batch_assemble(Ctx& c, const std::vector<BatchMember>& members, bool autotu
     rep->ms_tables = t1;
     rep->ms_values = t2;
     rep->shape = shape;
-    rep->total_entries = total;
+    rep->total_entries = total_full;
     int64_t codes = 0;
     for (const auto& m : members) codes += (int64_t)m.h->codes.size();
     rep->total_codes = codes;

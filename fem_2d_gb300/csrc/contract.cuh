@@ -79,7 +79,7 @@ __device__ __forceinline__ void contract1d_table(int basis, int P, int nivl, int
   }
 }
 
-// The value of one CSR entry of A and B: the sum of its visits k0..k1-1, each the product C * Gu * Gv that
+// The value of one upper-triangle entry of A and B: the sum of its visits k0..k1-1, each the product C * Gu * Gv that
 // equals the reference's 2-D Gauss sum (integrals.rs:26-92, 292-354). The FP64 pipe bounds the kernels that
 // call this (79% busy): the four direction pairs share one sequence of products, with the tables chosen by
 // index, since a warp of mixed pairs would run each branch's products, and the first visit is not added to
@@ -120,6 +120,17 @@ __device__ __forceinline__ void entry_values(int64_t k0, int64_t k1, const uint6
   }
   out_a = sa;
   out_b = sb;
+}
+
+// the value of an upper entry into the full CSR
+__device__ __forceinline__ void store_entry(EntryPos q, double va, double vb, double* __restrict__ A,
+                                            double* __restrict__ B) {
+  A[q.own] = va;
+  B[q.own] = vb;
+  if (q.mirror != q.own) {
+    A[q.mirror] = va;
+    B[q.mirror] = vb;
+  }
 }
 
 }  // namespace

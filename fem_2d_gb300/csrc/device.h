@@ -195,7 +195,8 @@ struct DArena {
 struct DeviceGEP {
   DArena arena;   // holds all of the buffers below
   DBuf<int64_t> row_ptr, vptr;
-  DBuf<int32_t> col, fsrc;
+  DBuf<int32_t> col;
+  DBuf<EntryPos> upos;
   DBuf<uint64_t> codes;
   DBuf<GBlock> blocks;
   DBuf<uint32_t> specs;

@@ -327,8 +327,8 @@ void build_symbolic(const Domain& d, int basis, int nq_u, int nq_v, HostGEP& g) 
   const int64_t nf = g.row_ptr[n];
   g.nnz_full = nf;
   g.col.resize(nf);
-  g.fsrc.resize(nf);
-  int32_t* src = g.fsrc.data();   // the upper entry of each full entry
+  g.upos.resize(nu);
+  EntryPos* upos = g.upos.data();   // the full entries of each upper entry (nf < 2^32, since nu < 2^31)
   parallel_for(n, [&](int64_t r0, int64_t r1) {
     for (int64_t r = r0; r < r1; r++) {
       int64_t o = g.row_ptr[r];
@@ -346,7 +346,7 @@ void build_symbolic(const Domain& d, int basis, int nq_u, int nq_v, HostGEP& g) 
         if (ucol[u] != r) {
           const int64_t p = pos[ucol[u]]++;
           g.col[p] = (int32_t)r;
-          src[p] = (int32_t)u;
+          upos[u].mirror = (uint32_t)p;
         }
   });
   parallel_for(n, [&](int64_t r0, int64_t r1) {
@@ -354,7 +354,8 @@ void build_symbolic(const Domain& d, int basis, int nq_u, int nq_v, HostGEP& g) 
       int64_t pos = g.row_ptr[r] + lcnt[r];
       for (int64_t u = uptr[r]; u < uptr[r + 1]; u++, pos++) {
         g.col[pos] = ucol[u];
-        src[pos] = (int32_t)u;
+        upos[u].own = (uint32_t)pos;
+        if (ucol[u] == r) upos[u].mirror = (uint32_t)pos;
       }
     }
   });

@@ -76,6 +76,10 @@ struct NoInitAlloc : std::allocator<T> {
 template <class T>
 using HostVec = std::vector<T, NoInitAlloc<T>>;
 
+struct alignas(8) EntryPos {   // positions in the full CSR
+  uint32_t own, mirror;
+};
+
 struct HostGEP {
   int64_t n = 0;                       // DoFs
   int64_t nnz_upper = 0, nnz_full = 0;
@@ -86,10 +90,10 @@ struct HostGEP {
   std::vector<int64_t> row_ptr;        // n + 1
   HostVec<int32_t> col;                // nnz_full
   // contributions: per upper-triangle entry u (rows in order, columns ascending within a row) its visit
-  // codes codes[vptr[u] .. vptr[u + 1]) in a fixed order; per full entry the upper entry it mirrors
-  // (an entry (r, c) and its transpose (c, r) sum the same visits)
+  // codes codes[vptr[u] .. vptr[u + 1]) in a fixed order, and the two full entries that take its value, (r, c)
+  // and (c, r) (the same one on the diagonal)
   HostVec<int64_t> vptr;               // nnz_upper + 1
-  HostVec<int32_t> fsrc;               // nnz_full
+  HostVec<EntryPos> upos;              // nnz_upper
   HostVec<uint64_t> codes;             // visits
   // visit blocks, packed specs, intervals
   std::vector<GBlock> blocks;
