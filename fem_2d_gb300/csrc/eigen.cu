@@ -110,7 +110,9 @@ __global__ void __launch_bounds__(256) spmm_kernel(int64_t n, const int64_t* __r
 // values ca*A + cb*B (rows x 48, each row's entries read contiguously) in shared memory, accumulates
 // every (row, column) output from shared memory only, and adds its partial sums to Y (zeroed before
 // the launch) with FP64 atomics. X is gathered once per run instead of once per row. Up to 64 rows x
-// 32 columns = 8 outputs per thread.
+// 32 columns = 8 outputs per thread. One CTA per item, taken as CTAs finish: items differ tenfold in work, and
+// dealing them out over six CTAs per SM in turn left SMs idle (18.4M entries x 20 columns, both matrices:
+// 1.15 ms, now 0.81, against 0.70 ms for the products at the FP64 pipe's rate).
 constexpr int kGrpChunk = 48;
 constexpr int kGrpRows = 64;
 constexpr int kGrpSeg = 256;
@@ -120,7 +122,7 @@ __global__ void zero_block_kernel(int64_t n, int nb, double* __restrict__ Y, int
     Y[(t / nb) * ldy + t % nb] = 0.0;
 }
 
-__global__ void __launch_bounds__(256) spmm_group_kernel(int nwork, const int2* __restrict__ work,
+__global__ void __launch_bounds__(256) spmm_group_kernel(const int2* __restrict__ work,
                                                          const int32_t* __restrict__ grp,
                                                          const int64_t* __restrict__ rp,
                                                          const int32_t* __restrict__ col,
@@ -129,53 +131,53 @@ __global__ void __launch_bounds__(256) spmm_group_kernel(int nwork, const int2* 
                                                          int64_t ldx, int nb, double* __restrict__ Y, int64_t ldy) {
   __shared__ double xs[kGrpChunk * 32];
   __shared__ double vs[kGrpRows * (kGrpChunk + 1)];
-  for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
-    const int2 it = work[w];
-    const int r0 = grp[it.x], R = grp[it.x + 1] - r0;
-    const int64_t c0 = rp[r0];
-    const int cend = min((int)(rp[r0 + 1] - c0), it.y + kGrpSeg);
-    const int32_t* cols = col + c0;
-    double acc[8];
+  const int2 it = work[blockIdx.x];
+  const int r0 = grp[it.x], R = grp[it.x + 1] - r0;
+  const int64_t c0 = rp[r0];
+  const int cend = min((int)(rp[r0 + 1] - c0), it.y + kGrpSeg);
+  const int32_t* cols = col + c0;
+  double acc[8];
 #pragma unroll
-    for (int o = 0; o < 8; o++) acc[o] = 0.0;
-    for (int q0 = it.y; q0 < cend; q0 += kGrpChunk) {
-      const int qn = min(kGrpChunk, cend - q0);
-      __syncthreads();
-      for (int t = threadIdx.x; t < qn * nb; t += blockDim.x) {
-        const int q = t / nb, j = t - q * nb;
-        xs[q * 32 + j] = __ldg(X + (int64_t)__ldg(cols + q0 + q) * ldx + j);
-      }
-      for (int t = threadIdx.x; t < R * kGrpChunk; t += blockDim.x) {
-        const int r = t / kGrpChunk, q = t - r * kGrpChunk;
-        double v = 0.0;
-        if (q < qn) {
-          const int64_t k = rp[r0 + r] + q0 + q;
-          if (ca != 0.0) v += ca * __ldg(va + k);
-          if (cb != 0.0) v += cb * __ldg(vb + k);
-        }
-        vs[r * (kGrpChunk + 1) + q] = v;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int o = 0; o < 8; o++) {
-        const int t = threadIdx.x + o * 256;
-        if (t < R * nb) {
-          const int r = t / nb, j = t - r * nb;
-          const double* vr = vs + r * (kGrpChunk + 1);
-          double s = acc[o];
-#pragma unroll 8
-          for (int q = 0; q < qn; q++) s += vr[q] * xs[q * 32 + j];
-          acc[o] = s;
-        }
-      }
+  for (int o = 0; o < 8; o++) acc[o] = 0.0;
+  for (int q0 = it.y; q0 < cend; q0 += kGrpChunk) {
+    const int qn = min(kGrpChunk, cend - q0);
+    __syncthreads();
+    for (int t = threadIdx.x; t < qn * nb; t += blockDim.x) {
+      const int q = t / nb, j = t - q * nb;
+      xs[q * 32 + j] = __ldg(X + (int64_t)__ldg(cols + q0 + q) * ldx + j);
     }
+    for (int t = threadIdx.x; t < R * kGrpChunk; t += blockDim.x) {
+      const int r = t / kGrpChunk, q = t - r * kGrpChunk;
+      double v = 0.0;
+      if (q < qn) {
+        const int64_t k = rp[r0 + r] + q0 + q;
+        // (a coefficient of one, the usual case, costs no FP64 operation per entry)
+        if (ca == 1.0) v = __ldg(va + k);
+        else if (ca != 0.0) v = ca * __ldg(va + k);
+        if (cb != 0.0) v += cb * __ldg(vb + k);
+      }
+      vs[r * (kGrpChunk + 1) + q] = v;
+    }
+    __syncthreads();
 #pragma unroll
     for (int o = 0; o < 8; o++) {
       const int t = threadIdx.x + o * 256;
       if (t < R * nb) {
         const int r = t / nb, j = t - r * nb;
-        atomicAdd(Y + (int64_t)(r0 + r) * ldy + j, acc[o]);
+        const double* vr = vs + r * (kGrpChunk + 1);
+        double s = acc[o];
+#pragma unroll 8
+        for (int q = 0; q < qn; q++) s += vr[q] * xs[q * 32 + j];
+        acc[o] = s;
       }
+    }
+  }
+#pragma unroll
+  for (int o = 0; o < 8; o++) {
+    const int t = threadIdx.x + o * 256;
+    if (t < R * nb) {
+      const int r = t / nb, j = t - r * nb;
+      atomicAdd(Y + (int64_t)(r0 + r) * ldy + j, acc[o]);
     }
   }
 }
@@ -571,8 +573,7 @@ struct Dev {
     if (d.nwork > 0 && nb <= 32) {
       const int64_t zb = std::min<int64_t>((h.n * nb + 255) / 256, (int64_t)c.num_sms * 8);
       zero_block_kernel<<<(int)std::max<int64_t>(zb, 1), 256, 0, c.stream>>>(h.n, nb, Y, ldy);
-      const int grid = std::max(1, std::min(d.nwork, c.num_sms * 6));
-      spmm_group_kernel<<<grid, 256, 0, c.stream>>>(d.nwork, d.gwork.p, d.grp.p, d.row_ptr.p, d.col.p, va, vb, ca,
+            spmm_group_kernel<<<d.nwork, 256, 0, c.stream>>>(d.gwork.p, d.grp.p, d.row_ptr.p, d.col.p, va, vb, ca,
                                                     cb, X, ldx, nb, Y, ldy);
       c.launches += 2;
       return;
