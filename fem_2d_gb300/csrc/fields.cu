@@ -6,7 +6,10 @@
 // ancestor's specs and their solution coefficients in shared memory, and every thread accumulates
 // its grid points in registers in the reference's order (ancestors, then specs). The products are
 // formed as the reference writes them, ((jac_inv * N) * T) * coefficient, with separate rounded
-// multiplies and adds.
+// multiplies and adds. The FP64 pipe bounds it, so jac_inv is tabulated with the u factor (three operations per spec
+// and point instead of four) and only the orders that the ancestor's specs have are tabulated (an ancestor
+// holds a few edge functions; tables of the mesh's largest order cost as much as its sums). 1,752 Elems of
+// orders 3 to 8, 16 x 15 points: 304 -> 214 us.
 #include <algorithm>
 
 #include "fields.h"
@@ -16,12 +19,12 @@ namespace fem2d {
 
 namespace {
 
-constexpr int kFieldThreads = 128;
+constexpr int kFieldMaxThreads = 128;   // fewer for grids that fewer threads cover
 constexpr int kFieldPts = 2;        // grid points per thread per pass
 constexpr int kSpecChunk = 256;     // specs staged per shared-memory pass
 
-__global__ void __launch_bounds__(kFieldThreads)
-fem2d_xy_fields_kernel(const FieldItem* __restrict__ items, const int32_t* __restrict__ item_ptr,
+template <int kFieldThreads>
+__global__ void __launch_bounds__(kFieldThreads) fem2d_xy_fields_kernel(const FieldItem* __restrict__ items, const int32_t* __restrict__ item_ptr,
                        const uint32_t* __restrict__ codes, const int32_t* __restrict__ dofs,
                        const double* __restrict__ sol, int basis, int d0, int d1, int imax, int jmax,
                        int64_t nleaves, double* __restrict__ ox, double* __restrict__ oy) {
@@ -56,13 +59,13 @@ fem2d_xy_fields_kernel(const FieldItem* __restrict__ items, const int32_t* __res
       for (int it = it0; it < it1; it++) {
         const FieldItem I = items[it];
         __syncthreads();   // the previous item's tables and specs are consumed
-        for (int k = tid; k < tu; k += kFieldThreads) {
+        for (int k = tid; k < (I.imax + 1) * d0; k += kFieldThreads) {
           const int a = k / d0, m = k % d0;
           const double u = __dadd_rn(__dmul_rn(__dadd_rn(__dmul_rn((double)m, stepu), -1.0), I.su), I.ou);
-          Nu[k] = shape(basis, 0, a, u);
-          Tu[k] = shape(basis, 2, a, u);
+          Nu[k] = __dmul_rn(I.jiu, shape(basis, 0, a, u));
+          Tu[k] = __dmul_rn(I.jiv, shape(basis, 2, a, u));
         }
-        for (int k = tid; k < tv; k += kFieldThreads) {
+        for (int k = tid; k < (I.jmax + 1) * d1; k += kFieldThreads) {
           const int b = k / d1, n = k % d1;
           const double v = __dadd_rn(__dmul_rn(__dadd_rn(__dmul_rn((double)n, stepv), -1.0), I.sv), I.ov);
           Nv[k] = shape(basis, 0, b, v);
@@ -83,13 +86,13 @@ fem2d_xy_fields_kernel(const FieldItem* __restrict__ items, const int32_t* __res
             if (dir == 0) {   // f_u: jac_inv.u * N_i(u) * T_j(v)   (basis.rs:225-228)
 #pragma unroll
               for (int q = 0; q < kFieldPts; q++) {
-                const double f = __dmul_rn(__dmul_rn(I.jiu, Nu[i * d0 + pm[q]]), Tv[j * d1 + pn[q]]);
+                const double f = __dmul_rn(Nu[i * d0 + pm[q]], Tv[j * d1 + pn[q]]);
                 ax[q] = __dadd_rn(ax[q], __dmul_rn(f, s));
               }
             } else if (dir == 1) {   // f_v: jac_inv.v * T_i(u) * N_j(v)   (basis.rs:230-233)
 #pragma unroll
               for (int q = 0; q < kFieldPts; q++) {
-                const double f = __dmul_rn(__dmul_rn(I.jiv, Tu[i * d0 + pm[q]]), Nv[j * d1 + pn[q]]);
+                const double f = __dmul_rn(Tu[i * d0 + pm[q]], Nv[j * d1 + pn[q]]);
                 ay[q] = __dadd_rn(ay[q], __dmul_rn(f, s));
               }
             }
@@ -163,6 +166,11 @@ void fields_plan(Ctx& c, const Domain& d, int basis, int d0, int d1, FieldSpace&
       I.jiv = jac[a].ji_v1;
       I.sp0 = (int32_t)d.spec_ptr[a];
       I.sp1 = (int32_t)d.spec_ptr[a + 1];
+      I.imax = I.jmax = -1;
+      for (int32_t k = I.sp0; k < I.sp1; k++) {
+        I.imax = std::max<int32_t>(I.imax, d.specs[k].i);
+        I.jmax = std::max<int32_t>(I.jmax, d.specs[k].j);
+      }
       f.h_items.push_back(I);
     }
     f.h_item_ptr.push_back((int32_t)f.h_items.size());
@@ -182,8 +190,12 @@ void fields_plan(Ctx& c, const Domain& d, int basis, int d0, int d1, FieldSpace&
   f.codes.upload(codes, c.stream);
   f.dofs.upload(dofs, c.stream);
   f.h2d_bytes = (int64_t)(f.h_items.size() * sizeof(FieldItem) + f.h_item_ptr.size() * 4 + codes.size() * 8);
-  FEM2D_CUDA(cudaFuncSetAttribute(fem2d_xy_fields_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)std::max<size_t>(f.smem, 48 * 1024)));
+  auto allow = [&](auto k) {
+    FEM2D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(f.smem, 48 * 1024)));
+  };
+  allow(fem2d_xy_fields_kernel<32>);
+  allow(fem2d_xy_fields_kernel<64>);
+  allow(fem2d_xy_fields_kernel<kFieldMaxThreads>);
   FEM2D_CUDA(cudaStreamSynchronize(c.stream));
 }
 
@@ -197,9 +209,16 @@ void fields_eval(FieldSpace& f, const double* d_solution, double* d_x, double* d
   for (const FieldItem& I : f.h_items) spec_visits += I.sp1 - I.sp0;
   const double bytes = 16.0 * P * nl + sizeof(FieldItem) * f.h_items.size() + 16.0 * spec_visits;
   ProfScope ps(c, "xy_fields", bytes);
-  const int64_t grid = std::min<int64_t>(nl, (int64_t)std::max(c.num_sms, 1) * 16);
-  fem2d_xy_fields_kernel<<<(unsigned)grid, kFieldThreads, f.smem, c.stream>>>(
-      f.items.p, f.item_ptr.p, f.codes.p, f.dofs.p, d_solution, f.basis, f.d0, f.d1, f.imax, f.jmax, nl, d_x, d_y);
+  const int64_t grid = std::min<int64_t>(nl, (int64_t)std::max(c.num_sms, 1) * 64);
+  auto launch = [&](auto k, int threads) {
+    k<<<(unsigned)grid, threads, f.smem, c.stream>>>(f.items.p, f.item_ptr.p, f.codes.p, f.dofs.p, d_solution, f.basis, f.d0,
+                                                     f.d1, f.imax, f.jmax, nl, d_x, d_y);
+  };
+  // as many threads as the grid's points need (two each): at 3 x 3 points 128 threads left all but five idle
+  const int points = f.d0 * f.d1;
+  if (points <= 32 * kFieldPts) launch(fem2d_xy_fields_kernel<32>, 32);
+  else if (points <= 64 * kFieldPts) launch(fem2d_xy_fields_kernel<64>, 64);
+  else launch(fem2d_xy_fields_kernel<kFieldMaxThreads>, kFieldMaxThreads);
   FEM2D_CUDA(cudaGetLastError());
   c.launches++;
 }

@@ -19,6 +19,7 @@ struct alignas(16) FieldItem {
   double su, ou, sv, ov;   // leaf parametric point x -> ancestor point x * s + o, per axis
   double jiu, jiv;         // ancestor inverse-Jacobian diagonal (jac_inv.u.x, jac_inv.v.y)
   int32_t sp0, sp1;        // the ancestor's spec range in the Domain's spec order
+  int32_t imax, jmax;      // largest orders among those specs (-1 without specs)
 };
 
 struct FieldSpace {

@@ -145,3 +145,21 @@ def test_fields_errors(ctx):
     dev = ufs._device(fg.HierPoly)
     with pytest.raises(fg.Fem2dError, match="does not match solution size"):
         dev.xy(np.zeros(3), 4, 4)
+
+
+@pytest.mark.parametrize("grid", [(2, 2), (3, 3), (8, 8), (13, 5), (9, 15), (16, 16), (24, 23)])
+def test_grid_sizes_agree(ctx, grid):
+    """Grids around the thread counts of the kernel: the corner points, which every grid has, are the same bit
+    for bit (same operations in the same order whatever the grid)."""
+    dom = fg.Domain.from_mesh(configs.build_mesh(configs.full_scale(seed=8, nx=4, ny=3, rounds=3, fraction=0.4, pmin=1,
+                                                                    pmax=6)))
+    u = np.random.default_rng(3).standard_normal(dom.num_dofs)
+    for basis in (fg.HierPoly, fg.KOLeg):
+        out = []
+        for densities in (grid, (12, 11)):
+            space = fg.UniformFieldSpace(dom, densities, ctx=ctx)
+            names = space.xy_fields(basis, "e", u)
+            out.append([space.quantity(q)[:, ::densities[0] - 1, ::densities[1] - 1] for q in names])
+        for a, b in zip(*out):
+            assert np.array_equal(a[:, 0, 0], b[:, 0, 0])
+            assert np.allclose(a, b, rtol=0, atol=1e-12 * np.max(np.abs(b)))
