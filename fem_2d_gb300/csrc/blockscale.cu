@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "blockscale.h"
+#include "dmma.h"
 
 namespace fem2d {
 
@@ -23,18 +24,23 @@ namespace {
 
 constexpr int kRun = 64;   // rows per run (the runs of device_upload are at most 64 long)
 
-// per run: Cholesky of B_gg in shared memory, then S_g = L^-1 (row-major, lower) to global
-__global__ void __launch_bounds__(256) run_cholinv_kernel(const int32_t* __restrict__ grp,
+// per listed run of at most LD rows: Cholesky of B_gg in shared memory, then S_g = L^-1 (row-major, lower) to
+// global. Runs of up to kSmallRun rows (60% of them at 1M DoFs) take small CTAs of their own: at the
+// 64 KB of the long ones three fit an SM.
+constexpr int kSmallRun = 16;
+template <int LD>
+__global__ void __launch_bounds__(4 * LD) run_cholinv_kernel(const int32_t* __restrict__ list,
+                                                          const int32_t* __restrict__ grp,
                                                           const int64_t* __restrict__ rp,
                                                           const int32_t* __restrict__ col,
                                                           const double* __restrict__ vb,
                                                           const int64_t* __restrict__ soff,
                                                           double* __restrict__ S, int* __restrict__ flag) {
   extern __shared__ double csm[];
-  double* M = csm;                 // kRun x kRun
-  double* Li = csm + kRun * kRun;  // kRun x kRun
+  double* M = csm;                 // LD x LD
+  double* Li = csm + LD * LD;  // LD x LD
   __shared__ int s_off;
-  const int g = blockIdx.x;
+  const int g = list[blockIdx.x];
   const int g0 = grp[g], R = grp[g + 1] - g0;
   if (threadIdx.x == 0) {   // position of column g0 in row g0 (every row of the run has the same list)
     int lo = 0, hi = (int)(rp[g0 + 1] - rp[g0]) - 1, at = -1;
@@ -51,102 +57,120 @@ __global__ void __launch_bounds__(256) run_cholinv_kernel(const int32_t* __restr
   if (s_off < 0) return;
   for (int t = threadIdx.x; t < R * R; t += blockDim.x) {
     const int r = t / R, q = t % R;
-    M[r * kRun + q] = vb[rp[g0 + r] + s_off + q];
+    M[r * LD + q] = vb[rp[g0 + r] + s_off + q];
   }
   __syncthreads();
   for (int j = 0; j < R; j++) {   // right-looking Cholesky, lower triangle
     if (threadIdx.x == 0) {
-      const double d = M[j * kRun + j];
+      const double d = M[j * LD + j];
       if (!(d > 0.0)) atomicOr(flag, 1);
-      M[j * kRun + j] = d > 0.0 ? sqrt(d) : 1.0;
+      M[j * LD + j] = d > 0.0 ? sqrt(d) : 1.0;
     }
     __syncthreads();
-    const double dj = M[j * kRun + j];
-    for (int i = j + 1 + threadIdx.x; i < R; i += blockDim.x) M[i * kRun + j] /= dj;
+    const double dj = M[j * LD + j];
+    for (int i = j + 1 + threadIdx.x; i < R; i += blockDim.x) M[i * LD + j] /= dj;
     __syncthreads();
     for (int t = threadIdx.x; t < (R - j - 1) * (R - j - 1); t += blockDim.x) {
       const int i = j + 1 + t / (R - j - 1), k = j + 1 + t % (R - j - 1);
-      if (k <= i) M[i * kRun + k] -= M[i * kRun + j] * M[k * kRun + j];
+      if (k <= i) M[i * LD + k] -= M[i * LD + j] * M[k * LD + j];
     }
     __syncthreads();
   }
   // column q of L^-1 per thread: L x = e_q
   for (int q = threadIdx.x; q < R; q += blockDim.x) {
-    for (int i = 0; i < q; i++) Li[i * kRun + q] = 0.0;
-    Li[q * kRun + q] = 1.0 / M[q * kRun + q];
+    for (int i = 0; i < q; i++) Li[i * LD + q] = 0.0;
+    Li[q * LD + q] = 1.0 / M[q * LD + q];
     for (int i = q + 1; i < R; i++) {
       double s = 0.0;
-      for (int k = q; k < i; k++) s += M[i * kRun + k] * Li[k * kRun + q];
-      Li[i * kRun + q] = -s / M[i * kRun + i];
+      for (int k = q; k < i; k++) s += M[i * LD + k] * Li[k * LD + q];
+      Li[i * LD + q] = -s / M[i * LD + i];
     }
   }
   __syncthreads();
   double* out = S + soff[g];
-  for (int t = threadIdx.x; t < R * R; t += blockDim.x) out[t] = Li[(t / R) * kRun + t % R];
+  for (int t = threadIdx.x; t < R * R; t += blockDim.x) out[t] = Li[(t / R) * LD + t % R];
 }
 
-// per run g and each column run h of its pattern: block <- S_g block S_h^T, for A and B (256 threads)
+// Per run g and matrix (blockIdx.y: A, B): block <- S_g block S_h^T for every column run h of its pattern, both
+// factors lower triangular, as FP64 MMAs on 8 x 8 tiles: U = block S_h^T with all operands read straight into
+// the fragments (rows of the CSR and of S are contiguous), U kept in shared memory, then S_g U. The column
+// runs go in groups of up to kGroupTiles tiles, so that the many runs of 4 to 8 functions fill the eight warps
+// together. One column run at a time through shared memory, with six barriers each, took 31.5 ms at 1M DoFs;
+// now 28, of which the FP64 pipe needs 20 (26 with the tiles' padding). Loading whole tiles ahead of their
+// products was slower (33 ms).
 constexpr int kTransformThreads = 256;
-constexpr int kT1Regs = kRun * kRun / kTransformThreads;
-__global__ void __launch_bounds__(kTransformThreads) run_transform_kernel(const int32_t* __restrict__ grp,
-                                                            const int64_t* __restrict__ rp,
-                                                            const int64_t* __restrict__ seg_ptr,
-                                                            const int2* __restrict__ seg,
-                                                            const int64_t* __restrict__ soff,
-                                                            const double* __restrict__ S,
-                                                            const double* __restrict__ va,
-                                                            const double* __restrict__ vb, double* __restrict__ sa,
-                                                            double* __restrict__ sb) {
-  extern __shared__ double smem[];
-  double* Sg = smem;                    // R x R
-  double* ShT = Sg + kRun * kRun;       // H x H, transposed: ShT[k H + q] = S_h[q][k]
-  double* Blk = ShT + kRun * kRun;      // R x H: the block, then T1 = S_g Blk in its place
-  const int g = blockIdx.x;
-  const int g0 = grp[g], R = grp[g + 1] - g0;
-  for (int t = threadIdx.x; t < R * R; t += blockDim.x) Sg[t] = S[soff[g] + t];
-  for (int64_t sgi = seg_ptr[g]; sgi < seg_ptr[g + 1]; sgi++) {
-    const int2 sh = seg[sgi];   // (column run h, offset of its first column in the rows of g)
-    const int h0 = grp[sh.x], H = grp[sh.x + 1] - h0;
-    __syncthreads();
-    // S_h is stored transposed so that the lanes of the second product (consecutive q) read consecutive
-    // doubles (row-major S_h would put all 32 lanes of a warp in one bank for H = 64)
-    for (int t = threadIdx.x; t < H * H; t += blockDim.x) ShT[(t % H) * H + t / H] = S[soff[sh.x] + t];
-    for (int m = 0; m < 2; m++) {
-      const double* src = m == 0 ? va : vb;
-      double* dst = m == 0 ? sa : sb;
-      __syncthreads();
-      for (int t = threadIdx.x; t < R * H; t += blockDim.x) {
-        const int r = t / H, q = t % H;
-        Blk[t] = src[rp[g0 + r] + sh.y + q];
-      }
-      __syncthreads();
-      // T1 = S_g Blk (S_g lower), held in registers (at most 16 entries a thread: 64 x 64 over 256
-      // threads) and written over Blk once every thread has read it: two CTAs fit an SM
-      double t1[kT1Regs];
-#pragma unroll
-      for (int i = 0; i < kT1Regs; i++) {
-        const int t = threadIdx.x + kTransformThreads * i;
-        t1[i] = 0.0;
-        if (t < R * H) {
-          const int r = t / H, q = t % H;
-          double s = 0.0;
-          for (int k = 0; k <= r; k++) s += Sg[r * R + k] * Blk[k * H + q];
-          t1[i] = s;
+constexpr int kGroupTiles = 12;
+constexpr int kUld = 8 * kGroupTiles + 4;   // rows 4 banks apart: fragments read without conflicts
+constexpr int kTransformSmem = kRun * kUld * (int)sizeof(double);
+__global__ void __launch_bounds__(kTransformThreads) run_transform_kernel(
+    const int32_t* __restrict__ grp, const int64_t* __restrict__ rp, const int64_t* __restrict__ seg_ptr,
+    const int2* __restrict__ seg, const int64_t* __restrict__ soff, const double* __restrict__ S,
+    const double* __restrict__ va, const double* __restrict__ vb, double* __restrict__ sa, double* __restrict__ sb) {
+  extern __shared__ double U[];
+  __shared__ int64_t tile_s[kGroupTiles];                               // S_h of the tile's column run
+  __shared__ int tile_h[kGroupTiles], tile_c[kGroupTiles], tile_j[kGroupTiles];   // its order, first column, tile in it
+  __shared__ int ntiles;
+  __shared__ int64_t next;
+  const double* src = blockIdx.y == 0 ? va : vb;
+  double* dst = blockIdx.y == 0 ? sa : sb;
+  const int g = blockIdx.x, g0 = grp[g], R = grp[g + 1] - g0, strips = (R + 7) >> 3;
+  const double* Sg = S + soff[g];
+  const int64_t r0 = rp[g0], len = rp[g0 + 1] - r0;   // the run's rows follow each other, len entries each
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q8 = lane >> 2, kl = lane & 3;
+  const int64_t end = seg_ptr[g + 1];
+  for (int64_t first = seg_ptr[g]; first < end; first = next) {
+    __syncthreads();   // U and the tile list of the previous group are read
+    if (threadIdx.x == 0) {
+      int n = 0;
+      int64_t s = first;
+      for (; s < end; s++) {
+        const int2 sh = seg[s];
+        const int H = grp[sh.x + 1] - grp[sh.x], ht = (H + 7) >> 3;
+        if (n + ht > kGroupTiles) break;   // (a column run has at most 8 tiles: every group makes progress)
+        for (int j = 0; j < ht; j++, n++) {
+          tile_s[n] = soff[sh.x];
+          tile_h[n] = H;
+          tile_c[n] = sh.y;
+          tile_j[n] = j;
         }
       }
-      __syncthreads();
-#pragma unroll
-      for (int i = 0; i < kT1Regs; i++) {
-        const int t = threadIdx.x + kTransformThreads * i;
-        if (t < R * H) Blk[t] = t1[i];
+      ntiles = n;
+      next = s;
+    }
+    __syncthreads();
+    const int nt = ntiles;
+    // U = block S_h^T: tile (strip i, tile j of h) sums the block's columns up to tile j
+    for (int w = warp; w < strips * nt; w += kTransformThreads / 32) {
+      const int i = w % strips, c = w / strips, H = tile_h[c], j = tile_j[c];
+      const double* Sh = S + tile_s[c];
+      const int row = 8 * i + q8, col = 8 * j + q8;
+      const double* a = src + r0 + (int64_t)row * len + tile_c[c];
+      double acc[2] = {0.0, 0.0};
+      for (int k0 = 0; k0 <= 8 * j + 4; k0 += 4) {
+        const int k = k0 + kl;
+        const double x = (row < R && k < H) ? __ldg(a + k) : 0.0;
+        const double y = (col < H && k <= col) ? __ldg(Sh + (int64_t)col * H + k) : 0.0;   // S_h[col][k]
+        dmma(acc, x, y);
       }
-      __syncthreads();
-      for (int t = threadIdx.x; t < R * H; t += blockDim.x) {   // out = T1 S_h^T (S_h lower)
-        const int r = t / H, q = t % H;
-        double s = 0.0;
-        for (int k = 0; k <= q; k++) s += Blk[r * H + k] * ShT[k * H + q];
-        dst[rp[g0 + r] + sh.y + q] = s;
+      double* u = U + row * kUld + 8 * c + 2 * kl;
+      u[0] = acc[0];
+      u[1] = acc[1];
+    }
+    __syncthreads();
+    // out = S_g U
+    for (int w = warp; w < strips * nt; w += kTransformThreads / 32) {
+      const int i = w % strips, c = w / strips;
+      const int row = 8 * i + q8;
+      double acc[2] = {0.0, 0.0};
+      for (int k0 = 0; k0 <= 8 * i + 4; k0 += 4) {
+        const int k = k0 + kl;
+        const double x = (row < R && k <= row) ? __ldg(Sg + row * R + k) : 0.0;
+        dmma(acc, x, U[k * kUld + 8 * c + q8]);
       }
+      const int col = 8 * tile_j[c] + 2 * kl;
+      double* o = dst + r0 + (int64_t)row * len + tile_c[c] + col;
+      if (row < R && col < tile_h[c]) o[0] = acc[0];
+      if (row < R && col + 1 < tile_h[c]) o[1] = acc[1];
     }
   }
 }
@@ -204,6 +228,11 @@ void BlockScale::build(Ctx& c, const HostGEP& h, const DeviceGEP& d, double* sa,
       sp[g + 1] = (int64_t)sg.size();
     }
     // kept in the GEP's plan across solves: plain (not stream-ordered) allocations
+    std::vector<int32_t> runs[2];   // short, long
+    for (int g = 0; g < ngrp; g++) runs[grp[g + 1] - grp[g] > kSmallRun].push_back(g);
+    nshort = (int)runs[0].size();
+    runs[0].insert(runs[0].end(), runs[1].begin(), runs[1].end());
+    list.upload(runs[0], c.stream);
     grp_d.upload(grp, c.stream);
     soff.upload(so, c.stream);
     seg_ptr.upload(sp, c.stream);
@@ -220,17 +249,21 @@ void BlockScale::build(Ctx& c, const HostGEP& h, const DeviceGEP& d, double* sa,
   {
     std::lock_guard<std::mutex> lk(mu);
     if (c.device >= 0 && c.device < 256 && !attr[c.device]) {
-      FEM2D_CUDA(cudaFuncSetAttribute(run_cholinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      FEM2D_CUDA(cudaFuncSetAttribute(run_cholinv_kernel<kRun>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       2 * kRun * kRun * (int)sizeof(double)));
       FEM2D_CUDA(cudaFuncSetAttribute(run_transform_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      3 * kRun * kRun * (int)sizeof(double)));
+                                      kTransformSmem));
       attr[c.device] = true;
     }
   }
-  run_cholinv_kernel<<<ngrp, 256, 2 * kRun * kRun * sizeof(double), c.stream>>>(grp_d.p, d.row_ptr.p, d.col.p, d.b.p,
-                                                                                soff.p, S.p, flag.p);
-  c.launches++;
-  run_transform_kernel<<<ngrp, kTransformThreads, 3 * kRun * kRun * sizeof(double), c.stream>>>(
+  if (nshort > 0)
+    run_cholinv_kernel<kSmallRun><<<nshort, 4 * kSmallRun, 2 * kSmallRun * kSmallRun * sizeof(double), c.stream>>>(
+        list.p, grp_d.p, d.row_ptr.p, d.col.p, d.b.p, soff.p, S.p, flag.p);
+  if (ngrp > nshort)
+    run_cholinv_kernel<kRun><<<ngrp - nshort, 4 * kRun, 2 * kRun * kRun * sizeof(double), c.stream>>>(
+        list.p + nshort, grp_d.p, d.row_ptr.p, d.col.p, d.b.p, soff.p, S.p, flag.p);
+  c.launches += 2;
+  run_transform_kernel<<<dim3(ngrp, 2), kTransformThreads, kTransformSmem, c.stream>>>(
       grp_d.p, d.row_ptr.p, seg_ptr.p, seg.p, soff.p, S.p, d.a.p, d.b.p, sa, sb);
   c.launches++;
   FEM2D_CUDA(cudaGetLastError());

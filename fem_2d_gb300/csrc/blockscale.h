@@ -9,6 +9,8 @@ namespace fem2d {
 struct BlockScale {
   int ngrp = 0;
   DBuf<int32_t> grp_d;     // run starts, ngrp + 1
+  DBuf<int32_t> list;      // the runs, short ones first
+  int nshort = 0;
   DBuf<int64_t> soff;      // offset of each run's |g| x |g| block of S
   DBuf<int64_t> seg_ptr;   // per run, its column-run segments
   DBuf<int2> seg;          // (column run, offset of its first column within the run's rows)

@@ -73,3 +73,18 @@ def test_scaling_and_damping_options_agree(ctx):
         assert r.stats["converged"]
         assert np.allclose(np.sort(r.values), ref, rtol=1e-11, atol=0)
     assert [r.stats["block_scaled"] for r in runs] == [0, 0, 1, 1]
+
+
+@pytest.mark.parametrize("orders", [(1, 1), (2, 3), (4, 4), (6, 5), (8, 8)])
+def test_block_scaling_run_lengths(ctx, oracle_lib, orders):
+    """Block scaling over runs from one row to 64, short and long in one mesh and column runs that do and do
+    not fill tiles of 8: the eigenvalues are those of LAPACK on the unscaled pencil."""
+    pm = configs.build_mesh(configs.full_scale(seed=2, nx=3, ny=2, rounds=1, fraction=0.5, pmin=1, pmax=2))
+    leaves = [int(e) for e in np.nonzero(pm.elem_info()[:, 0] == 1)[0]]
+    pm.set_expansion_on_elems(leaves[:max(1, len(leaves) // 2)], fg.Orders(*orders))
+    gep = fg.galerkin_sample_gep_hcurl(fg.KOLeg, fg.CurlCurl, fg.L2Inner, fg.Domain.from_mesh(pm), [10, 10], ctx=ctx)
+    A, B = gep.scipy()
+    ref, _ = oracle_lib.dense_nearest_physical(A, B, 5.0, 1)
+    r = fg.gpu_solve_gep_n(gep, 5.0, 1, scaling=2)
+    assert r.stats["block_scaled"] == 1
+    assert abs(r.values[0] - ref[0]) <= 1e-9 * abs(ref[0])
