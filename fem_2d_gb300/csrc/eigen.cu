@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <future>
 #include <cmath>
@@ -304,29 +305,45 @@ __global__ void copy_block_kernel(int64_t n, int b, const double* __restrict__ X
   }
 }
 
-// per CTA the largest absolute row sum of ka A + kb B over its rows (an upper bound of the 2-norm);
-// one warp per row (coalesced reads of the row's values)
+// per CTA the largest absolute row sums (upper bounds of the 2-norms) of A, B and, with `shifted`, of A + c B and
+// A - sigma B over its rows, in one pass; one warp per row (coalesced reads of the row's values)
 __global__ void __launch_bounds__(256) rowsum_max_kernel(int64_t n, const int64_t* __restrict__ rp,
                                                          const double* __restrict__ va, const double* __restrict__ vb,
-                                                         double ka, double kb, double* __restrict__ part) {
-  __shared__ double red[256];
-  const int lane = threadIdx.x & 31;
+                                                         double shift_p, double shift_m, int shifted,
+                                                         double* __restrict__ part) {
+  __shared__ double red[4][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t warp0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  double m = 0.0;
+  double m[4] = {0.0, 0.0, 0.0, 0.0};
   for (int64_t r = warp0; r < n; r += nwarps) {
-    double s = 0.0;
-    for (int64_t k = rp[r] + lane; k < rp[r + 1]; k += 32) s += fabs(ka * va[k] + kb * vb[k]);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    m = fmax(m, s);
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    const int64_t k1 = rp[r + 1];
+#pragma unroll 2
+    for (int64_t k = rp[r] + lane; k < k1; k += 32) {
+      const double a = va[k], b = vb[k];
+      s[0] += fabs(a);
+      s[1] += fabs(b);
+      if (shifted) {
+        s[2] += fabs(a + shift_p * b);
+        s[3] += fabs(a + shift_m * b);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (q >= 2 && !shifted) break;
+      for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+      m[q] = fmax(m[q], s[q]);
+    }
   }
-  red[threadIdx.x] = m;
+  if (lane == 0)
+    for (int q = 0; q < 4; q++) red[q][warp] = m[q];
   __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + st]);
-    __syncthreads();
+  if (threadIdx.x < 4) {
+    double v = red[threadIdx.x][0];
+    for (int q = 1; q < 8; q++) v = fmax(v, red[threadIdx.x][q]);
+    part[4 * blockIdx.x + threadIdx.x] = v;
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
 // Y = alpha X + beta Y on an n x b row-major block
@@ -340,45 +357,56 @@ __global__ void axpby_kernel(int64_t n, int b, double alpha, const double* __res
   }
 }
 
-// R = AX - BX * diag(theta) column by column, accumulating per CTA the column sums of squares of R, of
-// BX and of X: P[cta][0, b) = |R|^2, [b, 2b) = |BX|^2, [2b, 3b) = |X|^2
+// Per CTA and column j of R = AX - BX diag(theta) the sums of squares of R, of BX and of X over its rows:
+// P[cta][0, b) = |R|^2, [b, 2b) = |BX|^2, [2b, 3b) = |X|^2. Columns along the lanes (`w` of them, a power of
+// two), so that rows are read contiguously; one column after the other with rows along the lanes read 8 bytes
+// per 32-byte sector (127 us for 83,159 x 48, now 40)
 __global__ void __launch_bounds__(256) resid_partial_kernel(int64_t n, const double* __restrict__ AX,
                                                             const double* __restrict__ BX,
-                                                            const double* __restrict__ X, int64_t ld, int b,
+                                                            const double* __restrict__ X, int64_t ld, int b, int w,
                                                             const double* __restrict__ theta, int64_t rows_per_block,
                                                             double* __restrict__ P) {
   __shared__ double sr[256], sb[256], sx[256];
   const int64_t r0 = blockIdx.x * rows_per_block, r1 = min(n, r0 + rows_per_block);
-  for (int j = 0; j < b; j++) {
+  const int lane = threadIdx.x % w, part = threadIdx.x / w, parts = 256 / w;
+  for (int j0 = 0; j0 < b; j0 += w) {
+    const int j = j0 + lane;
     double a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    const double th = theta[j];
-    for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-      const double bx = BX[r * ld + j];
-      const double res = AX[r * ld + j] - th * bx;
-      const double x = X[r * ld + j];
-      a1 += res * res;
-      a2 += bx * bx;
-      a3 += x * x;
+    if (j < b) {
+      const double th = theta[j];
+#pragma unroll 4
+      for (int64_t r = r0 + part; r < r1; r += parts) {
+        const double bx = BX[r * ld + j];
+        const double res = AX[r * ld + j] - th * bx;
+        const double x = X[r * ld + j];
+        a1 += res * res;
+        a2 += bx * bx;
+        a3 += x * x;
+      }
     }
     sr[threadIdx.x] = a1;
     sb[threadIdx.x] = a2;
     sx[threadIdx.x] = a3;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-      if (threadIdx.x < s) {
-        sr[threadIdx.x] += sr[threadIdx.x + s];
-        sb[threadIdx.x] += sb[threadIdx.x + s];
-        sx[threadIdx.x] += sx[threadIdx.x + s];
+    if (part == 0 && j < b) {
+      for (int q = 1; q < parts; q++) {
+        a1 += sr[q * w + lane];
+        a2 += sb[q * w + lane];
+        a3 += sx[q * w + lane];
       }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      P[(int64_t)blockIdx.x * 3 * b + j] = sr[0];
-      P[(int64_t)blockIdx.x * 3 * b + b + j] = sb[0];
-      P[(int64_t)blockIdx.x * 3 * b + 2 * b + j] = sx[0];
+      P[(int64_t)blockIdx.x * 3 * b + j] = a1;
+      P[(int64_t)blockIdx.x * 3 * b + b + j] = a2;
+      P[(int64_t)blockIdx.x * 3 * b + 2 * b + j] = a3;
     }
     __syncthreads();
   }
+}
+
+// the column width of the kernel above: at most 32 lanes, as few as cover the columns
+inline int resid_width(int b) {
+  int w = 4;
+  while (w < b && w < 32) w <<= 1;
+  return w;
 }
 
 // s[i] = 1 / sqrt(B_ii) (B is SPD); one warp per row
@@ -710,24 +738,25 @@ void setup_gemm_smem(int device) {
 // splitmix64 -> standard normal (Box-Muller), deterministic start blocks
 // deterministic pseudo-random start blocks: a splitmix64 sequence turned into standard normals by
 // Box-Muller, generated on the device (element k of the row-major n x b block uses the generator's
-// calls 2 floor(k/2) + 1 and + 2, so every element is independent); written with leading dimension ld
+// calls 2 floor(k/2) + 1 and + 2: one thread per pair of elements); written with leading dimension ld
 __global__ void random_block_kernel(int64_t n, int b, uint64_t seed, double* __restrict__ out, int64_t ld) {
   const uint64_t s0 = seed * 0x9E3779B97F4A7C15ull + 0x2545F4914F6CDD1Dull;
   const int64_t total = n * b;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t pair = (uint64_t)(k >> 1);
-    auto mix = [](uint64_t z) {
-      z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-      z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-      return z ^ (z >> 31);
-    };
-    const uint64_t z1 = mix(s0 + (2 * pair + 1) * 0x9E3779B97F4A7C15ull);
-    const uint64_t z2 = mix(s0 + (2 * pair + 2) * 0x9E3779B97F4A7C15ull);
+  auto mix = [](uint64_t z) {
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return z ^ (z >> 31);
+  };
+  for (int64_t pair = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; 2 * pair < total;
+       pair += (int64_t)gridDim.x * blockDim.x) {
+    const uint64_t z1 = mix(s0 + (2 * (uint64_t)pair + 1) * 0x9E3779B97F4A7C15ull);
+    const uint64_t z2 = mix(s0 + (2 * (uint64_t)pair + 2) * 0x9E3779B97F4A7C15ull);
     const double u1 = ((double)(z1 >> 11) + 0.5) / 9007199254740992.0;
     const double u2 = ((double)(z2 >> 11) + 0.5) / 9007199254740992.0;
     const double r = sqrt(-2.0 * log(u1));
-    const double v = (k & 1) ? r * sinpi(2.0 * u2) : r * cospi(2.0 * u2);
-    out[(k / b) * ld + (k % b)] = v;
+    const int64_t k = 2 * pair;
+    out[(k / b) * ld + (k % b)] = r * cospi(2.0 * u2);
+    if (k + 1 < total) out[((k + 1) / b) * ld + ((k + 1) % b)] = r * sinpi(2.0 * u2);
   }
 }
 
@@ -799,6 +828,7 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
   const double spur = 1e-6 * std::max(1.0, std::fabs(sigma));
   if (sigma == 0.0) fail(FEM2D_E_INVALID_ARG, "target 0 is the null space of the curl-curl operator");
 
+  constexpr int64_t kLargeN = 10000;   // block scaling by default from here on (below)
   // symmetric Jacobi scaling: the whole solve runs on (D A D, D B D), D = diag(B)^-1/2 (same
   // eigenvalues, eigenvectors x = D x~); it keeps the unnormalised high-order bases well scaled
   DBuf<double> sc, sa, sb;
@@ -811,8 +841,11 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
   const int64_t jblocks = std::max<int64_t>(1, std::min<int64_t>((n * 32 + 255) / 256, (int64_t)c.num_sms * 16));
   {
     jacobi_scale_kernel<<<(int)jblocks, 256, 0, c.stream>>>(n, d.row_ptr.p, d.col.p, d.b.p, sc.p, bad.p);
-    scale_csr_kernel<<<(int)jblocks, 256, 0, c.stream>>>(n, d.row_ptr.p, d.col.p, d.a.p, d.b.p, sc.p, sa.p, sb.p);
-    c.launches += 2;
+    c.launches++;
+    if (!(o.scaling == 2 || (o.scaling == 0 && n >= kLargeN))) {   // else the block scaling writes sa and sb
+      scale_csr_kernel<<<(int)jblocks, 256, 0, c.stream>>>(n, d.row_ptr.p, d.col.p, d.a.p, d.b.p, sc.p, sa.p, sb.p);
+      c.launches++;
+    }
     int hb = 0;
     FEM2D_CUDA(cudaMemcpyAsync(&hb, bad.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     FEM2D_CUDA(cudaStreamSynchronize(c.stream));
@@ -826,7 +859,6 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
   // for). Below kLargeN DoFs the Jacobi scaling is kept unless the factorizations prove inaccurate
   // (below): there the rounding smear of the null space is small and the block set-up would cost more
   // than the solve gains (about 8 ms per solve at 2-4k DoFs).
-  constexpr int64_t kLargeN = 10000;
   const bool large = n >= kLargeN;
   // the pattern-only structures kept in the plan (block scaling, tensor-core products) belong to the
   // device they were built on
@@ -948,25 +980,25 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
   // solves (||K|| bounded by the largest absolute row sum): a backward-stable factorization keeps it
   // near the unit roundoff whatever cond(K) is, whereas the plain residual ||b - K x|| / ||b|| cannot
   // fall below about eps * cond(K) even for an exact-in-FP64 solve.
-  // ||ka A + kb B||_inf of the pencil in use (largest absolute row sum)
-  auto pencil_norm = [&](double ka, double kb) -> double {
-    const int nblk = std::max(1, std::min<int>(c.num_sms * 4, (int)((n + 7) / 8)));
+  // infinity norms (largest absolute row sums) of the pencil in use: A, B and, on request, A + c B, A - sigma B
+  auto pencil_norms = [&](bool shifted) -> std::array<double, 4> {
+    const int nblk = std::max(1, std::min<int>(c.num_sms * 16, (int)((n + 7) / 8)));
     DBuf<double> part;
-    part.alloc_on(nblk, c.stream);
-    rowsum_max_kernel<<<nblk, 256, 0, c.stream>>>(n, d.row_ptr.p, D.va, D.vb, ka, kb, part.p);
+    part.alloc_on(4 * (size_t)nblk, c.stream);
+    rowsum_max_kernel<<<nblk, 256, 0, c.stream>>>(n, d.row_ptr.p, D.va, D.vb, cshift, -sigma, shifted ? 1 : 0, part.p);
     c.launches++;
-    std::vector<double> hp(nblk);
-    FEM2D_CUDA(cudaMemcpyAsync(hp.data(), part.p, nblk * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    std::vector<double> hp(4 * (size_t)nblk);
+    FEM2D_CUDA(cudaMemcpyAsync(hp.data(), part.p, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     FEM2D_CUDA(cudaStreamSynchronize(c.stream));
-    double m = 0.0;
-    for (double v : hp) m = std::max(m, v);
+    std::array<double, 4> m{};
+    for (size_t q = 0; q < hp.size(); q++) m[q % 4] = std::max(m[q % 4], hp[q]);
     return m;
   };
   // normwise backward error below which the exact solves are used without refinement
   constexpr double kStableBwd = 1e-13;
-  auto calibrate = [&](const MFFactor& fac, double ka, double kb, double& rel_out) -> int {
+  std::array<double, 4> norms = pencil_norms(!iterative);   // of the scaled pencil
+  auto calibrate = [&](const MFFactor& fac, double ka, double kb, double knorm, double& rel_out) -> int {
     const int nb = 4;
-    const double knorm = pencil_norm(ka, kb);
     DBuf<double> Rb, Xb, Tb;
     Rb.alloc_on((size_t)n * nb, c.stream);
     Xb.alloc_on((size_t)n * nb, c.stream);
@@ -1001,8 +1033,8 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
     return 3;
   };
   double rel_p = 0, rel_m = 0;
-  int nref_p = iterative ? 0 : calibrate(fp, 1.0, cshift, rel_p);
-  int nref_m = iterative ? 0 : calibrate(fm, 1.0, -sigma, rel_m);
+  int nref_p = iterative ? 0 : calibrate(fp, 1.0, cshift, norms[2], rel_p);
+  int nref_m = iterative ? 0 : calibrate(fm, 1.0, -sigma, norms[3], rel_m);
   // a caller-fixed refinement count replaces the calibrated one after the checks below
   if (!iterative && (rel_p > 1e-11 || rel_m > 1e-11) && !blocked && !plan.dense && o.scaling == 0) {
     // the Jacobi-scaled factorizations lose too many digits: scale by row-run blocks of B instead
@@ -1015,14 +1047,16 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
       }
       blocked = true;
       factor_both();
-      nref_p = calibrate(fp, 1.0, cshift, rel_p);
-      nref_m = calibrate(fm, 1.0, -sigma, rel_m);
+      norms = pencil_norms(true);
+      nref_p = calibrate(fp, 1.0, cshift, norms[2], rel_p);
+      nref_m = calibrate(fm, 1.0, -sigma, norms[3], rel_m);
     } catch (const Error&) {
       scale_csr_kernel<<<(int)jblocks, 256, 0, c.stream>>>(n, d.row_ptr.p, d.col.p, d.a.p, d.b.p, sc.p, sa.p, sb.p);
       c.launches++;
       factor_both();
-      nref_p = calibrate(fp, 1.0, cshift, rel_p);
-      nref_m = calibrate(fm, 1.0, -sigma, rel_m);
+      norms = pencil_norms(true);
+      nref_p = calibrate(fp, 1.0, cshift, norms[2], rel_p);
+      nref_m = calibrate(fm, 1.0, -sigma, norms[3], rel_m);
     }
   }
   // small GEPs whose sparse factorization stays inaccurate after refinement (pivoting restricted to
@@ -1032,8 +1066,8 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
   if (!iterative && (rel_p > 1e-11 || rel_m > 1e-11) && !plan.dense && n <= kDenseMax) {
     M = &mf_plan_dense(plan, c, h);
     factor_both();
-    nref_p = calibrate(fp, 1.0, cshift, rel_p);
-    nref_m = calibrate(fm, 1.0, -sigma, rel_m);
+    nref_p = calibrate(fp, 1.0, cshift, norms[2], rel_p);
+    nref_m = calibrate(fm, 1.0, -sigma, norms[3], rel_m);
   }
   if (o.refine > 0) nref_p = nref_m = std::min(o.refine, 3);
   if (o.refine < 0) nref_p = nref_m = 0;
@@ -1133,7 +1167,7 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
     return keep;
   };
 
-  const double norm_a = pencil_norm(1.0, 0.0), norm_b = pencil_norm(0.0, 1.0);
+  const double norm_a = norms[0], norm_b = norms[1];
   // products with A or B alone (the T applications, the basis products) on the tensor cores from here
   // on: the scaled pencil is final, so its values are sliced once (by default from kTensorSpmmNnz
   // nonzeros, where the slicing is amortised; always with dense = 2)
@@ -1314,7 +1348,7 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
     P.alloc_on((size_t)nblk * 3 * nc, c.stream);
     {
       ProfScope ps_r(c, "vector_ops", 24.0 * n * nc);
-      resid_partial_kernel<<<nblk, 256, 0, c.stream>>>(n, AY.p, BY.p, XY.p, nc, nc, th_d.p, rpb, P.p);
+      resid_partial_kernel<<<nblk, 256, 0, c.stream>>>(n, AY.p, BY.p, XY.p, nc, nc, resid_width(nc), th_d.p, rpb, P.p);
       c.launches++;
     }
     std::vector<double> Ph((size_t)nblk * 3 * nc);
@@ -1498,9 +1532,10 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
     const int nblk = std::min<int64_t>(D.grid_rows(), std::max<int64_t>(1, (n + 255) / 256));
     const int64_t rpb = (n + nblk - 1) / nblk;
     P.alloc_on((size_t)nblk * 3 * kout, c.stream);
-    resid_partial_kernel<<<nblk, 256, 0, c.stream>>>(n, AX.p, BX.p, XO.p, 32, kout, th_d.p, rpb, P.p);
+    resid_partial_kernel<<<nblk, 256, 0, c.stream>>>(n, AX.p, BX.p, XO.p, 32, kout, resid_width(kout), th_d.p, rpb, P.p);
     c.launches++;
-    const double na0 = pencil_norm(1.0, 0.0), nb0 = pencil_norm(0.0, 1.0);
+    const std::array<double, 4> norms0 = pencil_norms(false);
+    const double na0 = norms0[0], nb0 = norms0[1];
     std::vector<double> Ph((size_t)nblk * 3 * kout);
     FEM2D_CUDA(cudaMemcpyAsync(Ph.data(), P.p, Ph.size() * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     FEM2D_CUDA(cudaStreamSynchronize(c.stream));
