@@ -266,10 +266,12 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const double* __re
   }
 }
 
-// Z = beta*Z + X * C; X n x a (ldx), C a x b row-major (device), Z n x b (ldz)
-__global__ void __launch_bounds__(256) gemm_nn_kernel(int64_t n, const double* __restrict__ X, int64_t ldx, int a,
-                                                      const double* __restrict__ C, int b, double alpha, double beta,
-                                                      double* __restrict__ Z, int64_t ldz) {
+// Z = beta*Z + alpha X C for each set (blockIdx.y); X n x a (ldx), C a x b row-major (device), Z n x b (ldz)
+__global__ void __launch_bounds__(256) gemm_nn_kernel(int64_t n, BlockSets sets, int a, const double* __restrict__ C,
+                                                      int b, double alpha, double beta) {
+  const double* __restrict__ X = sets.X[blockIdx.y];
+  double* __restrict__ Z = sets.Z[blockIdx.y];
+  const int64_t ldx = sets.ldx[blockIdx.y], ldz = sets.ldz[blockIdx.y];
   extern __shared__ double cs[];
   for (int t = threadIdx.x; t < a * b; t += blockDim.x) cs[t] = C[t];
   __syncthreads();
@@ -295,13 +297,16 @@ __global__ void __launch_bounds__(256) gemm_nn_kernel(int64_t n, const double* _
   }
 }
 
-__global__ void copy_block_kernel(int64_t n, int b, const double* __restrict__ X, int64_t ldx, double* __restrict__ Y,
-                                  int64_t ldy) {
+// Z = X (n x b) for each set (blockIdx.y)
+__global__ void copy_block_kernel(int64_t n, int b, BlockSets sets) {
+  const double* __restrict__ X = sets.X[blockIdx.y];
+  double* __restrict__ Z = sets.Z[blockIdx.y];
+  const int64_t ldx = sets.ldx[blockIdx.y], ldz = sets.ldz[blockIdx.y];
   const int64_t total = n * b;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = t / b;
     const int j = (int)(t % b);
-    Y[r * ldy + j] = X[r * ldx + j];
+    Z[r * ldz + j] = X[r * ldx + j];
   }
 }
 
@@ -544,7 +549,7 @@ struct Dev {
   TcSpmm* tcs = nullptr;  // products with A or B alone on the tensor cores when set (slices of va, vb)
   DBuf<double> ozw;      // tensor Gram workspace (partial tiles)
   DBuf<int> ozerr;       // set by the tensor Gram kernel when a bounded wait expired
-  DBuf<int> ozrow;       // row exponents of the tensor block update
+  DBuf<int> ozrow;       // row exponents of the tensor block update, per set
   int grid_rows() const { return std::max(1, c.num_sms * 2); }
 
   // C (device, a x b) = X^T Y on the tensor cores; false when the FP64 CUDA-core kernels must be used
@@ -560,17 +565,18 @@ struct Dev {
     ozaki_gram(c, h.n, X, ldx, a, Y, ldy, b, Cd, ozw.p, ozw.n, ozerr.p);
     return true;
   }
-  // Z = beta Z + alpha X C (C device, a x b) on the tensor cores; false when the FP64 kernel must be used
-  bool tensor_gemm(const double* X, int64_t ldx, int a, const double* Cd, int b, double alpha, double beta, double* Z,
-                   int64_t ldz) {
+  // Z = beta Z + alpha X C for each set (C device, a x b) on the tensor cores; false when the FP64 kernel must be
+  // used
+  bool tensor_gemm(const BlockSets& s, int a, const double* Cd, int b, double alpha, double beta) {
     if (dense_mode != 0 || a > 256 || b > 32 || a <= 0 || b <= 0) return false;
-    ProfScope ps(c, "gemm_tc", 8.0 * h.n * (a + (beta != 0.0 ? 2.0 : 1.0) * b), 2.0 * h.n * a * b);
+    ProfScope ps(c, "gemm_tc", s.count * 8.0 * h.n * (a + (beta != 0.0 ? 2.0 : 1.0) * b), s.count * 2.0 * h.n * a * b);
     if (ozerr.n == 0) {
       ozerr.alloc_on(1, c.stream);
       FEM2D_CUDA(cudaMemsetAsync(ozerr.p, 0, sizeof(int), c.stream));
     }
-    if (ozrow.n < (size_t)std::max<int64_t>(h.n, 1)) ozrow.alloc_on(std::max<int64_t>(h.n, 1), c.stream);
-    ozaki_gemm(c, h.n, X, ldx, a, Cd, b, alpha, beta, Z, ldz, ozrow.p, ozerr.p);
+    const size_t need = (size_t)std::max<int64_t>(h.n, 1) * s.count;
+    if (ozrow.n < need) ozrow.alloc_on(need, c.stream);
+    ozaki_gemm(c, h.n, s, a, Cd, b, alpha, beta, ozrow.p, ozerr.p);
     return true;
   }
   // the tensor Gram kernel's error flag (synchronises the stream)
@@ -653,41 +659,39 @@ struct Dev {
     FEM2D_CUDA(cudaMemcpyAsync(C.data(), small.p, ab * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     FEM2D_CUDA(cudaStreamSynchronize(c.stream));
   }
-  // Z = beta Z + X * C (C host a x b), tiled over the columns of C so a tile fits in shared memory
-  void gemm(const double* X, int64_t ldx, int a, const std::vector<double>& C, int b, double beta, double* Z,
-            int64_t ldz) {
+  // Z = beta Z + X C for each set (C host a x b), tiled over the columns of C so a tile fits in shared memory
+  void gemm(const BlockSets& s, int a, const std::vector<double>& C, int b, double beta) {
     if (a <= 0 || b <= 0) return;
-    if (dense_mode == 0 && a <= 256) {
-      // 32 columns of C at a time through the tensor-core kernel
-      std::vector<double> Ct;
-      for (int j0 = 0; j0 < b; j0 += 32) {
-        const int w = std::min(32, b - j0);
-        Ct.resize((size_t)a * w);
-        for (int i = 0; i < a; i++)
-          for (int j = 0; j < w; j++) Ct[(size_t)i * w + j] = C[(size_t)i * b + j0 + j];
-        if (small.n < Ct.size()) small.alloc_on(std::max<size_t>(Ct.size(), 16384), c.stream);
-        FEM2D_CUDA(cudaMemcpyAsync(small.p, Ct.data(), Ct.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-        tensor_gemm(X, ldx, a, small.p, w, 1.0, beta, Z + j0, ldz);
-        // (pageable copies are staged before cudaMemcpyAsync returns: Ct may be reused)
-      }
-      return;
-    }
-    ProfScope ps(c, "dense_block", 8.0 * h.n * (a + (beta != 0.0 ? 2.0 : 1.0) * b), 2.0 * h.n * a * b);
-    const int chunk = std::max(1, std::min(b, (int)((96 * 1024) / (sizeof(double) * a))));
+    // 32 columns of C at a time through the tensor-core kernel
+    const bool tensor = dense_mode == 0 && a <= 256;
+    const int chunk = tensor ? 32 : std::max(1, std::min(b, (int)((96 * 1024) / (sizeof(double) * a))));
     std::vector<double> Ct;
     for (int j0 = 0; j0 < b; j0 += chunk) {
       const int w = std::min(chunk, b - j0);
-      Ct.resize((size_t)a * w);
-      for (int i = 0; i < a; i++)
-        for (int j = 0; j < w; j++) Ct[(size_t)i * w + j] = C[(size_t)i * b + j0 + j];
-      if (small.n < Ct.size()) small.alloc_on(std::max<size_t>(Ct.size(), 16384), c.stream);
-      FEM2D_CUDA(cudaMemcpyAsync(small.p, Ct.data(), Ct.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-      const size_t smem = Ct.size() * sizeof(double);
-      const int64_t blocks = std::min<int64_t>((h.n * w + 255) / 256, (int64_t)c.num_sms * 8);
-      gemm_nn_kernel<<<(int)std::max<int64_t>(blocks, 1), 256, smem, c.stream>>>(h.n, X, ldx, a, small.p, w, 1.0, beta,
-                                                                                Z + j0, ldz);
-      c.launches++;   // (pageable copies are staged before cudaMemcpyAsync returns: Ct may be reused)
+      const double* src = C.data();
+      if (w < b) {
+        Ct.resize((size_t)a * w);
+        for (int i = 0; i < a; i++)
+          for (int j = 0; j < w; j++) Ct[(size_t)i * w + j] = C[(size_t)i * b + j0 + j];
+        src = Ct.data();
+      }
+      const size_t count = (size_t)a * w;
+      if (small.n < count) small.alloc_on(std::max<size_t>(count, 16384), c.stream);
+      FEM2D_CUDA(cudaMemcpyAsync(small.p, src, count * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+      if (!tensor || !tensor_gemm(s.columns(j0), a, small.p, w, 1.0, beta)) fp64_gemm(s.columns(j0), a, small.p, w, 1.0, beta);
+      // (pageable copies are staged before cudaMemcpyAsync returns: Ct may be reused)
     }
+  }
+  // the same on the FP64 pipe, C on the device (a * b * 8 bytes fit the kernel's smem)
+  void fp64_gemm(const BlockSets& s, int a, const double* Cd, int b, double alpha, double beta) {
+    ProfScope ps(c, "dense_block", s.count * 8.0 * h.n * (a + (beta != 0.0 ? 2.0 : 1.0) * b),
+                 s.count * 2.0 * h.n * a * b);
+    const size_t smem = (size_t)a * b * sizeof(double);
+    if (smem > 96 * 1024) fail(FEM2D_E_INVALID_ARG, "device-resident projection block too large");
+    const int64_t blocks = std::min<int64_t>((h.n * b + 255) / 256, (int64_t)c.num_sms * 8);
+    gemm_nn_kernel<<<dim3((unsigned)std::max<int64_t>(blocks, 1), s.count), 256, smem, c.stream>>>(h.n, s, a, Cd, b, alpha,
+                                                                                                  beta);
+    c.launches++;
   }
   void axpby(double alpha, const double* X, int64_t ldx, int b, double beta, double* Y, int64_t ldy) {
     ProfScope ps(c, "vector_ops", 8.0 * h.n * b * (beta != 0.0 ? 3.0 : 2.0));
@@ -699,23 +703,15 @@ struct Dev {
   void gram_dev(const double* X, int64_t ldx, int a, const double* Y, int64_t ldy, int b, double* Cd) {
     if (!tensor_gram(X, ldx, a, Y, ldy, b, Cd)) fp64_gram(X, ldx, a, Y, ldy, b, Cd);
   }
-  // Z = beta Z + alpha X C with C (a x b) already on the device (a * b * 8 bytes fit the kernel's smem)
-  void gemm_dev(const double* X, int64_t ldx, int a, const double* Cd, int b, double alpha, double beta, double* Z,
-                int64_t ldz) {
+  // Z = beta Z + alpha X C for each set with C (a x b) already on the device
+  void gemm_dev(const BlockSets& s, int a, const double* Cd, int b, double alpha, double beta) {
     if (a <= 0 || b <= 0) return;
-    if (tensor_gemm(X, ldx, a, Cd, b, alpha, beta, Z, ldz)) return;
-    ProfScope ps(c, "dense_block", 8.0 * h.n * (a + (beta != 0.0 ? 2.0 : 1.0) * b), 2.0 * h.n * a * b);
-    const size_t smem = (size_t)a * b * sizeof(double);
-    if (smem > 96 * 1024) fail(FEM2D_E_INVALID_ARG, "device-resident projection block too large");
-    const int64_t blocks = std::min<int64_t>((h.n * b + 255) / 256, (int64_t)c.num_sms * 8);
-    gemm_nn_kernel<<<(int)std::max<int64_t>(blocks, 1), 256, smem, c.stream>>>(h.n, X, ldx, a, Cd, b, alpha, beta, Z,
-                                                                              ldz);
-    c.launches++;
+    if (!tensor_gemm(s, a, Cd, b, alpha, beta)) fp64_gemm(s, a, Cd, b, alpha, beta);
   }
-  void copy(const double* X, int64_t ldx, int b, double* Y, int64_t ldy) {
-    ProfScope ps(c, "vector_ops", 16.0 * h.n * b);
+  void copy(const BlockSets& s, int b) {
+    ProfScope ps(c, "vector_ops", s.count * 16.0 * h.n * b);
     const int64_t blocks = std::min<int64_t>((h.n * b + 255) / 256, (int64_t)c.num_sms * 8);
-    copy_block_kernel<<<(int)std::max<int64_t>(blocks, 1), 256, 0, c.stream>>>(h.n, b, X, ldx, Y, ldy);
+    copy_block_kernel<<<dim3((unsigned)std::max<int64_t>(blocks, 1), s.count), 256, 0, c.stream>>>(h.n, b, s);
     c.launches++;
   }
 };
@@ -1123,13 +1119,12 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
     // coefficients stay on the device (no host round trip)
     auto project_w = [&](int cols) {
       D.gram_dev(BV.p, mmax, m0, Wb, mmax, cols, Cproj.p);
-      D.gemm_dev(V.p, mmax, m0, Cproj.p, cols, -1.0, 1.0, Wb, mmax);
+      D.gemm_dev(BlockSets().add(V.p, mmax, Wb, mmax), m0, Cproj.p, cols, -1.0, 1.0);
     };
     // W -= V (V^T B W), B W -= (B V)(V^T B W): B W tracked linearly through a late, small correction
     auto project = [&](int cols) {
       D.gram_dev(V.p, mmax, m0, BWb, mmax, cols, Cproj.p);
-      D.gemm_dev(V.p, mmax, m0, Cproj.p, cols, -1.0, 1.0, Wb, mmax);
-      D.gemm_dev(BV.p, mmax, m0, Cproj.p, cols, -1.0, 1.0, BWb, mmax);
+      D.gemm_dev(BlockSets().add(V.p, mmax, Wb, mmax).add(BV.p, mmax, BWb, mmax), m0, Cproj.p, cols, -1.0, 1.0);
     };
     if (m0 > 0) {
       project_w(r);
@@ -1155,10 +1150,8 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
       std::vector<double> T((size_t)keep * nk);
       for (int i = 0; i < keep; i++)
         for (int q = 0; q < nk; q++) T[(size_t)i * nk + q] = z[(size_t)i * keep + kept[q]] / std::sqrt(w[kept[q]]);
-      D.gemm(Wb, mmax, keep, T, nk, 0.0, W2.p, 32);
-      D.copy(W2.p, 32, nk, Wb, mmax);
-      D.gemm(BWb, mmax, keep, T, nk, 0.0, W2.p, 32);
-      D.copy(W2.p, 32, nk, BWb, mmax);
+      D.gemm(BlockSets().add(Wb, mmax, W2.p, 32).add(BWb, mmax, W3.p, 32), keep, T, nk, 0.0);
+      D.copy(BlockSets().add(W2.p, 32, Wb, mmax).add(W3.p, 32, BWb, mmax), nk);
       keep = nk;
       if (pass == 0 && m0 > 0) project(keep);
     }
@@ -1250,20 +1243,14 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
   for (; cycles < max_cycles; cycles++) {
     int m, last0, lastn;
     if (cycles == 0) {
-      D.copy(X.p, 32, bx, V.p, mmax);
+      D.copy(BlockSets().add(X.p, 32, V.p, mmax), bx);
       m = borth_new(0, bx);
       last0 = 0;
       lastn = m;
     } else {
       // V = [locked | active Ritz vectors | T^j (active)]; every active vector is unconverged
-      if (nl > 0) {
-        D.copy(XL.p, 32, nl, V.p, mmax);
-        D.copy(AXL.p, 32, nl, AV.p, mmax);
-        D.copy(BXL.p, 32, nl, BV.p, mmax);
-      }
-      D.copy(X.p, 32, bx, V.p + nl, mmax);
-      D.copy(AX.p, 32, bx, AV.p + nl, mmax);
-      D.copy(BX.p, 32, bx, BV.p + nl, mmax);
+      if (nl > 0) D.copy(BlockSets().add(XL.p, 32, V.p, mmax).add(AXL.p, 32, AV.p, mmax).add(BXL.p, 32, BV.p, mmax), nl);
+      D.copy(BlockSets().add(X.p, 32, V.p + nl, mmax).add(AX.p, 32, AV.p + nl, mmax).add(BX.p, 32, BV.p + nl, mmax), bx);
       m = nl + bx;
       if (m + bx > mmax) fail(FEM2D_E_NOT_CONVERGED, "gpu_solve_gep: basis capacity exceeded");
       // expand with T applied to the active Ritz vectors: T kills their null-space part and damps
@@ -1339,9 +1326,7 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
     AY.alloc_on((size_t)n * nc, c.stream);
     BY.alloc_on((size_t)n * nc, c.stream);
     XY.alloc_on((size_t)n * nc, c.stream);
-    D.gemm(AVa, mmax, ma, Ysub, nc, 0.0, AY.p, nc);
-    D.gemm(BVa, mmax, ma, Ysub, nc, 0.0, BY.p, nc);
-    D.gemm(Va, mmax, ma, Ysub, nc, 0.0, XY.p, nc);
+    D.gemm(BlockSets().add(AVa, mmax, AY.p, nc).add(BVa, mmax, BY.p, nc).add(Va, mmax, XY.p, nc), ma, Ysub, nc, 0.0);
     th_d.upload_on(thc, c.stream);
     const int nblk = std::min<int64_t>(D.grid_rows(), std::max<int64_t>(1, (n + 255) / 256));
     const int64_t rpb = (n + nblk - 1) / nblk;
@@ -1412,9 +1397,7 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
       std::vector<double> Ys((size_t)ma * w);
       for (int i = 0; i < ma; i++)
         for (int q = 0; q < w; q++) Ys[(size_t)i * w + q] = Y[(size_t)i * m2 + sel[idx[q]]];
-      D.gemm(Va, mmax, ma, Ys, w, 0.0, Xd, 32);
-      D.gemm(AVa, mmax, ma, Ys, w, 0.0, AXd, 32);
-      D.gemm(BVa, mmax, ma, Ys, w, 0.0, BXd, 32);
+      D.gemm(BlockSets().add(Va, mmax, Xd, 32).add(AVa, mmax, AXd, 32).add(BVa, mmax, BXd, 32), ma, Ys, w, 0.0);
     };
     gather(to_lock, XL.p + nl, AXL.p + nl, BXL.p + nl);
     for (int q : to_lock) {
@@ -1494,7 +1477,7 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
   for (int q = 0; q < kout; q++) {
     const auto& e = nearest[q];
     theta_out[q] = e.first ? theta_l[e.second] : theta_sel[e.second];
-    D.copy((e.first ? XL.p : X.p) + e.second, 32, 1, XO.p + q, 32);
+    D.copy(BlockSets().add((e.first ? XL.p : X.p) + e.second, 32, XO.p + q, 32), 1);
   }
   if (st) {
     st->outer_iters = cycles;
@@ -1762,7 +1745,7 @@ void block_gemm(Ctx& c, int method, int64_t n, const double* X, int64_t ldx, int
   Dev D{c, hg, dg, nullptr, nullptr};
   D.dense_mode = method == 0 ? 0 : 1;
   if (method == 0 && (a > 256 || b > 32)) fail(FEM2D_E_INVALID_ARG, "tensor update: a <= 256 and b <= 32");
-  D.gemm_dev(X, ldx, a, Cd, b, alpha, beta, Z, ldz);
+  D.gemm_dev(BlockSets().add(X, ldx, Z, ldz), a, Cd, b, alpha, beta);
   D.check_tensor();
   FEM2D_CUDA(cudaStreamSynchronize(c.stream));
 }

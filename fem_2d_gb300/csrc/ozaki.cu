@@ -487,8 +487,10 @@ __device__ __forceinline__ int core_off_k(int rg, int kg, int kc) { return (rg *
 // E[r] = biased exponent of max |X[r][k]| over k < a: a warp takes 4 rows at a time (lanes across the
 // rows, four independent loads in flight per lane: the pass is bound by load latency)
 constexpr int kRowExpRows = 4;
-__global__ void __launch_bounds__(256) row_exp_kernel(int64_t n, const double* __restrict__ X, int64_t ldx, int a,
-                                                       int* __restrict__ E) {
+__global__ void __launch_bounds__(256) row_exp_kernel(int64_t n, BlockSets sets, int a, int* __restrict__ E) {
+  const double* __restrict__ X = sets.X[blockIdx.y];
+  const int64_t ldx = sets.ldx[blockIdx.y];
+  E += (int64_t)blockIdx.y * n;
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t r0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * kRowExpRows; r0 < n;
@@ -509,10 +511,14 @@ __global__ void __launch_bounds__(256) row_exp_kernel(int64_t n, const double* _
   }
 }
 
-// rows of X tile `tile`, columns k0 .. k0 + 31, into the staging buffer sx (row r at r * kGemmRow);
-// entries outside X are zero-filled
-__device__ __forceinline__ void gemm_stage(const double* __restrict__ X, int64_t n, int64_t ldx, int a, int64_t tile,
-                                           int k0, double* sx) {
+// rows of tile `tile` (counted through all sets), columns k0 .. k0 + 31, into the staging buffer sx (row r at
+// r * kGemmRow); entries outside X are zero-filled
+__device__ __forceinline__ void gemm_stage(const BlockSets& sets, int64_t n, int a, int64_t tile, int64_t ntiles, int k0,
+                                           double* sx) {
+  const int set = (int)(tile / ntiles);
+  tile -= set * ntiles;
+  const double* __restrict__ X = sets.X[set];
+  const int64_t ldx = sets.ldx[set];
 #pragma unroll
   for (int i = 0; i < kM * kSub / kGemmThreads; i++) {
     const int e = threadIdx.x + kGemmThreads * i;
@@ -528,9 +534,8 @@ __device__ __forceinline__ void gemm_stage(const double* __restrict__ X, int64_t
 }
 
 __global__ void __launch_bounds__(kGemmThreads, 1)
-    ozaki_gemm_kernel(int64_t n, const double* __restrict__ X, int64_t ldx, int a, const double* __restrict__ C, int b,
-                      double alpha, double beta, double* __restrict__ Z, int64_t ldz, const int* __restrict__ EXr,
-                      int stages, int* __restrict__ err) {
+    ozaki_gemm_kernel(int64_t n, const __grid_constant__ BlockSets sets, int a, const double* __restrict__ C, int b,
+                      double alpha, double beta, const int* __restrict__ EXr, int stages, int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int kc = (a + kSub - 1) / kSub * kSub;     // K padded to whole sub-blocks
   const int planeC = kN * kc * 2;                  // one digit plane of C (32 x kc bf16, K-major)
@@ -542,7 +547,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
   const int tid = threadIdx.x, warp = tid >> 5;
   const int rl = tid & (kM - 1), part = tid >> 7;  // row of the tile (TMEM lane), column quarter
-  const int64_t ntiles = (n + kM - 1) / kM;
+  const int64_t ntiles = (n + kM - 1) / kM, total = sets.count * ntiles;
   const int nsub = kc / kSub;
 
   if (warp == 0) {
@@ -557,7 +562,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   }
   // the first sub-block's copies, then C's column exponents and digit planes (row j of the B operand =
   // column j of C)
-  if (blockIdx.x < ntiles) gemm_stage(X, n, ldx, a, blockIdx.x, 0, sX);
+  if (blockIdx.x < total) gemm_stage(sets, n, a, blockIdx.x, ntiles, 0, sX);
   if (tid < kN) eC[tid] = 0;
   __syncthreads();
   {
@@ -598,10 +603,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   bool pending = false;   // MMAs committed and not yet waited for (they read sA)
   int sbc = 0;            // sub-blocks staged so far (selects the staging buffer)
 
-  for (int64_t tile = blockIdx.x; tile < ntiles && !failed; tile += gridDim.x) {
-    const int64_t row = tile * kM + rl;
+  for (int64_t tile = blockIdx.x; tile < total && !failed; tile += gridDim.x) {
+    const int set = (int)(tile / ntiles);
+    const int64_t row = (tile - set * ntiles) * kM + rl;
     const bool row_ok = row < n;
-    const int Ex = row_ok ? EXr[row] : 0;
+    const int Ex = row_ok ? EXr[set * n + row] : 0;
+    double* Zr = sets.Z[set] + row * sets.ldz[set] + part * kGemmCols;
     long long Th[kGemmCols], Tl[kGemmCols];
 #pragma unroll
     for (int j = 0; j < kGemmCols; j++) Th[j] = Tl[j] = 0;
@@ -616,9 +623,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         nt = tile + gridDim.x;
         nk = 0;
       }
-      const bool more = nt < ntiles;
+      const bool more = nt < total;
       if (stages == 2 && more) {
-        gemm_stage(X, n, ldx, a, nt, nk, sX + ((sbc + 1) & 1) * (kGemmStage / 8));
+        gemm_stage(sets, n, a, nt, ntiles, nk, sX + ((sbc + 1) & 1) * (kGemmStage / 8));
         asm volatile("cp.async.wait_group 1;" ::: "memory");
       } else {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -658,7 +665,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // with one staging buffer the next sub-block's copies start now (its slot was read above)
-      if (stages == 1 && more) gemm_stage(X, n, ldx, a, nt, nk, sX);
+      if (stages == 1 && more) gemm_stage(sets, n, a, nt, ntiles, nk, sX);
       const bool first = (k0 % kChunk) == 0;   // the accumulators restart every 128 columns of K
       if (tid == 0) {
 #pragma unroll 1
@@ -678,9 +685,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const bool last = (k0 + kSub) % kChunk == 0 || k0 + kSub >= kc;
       if (last) {   // the accumulators are read back: wait for these MMAs now (the old Z in flight meanwhile)
         if (beta != 0.0 && k0 + kSub >= kc && row_ok) {
-          const double* zr = Z + row * ldz + part * kGemmCols;
 #pragma unroll
-          for (int q = 0; q < kGemmCols; q++) zv[q] = part * kGemmCols + q < b ? zr[q] : 0.0;
+          for (int q = 0; q < kGemmCols; q++) zv[q] = part * kGemmCols + q < b ? Zr[q] : 0.0;
         }
         if (mbar_wait(smem_addr(bar), ph)) {
           ph ^= 1u;
@@ -719,14 +725,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     if (row_ok) {
       // one conversion and one multiply (or FMA) per output: alpha and the power-of-two scale are
       // combined exactly in the exponent field
-      double* zr = Z + row * ldz + part * kGemmCols;
 #pragma unroll
       for (int q = 0; q < kGemmCols; q++) {
         const int j = part * kGemmCols + q;
         if (j >= b) break;
         const double t = (double)fuse_digit_sums<kFuseGemm>(Th[q], Tl[q]);
         const double m = scale_pow2(alpha, Ex + eC[j] - 2044 - 35 - kFuseGemm);
-        zr[q] = beta == 0.0 ? t * m : fma(t, m, beta == 1.0 ? zv[q] : beta * zv[q]);
+        Zr[q] = beta == 0.0 ? t * m : fma(t, m, beta == 1.0 ? zv[q] : beta * zv[q]);
       }
     }
   }
@@ -1217,9 +1222,9 @@ size_t ozaki_gram_workspace(int64_t n, int a, int b, int num_sms) {
   return (size_t)ozaki_gram_partials(n, a, b, num_sms) * tiles * kM * kN + (size_t)(chunks * (a + b) + 1) / 2 + 1;
 }
 
-void ozaki_gemm(Ctx& c, int64_t n, const double* X, int64_t ldx, int a, const double* C, int b, double alpha,
-                double beta, double* Z, int64_t ldz, int* rowexp, int* err) {
-  if (n <= 0 || b <= 0) return;
+void ozaki_gemm(Ctx& c, int64_t n, const BlockSets& s, int a, const double* C, int b, double alpha, double beta,
+                int* rowexp, int* err) {
+  if (n <= 0 || b <= 0 || s.count <= 0) return;
   if (a < 1 || a > kGemmKMax || b > kN) fail(FEM2D_E_INVALID_ARG, "ozaki_gemm: a <= 256 and b <= 32");
   static std::mutex mu;
   static bool done[256] = {};
@@ -1232,12 +1237,12 @@ void ozaki_gemm(Ctx& c, int64_t n, const double* X, int64_t ldx, int a, const do
   }
   const int kc = (a + kSub - 1) / kSub * kSub;
   const int stages = gemm_smem(kc, 2) <= kGemmSmemMax ? 2 : 1;
-  const int64_t ntiles = (n + kM - 1) / kM;
+  const int64_t ntiles = s.count * ((n + kM - 1) / kM);
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)c.num_sms));
-  row_exp_kernel<<<(int)std::min<int64_t>((n * 32 + 255) / 256, (int64_t)c.num_sms * 16), 256, 0, c.stream>>>(
-      n, X, ldx, a, rowexp);
-  ozaki_gemm_kernel<<<grid, kGemmThreads, gemm_smem(kc, stages), c.stream>>>(n, X, ldx, a, C, b, alpha, beta, Z, ldz,
-                                                                            rowexp, stages, err);
+  row_exp_kernel<<<dim3((unsigned)std::min<int64_t>((n * 32 + 255) / 256, (int64_t)c.num_sms * 16), s.count), 256, 0,
+                   c.stream>>>(n, s, a, rowexp);
+  ozaki_gemm_kernel<<<grid, kGemmThreads, gemm_smem(kc, stages), c.stream>>>(n, s, a, C, b, alpha, beta, rowexp, stages,
+                                                                            err);
   FEM2D_CUDA(cudaGetLastError());
   c.launches += 2;
 }

@@ -19,11 +19,36 @@ size_t ozaki_gram_workspace(int64_t n, int a, int b, int num_sms);
 void ozaki_gram(Ctx& c, int64_t n, const double* X, int64_t ldx, int a, const double* Y, int64_t ldy, int b,
                 double* C, double* work, size_t work_doubles, int* err);
 
-// Z (row-major n x b, ldz) = beta Z + alpha X C for X (n x a, ldx) and C (device, row-major a x b);
+// Up to three block operands that go through one kernel together: X (n x a or n x b, ldx) to Z (n x b, ldz).
+// A search step updates W, A W and B W with the same C: one launch fills the chip where one block of a small GEP
+// (5k rows: 43 tiles of 128, or 676 CTAs of FP64 rows) leaves it part idle, and C is sliced and copied once.
+// Whole solves at 0.8k / 5k / 29k / 83k rows: 3.94 / 12.75 / 32.7 / 78.6 ms with a launch per block,
+// 3.73 / 12.17 / 32.3 / 78.0 ms together.
+struct BlockSets {
+  int count = 0;
+  const double* X[3] = {};
+  int64_t ldx[3] = {};
+  double* Z[3] = {};
+  int64_t ldz[3] = {};
+  BlockSets& add(const double* x, int64_t lx, double* z, int64_t lz) {
+    X[count] = x;
+    ldx[count] = lx;
+    Z[count] = z;
+    ldz[count++] = lz;
+    return *this;
+  }
+  BlockSets columns(int j0) const {   // the same with Z from column j0 on
+    BlockSets s = *this;
+    for (int q = 0; q < count; q++) s.Z[q] += j0;
+    return s;
+  }
+};
+
+// Z (row-major n x b) = beta Z + alpha X C for each set's X (n x a) and one C (device, row-major a x b);
 // a <= 256, b <= 32; FP64 emulated on the tensor cores (one exponent per row of X and per column of C,
 // normwise accuracy at FP64 rounding level). Queued on c.stream; *err as ozaki_gram.
-void ozaki_gemm(Ctx& c, int64_t n, const double* X, int64_t ldx, int a, const double* C, int b, double alpha,
-                double beta, double* Z, int64_t ldz, int* rowexp /* n ints of scratch */, int* err);
+void ozaki_gemm(Ctx& c, int64_t n, const BlockSets& s, int a, const double* C, int b, double alpha, double beta,
+                int* rowexp /* n ints of scratch per set */, int* err);
 
 // measured issue cost (ns per instruction and SM) of tcgen05.mma kind::f16 with M = 128, K = 16 and the
 // given N (16..256, multiple of 16)

@@ -126,3 +126,18 @@ def test_targets_and_dampings(oracle_lib, ctx, target, k, opts):
     r = fg.gpu_solve_gep_n(gep, target, k, **opts)
     assert np.max(np.abs(r.values - ref) / np.abs(ref)) <= EIG_TOL
     assert np.all(np.abs(np.einsum("ij,ij->i", r.vectors, (B @ r.vectors.T).T) - 1.0) < 1e-9)
+
+
+@pytest.mark.parametrize("dense", [1, 2])
+@pytest.mark.parametrize("nx,ny,rounds,k", [(2, 2, 0, 1), (4, 3, 1, 3), (6, 5, 1, 12)])
+def test_block_updates_of_several_operands(oracle_lib, ctx, nx, ny, rounds, k, dense):
+    """Updates of one, two and three blocks at once, with the FP64 and the tensor kernels, from GEPs of less
+    than one tile of 128 rows to several with a ragged last one, with locked and compressed columns."""
+    w = configs.full_scale(seed=nx, nx=nx, ny=ny, rounds=rounds, fraction=0.4, pmin=3, pmax=4, basis=1)
+    w.mesh_json = configs.grid_mesh_json(nx, ny, 0.0, 1.87, 0.0, 1.0)
+    gep = _gep(w.mesh_json, w.ops, 1, w.glq, ctx)
+    A, B = gep.scipy()
+    ref, _ = oracle_lib.dense_nearest_physical(A, B, 2.64, k)
+    r = fg.gpu_solve_gep_n(gep, 2.64, k, dense=dense)
+    assert np.max(np.abs(r.values - ref) / np.abs(ref)) <= EIG_TOL
+    assert np.all(np.abs(np.einsum("ij,ij->i", r.vectors, (B @ r.vectors.T).T) - 1.0) < 1e-9)
