@@ -1046,25 +1046,43 @@ __global__ void __launch_bounds__(128) mf_partinv_kernel(const int4* __restrict_
 
 constexpr size_t inverse_smem(int p) { return sizeof(double) * 8 * (size_t)((((p + 7) / 8 * 8) | 4) + (p + 7) / 8 * 8); }
 
-// sum_{k = k0}^{k1 - 1} A[k * f] * v[k] with four independent accumulators (eight loads in flight per
-// thread): the solve loops are latency-bound on the factor reads, not FP64-bound
-__device__ __forceinline__ double col_dot(const double* __restrict__ A, int f, const double* __restrict__ v, int k0,
-                                          int k1) {
-  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-  int k = k0;
-#pragma unroll 2
-  for (; k + 4 <= k1; k += 4) {
+// sum_{k = 0}^{n - 1} A[k * f] * v[k]; the FP64 pipe issues one warp instruction in some 19 clocks per SM, so
+// two accumulators hide its latency and cost one addition per row (four cost three)
+__device__ __forceinline__ double col_dot(const double* __restrict__ A, int f, const double* __restrict__ v, int n) {
+  double a0 = 0.0, a1 = 0.0;
+  int k = 0;
+#pragma unroll 4
+  for (; k + 2 <= n; k += 2) {
     a0 += A[(int64_t)k * f] * v[k];
     a1 += A[(int64_t)(k + 1) * f] * v[k + 1];
-    a2 += A[(int64_t)(k + 2) * f] * v[k + 2];
-    a3 += A[(int64_t)(k + 3) * f] * v[k + 3];
   }
-  for (; k < k1; k++) a0 += A[(int64_t)k * f] * v[k];
-  return (a0 + a1) + (a2 + a3);
+  if (k < n) a0 += A[(int64_t)k * f] * v[k];
+  return a0 + a1;
 }
 
-// One factorization of the plan and what a solve with it writes. A launch serves one or two of them
-// (blockIdx.z): the solves of one right-hand side with both shifted matrices go level by level together.
+// Two rows of a triangle as one loop of n steps: r1 = the first n1 products, r2 = the others. Step j takes
+// A[o1 + j s1] v[x1 + j e1] before n1 and A[o2 + j s2] v[x2 + j e2] from n1 on. The rows q and p - 1 - q have
+// the same number of products together for every q, so the lanes of a warp stay together although n1 differs:
+// with one loop per row a warp issued as many FP64 instructions as its longest rows have products, and
+// a fifth of the lanes in them were idle.
+__device__ __forceinline__ void pair_dot(const double* __restrict__ A, const double* __restrict__ v, int n, int n1, int o1,
+                                         int s1, int x1, int e1, int o2, int s2, int x2, int e2, double& r1,
+                                         double& r2) {
+  double acc = 0.0;
+  r1 = 0.0;
+#pragma unroll 4
+  for (int j = 0; j < n; j++) {
+    r1 = j == n1 ? acc : r1;
+    acc = j == n1 ? 0.0 : acc;
+    const int o = j < n1 ? o1 : o2, x = j < n1 ? x1 : x2;
+    acc += A[o] * v[x];
+    o1 += s1, o2 += s2, x1 += e1, x2 += e2;
+  }
+  r2 = n1 < n ? acc : 0.0;
+  r1 = n1 < n ? r1 : acc;
+}
+
+// One factorization of the plan and what a solve with it writes. A launch serves one or two of them: the solves of one right-hand side with both shifted matrices go level by level together.
 struct SolveSet {
   const int32_t *perm, *iperm;
   const double* F;
@@ -1081,7 +1099,8 @@ struct SolveArgs {
   int64_t ldb;
   SolveSet set[2];
   int nb;
-  int per;   // right-hand sides per CTA: blockIdx.y takes the columns from blockIdx.y * per on
+  int per;          // right-hand sides per CTA
+  int sets, parts;  // CTAs per front, one after another: a set (the low bit, when there are two) and a column range
 };
 
 // One CTA solves a front for `per` right-hand sides. The kernels are bound by the FP64 pipe (under two
@@ -1089,11 +1108,15 @@ struct SolveArgs {
 //   - global rows (B, X, the workspace) are read and written with the right-hand sides along the lanes, so
 //     a row is one contiguous access; the dot products take the rows along the lanes and read the factor
 //     contiguously. Shared columns have odd length, so both orders are free of bank conflicts.
-//   - a level with few fronts per SM splits the right-hand sides over CTAs (blockIdx.y): the SMs then
+//   - a level's largest fronts go first, and one with few fronts per SM splits the right-hand sides over
+//     CTAs: the SMs then
 //     finish together, and one CTA's gathers overlap another's dot products.
 // At 83k DoFs (1,179 leaf fronts, 24 right-hand sides) the leaf level took 348 / 315 us forward / backward
 // with column-major rows and one CTA per front; a whole solve went from 0.99 to 0.70 ms there, from 0.48 to
 // 0.31 ms at 29k DoFs and from 5.95 to 4.93 ms at 1M (13 right-hand sides on average), upper levels included.
+// With both shifted matrices in one launch it took 542 / 557 us at 95% of the FP64 issue rate; the paired
+// triangle rows, two accumulators for four and the order by size brought it to 391 / 393 us (1M: a whole
+// solve from 10.8 to 9.5 ms), at 92% of that rate while it runs: what is left is the products themselves.
 
 // the front's gathered right-hand side v[c * ld + i] (pivot rows permuted): the pivot rows' entries of
 // B, then each child's update vector added in slot order (rows are distinct within one child, so no
@@ -1136,9 +1159,9 @@ __host__ __device__ constexpr int backward_cols(int f, int p) { return (p | 1) +
 template <int NT>
 __global__ void __launch_bounds__(NT) mf_forward_small_kernel(const int32_t* __restrict__ lf, SolveArgs a) {
   extern __shared__ double sm[];
-  const int fr = lf[blockIdx.x];
-  const SolveSet set = a.set[blockIdx.z];
-  const int c0 = blockIdx.y * a.per, w = min(a.per, a.nb - c0);
+  const int fr = lf[blockIdx.x / a.parts], part = blockIdx.x % a.parts;
+  const SolveSet set = a.set[part & (a.sets - 1)];
+  const int c0 = part / a.sets * a.per, w = min(a.per, a.nb - c0);
   const FrontDesc d = a.fd[fr];
   const int f = d.f, p = d.p, lv = f | 1, ly = p | 1;
   double* v = sm;            // v[c * lv + i]
@@ -1146,21 +1169,23 @@ __global__ void __launch_bounds__(NT) mf_forward_small_kernel(const int32_t* __r
   const double* A = set.F + d.off;
   gather_front_rhs(d, a.fd, a.emap, set.iperm + a.piv_off[fr], set.W, a.woff, a.B, a.ldb, a.dofs + d.dptr,
                    set.perm + a.piv_off[fr], c0, w, lv, v);
-  // the unit lower triangle: row i is a dot product of length i, so a thread takes the rows q and
-  // p - 1 - q (p - 1 terms together) and the lanes of a warp run equally long
+  // the unit lower triangle: row i is a dot product of length i, so a thread takes the rows p - 1 - q and q
+  // (p - 1 products together), the first by rising and the second by falling columns: a warp then reads one
+  // or two columns in a step
   const int hp = (p + 1) >> 1;
   for (int t = threadIdx.x; t < hp * w; t += blockDim.x) {
-    const int c = t / hp, q = t - c * hp;
+    const int c = t / hp, q = t - c * hp, i2 = p - 1 - q;
     const double* vc = v + c * lv;
-    y[c * ly + q] = vc[q] + col_dot(A + q, f, vc, 0, q);
-    const int i2 = p - 1 - q;
-    if (i2 != q) y[c * ly + i2] = vc[i2] + col_dot(A + i2, f, vc, 0, i2);
+    double r1, r2;
+    pair_dot(A, vc, p - 1, i2, i2, f, 0, 1, q + (p - 2) * f, -f, p - 2, -1, r1, r2);
+    y[c * ly + i2] = vc[i2] + r1;
+    if (i2 != q) y[c * ly + q] = vc[q] + r2;
   }
   __syncthreads();
   const int s = f - p;
   for (int t = threadIdx.x; t < s * w; t += blockDim.x) {
     const int c = t / s, i = p + t - c * s;
-    v[c * lv + i] -= col_dot(A + i, f, y + c * ly, 0, p);
+    v[c * lv + i] -= col_dot(A + i, f, y + c * ly, p);
   }
   __syncthreads();
   double* out = set.W + a.woff[fr] + c0;
@@ -1173,9 +1198,9 @@ __global__ void __launch_bounds__(NT) mf_forward_small_kernel(const int32_t* __r
 template <int NT>
 __global__ void __launch_bounds__(NT) mf_backward_small_kernel(const int32_t* __restrict__ lf, SolveArgs a) {
   extern __shared__ double sm[];
-  const int fr = lf[blockIdx.x];
-  const SolveSet set = a.set[blockIdx.z];
-  const int c0 = blockIdx.y * a.per, w = min(a.per, a.nb - c0);
+  const int fr = lf[blockIdx.x / a.parts], part = blockIdx.x % a.parts;
+  const SolveSet set = a.set[part & (a.sets - 1)];
+  const int c0 = part / a.sets * a.per, w = min(a.per, a.nb - c0);
   const FrontDesc d = a.fd[fr];
   const int f = d.f, p = d.p;
   if (p == 0) return;
@@ -1194,17 +1219,18 @@ __global__ void __launch_bounds__(NT) mf_backward_small_kernel(const int32_t* __
   __syncthreads();
   for (int t = threadIdx.x; t < p * w; t += blockDim.x) {
     const int c = t / p, i = t - c * p;
-    z[c * lz + i] -= col_dot(A + (int64_t)p * f + i, f, xs + c * lx, 0, s);
+    z[c * lz + i] -= col_dot(A + (int64_t)p * f + i, f, xs + c * lx, s);
   }
   __syncthreads();
-  // the upper triangle: row i is a dot product of length p - i; rows q and p - 1 - q share a thread
+  // the upper triangle: row i is a dot product of length p - i; the rows q (by falling columns) and p - 1 - q
+  // (by rising ones) share a thread, p + 1 products together
   const int hp = (p + 1) >> 1;
   for (int t = threadIdx.x; t < hp * w; t += blockDim.x) {
-    const int c = t / hp, q = t - c * hp;
-    const double* zc = z + c * lz;
-    xs[c * lx + q] = col_dot(A + q, f, zc, q, p);
-    const int i2 = p - 1 - q;
-    if (i2 != q) xs[c * lx + i2] = col_dot(A + i2, f, zc, i2, p);
+    const int c = t / hp, q = t - c * hp, i2 = p - 1 - q;
+    double r1, r2;
+    pair_dot(A, z + c * lz, p + 1, p - q, q + (p - 1) * f, -f, p - 1, -1, i2 - f, f, -1, 1, r1, r2);
+    xs[c * lx + q] = r1;
+    if (i2 != q) xs[c * lx + i2] = r2;
   }
   __syncthreads();
   for (int t = threadIdx.x; t < p * w; t += blockDim.x) {
@@ -1708,6 +1734,8 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
         ll.push_back(fr);
       }
     }
+    const auto cost = [&](int32_t fr) { return (int64_t)s.p[fr] * (2 * s.f[fr] - s.p[fr]); };
+    std::stable_sort(ls.begin() + small_ptr[l], ls.end(), [&](int32_t x, int32_t y) { return cost(x) > cost(y); });
   }
   small_ptr[nlevels] = (int32_t)ls.size();
   large_ptr[nlevels] = (int32_t)ll.size();
@@ -1849,9 +1877,9 @@ void MFDevice::factor(Ctx& c, const double* va, const double* vb, double ca, dou
   }
 }
 
-// The leaf level of a tree with fewer than kSplitFronts fronts per SM splits its right-hand sides over two
-// CTAs: 1,179 fronts and 24 right-hand sides took 0.75 ms per solve instead of 0.81 (three CTAs: 0.74), while
-// at 18,502 fronts, where the level fills the chip many times over, splitting cost 3 to 10%.
+// A level with fewer than kSplitFronts CTAs per SM splits its right-hand sides over two CTAs per front and set:
+// 1,179 leaf fronts and two sets took 0.92 ms per solve instead of 0.94 (three CTAs: 1.00), 414 leaf fronts
+// 0.386 instead of 0.381; at 18,502 fronts, where the level fills the chip many times over, it cost 2 to 9%.
 constexpr int kSplitFronts = 16;
 
 // How a level of ns small fronts with `cols` doubles of shared memory per right-hand side is solved, one CTA
@@ -1915,7 +1943,7 @@ void MFDevice::solve_sets(Ctx& c, int sets, const MFFactor* f1, const MFFactor* 
   ProfScope ps(c, "mf_solve", sets * 2.0 * fbytes, sets * 2.0 * 2.0 * (fbytes / 8.0) * nb);
   const SolveSet s1{f1->perm.p, f1->iperm.p, f1->F.p, work.p, X1, ldx1};
   const SolveSet s2 = sets == 2 ? SolveSet{f2->perm.p, f2->iperm.p, f2->F.p, work2.p, X2, ldx2} : s1;
-  SolveArgs a{fd, dofs.p, ea_map.p, piv_off.p, woff.p, B, ldb, {s1, s2}, nb, nb};
+  SolveArgs a{fd, dofs.p, ea_map.p, piv_off.p, woff.p, B, ldb, {s1, s2}, nb, nb, sets, sets};
   TiledArgs ta{fd, dofs.p, piv_off.p, woff.p, reinterpret_cast<const int4*>(pull.p), B, ldb, {s1, s2}, nb, 0};
   auto tiled = [&](bool fwd, int l, const int2* items, int ni) {
     const int nt = tile_groups(sets * ni, nb, c.num_sms);
@@ -1939,7 +1967,8 @@ void MFDevice::solve_sets(Ctx& c, int sets, const MFFactor* f1, const MFFactor* 
     const int cols = fwd ? level_fwd_cols[l] : level_bwd_cols[l];
     const SmallShape s = small_shape(sets * ns, cols, nb, c.num_sms);
     a.per = s.per;
-    const dim3 grid(ns, (nb + s.per - 1) / s.per, sets);
+    a.parts = sets * ((nb + s.per - 1) / s.per);
+    const unsigned grid = (unsigned)ns * a.parts;
     const size_t smem = (size_t)cols * s.per * sizeof(double);
     const int32_t* lf = lsmall.p + small_ptr[l];
     if (fwd) {
