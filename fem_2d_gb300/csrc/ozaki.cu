@@ -177,6 +177,16 @@ template <int SH>
 __device__ __forceinline__ long long fuse_digit_sums(long long th, long long tl) {
   return (long long)((unsigned long long)th << SH) + ((tl + (1ll << (27 - SH))) >> (28 - SH));
 }
+
+// t + 2^21 v0 + 2^14 v1 + 2^7 v2 + v3 for digit sums v0 .. v3 of consecutive groups over at most 128 products:
+// group g holds g + 1 digit pairs, |v_g| <= (g + 1) 128 127^2 < 2^24, so 128 v_g + v_{g+1} stays below
+// 7 128^2 127^2 + 8 128 127^2 < 2^31 for g = 0, 2, 4, 6 and only the pairs are joined in 64 bits: half the
+// instructions of eight shifts and adds of 64 bits, which were a third of the Gram and update kernels'.
+__device__ __forceinline__ long long digit_sum(float v0, float v1, float v2, float v3, long long t) {
+  const int p = __float2int_rn(v0) * 128 + __float2int_rn(v1), q = __float2int_rn(v2) * 128 + __float2int_rn(v3);
+  return t + (long long)p * 16384 + (long long)q;
+}
+
 constexpr int kFuseGram = 20, kFuseGemm = 19, kFuseSpmm = 20;
 
 // a 2^k, exact, by an integer add to a's exponent field when a and the result are normal; otherwise by
@@ -396,18 +406,13 @@ __global__ void __launch_bounds__(kGramThreads, 2)
       const int jc = half * kHalf + cb;   // first column of this group in the C tile
       long long Th[8], Tl[8];
 #pragma unroll
-      for (int q = 0; q < 8; q++) Th[q] = Tl[q] = 0;
+      for (int g0 = 0; g0 < kDigits; g0 += 4) {
+        float v[4][8];
 #pragma unroll
-      for (int g = 0; g < kDigits; g++) {
-        float v[8];
-        tmem_ld8(lane_base + (uint32_t)(g * kN + jc), v);
+        for (int g = 0; g < 4; g++) tmem_ld8(lane_base + (uint32_t)((g0 + g) * kN + jc), v[g]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-          const long long iv = (long long)__float2int_rn(v[q]);
-          if (g < 4) Th[q] += iv << (7 * (3 - g));
-          else Tl[q] += iv << (7 * (7 - g));
-        }
+        for (int q = 0; q < 8; q++) (g0 == 0 ? Th : Tl)[q] = digit_sum(v[0][q], v[1][q], v[2][q], v[3][q], 0);
       }
 #pragma unroll
       for (int q = 0; q < 8; q++)
@@ -466,15 +471,14 @@ __global__ void __launch_bounds__(256) ozaki_reduce_kernel(const double* __restr
 // in int64, fused into one integer (fuse_digit_sums) and converted to FP64 once per output element, with
 // alpha and the power-of-two scale joined exactly in the exponent field. C's digit planes (K padded to
 // kc) stay in shared memory for all tiles. Each 128 x 32 sub-block of X is brought in by coalesced
-// asynchronous copies (cp.async, a whole row segment per warp instruction) into a padded staging
+// asynchronous copies (cp.async, whole row segments per warp instruction) into a swizzled staging
 // buffer, one sub-block ahead of its slicing when two staging buffers fit. The row exponents come from
 // a coalesced pre-pass (row_exp_kernel).
 constexpr int kGemmKMax = 256;
 constexpr int kGemmThreads = 512;
 constexpr int kGemmCols = kN / 4;                // columns of Z per thread
 constexpr int kGemmPlanes = kDigits * kPlaneA;   // digit planes of one 128 x 32 sub-block of X (64 KB)
-constexpr int kGemmRow = kSub + 1;               // staged doubles per row (padded: no bank conflicts)
-constexpr int kGemmStage = kM * kGemmRow * 8;    // one staged 128 x 32 sub-block of X (33 KB)
+constexpr int kGemmStage = kM * kSub * 8;        // one staged 128 x 32 sub-block of X (32 KB)
 constexpr int kGemmSmemMax = 227 * 1024;
 // shared memory of the block update for K padded to kc, with `stages` staging buffers
 __host__ __device__ constexpr int gemm_smem(int kc, int stages) {
@@ -511,24 +515,42 @@ __global__ void __launch_bounds__(256) row_exp_kernel(int64_t n, BlockSets sets,
   }
 }
 
-// rows of tile `tile` (counted through all sets), columns k0 .. k0 + 31, into the staging buffer sx (row r at
-// r * kGemmRow); entries outside X are zero-filled
+// double q of row r in a staging buffer: the 16-byte units of a row are permuted by the row, so eight threads
+// of consecutive rows read the same unit index without bank conflicts
+__device__ __forceinline__ int staged(int r, int q) { return r * kSub + (((q >> 1) ^ (r & 15)) << 1) + (q & 1); }
+
+// rows of tile `tile` (counted through all sets), columns k0 .. k0 + 31, into the staging buffer sx; entries
+// outside X are zero-filled. Two columns per copy where every row of X starts on a 16-byte boundary.
 __device__ __forceinline__ void gemm_stage(const BlockSets& sets, int64_t n, int a, int64_t tile, int64_t ntiles, int k0,
                                            double* sx) {
   const int set = (int)(tile / ntiles);
   tile -= set * ntiles;
   const double* __restrict__ X = sets.X[set];
   const int64_t ldx = sets.ldx[set];
+  if (((reinterpret_cast<uintptr_t>(X) & 15) | (uintptr_t)(ldx & 1)) == 0) {
 #pragma unroll
-  for (int i = 0; i < kM * kSub / kGemmThreads; i++) {
-    const int e = threadIdx.x + kGemmThreads * i;
-    const int r = e >> 5, q = e & 31;
-    const int64_t row = tile * kM + r;
-    const bool ok = row < n && k0 + q < a;
-    const double* src = ok ? X + row * ldx + k0 + q : X;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_addr(sx + r * kGemmRow + q)), "l"(src),
-                 "r"(ok ? 8 : 0)
-                 : "memory");
+    for (int i = 0; i < kM * kSub / 2 / kGemmThreads; i++) {
+      const int e = threadIdx.x + kGemmThreads * i;
+      const int r = e >> 4, q = 2 * (e & 15);
+      const int64_t row = tile * kM + r;
+      const int cols = row < n ? min(2, max(0, a - k0 - q)) : 0;
+      const double* src = cols > 0 ? X + row * ldx + k0 + q : X;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(sx + staged(r, q))), "l"(src),
+                   "r"(8 * cols)
+                   : "memory");
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < kM * kSub / kGemmThreads; i++) {
+      const int e = threadIdx.x + kGemmThreads * i;
+      const int r = e >> 5, q = e & 31;
+      const int64_t row = tile * kM + r;
+      const bool ok = row < n && k0 + q < a;
+      const double* src = ok ? X + row * ldx + k0 + q : X;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_addr(sx + staged(r, q))), "l"(src),
+                   "r"(ok ? 8 : 0)
+                   : "memory");
+    }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -633,7 +655,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       __syncthreads();   // every thread's copies of this sub-block have landed
       double xv[8];
 #pragma unroll
-      for (int q = 0; q < 8; q++) xv[q] = sx[rl * kGemmRow + part * 8 + q];
+      for (int q = 0; q < 8; q += 2) {
+        const double2 x2 = *reinterpret_cast<const double2*>(sx + staged(rl, part * 8 + q));
+        xv[q] = x2.x;
+        xv[q + 1] = x2.y;
+      }
       if (pending) {   // the digit planes are free once the previous MMAs completed
         if (mbar_wait(smem_addr(bar), ph)) {
           ph ^= 1u;
@@ -707,13 +733,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           for (int g = 0; g < 4; g++) tmem_ld8(lane_base + (uint32_t)((g0 + g) * kN + part * kGemmCols), v[g]);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int g = 0; g < 4; g++)
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-              const long long iv = (long long)__float2int_rn(v[g][q]) << (7 * (3 - g));
-              if (g0 == 0) Th[q] += iv;
-              else Tl[q] += iv;
-            }
+          for (int q = 0; q < 8; q++) {
+            long long& T = (g0 == 0 ? Th : Tl)[q];
+            T = digit_sum(v[0][q], v[1][q], v[2][q], v[3][q], T);
+          }
         }
         // every thread's reads of the accumulators precede the next MMAs
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -780,6 +803,8 @@ constexpr int kSpXPlaneP = 16 * kSpK * 2;               // 16 columns (2 KB)
 constexpr int kSpXBytes = 11 * kSpXPlaneW;              // 3 zero + 8 digit planes (wide); 7 + 8 (packed)
 constexpr int kSpMBytes = 2 * kDigits * 64 * 64 + 2048; // planes of a 64-row item + row-block overrun
 constexpr int kSpSmem = kSpXBytes + kSpMBytes + 1536;   // one stage; two CTAs per SM
+constexpr int kSpDPlaneW = 64 * 32;        // floats of a group's digit sums in the M buffer, 32 columns
+constexpr int kSpDPlaneP = 64 * 16 + 16;   // 16 columns (a warp writes two planes: 16 banks apart)
 constexpr uint32_t kSpTmemCols = 128;
 
 // uint4 units of one item's digit planes: 2 sub-blocks of 32 K x 8 planes x R8 rows x 4 k-groups
@@ -981,7 +1006,7 @@ __global__ void __launch_bounds__(kSpThreads, 2)
   for (int idx = i0, k = 0; idx < i1; idx++, k++) {
     const TcSpmmItem w = items[idx];
     const bool more = idx + 1 < i1;
-    const int R = w.R, R8 = (R + 7) & ~7, nrb = (R + 31) >> 5;
+    const int R = w.R, R8 = (R + 7) & ~7;
     int* ecs = ecol + 32 * (k & 1);
     int* ems = em + 64 * (k & 1);
     // the item's digit planes of M (the buffer's previous readers finished before the last barrier)
@@ -1058,77 +1083,61 @@ __global__ void __launch_bounds__(kSpThreads, 2)
       failed = true;
       break;
     }
-    // readout into the M buffer (its planes are consumed): per lane (group g, column j) the exact int64
-    // digit sums T_hi = sum_{g<4} D_g 2^(7 (3 - g)), T_lo = sum_{g>=4} D_g 2^(7 (7 - g)), one partial per
-    // warp; D_g < 8 * 64 * 127^2 < 2^23, so the partials stay below 2^46. Lanes stay in integers: the FP64
-    // conversion is done once per output by its owner (GB300's FP64 pipe is the scarce unit)
-    long long* PH = reinterpret_cast<long long*>(ms);
-    long long* PL = PH + 4096;
-    const int rounds = packed ? 1 : nrb;
-    for (int rb = 0; rb < rounds; rb++) {
-      if (!packed) {
-        // lane (r = warp % 4, column j = lane): groups r (block 0) and 4 + r (block 1) of row block rb;
-        // warps 0-3 take the first half of its row groups, 4-7 the second
-        const int r = warp & 3, j = lane;
-        const int ngr = min(32, R - 32 * rb) > 16 ? 4 : 2;
-        const int g0 = warp < 4 ? 0 : ngr / 2, g1 = warp < 4 ? ngr / 2 : ngr;
-        for (int ig = g0; ig < g1; ig++) {
-          float v0[8], v1[8];
-          tmem_ld8(lane_base + (uint32_t)(rb * 32 + ig * 8), v0);
-          tmem_ld8(lane_base + (uint32_t)(64 + rb * 32 + ig * 8), v1);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    // readout into the M buffer (its planes are consumed): the digit sums D_g of the run's rows as they are, one
+    // plane per group g; |D_g| <= 8 * 64 * 127^2 < 2^23. Their owners join them in integers and convert once
+    // per output (GB300's FP64 pipe is the scarce unit).
+    float* D = reinterpret_cast<float*>(ms);
+    const int ng = (R + 7) >> 3;   // groups of 8 rows = TMEM columns
+    if (!packed) {
+      // lane (r = warp % 4, column j = lane): group r at TMEM column 0 (warps 0-3), 4 + r at 64 (warps 4-7)
+      const uint32_t src = lane_base + (uint32_t)((warp >> 2) * 64);
+      float* dst = D + warp * kSpDPlaneW + lane;
+      int ig = 0;
+      for (; ig + 2 <= ng; ig += 2) {
+        float v0[8], v1[8];
+        tmem_ld8(src + (uint32_t)(ig * 8), v0);
+        tmem_ld8(src + (uint32_t)(ig * 8 + 8), v1);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int q = 0; q < 8; q++) {
-            const int e = (r * 32 + ig * 8 + q) * 32 + j;
-            PH[e] = (long long)__float2int_rn(v0[q]) << (7 * (3 - r));
-            PL[e] = (long long)__float2int_rn(v1[q]) << (7 * (3 - r));
-          }
-        }
-      } else {
-        // lane (group g = 2 (warp % 4) + lane / 16, column j = lane % 16); the two groups of a warp are
-        // both below 4 (warps 0, 1) or both above (2, 3) and are added by a shuffle; warps 0-3 and 4-7
-        // split the row groups (the two row blocks, or the halves of one)
-        const int g = 2 * (warp & 3) + (lane >> 4), j = lane & 15;
-        const int sh = g < 4 ? 7 * (3 - g) : 7 * (7 - g);
-        const int ngr_total = nrb == 2 ? 4 + ((R - 32) > 16 ? 4 : 2) : (R > 16 ? 4 : 2);
-        const int first = warp < 4 ? 0 : (nrb == 2 ? 4 : ngr_total / 2);
-        const int last = warp < 4 ? (nrb == 2 ? 4 : ngr_total / 2) : ngr_total;
-        for (int gi = first; gi < last; gi++) {
-          const int b = gi >> 2, ig = gi & 3;
-          float v[8];
-          tmem_ld8(lane_base + (uint32_t)(b * 32 + ig * 8), v);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int q = 0; q < 8; q++) {
-            long long t = (long long)__float2int_rn(v[q]) << sh;
-            t += __shfl_xor_sync(0xffffffffu, t, 16);
-            if (lane < 16) PH[((warp & 3) * 64 + b * 32 + ig * 8 + q) * 16 + j] = t;
-          }
+        for (int q = 0; q < 8; q++) {
+          dst[(ig * 8 + q) * 32] = v0[q];
+          dst[(ig * 8 + 8 + q) * 32] = v1[q];
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncthreads();
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // convert: thread tid owns pairs p = tid + 256 o of the run (row p / 32 and column p % 32, or
-      // row p / 16 and column p % 16 with nb <= 16); the partials are added in a fixed order
+      if (ig < ng) {
+        float v0[8];
+        tmem_ld8(src + (uint32_t)(ig * 8), v0);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int o = 0; o < 8; o++) {
-        const int p = tid + 256 * o;
-        const int i = packed ? p >> 4 : p >> 5, j = packed ? p & 15 : p & 31;
-        const bool mine = packed ? o < 4 : (o >> 2) == rb;
-        if (!mine || i >= R || j >= nb) continue;
-        long long th, tl;
-        if (packed) {
-          th = PH[i * 16 + j] + PH[(64 + i) * 16 + j];
-          tl = PH[(128 + i) * 16 + j] + PH[(192 + i) * 16 + j];
-        } else {
-          const int e = (i - 32 * rb) * 32 + j;
-          th = PH[e] + PH[1024 + e] + PH[2048 + e] + PH[3072 + e];
-          tl = PL[e] + PL[1024 + e] + PL[2048 + e] + PL[3072 + e];
-        }
-        acc[o] = fma((double)fuse_digit_sums<kFuseSpmm>(th, tl), pow2(ecs[j] + ems[i] - 2044 - 35 - kFuseSpmm), acc[o]);
+        for (int q = 0; q < 8; q++) dst[(ig * 8 + q) * 32] = v0[q];
       }
-      if (rb + 1 < rounds) __syncthreads();
+    } else {
+      // lane (group g = 2 (warp % 4) + lane / 16, column j = lane % 16); warps 0-3 and 4-7 take the even and
+      // the odd row groups
+      float* dst = D + (2 * (warp & 3) + (lane >> 4)) * kSpDPlaneP + (lane & 15);
+      for (int ig = warp >> 2; ig < ng; ig += 2) {
+        float v[8];
+        tmem_ld8(lane_base + (uint32_t)(ig * 8), v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int q = 0; q < 8; q++) dst[(ig * 8 + q) * 16] = v[q];
+      }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // convert: thread tid owns pairs p = tid + 256 o of the run (row p / 32 and column p % 32, or row p / 16 and
+    // column p % 16 with nb <= 16)
+#pragma unroll
+    for (int o = 0; o < 8; o++) {
+      const int p = tid + 256 * o;
+      const int i = packed ? p >> 4 : p >> 5, j = packed ? p & 15 : p & 31;
+      if ((packed && o >= 4) || i >= R || j >= nb) continue;
+      const float* d = D + p;
+      const int ld = packed ? kSpDPlaneP : kSpDPlaneW;
+      const long long th = digit_sum(d[0], d[ld], d[2 * ld], d[3 * ld], 0);
+      const long long tl = digit_sum(d[4 * ld], d[5 * ld], d[6 * ld], d[7 * ld], 0);
+      acc[o] = fma((double)fuse_digit_sums<kFuseSpmm>(th, tl), pow2(ecs[j] + ems[i] - 2044 - 35 - kFuseSpmm), acc[o]);
     }
     if (w.last) {   // the run is complete: its rows of Y
 #pragma unroll
