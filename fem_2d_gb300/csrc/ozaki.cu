@@ -463,27 +463,37 @@ __global__ void __launch_bounds__(256) ozaki_reduce_kernel(const double* __restr
 // ---------------------------------------------------------------------------------------------------
 // Z = beta Z + alpha X C for a tall X (n x a, a <= 256) and a small C (a x b, b <= 32): the block
 // updates of the B-orthogonalisation and the Ritz-vector products. Each CTA owns 128-row tiles of X
-// and Z (TMEM lane = row; 16 warps, four threads per row, each slicing 8 of a sub-block's 32 columns of
-// X and owning 8 of the 32 columns of Z: with two threads per row one CTA of 8 warps, all that fits an SM,
-// issued on 28% of its cycles and waited on loads and barriers for the rest). X is sliced with one exponent per row (over its a entries)
-// and C with one per column (over its a entries), so every K sub-block's digit sums share one scale:
-// they are read from TMEM after each 128 columns of K (the exact-accumulation limit) and summed exactly
-// in int64, fused into one integer (fuse_digit_sums) and converted to FP64 once per output element, with
-// alpha and the power-of-two scale joined exactly in the exponent field. C's digit planes (K padded to
-// kc) stay in shared memory for all tiles. Each 128 x 32 sub-block of X is brought in by coalesced
-// asynchronous copies (cp.async, whole row segments per warp instruction) into a swizzled staging
-// buffer, one sub-block ahead of its slicing when two staging buffers fit. The row exponents come from
-// a coalesced pre-pass (row_exp_kernel).
+// and Z (TMEM lane = row) and goes through X in sub-blocks of 8 PARTS columns. X is sliced with one exponent
+// per row (over its a entries) and C with one per column (over its a entries), so every K sub-block's digit
+// sums share one scale: they are read from TMEM after each 128 columns of K (the exact-accumulation limit) and
+// summed exactly in int64, fused into one integer (fuse_digit_sums) and converted to FP64 once per output
+// element, with alpha and the power-of-two scale joined exactly in the exponent field. C's digit planes (K
+// padded to kc) stay in shared memory for all tiles. Each sub-block of X is brought in by coalesced
+// asynchronous copies (cp.async, whole row segments per warp instruction) into a swizzled staging buffer, one
+// sub-block ahead of its slicing when two staging buffers fit. The row exponents come from a coalesced
+// pre-pass (row_exp_kernel).
+//
+// The phases of a sub-block (copies, slicing, MMAs, read-out) depend on one another, so one CTA alone waits at
+// barriers for half of its time (issuing on 41% of its cycles). Up to 128 columns of K two CTAs of 256
+// threads with sub-blocks of 16 columns share an SM and fill each other's waits: 72 columns at 83k rows took
+// 70 us on average with one CTA of 512 threads, 53 us with two (1M rows, with the exponent pass: 965 and
+// 792 us). Above 128 columns the planes of C leave no room for two, and one CTA of 512 threads is the
+// better half: with 256 threads it issued on 28% of its cycles.
 constexpr int kGemmKMax = 256;
-constexpr int kGemmThreads = 512;
-constexpr int kGemmCols = kN / 4;                // columns of Z per thread
-constexpr int kGemmPlanes = kDigits * kPlaneA;   // digit planes of one 128 x 32 sub-block of X (64 KB)
-constexpr int kGemmStage = kM * kSub * 8;        // one staged 128 x 32 sub-block of X (32 KB)
-constexpr int kGemmSmemMax = 227 * 1024;
-// shared memory of the block update for K padded to kc, with `stages` staging buffers
-__host__ __device__ constexpr int gemm_smem(int kc, int stages) {
-  return kGemmPlanes + stages * kGemmStage + kDigits * kN * kc * 2 + 1024;
-}
+// The two shapes of the kernel: PARTS threads per row of a tile, each slicing 8 of a sub-block's 8 PARTS columns
+// of X and owning 32 / PARTS columns of Z.
+template <int PARTS>
+struct GemmShape {
+  static constexpr int threads = kM * PARTS, sub = 8 * PARTS, cols = kN / PARTS;
+  static constexpr int plane = kM * sub * 2;   // one digit plane of a sub-block of X
+  static constexpr int stage = kM * sub * 8;   // one staged sub-block of X
+  // shared memory for K padded to kc, with `stages` staging buffers
+  static constexpr int smem(int kc, int stages) {
+    return kDigits * plane + stages * stage + kDigits * kN * kc * 2 + 1024;
+  }
+};
+constexpr int kGemmSmemMax = 227 * 1024;    // one CTA per SM
+constexpr int kGemmSmemHalf = 113 * 1024;   // two
 
 // byte offset of core matrix (row group rg, k group kg) in a K-major tile with kc columns
 __device__ __forceinline__ int core_off_k(int rg, int kg, int kc) { return (rg * (kc / 8) + kg) * 128; }
@@ -517,37 +527,42 @@ __global__ void __launch_bounds__(256) row_exp_kernel(int64_t n, BlockSets sets,
 
 // double q of row r in a staging buffer: the 16-byte units of a row are permuted by the row, so eight threads
 // of consecutive rows read the same unit index without bank conflicts
-__device__ __forceinline__ int staged(int r, int q) { return r * kSub + (((q >> 1) ^ (r & 15)) << 1) + (q & 1); }
+template <int SUB>
+__device__ __forceinline__ int staged(int r, int q) {
+  return r * SUB + (((q >> 1) ^ (r & (SUB / 2 - 1))) << 1) + (q & 1);
+}
 
-// rows of tile `tile` (counted through all sets), columns k0 .. k0 + 31, into the staging buffer sx; entries
-// outside X are zero-filled. Two columns per copy where every row of X starts on a 16-byte boundary.
+// rows of tile `tile` (counted through all sets), columns k0 .. k0 + sub - 1, into the staging buffer sx;
+// entries outside X are zero-filled. Two columns per copy where every row of X starts on a 16-byte boundary.
+template <int PARTS>
 __device__ __forceinline__ void gemm_stage(const BlockSets& sets, int64_t n, int a, int64_t tile, int64_t ntiles, int k0,
                                            double* sx) {
+  constexpr int SUB = GemmShape<PARTS>::sub, NT = GemmShape<PARTS>::threads;
   const int set = (int)(tile / ntiles);
   tile -= set * ntiles;
   const double* __restrict__ X = sets.X[set];
   const int64_t ldx = sets.ldx[set];
   if (((reinterpret_cast<uintptr_t>(X) & 15) | (uintptr_t)(ldx & 1)) == 0) {
 #pragma unroll
-    for (int i = 0; i < kM * kSub / 2 / kGemmThreads; i++) {
-      const int e = threadIdx.x + kGemmThreads * i;
-      const int r = e >> 4, q = 2 * (e & 15);
+    for (int i = 0; i < kM * SUB / 2 / NT; i++) {
+      const int e = threadIdx.x + NT * i;
+      const int r = e / (SUB / 2), q = 2 * (e % (SUB / 2));
       const int64_t row = tile * kM + r;
       const int cols = row < n ? min(2, max(0, a - k0 - q)) : 0;
       const double* src = cols > 0 ? X + row * ldx + k0 + q : X;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(sx + staged(r, q))), "l"(src),
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(sx + staged<SUB>(r, q))), "l"(src),
                    "r"(8 * cols)
                    : "memory");
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < kM * kSub / kGemmThreads; i++) {
-      const int e = threadIdx.x + kGemmThreads * i;
-      const int r = e >> 5, q = e & 31;
+    for (int i = 0; i < kM * SUB / NT; i++) {
+      const int e = threadIdx.x + NT * i;
+      const int r = e / SUB, q = e % SUB;
       const int64_t row = tile * kM + r;
       const bool ok = row < n && k0 + q < a;
       const double* src = ok ? X + row * ldx + k0 + q : X;
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_addr(sx + staged(r, q))), "l"(src),
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_addr(sx + staged<SUB>(r, q))), "l"(src),
                    "r"(ok ? 8 : 0)
                    : "memory");
     }
@@ -555,22 +570,25 @@ __device__ __forceinline__ void gemm_stage(const BlockSets& sets, int64_t n, int
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-__global__ void __launch_bounds__(kGemmThreads, 1)
+template <int PARTS>
+__global__ void __launch_bounds__(GemmShape<PARTS>::threads, PARTS == 4 ? 1 : 2)
     ozaki_gemm_kernel(int64_t n, const __grid_constant__ BlockSets sets, int a, const double* __restrict__ C, int b,
                       double alpha, double beta, const int* __restrict__ EXr, int stages, int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  const int kc = (a + kSub - 1) / kSub * kSub;     // K padded to whole sub-blocks
+  using S = GemmShape<PARTS>;
+  constexpr int SUB = S::sub, COLS = S::cols;
+  const int kc = (a + SUB - 1) / SUB * SUB;        // K padded to whole sub-blocks
   const int planeC = kN * kc * 2;                  // one digit plane of C (32 x kc bf16, K-major)
   uint8_t* sA = smem;                              // digit planes of the current sub-block of X
-  double* sX = reinterpret_cast<double*>(smem + kGemmPlanes);   // staging buffers
-  uint8_t* sC = smem + kGemmPlanes + stages * kGemmStage;
+  double* sX = reinterpret_cast<double*>(smem + kDigits * S::plane);   // staging buffers
+  uint8_t* sC = smem + kDigits * S::plane + stages * S::stage;
   int* eC = reinterpret_cast<int*>(sC + kDigits * planeC);   // kN column exponents of C
   uint64_t* bar = reinterpret_cast<uint64_t*>(eC + kN);       // MMAs committed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int rl = tid & (kM - 1), part = tid >> 7;  // row of the tile (TMEM lane), column quarter
+  const int rl = tid & (kM - 1), part = tid >> 7;  // row of the tile (TMEM lane), column part
   const int64_t ntiles = (n + kM - 1) / kM, total = sets.count * ntiles;
-  const int nsub = kc / kSub;
+  const int nsub = kc / SUB;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
@@ -584,18 +602,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   }
   // the first sub-block's copies, then C's column exponents and digit planes (row j of the B operand =
   // column j of C)
-  if (blockIdx.x < total) gemm_stage(sets, n, a, blockIdx.x, ntiles, 0, sX);
+  if (blockIdx.x < total) gemm_stage<PARTS>(sets, n, a, blockIdx.x, ntiles, 0, sX);
   if (tid < kN) eC[tid] = 0;
   __syncthreads();
   {
     const int j = tid % kN;
     int e = 0;
     if (j < b)
-      for (int k = tid / kN; k < a; k += kGemmThreads / kN) e = max(e, biased_exp(C[(int64_t)k * b + j]));
+      for (int k = tid / kN; k < a; k += S::threads / kN) e = max(e, biased_exp(C[(int64_t)k * b + j]));
     atomicMax(&eC[j], e);
   }
   __syncthreads();
-  for (int t = tid; t < kN * (kc / 8); t += kGemmThreads) {
+  for (int t = tid; t < kN * (kc / 8); t += S::threads) {
     const int j = t % kN, kg = t / kN;
     uint32_t pk[kDigits][4];
 #pragma unroll
@@ -619,7 +637,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const uint32_t tmem = *tmem_slot;
   bool failed = false;
   const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  const uint64_t dA = smem_desc(smem_addr(sA), 128, (kSub / 8) * 128);
+  const uint64_t dA = smem_desc(smem_addr(sA), 128, (SUB / 8) * 128);
   const uint64_t dC = smem_desc(smem_addr(sC), 128, (uint32_t)kc * 16u);
   uint32_t ph = 0u;
   bool pending = false;   // MMAs committed and not yet waited for (they read sA)
@@ -630,24 +648,42 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const int64_t row = (tile - set * ntiles) * kM + rl;
     const bool row_ok = row < n;
     const int Ex = row_ok ? EXr[set * n + row] : 0;
-    double* Zr = sets.Z[set] + row * sets.ldz[set] + part * kGemmCols;
-    long long Th[kGemmCols], Tl[kGemmCols];
+    double* Zr = sets.Z[set] + row * sets.ldz[set] + part * COLS;
+    long long Th[8], Tl[8];
 #pragma unroll
-    for (int j = 0; j < kGemmCols; j++) Th[j] = Tl[j] = 0;
-    double zv[kGemmCols];
+    for (int q = 0; q < 8; q++) Th[q] = Tl[q] = 0;
+    double zv[8];
+    const auto load_z = [&](int cb) {
+      if (beta == 0.0 || !row_ok) return;
+#pragma unroll
+      for (int q = 0; q < 8; q++) zv[q] = part * COLS + cb + q < b ? Zr[cb + q] : 0.0;
+    };
+    // one conversion and one multiply (or FMA) per output: alpha and the power-of-two scale are combined
+    // exactly in the exponent field
+    const auto store_z = [&](int cb) {
+      if (!row_ok) return;
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int j = part * COLS + cb + q;
+        if (j >= b) break;
+        const double t = (double)fuse_digit_sums<kFuseGemm>(Th[q], Tl[q]);
+        const double m = scale_pow2(alpha, Ex + eC[j] - 2044 - 35 - kFuseGemm);
+        Zr[cb + q] = beta == 0.0 ? t * m : fma(t, m, beta == 1.0 ? zv[q] : beta * zv[q]);
+      }
+    };
     for (int sb = 0; sb < nsub && !failed; sb++, sbc++) {
-      const int k0 = sb * kSub;
-      const double* sx = sX + (stages == 2 ? (sbc & 1) : 0) * (kGemmStage / 8);
+      const int k0 = sb * SUB;
+      const double* sx = sX + (stages == 2 ? (sbc & 1) : 0) * (S::stage / 8);
       // the next sub-block's copies into the other staging buffer (with one buffer, after the slicing)
       int64_t nt = tile;
-      int nk = k0 + kSub;
+      int nk = k0 + SUB;
       if (nk >= kc) {
         nt = tile + gridDim.x;
         nk = 0;
       }
       const bool more = nt < total;
       if (stages == 2 && more) {
-        gemm_stage(sets, n, a, nt, ntiles, nk, sX + ((sbc + 1) & 1) * (kGemmStage / 8));
+        gemm_stage<PARTS>(sets, n, a, nt, ntiles, nk, sX + ((sbc + 1) & 1) * (S::stage / 8));
         asm volatile("cp.async.wait_group 1;" ::: "memory");
       } else {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -656,7 +692,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       double xv[8];
 #pragma unroll
       for (int q = 0; q < 8; q += 2) {
-        const double2 x2 = *reinterpret_cast<const double2*>(sx + staged(rl, part * 8 + q));
+        const double2 x2 = *reinterpret_cast<const double2*>(sx + staged<SUB>(rl, part * 8 + q));
         xv[q] = x2.x;
         xv[q + 1] = x2.y;
       }
@@ -678,10 +714,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 #pragma unroll
           for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = d[s2];
         }
-        const int off = core_off(rl >> 3, part) + (rl & 7) * 16;
+        const int off = ((rl >> 3) * (SUB / 8) + part) * 128 + (rl & 7) * 16;
 #pragma unroll
         for (int s2 = 0; s2 < kDigits; s2++)
-          *reinterpret_cast<uint4*>(sA + s2 * kPlaneA + off) = make_uint4(pk[s2][0], pk[s2][1], pk[s2][2], pk[s2][3]);
+          *reinterpret_cast<uint4*>(sA + s2 * S::plane + off) = make_uint4(pk[s2][0], pk[s2][1], pk[s2][2], pk[s2][3]);
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -691,7 +727,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // with one staging buffer the next sub-block's copies start now (its slot was read above)
-      if (stages == 1 && more) gemm_stage(sets, n, a, nt, ntiles, nk, sX);
+      if (stages == 1 && more) gemm_stage<PARTS>(sets, n, a, nt, ntiles, nk, sX);
       const bool first = (k0 % kChunk) == 0;   // the accumulators restart every 128 columns of K
       if (tid == 0) {
 #pragma unroll 1
@@ -700,20 +736,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 #pragma unroll 1
         for (int s2 = 0; s2 < kDigits; s2++)
 #pragma unroll
-          for (int kk = 0; kk < kSub / 16; kk++) {
+          for (int kk = 0; kk < SUB / 16; kk++) {
             const uint32_t accum = (!first || s2 > 0 || kk > 0) ? 1u : 0u;
-            mma_bf16(tmem + (uint32_t)(s2 * kN), dA + (uint64_t)((s2 * kPlaneA + kk * 256) >> 4),
+            mma_bf16(tmem + (uint32_t)(s2 * kN), dA + (uint64_t)((s2 * S::plane + kk * 256) >> 4),
                      dC + (uint64_t)((((k0 / 8) + 2 * kk) * 128) >> 4), instr_desc(kM, (kDigits - s2) * kN), accum);
           }
         mma_commit(smem_addr(bar));
       }
       pending = true;
-      const bool last = (k0 + kSub) % kChunk == 0 || k0 + kSub >= kc;
+      const bool all = k0 + SUB >= kc, last = (k0 + SUB) % kChunk == 0 || all;
       if (last) {   // the accumulators are read back: wait for these MMAs now (the old Z in flight meanwhile)
-        if (beta != 0.0 && k0 + kSub >= kc && row_ok) {
-#pragma unroll
-          for (int q = 0; q < kGemmCols; q++) zv[q] = part * kGemmCols + q < b ? Zr[q] : 0.0;
-        }
+        if (all) load_z(0);
         if (mbar_wait(smem_addr(bar), ph)) {
           ph ^= 1u;
           pending = false;
@@ -727,16 +760,25 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         }
         // exact digit sums of these (at most 128) columns of K into the int64 accumulators
 #pragma unroll
-        for (int g0 = 0; g0 < kDigits; g0 += 4) {
-          float v[4][8];
+        for (int cb = 0; cb < COLS; cb += 8) {
+          if (PARTS == 2) {   // one chunk: eight columns of Z at a time
+            if (cb > 0) load_z(cb);
 #pragma unroll
-          for (int g = 0; g < 4; g++) tmem_ld8(lane_base + (uint32_t)((g0 + g) * kN + part * kGemmCols), v[g]);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int q = 0; q < 8; q++) {
-            long long& T = (g0 == 0 ? Th : Tl)[q];
-            T = digit_sum(v[0][q], v[1][q], v[2][q], v[3][q], T);
+            for (int q = 0; q < 8; q++) Th[q] = Tl[q] = 0;
           }
+#pragma unroll
+          for (int g0 = 0; g0 < kDigits; g0 += 4) {
+            float v[4][8];
+#pragma unroll
+            for (int g = 0; g < 4; g++) tmem_ld8(lane_base + (uint32_t)((g0 + g) * kN + part * COLS + cb), v[g]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+              long long& T = (g0 == 0 ? Th : Tl)[q];
+              T = digit_sum(v[0][q], v[1][q], v[2][q], v[3][q], T);
+            }
+          }
+          if (PARTS == 2) store_z(cb);
         }
         // every thread's reads of the accumulators precede the next MMAs
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -745,18 +787,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
     }
     if (failed) break;
-    if (row_ok) {
-      // one conversion and one multiply (or FMA) per output: alpha and the power-of-two scale are
-      // combined exactly in the exponent field
-#pragma unroll
-      for (int q = 0; q < kGemmCols; q++) {
-        const int j = part * kGemmCols + q;
-        if (j >= b) break;
-        const double t = (double)fuse_digit_sums<kFuseGemm>(Th[q], Tl[q]);
-        const double m = scale_pow2(alpha, Ex + eC[j] - 2044 - 35 - kFuseGemm);
-        Zr[q] = beta == 0.0 ? t * m : fma(t, m, beta == 1.0 ? zv[q] : beta * zv[q]);
-      }
-    }
+    if (PARTS == 4) store_z(0);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");   // no copy outlives the kernel
   if (failed && tid == 0) {   // every thread arrives here (uniform exits)
@@ -1240,18 +1271,23 @@ void ozaki_gemm(Ctx& c, int64_t n, const BlockSets& s, int a, const double* C, i
   {
     std::lock_guard<std::mutex> lk(mu);
     if (c.device >= 0 && c.device < 256 && !done[c.device]) {
-      FEM2D_CUDA(cudaFuncSetAttribute(ozaki_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemMax));
+      FEM2D_CUDA(cudaFuncSetAttribute(ozaki_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemHalf));
+      FEM2D_CUDA(cudaFuncSetAttribute(ozaki_gemm_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemMax));
       done[c.device] = true;
     }
   }
-  const int kc = (a + kSub - 1) / kSub * kSub;
-  const int stages = gemm_smem(kc, 2) <= kGemmSmemMax ? 2 : 1;
   const int64_t ntiles = s.count * ((n + kM - 1) / kM);
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)c.num_sms));
   row_exp_kernel<<<dim3((unsigned)std::min<int64_t>((n * 32 + 255) / 256, (int64_t)c.num_sms * 16), s.count), 256, 0,
                    c.stream>>>(n, s, a, rowexp);
-  ozaki_gemm_kernel<<<grid, kGemmThreads, gemm_smem(kc, stages), c.stream>>>(n, s, a, C, b, alpha, beta, rowexp, stages,
-                                                                            err);
+  const auto launch = [&](auto kernel, auto shape, int per_sm, int limit) {
+    using S = decltype(shape);
+    const int kc = (a + S::sub - 1) / S::sub * S::sub;
+    const int stages = S::smem(kc, 2) <= limit ? 2 : 1;
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)c.num_sms * per_sm));
+    kernel<<<grid, S::threads, S::smem(kc, stages), c.stream>>>(n, s, a, C, b, alpha, beta, rowexp, stages, err);
+  };
+  if (a <= kChunk) launch(ozaki_gemm_kernel<2>, GemmShape<2>{}, 2, kGemmSmemHalf);
+  else launch(ozaki_gemm_kernel<4>, GemmShape<4>{}, 1, kGemmSmemMax);
   FEM2D_CUDA(cudaGetLastError());
   c.launches += 2;
 }
