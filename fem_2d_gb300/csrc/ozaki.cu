@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(256) chunk_exp_kernel(int64_t n, const double*
 // w + 4 read the two column halves of the same TMEM lanes back
 constexpr int kGramThreads = 256;
 
+constexpr int kGramUnits = (kM / 32 + 1) * 4 * 32 / kGramThreads + 1;   // most units of a warp
 __global__ void __launch_bounds__(kGramThreads, 2)
     ozaki_gram_kernel(int64_t n, const double* __restrict__ X, int64_t ldx, int a, const double* __restrict__ Y,
                       int64_t ldy, int b, int64_t rows_per_cta, const int* __restrict__ EX, const int* __restrict__ EY,
@@ -247,10 +248,11 @@ __global__ void __launch_bounds__(kGramThreads, 2)
   uint8_t* sA = smem;                                   // kDigits planes of kM x kSub bf16
   uint8_t* sB = smem + kDigits * kPlaneA;               // kDigits planes of kN x kSub bf16
   int* eY = reinterpret_cast<int*>(sB + kDigits * kPlaneB);   // kN column exponents of Y in the chunk
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(eY + kN);
+  int* eX = eY + kN;                                          // kM of X
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(eX + kM);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row = tid & (kM - 1), half = tid >> 7;   // row of the C tile (TMEM lane), column half
   const int col0 = blockIdx.z * kM;    // first column of X in this tile
   const int cy0 = blockIdx.y * kN;     // first column of Y
@@ -284,34 +286,35 @@ __global__ void __launch_bounds__(kGramThreads, 2)
 #pragma unroll
   for (int j = 0; j < kHalf; j++) acc[j] = 0.0;
 
-  const int my_col = col0 + row;   // this thread's column of X (its row of C)
-  const bool col_ok = my_col < a;
-  // warps whose 32 rows of the tile all lie past column a of X skip their loads, slicing and readout
+  // warps whose 32 rows of the tile all lie past column a of X skip the readout
   const bool xw = col0 + 32 * (warp & 3) < a;
-  const int yj = tid % kN, ykg = tid / kN;   // threads 0..127: a column of Y and its 8-row group
-  const bool y_ok = tid < kN * (kSub / 8) && cy0 + yj < b;
+  // a sub-block is sliced in units of 32 columns x 8 rows, four per group of columns: first the tile's groups
+  // of X that hold columns, then Y. Warp w takes the units w, w + 8, ...: at most one with up to 32 columns
+  // of X in the tile, two up to 96 and three beyond, where a fixed share of X and Y per thread left the first
+  // warps three at every width and the others waiting (a product with its exponents and sums, on average:
+  // 88.5 us at 83k rows and 755 at 1M, now 81.6 and 684).
+  const int xgroups = min(kM / 32, (a - col0 + 31) / 32), units = 4 * (xgroups + 1);
 
   for (int64_t c0 = r0; c0 < r1 && !failed; c0 += kChunk) {
     const int64_t chunk = c0 / kChunk;
-    const int Ex = col_ok ? EX[chunk * a + my_col] : 0;
-    if (tid < kN) eY[tid] = (cy0 + tid < b) ? EY[chunk * b + cy0 + tid] : 0;
+    if (tid < kM) eX[tid] = col0 + tid < a ? EX[chunk * a + col0 + tid] : 0;
+    else if (tid < kM + kN) eY[tid - kM] = cy0 + tid - kM < b ? EY[chunk * b + cy0 + tid - kM] : 0;
     __syncthreads();
-    const int Ey = eY[yj];
+    const int Ex = eX[row];
     for (int sb = 0; sb < kChunk / kSub; sb++) {
-      const int64_t s0 = c0 + sb * kSub + half * (kSub / 2);
-      // this thread's 16 rows of the sub-block, loaded before waiting on the previous MMAs
-      double xv[kSub / 2], yv[8];
-      if (xw) {
+      // this warp's units of the sub-block, loaded before waiting on the previous MMAs
+      double uv[kGramUnits][8];
 #pragma unroll
-        for (int r = 0; r < kSub / 2; r++) {
-          const int64_t ra = s0 + r;
-          xv[r] = (col_ok && ra < r1) ? __ldg(X + ra * ldx + my_col) : 0.0;
-        }
-      }
+      for (int i = 0; i < kGramUnits; i++) {
+        const int unit = warp + 8 * i, cg = unit >> 2;
+        if (unit >= units) break;
+        const bool x = cg < xgroups;
+        const int cl = (x ? col0 + 32 * cg : cy0) + lane;
+        const bool ok = cl < (x ? a : b);
+        const int64_t ld = x ? ldx : ldy, ra = c0 + sb * kSub + (unit & 3) * 8;
+        const double* src = (x ? X : Y) + ra * ld + cl;
 #pragma unroll
-      for (int r = 0; r < 8; r++) {
-        const int64_t ra = c0 + sb * kSub + ykg * 8 + r;
-        yv[r] = (y_ok && ra < r1) ? __ldg(Y + ra * ldy + cy0 + yj) : 0.0;
+        for (int r = 0; r < 8; r++) uv[i][r] = ok && ra + r < r1 ? __ldg(src + r * ld) : 0.0;
       }
       if (pending) {   // the digit planes are free once the previous sub-block's MMAs have completed
         if (mbar_wait(mb, phase)) {
@@ -323,35 +326,25 @@ __global__ void __launch_bounds__(kGramThreads, 2)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       }
 #pragma unroll
-      for (int kh = 0; kh < kSub / 16; kh++) {
-        if (!xw) break;
-        const int kg = half * (kSub / 16) + kh;
+      for (int i = 0; i < kGramUnits; i++) {
+        const int unit = warp + 8 * i, cg = unit >> 2, kg = unit & 3;
+        if (unit >= units) break;
+        const bool x = cg < xgroups;
+        const int rr = x ? 32 * cg + lane : lane;   // row of the operand's tile
+        const int E = (x ? eX : eY)[rr];
         uint32_t pk[kDigits][4];
 #pragma unroll
         for (int r8 = 0; r8 < 8; r8 += 2) {
           uint32_t d[kDigits];
-          digits8_pair(xv[kh * 8 + r8], xv[kh * 8 + r8 + 1], Ex, d);
+          digits8_pair(uv[i][r8], uv[i][r8 + 1], E, d);
 #pragma unroll
           for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = d[s2];
         }
-        const int off = core_off(row >> 3, kg) + (row & 7) * 16;
+        uint8_t* dst = (x ? sA : sB) + core_off(rr >> 3, kg) + (rr & 7) * 16;
+        const int plane = x ? kPlaneA : kPlaneB;
 #pragma unroll
         for (int s2 = 0; s2 < kDigits; s2++)
-          *reinterpret_cast<uint4*>(sA + s2 * kPlaneA + off) = make_uint4(pk[s2][0], pk[s2][1], pk[s2][2], pk[s2][3]);
-      }
-      if (tid < kN * (kSub / 8)) {
-        uint32_t pk[kDigits][4];
-#pragma unroll
-        for (int r8 = 0; r8 < 8; r8 += 2) {
-          uint32_t d[kDigits];
-          digits8_pair(yv[r8], yv[r8 + 1], Ey, d);
-#pragma unroll
-          for (int s2 = 0; s2 < kDigits; s2++) pk[s2][r8 >> 1] = d[s2];
-        }
-        const int off = core_off(yj >> 3, ykg) + (yj & 7) * 16;
-#pragma unroll
-        for (int s2 = 0; s2 < kDigits; s2++)
-          *reinterpret_cast<uint4*>(sB + s2 * kPlaneB + off) = make_uint4(pk[s2][0], pk[s2][1], pk[s2][2], pk[s2][3]);
+          *reinterpret_cast<uint4*>(dst + s2 * plane) = make_uint4(pk[s2][0], pk[s2][1], pk[s2][2], pk[s2][3]);
       }
       // the generic-proxy stores above must be visible to the tensor core's (async) proxy
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
