@@ -808,16 +808,17 @@ __global__ void __launch_bounds__(GemmShape<PARTS>::threads, PARTS == 4 ? 1 : 2)
 // s + t = g -- at most 8 pairs x 64 columns x 127^2 < 2^24, exact in FP32 -- and each TMEM lane holds
 // one or two such sums per run row. With nb <= 16 the eight groups x 16 columns fill one 128-row
 // operand (8 MMAs per plane step); with nb <= 32, groups 0..3 and 4..7 x 32 columns fill two (4 and 8
-// MMAs). Sums are combined exactly in int64 across lanes and warps (fixed order), fused into one integer
-// and converted once per item and output to FP64 (one conversion and one FMA) and summed per run in
+// MMAs). Sums are joined exactly in int64 by their output's owner, fused into one integer and converted once per item and output to FP64 (one conversion and one FMA) and summed per run in
 // registers; every run is owned by one CTA, which writes
 // its rows of Y once (no atomics, no zero fill, deterministic). Pairs with s + t >= 8 are dropped: below
 // 2^-52 of max|m| max|x| of the item per term, FP64 rounding level in the normwise sense.
 //
-// Pipeline: two CTAs per SM, one shared-memory stage each, so one CTA's gathers and slicing overlap the
-// other's MMAs and readout. Per item, thread 0 has its digit planes of M brought in by one bulk
-// asynchronous copy while all threads gather and slice its rows of X (the next item's record, column
-// indices and row exponents are loaded one item ahead, and its rows of X prefetched into L2). Every
+// Pipeline: two CTAs per SM, one shared-memory stage each, so one CTA's slicing overlaps the other's MMAs and
+// readout. Per item, thread 0 has its digit planes of M brought in by one bulk asynchronous copy while all
+// threads slice its rows of X, gathered into registers behind the MMAs of the item before; the next
+// item's record, column indices and row exponents are loaded one item ahead, and its digit planes of M
+// prefetched into L2 (the copy's wait was the longest of an item). 24 columns at 83k rows took 182 us with the
+// gathers in line and 64-bit sums in the readout, 172 us so; at 1M rows 2.36 and 2.15 ms. Every
 // mbarrier wait is bounded (one second): on expiry the kernel raises the error flag, lets its copies
 // and MMAs in flight finish (bounded), frees its TMEM and returns.
 constexpr int kSpK = 64;                                // columns of a run's list per item
@@ -896,26 +897,34 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
                : "memory");
 }
 
-// gather the item's 64 rows of X (their indices in cq, -1 past the item's columns), find each column's
-// exponent (ecol: zeroed by the caller) and write the digit planes of X into xs (after its zero planes)
-__device__ __forceinline__ void sp_stage_x(const int* cq, const double* __restrict__ X, int64_t ldx, int nb,
-                                           bool packed, uint8_t* xs, int* ecol) {
-  const int tid = threadIdx.x;
+__device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
+// An item's 64 rows of X (their indices in cq, -1 past the item's columns) are gathered into registers one item
+// ahead (sp_gather), so the loads run behind the MMAs and the read-out of the item before; sp_stage_x finds
+// each column's exponent (ecol: zeroed by the caller) and writes the digit planes into xs (after its zero
+// planes). Thread: column tid % 32 and rows 8 part .. 8 part + 7 (one core-matrix row of 8 K values per digit),
+// or packed column tid % 16 and rows 4 part .. 4 part + 3 (half of one).
+__device__ __forceinline__ void sp_gather(const int* cq, const double* __restrict__ X, int64_t ldx, int nb, bool packed,
+                                          double (&xv)[8]) {
+  const int tid = threadIdx.x, j = packed ? tid & 15 : tid & 31, q0 = packed ? (tid >> 4) * 4 : (tid >> 5) * 8;
+#pragma unroll
+  for (int r = 0; r < 8; r++) {
+    const int c = packed && r >= 4 ? -1 : cq[q0 + r];
+    xv[r] = (j < nb && c >= 0) ? __ldg(X + (int64_t)c * ldx + j) : 0.0;
+  }
+}
+
+__device__ __forceinline__ void sp_stage_x(const double (&xv)[8], int nb, bool packed, uint8_t* xs, int* ecol) {
+  const int tid = threadIdx.x, j = packed ? tid & 15 : tid & 31, part = packed ? tid >> 4 : tid >> 5;
+  int e = 0;
+#pragma unroll
+  for (int r = 0; r < 8; r++) e = max(e, biased_exp(xv[r]));
+  if (j < nb) atomicMax(&ecol[j], e);
+  __syncthreads();
+  const int E = ecol[j];
   if (!packed) {
-    // thread: column j, rows q = 8 part .. 8 part + 7 (one core-matrix row of 8 K values per digit)
-    const int j = tid & 31, part = tid >> 5;
-    double xv[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const int c = cq[part * 8 + r];
-      xv[r] = (j < nb && c >= 0) ? __ldg(X + (int64_t)c * ldx + j) : 0.0;
-    }
-    int e = 0;
-#pragma unroll
-    for (int r = 0; r < 8; r++) e = max(e, biased_exp(xv[r]));
-    if (j < nb) atomicMax(&ecol[j], e);
-    __syncthreads();
-    const int E = ecol[j];
     uint32_t pk[kDigits][4];
 #pragma unroll
     for (int r = 0; r < 8; r += 2) {
@@ -930,20 +939,6 @@ __device__ __forceinline__ void sp_stage_x(const int* cq, const double* __restri
       *reinterpret_cast<uint4*>(xs + (3 + s) * kSpXPlaneW + (j >> 3) * 1024 + part * 128 + (j & 7) * 16) =
           make_uint4(pk[s][0], pk[s][1], pk[s][2], pk[s][3]);
   } else {
-    // thread: column j < 16, rows q = 4 part .. 4 part + 3 (half a core-matrix row per digit)
-    const int j = tid & 15, part = tid >> 4;
-    double xv[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const int c = cq[part * 4 + r];
-      xv[r] = (j < nb && c >= 0) ? __ldg(X + (int64_t)c * ldx + j) : 0.0;
-    }
-    int e = 0;
-#pragma unroll
-    for (int r = 0; r < 4; r++) e = max(e, biased_exp(xv[r]));
-    if (j < nb) atomicMax(&ecol[j], e);
-    __syncthreads();
-    const int E = ecol[j];
     uint32_t pk[kDigits][2];
 #pragma unroll
     for (int r = 0; r < 4; r += 2) {
@@ -1027,6 +1022,8 @@ __global__ void __launch_bounds__(kSpThreads, 2)
   // indices, row exponents) start at the top of an iteration and are consumed after its gathers
   TcSpmmItem wn_next{};
   if (tid < 64 && i0 + 1 < i1) wn_next = items[i0 + 1];
+  double xv[8] = {};
+  if (i0 < i1) sp_gather(cq, X, ldx, nb, packed, xv);
   for (int idx = i0, k = 0; idx < i1; idx++, k++) {
     const TcSpmmItem w = items[idx];
     const bool more = idx + 1 < i1;
@@ -1038,23 +1035,19 @@ __global__ void __launch_bounds__(kSpThreads, 2)
       bulk_copy_g2s(smem_addr(ms), planes + w.poff, (uint32_t)sp_item_units(R8) * 16u, mbf);
       copy_out = true;
     }
-    // the next item's column indices (used after this item's gathers for an L2 prefetch of its rows of
-    // X, and by its own gathers), exponent slots of the other parity
+    // the next item's column indices (its rows of X are gathered behind this item's MMAs) and the exponent
+    // slots of the other parity
     int nc = -1, emv = 0;
     TcSpmmItem wn_after{};
     if (more && tid < 64) {
       const TcSpmmItem wn = wn_next;
+      if (tid == 0) bulk_prefetch_l2(planes + wn.poff, (uint32_t)sp_item_units((wn.R + 7) & ~7) * 16u);
       nc = tid < wn.Lc ? __ldg(col + wn.cbase + tid) : -1;
       emv = tid < wn.R ? __ldg(ex + wn.eoff + tid) : 0;
       ecol[32 * ((k + 1) & 1) + (tid & 31)] = 0;
       if (idx + 2 < i1) wn_after = items[idx + 2];
     }
-    sp_stage_x(cq + 64 * (k & 1), X, ldx, nb, packed, xs, ecs);
-    if (nc >= 0) {
-      const double* xr = X + (int64_t)nc * ldx;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(xr));
-      if (nb > 16) asm volatile("prefetch.global.L2 [%0];" ::"l"(xr + 16));
-    }
+    sp_stage_x(xv, nb, packed, xs, ecs);
     if (more && tid < 64) {
       cq[64 * ((k + 1) & 1) + tid] = nc;
       em[64 * ((k + 1) & 1) + tid] = emv;
@@ -1100,6 +1093,7 @@ __global__ void __launch_bounds__(kSpThreads, 2)
       }
       mma_commit(mbm);
     }
+    if (more) sp_gather(cq + 64 * ((k + 1) & 1), X, ldx, nb, packed, xv);
     const bool ok = mbar_wait(mbm, ph_mma);
     ph_mma ^= 1u;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
