@@ -1150,8 +1150,12 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
       std::vector<double> T((size_t)keep * nk);
       for (int i = 0; i < keep; i++)
         for (int q = 0; q < nk; q++) T[(size_t)i * nk + q] = z[(size_t)i * keep + kept[q]] / std::sqrt(w[kept[q]]);
-      D.gemm(BlockSets().add(Wb, mmax, W2.p, 32).add(BWb, mmax, W3.p, 32), keep, T, nk, 0.0);
-      D.copy(BlockSets().add(W2.p, 32, Wb, mmax).add(W3.p, 32, BWb, mmax), nk);
+      if (D.dense_mode == 0) {   // the tensor update writes over its own operand
+        D.gemm(BlockSets().add(Wb, mmax, Wb, mmax).add(BWb, mmax, BWb, mmax), keep, T, nk, 0.0);
+      } else {
+        D.gemm(BlockSets().add(Wb, mmax, W2.p, 32).add(BWb, mmax, W3.p, 32), keep, T, nk, 0.0);
+        D.copy(BlockSets().add(W2.p, 32, Wb, mmax).add(W3.p, 32, BWb, mmax), nk);
+      }
       keep = nk;
       if (pass == 0 && m0 > 0) project(keep);
     }
