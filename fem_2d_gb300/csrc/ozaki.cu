@@ -494,10 +494,10 @@ __device__ __forceinline__ int core_off_k(int rg, int kg, int kc) { return (rg *
 // E[r] = biased exponent of max |X[r][k]| over k < a: a warp takes 4 rows at a time (lanes across the
 // rows, four independent loads in flight per lane: the pass is bound by load latency)
 constexpr int kRowExpRows = 4;
-__global__ void __launch_bounds__(256) row_exp_kernel(int64_t n, BlockSets sets, int a, int* __restrict__ E) {
+__global__ void __launch_bounds__(256) row_exp_kernel(int64_t n, BlockSets sets, int a) {
   const double* __restrict__ X = sets.X[blockIdx.y];
   const int64_t ldx = sets.ldx[blockIdx.y];
-  E += (int64_t)blockIdx.y * n;
+  int* __restrict__ E = sets.E[blockIdx.y];
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t r0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * kRowExpRows; r0 < n;
@@ -566,7 +566,7 @@ __device__ __forceinline__ void gemm_stage(const BlockSets& sets, int64_t n, int
 template <int PARTS>
 __global__ void __launch_bounds__(GemmShape<PARTS>::threads, PARTS == 4 ? 1 : 2)
     ozaki_gemm_kernel(int64_t n, const __grid_constant__ BlockSets sets, int a, const double* __restrict__ C, int b,
-                      double alpha, double beta, const int* __restrict__ EXr, int stages, int* __restrict__ err) {
+                      double alpha, double beta, int stages, int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
   using S = GemmShape<PARTS>;
   constexpr int SUB = S::sub, COLS = S::cols;
@@ -640,7 +640,7 @@ __global__ void __launch_bounds__(GemmShape<PARTS>::threads, PARTS == 4 ? 1 : 2)
     const int set = (int)(tile / ntiles);
     const int64_t row = (tile - set * ntiles) * kM + rl;
     const bool row_ok = row < n;
-    const int Ex = row_ok ? EXr[set * n + row] : 0;
+    const int Ex = row_ok ? __ldg(sets.E[set] + row) : 0;
     double* Zr = sets.Z[set] + row * sets.ldz[set] + part * COLS;
     long long Th[8], Tl[8];
 #pragma unroll
@@ -1264,19 +1264,27 @@ void ozaki_gemm(Ctx& c, int64_t n, const BlockSets& s, int a, const double* C, i
     }
   }
   const int64_t ntiles = s.count * ((n + kM - 1) / kM);
-  row_exp_kernel<<<dim3((unsigned)std::min<int64_t>((n * 32 + 255) / 256, (int64_t)c.num_sms * 16), s.count), 256, 0,
-                   c.stream>>>(n, s, a, rowexp);
+  BlockSets sets = s, todo;
+  for (int q = 0; q < s.count; q++) {
+    if (!sets.E[q]) sets.E[q] = rowexp + q * n;
+    if (!s.known[q]) todo.add(s.X[q], s.ldx[q], nullptr, 0, sets.E[q]);
+  }
+  if (todo.count > 0) {
+    row_exp_kernel<<<dim3((unsigned)std::min<int64_t>((n * 32 + 255) / 256, (int64_t)c.num_sms * 16), todo.count), 256, 0,
+                     c.stream>>>(n, todo, a);
+    c.launches++;
+  }
   const auto launch = [&](auto kernel, auto shape, int per_sm, int limit) {
     using S = decltype(shape);
     const int kc = (a + S::sub - 1) / S::sub * S::sub;
     const int stages = S::smem(kc, 2) <= limit ? 2 : 1;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)c.num_sms * per_sm));
-    kernel<<<grid, S::threads, S::smem(kc, stages), c.stream>>>(n, s, a, C, b, alpha, beta, rowexp, stages, err);
+    kernel<<<grid, S::threads, S::smem(kc, stages), c.stream>>>(n, sets, a, C, b, alpha, beta, stages, err);
   };
   if (a <= kChunk) launch(ozaki_gemm_kernel<2>, GemmShape<2>{}, 2, kGemmSmemHalf);
   else launch(ozaki_gemm_kernel<4>, GemmShape<4>{}, 1, kGemmSmemMax);
   FEM2D_CUDA(cudaGetLastError());
-  c.launches += 2;
+  c.launches++;
 }
 
 void TcSpmm::build(Ctx& c, int64_t n, const std::vector<int32_t>& grp_h, const std::vector<int64_t>& row_ptr) {
@@ -1417,7 +1425,7 @@ void TcSpmm::apply(Ctx& c, int k, double coef, const int32_t* grp, const int64_t
 }
 
 void ozaki_gram(Ctx& c, int64_t n, const double* X, int64_t ldx, int a, const double* Y, int64_t ldy, int b,
-                double* C, double* work, size_t work_doubles, int* err) {
+                double* C, double* work, size_t work_doubles, int* err, bool x_known) {
   if (a <= 0 || b <= 0) return;
   if (a > 4 * kM || b > 8 * kN) fail(FEM2D_E_INVALID_ARG, "ozaki_gram: block wider than 512 x 256");
   {
@@ -1434,8 +1442,9 @@ void ozaki_gram(Ctx& c, int64_t n, const double* X, int64_t ldx, int a, const do
   int* EX = reinterpret_cast<int*>(work + (size_t)nrb * mz * ny * kM * kN);
   int* EY = EX + chunks * a;
   if (n > 0) {
-    chunk_exp_kernel<<<dim3((unsigned)chunks, (a + 31) / 32 + (b + 31) / 32), 256, 0, c.stream>>>(n, X, ldx, a, EX, Y,
-                                                                                                   ldy, b, EY);
+    const int ax = x_known ? 0 : a;
+    chunk_exp_kernel<<<dim3((unsigned)chunks, (ax + 31) / 32 + (b + 31) / 32), 256, 0, c.stream>>>(n, X, ldx, ax, EX, Y,
+                                                                                                    ldy, b, EY);
     FEM2D_CUDA(cudaGetLastError());
     c.launches++;
   }

@@ -15,9 +15,10 @@ int ozaki_gram_partials(int64_t n, int a, int b, int num_sms);
 size_t ozaki_gram_workspace(int64_t n, int a, int b, int num_sms);
 // C (device, row-major a x b) = X^T Y for row-major X (n x a, ldx) and Y (n x b, ldy), accurate to
 // FP64 rounding in the normwise sense; a <= 512, b <= 256. Queued on c.stream; *err (device) is set
-// nonzero if a bounded wait inside the kernel expired.
+// nonzero if a bounded wait inside the kernel expired. x_known: the last product in this workspace had the same X
+// and widths, and its exponents of X are still there.
 void ozaki_gram(Ctx& c, int64_t n, const double* X, int64_t ldx, int a, const double* Y, int64_t ldy, int b,
-                double* C, double* work, size_t work_doubles, int* err);
+                double* C, double* work, size_t work_doubles, int* err, bool x_known = false);
 
 // Up to three block operands that go through one kernel together: X (n x a or n x b, ldx) to Z (n x b, ldz).
 // A search step updates W, A W and B W with the same C: one launch fills the chip where one block of a small GEP
@@ -30,16 +31,23 @@ struct BlockSets {
   int64_t ldx[3] = {};
   double* Z[3] = {};
   int64_t ldz[3] = {};
-  BlockSets& add(const double* x, int64_t lx, double* z, int64_t lz) {
+  int* E[3] = {};          // tensor update: where X's row exponents stand (n ints); null: in the call's scratch
+  bool known[3] = {};      // they are there already, from a call with the same X and a
+  BlockSets& add(const double* x, int64_t lx, double* z, int64_t lz, int* e = nullptr, bool has_e = false) {
     X[count] = x;
     ldx[count] = lx;
+    E[count] = e;
+    known[count] = has_e;
     Z[count] = z;
     ldz[count++] = lz;
     return *this;
   }
-  BlockSets columns(int j0) const {   // the same with Z from column j0 on
+  BlockSets columns(int j0) const {   // the same with Z from column j0 on, called after the columns before
     BlockSets s = *this;
-    for (int q = 0; q < count; q++) s.Z[q] += j0;
+    for (int q = 0; q < count; q++) {
+      s.Z[q] += j0;
+      s.known[q] = s.known[q] || j0 > 0;
+    }
     return s;
   }
 };
