@@ -9,8 +9,9 @@
 // multiplies and adds. The FP64 pipe bounds it, so jac_inv is tabulated with the u factor (three operations per spec
 // and point instead of four) and only the orders that the ancestor's specs have are tabulated (an ancestor
 // holds a few edge functions; tables of the mesh's largest order cost as much as its sums). 1,752 Elems of
-// orders 3 to 8, 16 x 15 points: 304 -> 214 us.
+// orders 3 to 8, 16 x 15 points: 304 -> 214 us (and 182, see fields_plan).
 #include <algorithm>
+#include <numeric>
 
 #include "fields.h"
 #include "shape.cuh"
@@ -25,6 +26,7 @@ constexpr int kSpecChunk = 256;     // specs staged per shared-memory pass
 
 template <int kFieldThreads>
 __global__ void __launch_bounds__(kFieldThreads) fem2d_xy_fields_kernel(const FieldItem* __restrict__ items, const int32_t* __restrict__ item_ptr,
+                       const int32_t* __restrict__ order,
                        const uint32_t* __restrict__ codes, const int32_t* __restrict__ dofs,
                        const double* __restrict__ sol, int basis, int d0, int d1, int imax, int jmax,
                        int64_t nleaves, double* __restrict__ ox, double* __restrict__ oy) {
@@ -42,7 +44,8 @@ __global__ void __launch_bounds__(kFieldThreads) fem2d_xy_fields_kernel(const Fi
   const double stepu = (1.0 - -1.0) / (double)(d0 - 1);
   const double stepv = (1.0 - -1.0) / (double)(d1 - 1);
 
-  for (int64_t leaf = blockIdx.x; leaf < nleaves; leaf += gridDim.x) {
+  for (int64_t k0 = blockIdx.x; k0 < nleaves; k0 += gridDim.x) {
+    const int64_t leaf = order[k0];
     const int it0 = item_ptr[leaf], it1 = item_ptr[leaf + 1];
     for (int pass = 0; pass < P; pass += kFieldThreads * kFieldPts) {
       int pm[kFieldPts], pn[kFieldPts];
@@ -187,9 +190,23 @@ void fields_plan(Ctx& c, const Domain& d, int basis, int d0, int d1, FieldSpace&
   FEM2D_CUDA(cudaSetDevice(c.device));
   f.items.upload(f.h_items, c.stream);
   f.item_ptr.upload(f.h_item_ptr, c.stream);
+  // The leaves with the most work first (products per grid point, and the tables at some ten operations an
+  // entry): a mesh of a thousand leaves fills the chip little more than once, and a long leaf that starts last
+  // sets the time. 1,163 leaves at 70k DoFs: 214 -> 182 us.
+  const int64_t nl = (int64_t)f.leaves.size();
+  std::vector<int64_t> work(nl, 0);
+  std::vector<int32_t> order(nl);
+  std::iota(order.begin(), order.end(), 0);
+  for (int64_t l = 0; l < nl; l++)
+    for (int32_t it = f.h_item_ptr[l]; it < f.h_item_ptr[l + 1]; it++) {
+      const FieldItem& I = f.h_items[it];
+      work[l] += (int64_t)(I.sp1 - I.sp0) * 3 * d0 * d1 + 20 * ((int64_t)(I.imax + 1) * d0 + (int64_t)(I.jmax + 1) * d1);
+    }
+  std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return work[x] > work[y]; });
+  f.order.upload(order, c.stream);
   f.codes.upload(codes, c.stream);
   f.dofs.upload(dofs, c.stream);
-  f.h2d_bytes = (int64_t)(f.h_items.size() * sizeof(FieldItem) + f.h_item_ptr.size() * 4 + codes.size() * 8);
+  f.h2d_bytes = (int64_t)(f.h_items.size() * sizeof(FieldItem) + (f.h_item_ptr.size() + order.size()) * 4 + codes.size() * 8);
   auto allow = [&](auto k) {
     FEM2D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(f.smem, 48 * 1024)));
   };
@@ -211,8 +228,8 @@ void fields_eval(FieldSpace& f, const double* d_solution, double* d_x, double* d
   ProfScope ps(c, "xy_fields", bytes);
   const int64_t grid = std::min<int64_t>(nl, (int64_t)std::max(c.num_sms, 1) * 64);
   auto launch = [&](auto k, int threads) {
-    k<<<(unsigned)grid, threads, f.smem, c.stream>>>(f.items.p, f.item_ptr.p, f.codes.p, f.dofs.p, d_solution, f.basis, f.d0,
-                                                     f.d1, f.imax, f.jmax, nl, d_x, d_y);
+    k<<<(unsigned)grid, threads, f.smem, c.stream>>>(f.items.p, f.item_ptr.p, f.order.p, f.codes.p, f.dofs.p, d_solution, f.basis,
+                                                     f.d0, f.d1, f.imax, f.jmax, nl, d_x, d_y);
   };
   // as many threads as the grid's points need (two each): at 3 x 3 points 128 threads left all but five idle
   const int points = f.d0 * f.d1;

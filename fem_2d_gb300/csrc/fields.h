@@ -33,7 +33,7 @@ struct FieldSpace {
   std::vector<FieldItem> h_items;
   std::vector<int32_t> h_item_ptr;    // leaves + 1
   DBuf<FieldItem> items;
-  DBuf<int32_t> item_ptr, dofs;
+  DBuf<int32_t> item_ptr, order, dofs;   // order: leaves by falling work
   DBuf<uint32_t> codes;               // i | j << 8 | dir << 16
   DBuf<double> sol, out;              // staging for the host-pointer entry point
   size_t smem = 0;
