@@ -1607,9 +1607,6 @@ void dense_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& d
   const int64_t n = h.n;
   if (n > 1000) fail(FEM2D_E_TOO_LARGE, "Matrices Exceeded Maximum Size (1000x1000); Cannot Solve!");
   MFDevice& mf = mf_plan(plan, c, dom, h);
-  MFFactor fb;
-  mf.factor(c, d.a.p, d.b.p, 0.0, 1.0, true, fb);
-  if (fb.flags & 2) fail(FEM2D_E_B_NOT_SPD, "Failed to invert B-matrix (via cholesky); likely ill-conditioned!");
   DBuf<double> Ad, Z;
   Ad.alloc_on((size_t)n * n, c.stream);
   Z.alloc_on((size_t)n * n, c.stream);
@@ -1617,7 +1614,17 @@ void dense_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& d
   densify_kernel<<<(int)std::min<int64_t>(n, 4096), 128, 0, c.stream>>>(n, d.row_ptr.p, d.col.p, d.a.p, d.b.p, 1.0,
                                                                         0.0, Ad.p);
   c.launches++;
-  for (int64_t c0 = 0; c0 < n; c0 += 32) {
+  int flags = 0;
+  // (a plan of one dense front is inverted whole, and one with a front of more than 768 pivots is past the
+  // ordered kernels)
+  const bool ordered = !(mf.nf == 1 && mf.max_p == mf.max_f) && mf.solve_ordered(c, d.b.p, n, Ad.p, Z.p, &flags);
+  MFFactor fb;
+  if (!ordered) {
+    mf.factor(c, d.a.p, d.b.p, 0.0, 1.0, true, fb);
+    flags = fb.flags;
+  }
+  if (flags & 2) fail(FEM2D_E_B_NOT_SPD, "Failed to invert B-matrix (via cholesky); likely ill-conditioned!");
+  for (int64_t c0 = 0; !ordered && c0 < n; c0 += 32) {
     const int w = (int)std::min<int64_t>(32, n - c0);
     mf.solve(c, fb, Ad.p + c0, n, Z.p + c0, n, w);
   }

@@ -1711,10 +1711,14 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   arena.reserve(weak_list, std::max<int64_t>(s.n, 1));
   arena.reserve(weak_count, 1);
   level_factor_bytes.assign(nlevels, 0.0);
+  level_max_f.assign(nlevels, 0);
+  level_max_p.assign(nlevels, 0);
   for (int l = 0; l < nlevels; l++)
     for (int k = s.level_ptr[l]; k < s.level_ptr[l + 1]; k++) {
       const double F = s.f[s.level_fronts[k]], P = s.p[s.level_fronts[k]];
       level_factor_bytes[l] += 8.0 * (0.5 * P * P + P * (F - P));
+      level_max_f[l] = std::max(level_max_f[l], s.f[s.level_fronts[k]]);
+      level_max_p[l] = std::max(level_max_p[l], s.p[s.level_fronts[k]]);
     }
   std::vector<int32_t> ls, ll;
   small_ptr.assign(nlevels + 1, 0);
@@ -2019,6 +2023,252 @@ void MFDevice::solve_sets(Ctx& c, int sets, const MFFactor* f1, const MFFactor* 
     }
   }
   FEM2D_CUDA(cudaGetLastError());
+}
+
+// ------------------------------------------------------------------ ordered solves (dense eigensolve)
+// The dense eigensolve reads the lower triangle of B^-1 A, whose structurally zero entries are rounding noise of
+// 1e-17, and the sign of its eigenvector follows the signs of that noise through the Householder reflectors: one
+// ulp in four of the 55 entries of a 10-DoF problem turns the vector round. The order of the sums is part
+// of that result, so it does not follow the tuned kernels (with them 37 of 120 small problems changed sign): LU in panels of 32 columns without pivoting, a
+// column's sums in plain loops, inverted squares, and on the levels whose fronts the chip could take row by row
+// (`parted`) the partitioned inverse. At most 1,000 DoFs: one CTA per front, then one per front and 32
+// columns; bound by the latency of a level (123 DoFs: 2.25 ms a solve with the tuned kernels, 2.27 with these).
+constexpr int kOrderedPanel = 32, kOrderedMaxP = 768;
+
+__global__ void __launch_bounds__(256) mf_ordered_factor_kernel(const int32_t* __restrict__ lf,
+                                                                const FrontDesc* __restrict__ fd,
+                                                                const int64_t* __restrict__ apos,
+                                                                const int64_t* __restrict__ acsr,
+                                                                const int32_t* __restrict__ emap,
+                                                                const double* __restrict__ vals, int parted, double* F,
+                                                                double* G, int* __restrict__ flags) {
+  const FrontDesc d = fd[lf[blockIdx.x]];
+  const int f = d.f, p = d.p, s = f - p, tid = threadIdx.x, nt = blockDim.x;
+  double* A = F + d.off;
+  for (int t = tid; t < f * f; t += nt) A[t] = 0.0;
+  __syncthreads();
+  for (int64_t k = d.aptr + tid; k < d.aend; k += nt) A[apos[k]] = vals[acsr[k]];
+  for (int slot = 0; slot < MAXKIDS; slot++) {
+    __syncthreads();
+    if (d.kid[slot] < 0) continue;   // uniform across the CTA
+    const FrontDesc cd = fd[d.kid[slot]];
+    const int cs = cd.f - cd.p;
+    const int32_t* m = emap + cd.eptr;
+    for (int t = tid; t < cs * cs; t += nt) {
+      const int i = t % cs, j = t / cs;
+      A[m[j] * f + m[i]] += F[cd.off + (int64_t)(cd.p + j) * cd.f + cd.p + i];
+    }
+  }
+  __syncthreads();
+  for (int k0 = 0; k0 < p; k0 += kOrderedPanel) {
+    const int w = min(kOrderedPanel, p - k0), base = k0 + w;
+    for (int k = k0; k < base; k++) {
+      double* col = A + k * f;
+      double dk = col[k];
+      __syncthreads();
+      if (dk == 0.0) dk = 1e-300;
+      if (tid == 0 && !(col[k] > 0.0)) {
+        atomicOr(flags, 2);
+        col[k] = dk;
+      }
+      const double inv = 1.0 / dk;
+      for (int i = k + 1 + tid; i < f; i += nt) col[i] *= inv;
+      __syncthreads();
+      const int rows = f - (k + 1);
+      for (int t = tid; t < (base - (k + 1)) * rows; t += nt) {
+        const int jj = k + 1 + t / rows, ii = k + 1 + t % rows;
+        A[jj * f + ii] = fma(-col[ii], A[jj * f + k], A[jj * f + ii]);
+      }
+      __syncthreads();
+    }
+    for (int j = base + tid; j < f; j += nt) {   // U12 of the panel's rows
+      double* x = A + j * f + k0;
+      for (int r = 1; r < w; r++) {
+        double sum = x[r];
+        for (int q = 0; q < r; q++) sum = fma(-A[(k0 + q) * f + k0 + r], x[q], sum);
+        x[r] = sum;
+      }
+    }
+    __syncthreads();
+    const int rest = f - base;
+    for (int t = tid; t < rest * rest; t += nt) {
+      const int r = base + t % rest, q = base + t / rest;
+      double acc = 0.0;
+      for (int k = k0; k < base; k++) acc = fma(A[k * f + r], A[q * f + k], acc);
+      A[q * f + r] -= acc;
+    }
+    __syncthreads();
+  }
+  // the pivot square, L21 by rows and U12 by columns, as the inverses below read them
+  double *S = G + d.off, *Lr = S + p * p, *Uc = Lr + s * p;
+  for (int t = tid; t < p * p; t += nt) S[t] = A[t / p * f + t % p];
+  for (int t = tid; t < s * p; t += nt) {
+    const int q = t / p, k = t % p;
+    Lr[t] = A[k * f + p + q];
+    Uc[t] = A[(p + q) * f + k];
+  }
+  __syncthreads();
+  const bool two = p > kSmallP;   // two sums by turns
+  for (int j = tid; j < p; j += nt) {
+    double* out = A + j * f;   // column j; only this thread writes it
+    for (int i = j + 1; i < p; i++) {
+      double a[2] = {-S[j * p + i], 0.0};
+      for (int k = j + 1; k < i; k++) {
+        const int z = two ? (k - j - 1) & 1 : 0;
+        a[z] = fma(-S[k * p + i], out[k], a[z]);
+      }
+      out[i] = two ? a[0] + a[1] : a[0];
+    }
+    out[j] = 1.0 / S[j * p + j];
+    for (int i = j - 1; i >= 0; i--) {
+      double a[2] = {0.0, 0.0};
+      for (int k = i + 1; k <= j; k++) {
+        const int z = two ? (k - i - 1) & 1 : 0;
+        a[z] = fma(S[k * p + i], out[k], a[z]);
+      }
+      out[i] = -(two ? a[0] + a[1] : a[0]) / S[i * p + i];
+    }
+  }
+  if (!parted) return;
+  __syncthreads();
+  const int lane = tid & 31;
+  for (int q = tid >> 5; q < s; q += nt >> 5) {
+    const double *b = Lr + q * p, *u = Uc + q * p;
+    for (int k = 0; k < p; k++) {
+      double sum = 0.0;
+      for (int i = k + 1 + lane; i < p; i += 32) sum = fma(b[i], A[k * f + i], sum);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+      if (lane == 0) A[k * f + p + q] = -(b[k] + sum);
+    }
+    for (int i = lane; i < p; i += 32) {
+      double a[2] = {0.0, 0.0};
+      for (int k = i; k < p; k++) a[(k - i) & 1] = fma(A[k * f + i], u[k], a[(k - i) & 1]);
+      A[(p + q) * f + i] = -(a[0] + a[1]);
+    }
+  }
+}
+
+// sum over k0 <= k < k1 of A[k f] v(k): four sums by turns and the rest with the first; or, on a parted level,
+// two sums by turns that start again at every 128 from `from` on
+template <class V>
+__device__ __forceinline__ double ordered_dot(const double* A, int f, int k0, int k1, int parted, int from, const V& v) {
+  double a[4] = {0.0, 0.0, 0.0, 0.0};
+  if (!parted) {
+    for (int k = k0; k < k1; k++) {
+      const int z = k0 + ((k1 - k0) & ~3) > k ? (k - k0) & 3 : 0;
+      a[z] = fma(A[(int64_t)k * f], v(k), a[z]);
+    }
+    return (a[0] + a[1]) + (a[2] + a[3]);
+  }
+  for (int c0 = from; c0 < k1; c0 += 128) {
+    const int b = max(c0, k0), e = min(c0 + 128, k1);
+    for (int k = b; k < e; k++) a[(k - b) & 1] = fma(A[(int64_t)k * f], v(k), a[(k - b) & 1]);
+  }
+  return a[0] + a[1];
+}
+
+// one front and 32 columns per CTA; V: gathered right-hand sides, W: solved rows and updates (per 32 columns)
+__global__ void __launch_bounds__(256) mf_ordered_forward_kernel(const int32_t* __restrict__ lf,
+                                                                 const FrontDesc* __restrict__ fd,
+                                                                 const int32_t* __restrict__ dofs,
+                                                                 const int32_t* __restrict__ emap,
+                                                                 const int64_t* __restrict__ woff, int parted,
+                                                                 const double* __restrict__ F, int64_t wsize, int64_t n,
+                                                                 const double* __restrict__ B, double* V, double* W) {
+  const int fr = lf[blockIdx.x];
+  const FrontDesc d = fd[fr];
+  const int f = d.f, p = d.p, c0 = blockIdx.y * kLdW, w = (int)min((int64_t)kLdW, n - c0), c = threadIdx.x & 31;
+  const double* A = F + d.off;
+  double *v = V + blockIdx.y * wsize + woff[fr] + c, *o = W + blockIdx.y * wsize + woff[fr] + c;
+  const int row0 = threadIdx.x >> 5, rows = blockDim.x >> 5;
+  for (int i = row0; i < f; i += rows) v[i * kLdW] = i < p && c < w ? B[(int64_t)dofs[d.dptr + i] * n + c0 + c] : 0.0;
+  for (int slot = 0; slot < MAXKIDS; slot++) {
+    __syncthreads();
+    if (d.kid[slot] < 0) continue;   // uniform across the CTA
+    const FrontDesc cd = fd[d.kid[slot]];
+    const double* cw = W + blockIdx.y * wsize + woff[d.kid[slot]] + cd.p * kLdW + c;
+    for (int i = row0; i < cd.f - cd.p; i += rows) v[emap[cd.eptr + i] * kLdW] += cw[i * kLdW];
+  }
+  __syncthreads();
+  const auto gathered = [&](int k) { return v[k * kLdW]; };
+  const auto solved = [&](int k) { return o[k * kLdW]; };
+  for (int i = row0; i < (parted ? f : p); i += rows)
+    o[i * kLdW] = v[i * kLdW] + ordered_dot(A + i, f, 0, min(i, p), parted, 0, gathered);
+  __syncthreads();
+  if (!parted)
+    for (int i = p + row0; i < f; i += rows) o[i * kLdW] = v[i * kLdW] - ordered_dot(A + i, f, 0, p, 0, 0, solved);
+}
+
+__global__ void __launch_bounds__(256) mf_ordered_backward_kernel(const int32_t* __restrict__ lf,
+                                                                  const FrontDesc* __restrict__ fd,
+                                                                  const int32_t* __restrict__ dofs,
+                                                                  const int64_t* __restrict__ woff, int parted,
+                                                                  const double* __restrict__ F, int64_t wsize, int64_t n,
+                                                                  double* V, const double* W, double* X) {
+  const int fr = lf[blockIdx.x];
+  const FrontDesc d = fd[fr];
+  const int f = d.f, p = d.p, c0 = blockIdx.y * kLdW, w = (int)min((int64_t)kLdW, n - c0), c = threadIdx.x & 31;
+  const double* A = F + d.off;
+  const int32_t* D = dofs + d.dptr;
+  double* z = V + blockIdx.y * wsize + woff[fr] + c;
+  const double* y = W + blockIdx.y * wsize + woff[fr] + c;
+  const int row0 = threadIdx.x >> 5, rows = blockDim.x >> 5;
+  for (int k = row0; k < f; k += rows)
+    z[k * kLdW] = k < p ? y[k * kLdW] : (c < w ? X[(int64_t)D[k] * n + c0 + c] : 0.0);
+  __syncthreads();
+  const auto value = [&](int k) { return z[k * kLdW]; };
+  if (!parted) {
+    for (int i = row0; i < p; i += rows)
+      z[i * kLdW] -= ordered_dot(A + (int64_t)p * f + i, f, 0, f - p, 0, 0, [&](int k) { return z[(p + k) * kLdW]; });
+    __syncthreads();
+  }
+  for (int i = row0; i < p; i += rows) {
+    const double x = ordered_dot(A + i, f, i, parted ? f : p, parted, i & ~7, value);
+    if (c < w) X[(int64_t)D[i] * n + c0 + c] = x;
+  }
+}
+
+bool MFDevice::solve_ordered(Ctx& c, const double* vals, int64_t n, const double* B, double* X, int* flags_out) {
+  // parted: the levels of few or large fronts, row by row over the chip
+  std::vector<int> parted(nlevels, 0);
+  for (int l = 0; l < nlevels; l++) {
+    const int count = level_ptr[l + 1] - level_ptr[l];
+    if (level_max_p[l] > kOrderedMaxP) return false;
+    const bool large = level_max_p[l] > kSmallP || level_max_f[l] > kSmallF;
+    parted[l] = large || count * CL <= 2 * c.num_sms;
+  }
+  const cudaStream_t st = c.stream;
+  const FrontDesc* fd = reinterpret_cast<const FrontDesc*>(desc.p);
+  const int groups = (int)((n + kLdW - 1) / kLdW);
+  const int64_t wsize = (int64_t)work.n;
+  DBuf<double> F, G, V, W;
+  F.alloc_on(std::max<int64_t>(mat_total, 1), st);
+  G.alloc_on(std::max<int64_t>(mat_total, 1), st);
+  V.alloc_on(wsize * groups, st);
+  W.alloc_on(wsize * groups, st);
+  FEM2D_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(int), st));
+  {
+    ProfScope ps(c, "mf_factor", 8.0 * (double)mat_total, 0.5 * factor_flops);
+    for (int l = 0; l < nlevels; l++) {
+      const int count = level_ptr[l + 1] - level_ptr[l];
+      mf_ordered_factor_kernel<<<count, 256, 0, st>>>(lfronts.p + level_ptr[l], fd, asm_pos.p, asm_csr.p, ea_map.p, vals,
+                                                      parted[l], F.p, G.p, flags.p);
+    }
+  }
+  double fbytes = 0.0;
+  for (double b : level_factor_bytes) fbytes += b;
+  ProfScope ps(c, "mf_solve", 2.0 * fbytes, 2.0 * 2.0 * (fbytes / 8.0) * n);
+  for (int l = 0; l < nlevels; l++)
+    mf_ordered_forward_kernel<<<dim3(level_ptr[l + 1] - level_ptr[l], groups), 256, 0, st>>>(
+        lfronts.p + level_ptr[l], fd, dofs.p, ea_map.p, woff.p, parted[l], F.p, wsize, n, B, V.p, W.p);
+  for (int l = nlevels - 1; l >= 0; l--)
+    mf_ordered_backward_kernel<<<dim3(level_ptr[l + 1] - level_ptr[l], groups), 256, 0, st>>>(
+        lfronts.p + level_ptr[l], fd, dofs.p, woff.p, parted[l], F.p, wsize, n, V.p, W.p, X);
+  c.launches += 3 * nlevels;
+  FEM2D_CUDA(cudaGetLastError());
+  *flags_out = read_flags(c);
+  return true;
 }
 
 int MFDevice::read_flags(Ctx& c) {

@@ -29,7 +29,7 @@ struct MFDevice {
   int nf = 0, nlevels = 0, max_f = 0, max_p = 0, nb_cap = 0;
   int64_t mat_total = 0, piv_total = 0;
   double factor_flops = 0;   // LU flops of all fronts, 2/3 (f^3 - (f - p)^3) each (half for Cholesky)
-  std::vector<int32_t> level_ptr;
+  std::vector<int32_t> level_ptr, level_max_f, level_max_p;
   std::vector<int64_t> level_off;
   std::vector<int64_t> level_big_end;   // end of the storage of a level's fronts factored in global memory
   std::vector<double> level_factor_bytes;   // L (forward) or U (backward) bytes read per level
@@ -75,6 +75,10 @@ struct MFDevice {
   void solve_pair(Ctx& c, const MFFactor& f1, const MFFactor& f2, const double* B, int64_t ldb, double* X1, int64_t ldx1,
                   double* X2, int64_t ldx2, int nb);
   int read_flags(Ctx& c);
+  // X = K^-1 B for all n columns of B (row-major, ld n; X likewise) and K = A's or B's SPD values, every sum in
+  // the fixed order of plain loops over each front (see mf_ordered_factor_kernel); false when a front is too
+  // large for them. Returns the flags of factor() in *flags_out.
+  bool solve_ordered(Ctx& c, const double* vals, int64_t n, const double* B, double* X, int* flags_out);
 
  private:
   void solve_sets(Ctx& c, int sets, const MFFactor* f1, const MFFactor* f2, const double* B, int64_t ldb, double* X1,

@@ -53,7 +53,9 @@ bool symeig(int n, const std::vector<double>& a, std::vector<double>& w, std::ve
         for (int j = 0; j <= l; j++) {
           double* vj = &V[(size_t)j * n];
           const double fj = vi[j], gj = e[j];
-          for (int k = 0; k <= l; k++) vj[k] -= fj * e[k] + gj * vi[k];
+          for (int k = 0; k <= j; k++) vj[k] -= fj * e[k] + gj * vi[k];
+          // the upper entry (j, k) rounds as its mirror (k, j) does, also where the compiler fuses a product
+          for (int k = j + 1; k <= l; k++) vj[k] -= vi[k] * gj + e[k] * fj;
         }
       }
     } else {

@@ -141,3 +141,23 @@ def test_block_updates_of_several_operands(oracle_lib, ctx, nx, ny, rounds, k, d
     r = fg.gpu_solve_gep_n(gep, 2.64, k, dense=dense)
     assert np.max(np.abs(r.values - ref) / np.abs(ref)) <= EIG_TOL
     assert np.all(np.abs(np.einsum("ij,ij->i", r.vectors, (B @ r.vectors.T).T) - 1.0) < 1e-9)
+
+
+@pytest.mark.parametrize("nx,ny,p,rounds", [(2, 1, 2, 0), (2, 1, 4, 1), (3, 2, 3, 1), (7, 6, 2, 1), (9, 7, 2, 2),
+                                            (6, 4, 4, 0)])
+def test_dense_solve_tree_shapes(oracle_lib, ctx, nx, ny, p, rounds):
+    """The dense solve on trees of one to several levels, with few fronts (partitioned inverses) and with more
+    than the chip's SMs take row by row: the mode nearest the target of the same lower triangle, to rounding
+    (n 2^-53 cond(B), below 1e-10 for orders up to 4), and its vector up to the sign."""
+    w = configs.full_scale(seed=nx + p, nx=nx, ny=ny, rounds=rounds, fraction=0.3, pmin=p, pmax=p, basis=0)
+    w.mesh_json = configs.grid_mesh_json(nx, ny, 0.0, 1.87, 0.0, 1.0)
+    gep = _gep(w.mesh_json, w.ops, 0, [8, 8], ctx)
+    assert gep.dimension <= 1000
+    A, B = (m.toarray() for m in gep.scipy())
+    S = np.linalg.solve(B, A)
+    val, vec = np.linalg.eigh(np.tril(S) + np.tril(S, -1).T)
+    best = np.argmin(np.abs(val - 10.0))
+    pair = fg.nalgebra_solve_gep(gep, 10.0)
+    assert abs(pair.value - val[best]) <= 1e-10 * np.max(np.abs(val))
+    gap = np.min(np.abs(np.delete(val, best) - val[best]))
+    assert 1.0 - abs(vec[:, best] @ pair.vector) <= (1e-10 * np.max(np.abs(val)) / gap) ** 2 + 1e-12
