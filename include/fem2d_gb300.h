@@ -277,7 +277,8 @@ typedef struct fem2d_solve_opts {
   int verbose;
   int krylov_steps;     /* block Krylov steps per restart cycle (at most 8), 0 = default (5 from 100,000
                            DoFs, else 4) */
-  double damping;       /* null-space damping c / |sigma| of T = (A - sigma B)^-1 A (A + c B)^-1 B,
+  double damping;       /* null-space damping c / |sigma| of T = (A - sigma B)^-1 A (A + c B)^-1 B (for sigma > 0
+                           applied as (c (A + c B)^-1 B + sigma (A - sigma B)^-1 B) / (c + sigma)),
                            0 = default (1 from 10,000 DoFs, 0.05 below) */
   int scaling;          /* 0 = automatic (row-run blocks from 10,000 DoFs; below, Jacobi, switching to
                            row-run blocks when the Jacobi-scaled factorizations are inaccurate),
