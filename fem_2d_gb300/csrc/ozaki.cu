@@ -235,8 +235,8 @@ __global__ void __launch_bounds__(256) chunk_exp_kernel(int64_t n, const double*
 }
 
 // 8 warps per CTA: thread t owns row t % 128 of the C tile (the TMEM lane) and column half t / 128
-// (16 FP64 accumulators), slices 16 of each sub-block's 32 rows of its column of X, and warps w and
-// w + 4 read the two column halves of the same TMEM lanes back
+// (16 FP64 accumulators), and warps w and w + 4 read the two column halves of the same TMEM lanes back; the
+// slicing goes round the warps in units (see the kernel)
 constexpr int kGramThreads = 256;
 
 constexpr int kGramUnits = (kM / 32 + 1) * 4 * 32 / kGramThreads + 1;   // most units of a warp
