@@ -79,11 +79,18 @@ __device__ __forceinline__ void contract1d_table(int basis, int P, int nivl, int
   }
 }
 
+// v, with +0 for -0 (in integers: these kernels have no FP64 operation to spare)
+__device__ __forceinline__ double positive_zero(double v) {
+  const long long bits = __double_as_longlong(v);
+  return (bits << 1) == 0 ? 0.0 : v;
+}
+
 // The value of one upper-triangle entry of A and B: the sum of its visits k0..k1-1, each the product C * Gu * Gv that
 // equals the reference's 2-D Gauss sum (integrals.rs:26-92, 292-354). The FP64 pipe bounds the kernels that
 // call this (79% busy): the four direction pairs share one sequence of products, with the tables chosen by
 // index, since a warp of mixed pairs would run each branch's products, and the first visit is not added to
-// zero (nearly every entry has one visit).
+// zero (nearly every entry has one visit). A sum that starts from zero is never -0, and the values are written to
+// files bit for bit, so a first visit of -0 (a zero table entry times a negative coefficient) is stored as +0.
 __device__ __forceinline__ void entry_values(int64_t k0, int64_t k1, const uint64_t* __restrict__ codes,
                                              const GBlock* __restrict__ blocks, const uint32_t* __restrict__ specs,
                                              const double* __restrict__ tables, int P, int nivl, double& out_a,
@@ -118,8 +125,8 @@ __device__ __forceinline__ void entry_values(int64_t k0, int64_t k1, const uint6
       sb += vb;
     }
   }
-  out_a = sa;
-  out_b = sb;
+  out_a = positive_zero(sa);
+  out_b = positive_zero(sb);
 }
 
 // the value of an upper entry into the full CSR

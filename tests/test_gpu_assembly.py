@@ -158,3 +158,20 @@ def test_print_to_petsc_binary_files(oracle_lib, kat, ctx, tmp_path):
         for i, j, v in zip(r, c, a if which == 0 else b):
             sm.insert((i, j), float(v))
         assert open(os.path.join(tmp_path, "tmp", "p_00000001_%s.dat" % tag), "rb").read() == sm.aij_bytes()
+
+
+@pytest.mark.parametrize("basis,glq,orders,rounds", [(fg.KOLeg, 10, (3, 8), 3), (fg.KOLeg, 14, (9, 12), 1),
+                                                     (fg.HierPoly, 14, (9, 12), 1)])
+def test_zero_entries_are_positive(ctx, basis, glq, orders, rounds, tmp_path):
+    """An entry is a sum that starts from zero, so it is never -0.0, whatever the sign of a visit that is zero:
+    the sign shows in the files of the external solver's hand-off, which hold the values bit for bit."""
+    w = configs.full_scale(seed=0, nx=5, ny=4, rounds=rounds, fraction=0.4, pmin=orders[0], pmax=orders[1])
+    dom = fg.Domain.from_mesh(configs.build_mesh(w))
+    gep = fg.galerkin_sample_gep_hcurl(basis, fg.CurlCurl, fg.L2Inner, dom, [glq, glq], ctx=ctx)
+    batch, _ = fg.galerkin_sample_gep_hcurl_batch(basis, fg.CurlCurl, fg.L2Inner, [dom], [glq, glq], ctx=ctx)
+    (tmp_path / "tmp").mkdir()
+    gep.print_to_petsc_binary_files(tmp_path, "z")
+    for name, which in (("a", "A"), ("b", "B")):
+        for v in (gep.csr(which)[2], batch[0].csr(which)[2], fg.aij_read(tmp_path / "tmp" / ("z_%s.dat" % name))[2]):
+            assert np.any(v == 0.0)
+            assert not np.any(np.signbit(v[v == 0.0]))
