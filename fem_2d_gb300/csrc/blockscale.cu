@@ -92,8 +92,11 @@ __global__ void __launch_bounds__(4 * LD) run_cholinv_kernel(const int32_t* __re
 }
 
 // Per run g and matrix (blockIdx.y: A, B): block <- S_g block S_h^T for every column run h of its pattern, both
-// factors lower triangular, as FP64 MMAs on 8 x 8 tiles: U = block S_h^T with all operands read straight into
-// the fragments (rows of the CSR and of S are contiguous), U kept in shared memory, then S_g U. The column
+// factors lower triangular, as FP64 MMAs on 8 x 8 tiles: U = S_g block with all operands read straight into
+// the fragments (rows of the CSR and of S are contiguous), U kept in shared memory, then U S_h^T. In this order:
+// the result multiplies y = S^-T x from the left, so that the rounding of S_g block meets the smooth S_h^T y = x,
+// where that of block S_h^T would meet y itself, which is large for a monomial basis (eigenvectors of HierPoly
+// pencils at 12,430 DoFs: 1 to 2e-8 from the exact ones, 8 to 9e-8 the other way). The column
 // runs go in groups of up to kGroupTiles tiles, so that the many runs of 4 to 8 functions fill the eight warps
 // together. One column run at a time through shared memory, with six barriers each, took 31.5 ms at 1M DoFs;
 // now 28, of which the FP64 pipe needs 20 (26 with the tiles' padding). Loading whole tiles ahead of their
@@ -139,17 +142,16 @@ __global__ void __launch_bounds__(kTransformThreads) run_transform_kernel(
     }
     __syncthreads();
     const int nt = ntiles;
-    // U = block S_h^T: tile (strip i, tile j of h) sums the block's columns up to tile j
+    // U = S_g block: tile (strip i, tile j of h) sums the rows of g up to strip i
     for (int w = warp; w < strips * nt; w += kTransformThreads / 32) {
-      const int i = w % strips, c = w / strips, H = tile_h[c], j = tile_j[c];
-      const double* Sh = S + tile_s[c];
-      const int row = 8 * i + q8, col = 8 * j + q8;
-      const double* a = src + r0 + (int64_t)row * len + tile_c[c];
+      const int i = w % strips, c = w / strips, H = tile_h[c];
+      const int row = 8 * i + q8, col = 8 * tile_j[c] + q8;
+      const double* b = src + r0 + tile_c[c] + col;
       double acc[2] = {0.0, 0.0};
-      for (int k0 = 0; k0 <= 8 * j + 4; k0 += 4) {
+      for (int k0 = 0; k0 <= 8 * i + 4; k0 += 4) {
         const int k = k0 + kl;
-        const double x = (row < R && k < H) ? __ldg(a + k) : 0.0;
-        const double y = (col < H && k <= col) ? __ldg(Sh + (int64_t)col * H + k) : 0.0;   // S_h[col][k]
+        const double x = (row < R && k <= row) ? __ldg(Sg + row * R + k) : 0.0;
+        const double y = (k < R && col < H) ? __ldg(b + (int64_t)k * len) : 0.0;
         dmma(acc, x, y);
       }
       double* u = U + row * kUld + 8 * c + 2 * kl;
@@ -157,20 +159,22 @@ __global__ void __launch_bounds__(kTransformThreads) run_transform_kernel(
       u[1] = acc[1];
     }
     __syncthreads();
-    // out = S_g U
+    // out = U S_h^T: tile j sums U's columns of h up to tile j
     for (int w = warp; w < strips * nt; w += kTransformThreads / 32) {
-      const int i = w % strips, c = w / strips;
-      const int row = 8 * i + q8;
+      const int i = w % strips, c = w / strips, H = tile_h[c], j = tile_j[c];
+      const double* Sh = S + tile_s[c];
+      const int row = 8 * i + q8, scol = 8 * j + q8;
+      const double* u = U + row * kUld + 8 * (c - j);
       double acc[2] = {0.0, 0.0};
-      for (int k0 = 0; k0 <= 8 * i + 4; k0 += 4) {
+      for (int k0 = 0; k0 <= 8 * j + 4; k0 += 4) {
         const int k = k0 + kl;
-        const double x = (row < R && k <= row) ? __ldg(Sg + row * R + k) : 0.0;
-        dmma(acc, x, U[k * kUld + 8 * c + q8]);
+        const double y = (scol < H && k <= scol) ? __ldg(Sh + (int64_t)scol * H + k) : 0.0;   // S_h[scol][k]
+        dmma(acc, u[k], y);
       }
-      const int col = 8 * tile_j[c] + 2 * kl;
+      const int col = 8 * j + 2 * kl;
       double* o = dst + r0 + (int64_t)row * len + tile_c[c] + col;
-      if (row < R && col < tile_h[c]) o[0] = acc[0];
-      if (row < R && col + 1 < tile_h[c]) o[1] = acc[1];
+      if (row < R && col < H) o[0] = acc[0];
+      if (row < R && col + 1 < H) o[1] = acc[1];
     }
   }
 }

@@ -38,15 +38,18 @@ struct FrontDesc {   // device copy of the per-front scalars
   int64_t aux;    // fronts factored in global memory: offset of the p x p scratch square of their inverses
 };
 
+// the CSR values of the listed fronts to their positions row * f + col: `by_rows` keeps the fronts row-major (one
+// dense front, inverted in that layout), otherwise they are column-major like all fronts. (The scaled pencil is
+// symmetric up to rounding only, and the solves are to be those of the matrix that the products multiply with.)
 __global__ void mf_assemble_kernel(const int32_t* __restrict__ lf, const FrontDesc* __restrict__ fd,
                                    const int64_t* __restrict__ apos, const int64_t* __restrict__ acsr,
                                    const double* __restrict__ va, const double* __restrict__ vb, double ca, double cb,
-                                   double* __restrict__ F) {
+                                   int by_rows, double* __restrict__ F) {
   const FrontDesc d = fd[lf[blockIdx.y]];
   for (int64_t k = d.aptr + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < d.aend;
        k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = acsr[k];
-    F[d.off + apos[k]] = ca * va[c] + cb * vb[c];
+    const int64_t c = acsr[k], pos = apos[k], row = pos / d.f;
+    F[d.off + (by_rows ? pos : (pos - row * d.f) * d.f + row)] = ca * va[c] + cb * vb[c];
   }
 }
 
@@ -586,9 +589,9 @@ __global__ void __launch_bounds__(NT, 768 / NT) mf_front_kernel(const int32_t* _
   __syncthreads();
 #pragma unroll 4
   for (int64_t k = d.aptr + tid; k < d.aend; k += NT) {
-    const int pos = (int)__ldg(a.apos + k), j = pos / f;
+    const int pos = (int)__ldg(a.apos + k), i = pos / f;   // row i, column pos - i f
     const int64_t c = __ldg(a.acsr + k);
-    A[j * ld + (pos - j * f)] = a.ca * __ldg(a.va + c) + a.cb * __ldg(a.vb + c);
+    A[(pos - i * f) * ld + i] = a.ca * __ldg(a.va + c) + a.cb * __ldg(a.vb + c);
   }
   for (int slot = 0; slot < MAXKIDS; slot++) {
     const int ch = d.kid[slot];
@@ -1791,7 +1794,7 @@ void MFDevice::factor(Ctx& c, const double* va, const double* vb, double ca, dou
     // one dense product
     const int n = max_f;
     FEM2D_CUDA(cudaMemsetAsync(Fbuf.p, 0, (size_t)n * n * sizeof(double), st));
-    mf_assemble_kernel<<<dim3(8, 1), 256, 0, st>>>(lfronts.p, fd, asm_pos.p, asm_csr.p, va, vb, ca, cb, Fbuf.p);
+    mf_assemble_kernel<<<dim3(8, 1), 256, 0, st>>>(lfronts.p, fd, asm_pos.p, asm_csr.p, va, vb, ca, cb, 1, Fbuf.p);
     c.launches++;
     const int gu = (int)std::min<int64_t>(((int64_t)n * n + 255) / 256, (int64_t)c.num_sms * 8);
     const int pivoting = cholesky ? 0 : 1;
@@ -1831,7 +1834,7 @@ void MFDevice::factor(Ctx& c, const double* va, const double* vb, double ca, dou
     if (nbig == 0) continue;
     const int32_t* lf = lbig.p + big_ptr[l];
     FEM2D_CUDA(cudaMemsetAsync(Fbuf.p + level_off[l], 0, (level_big_end[l] - level_off[l]) * sizeof(double), st));
-    mf_assemble_kernel<<<dim3(8, nbig), 256, 0, st>>>(lf, fd, asm_pos.p, asm_csr.p, va, vb, ca, cb, Fbuf.p);
+    mf_assemble_kernel<<<dim3(8, nbig), 256, 0, st>>>(lf, fd, asm_pos.p, asm_csr.p, va, vb, ca, cb, 0, Fbuf.p);
     c.launches++;
     const int mf = level_big_f[l], mp = level_big_p[l], strips = (mf + 7) / 8;
     if (l > 0) {
