@@ -11,6 +11,7 @@
 // holds a few edge functions; tables of the mesh's largest order cost as much as its sums). 1,752 Elems of
 // orders 3 to 8, 16 x 15 points: 304 -> 214 us (and 182, see fields_plan).
 #include <algorithm>
+#include <mutex>
 #include <numeric>
 
 #include "fields.h"
@@ -23,6 +24,7 @@ namespace {
 constexpr int kFieldMaxThreads = 128;   // fewer for grids that fewer threads cover
 constexpr int kFieldPts = 2;        // grid points per thread per pass
 constexpr int kSpecChunk = 256;     // specs staged per shared-memory pass
+constexpr size_t kFieldSmemMax = 200 * 1024;   // tables and staged specs
 
 template <int kFieldThreads>
 __global__ void __launch_bounds__(kFieldThreads) fem2d_xy_fields_kernel(const FieldItem* __restrict__ items, const int32_t* __restrict__ item_ptr,
@@ -117,6 +119,22 @@ __global__ void __launch_bounds__(kFieldThreads) fem2d_xy_fields_kernel(const Fi
 
 }  // namespace
 
+// the kernels' shared-memory limit, once per device and for every plan (the limit belongs to the device's context:
+// set to one plan's need, it would fall below another's)
+static void allow_tables(int device) {
+  static std::mutex mu;
+  static bool done[256] = {};
+  std::lock_guard<std::mutex> lk(mu);
+  if (device >= 0 && device < 256 && done[device]) return;
+  auto allow = [](auto k) {
+    FEM2D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFieldSmemMax));
+  };
+  allow(fem2d_xy_fields_kernel<32>);
+  allow(fem2d_xy_fields_kernel<64>);
+  allow(fem2d_xy_fields_kernel<kFieldMaxThreads>);
+  if (device >= 0 && device < 256) done[device] = true;
+}
+
 void fields_plan(Ctx& c, const Domain& d, int basis, int d0, int d1, FieldSpace& f) {
   if (basis != FEM2D_BASIS_HIERPOLY && basis != FEM2D_BASIS_KOLEG) fail(FEM2D_E_INVALID_ARG, "unknown basis space");
   if (d.cc != FEM2D_CC_HCURL) fail(FEM2D_E_WRONG_CC, "xy fields need an H(curl) Domain");
@@ -186,7 +204,7 @@ void fields_plan(Ctx& c, const Domain& d, int basis, int d0, int d1, FieldSpace&
   }
   const size_t tu = (size_t)(f.imax + 1) * d0, tv = (size_t)(f.jmax + 1) * d1;
   f.smem = (2 * tu + 2 * tv + kSpecChunk) * sizeof(double) + kSpecChunk * sizeof(uint32_t);
-  if (f.smem > 200 * 1024) fail(FEM2D_E_TOO_LARGE, "field grid too dense for the shape tables");
+  if (f.smem > kFieldSmemMax) fail(FEM2D_E_TOO_LARGE, "field grid too dense for the shape tables");
   FEM2D_CUDA(cudaSetDevice(c.device));
   f.items.upload(f.h_items, c.stream);
   f.item_ptr.upload(f.h_item_ptr, c.stream);
@@ -207,12 +225,7 @@ void fields_plan(Ctx& c, const Domain& d, int basis, int d0, int d1, FieldSpace&
   f.codes.upload(codes, c.stream);
   f.dofs.upload(dofs, c.stream);
   f.h2d_bytes = (int64_t)(f.h_items.size() * sizeof(FieldItem) + (f.h_item_ptr.size() + order.size()) * 4 + codes.size() * 8);
-  auto allow = [&](auto k) {
-    FEM2D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(f.smem, 48 * 1024)));
-  };
-  allow(fem2d_xy_fields_kernel<32>);
-  allow(fem2d_xy_fields_kernel<64>);
-  allow(fem2d_xy_fields_kernel<kFieldMaxThreads>);
+  allow_tables(c.device);
   FEM2D_CUDA(cudaStreamSynchronize(c.stream));
 }
 

@@ -163,3 +163,17 @@ def test_grid_sizes_agree(ctx, grid):
         for a, b in zip(*out):
             assert np.array_equal(a[:, 0, 0], b[:, 0, 0])
             assert np.allclose(a, b, rtol=0, atol=1e-12 * np.max(np.abs(b)))
+
+
+@pytest.mark.parametrize("grid", [(60, 60), (200, 200)])
+def test_plans_of_several_sizes_stay_usable(ctx, grid):
+    """A plan whose tables need much shared memory (some 20 and 60 KB at order 8) evaluates the same after a
+    plan that needs little was made."""
+    dom = fg.Domain.from_mesh(configs.build_mesh(configs.full_scale(seed=8, nx=2, ny=2, rounds=1, fraction=0.4, pmin=8,
+                                                                    pmax=8)))
+    u = np.random.default_rng(3).standard_normal(dom.num_dofs)
+    dense = fg.UniformFieldSpace(dom, grid, ctx=ctx)._device(fg.HierPoly)
+    before = dense.xy(u, *grid)
+    fg.UniformFieldSpace(dom, (3, 3), ctx=ctx)._device(fg.HierPoly)
+    for a, b in zip(before, dense.xy(u, *grid)):
+        assert np.array_equal(a, b)
