@@ -244,10 +244,14 @@ void fields_eval(FieldSpace& f, const double* d_solution, double* d_x, double* d
     k<<<(unsigned)grid, threads, f.smem, c.stream>>>(f.items.p, f.item_ptr.p, f.order.p, f.codes.p, f.dofs.p, d_solution, f.basis,
                                                      f.d0, f.d1, f.imax, f.jmax, nl, d_x, d_y);
   };
-  // as many threads as the grid's points need (two each): at 3 x 3 points 128 threads left all but five idle
-  const int points = f.d0 * f.d1;
-  if (points <= 32 * kFieldPts) launch(fem2d_xy_fields_kernel<32>, 32);
-  else if (points <= 64 * kFieldPts) launch(fem2d_xy_fields_kernel<64>, 64);
+  // As many threads as the grid's points need (two each): at 3 x 3 points 128 threads left all but five idle. A
+  // mesh of few leaves leaves SMs idle anyway, and what counts is how soon a leaf's tables are filled: there also
+  // as many as the longer axis has table entries (one leaf of order 3, KOLeg, 2 x 30 points: 16 us with 128
+  // threads, 33 with 32; 120 leaves of orders 5 to 8: 148 and 225; at 371 leaves fewer threads win at every grid).
+  int need = (f.d0 * f.d1 + kFieldPts - 1) / kFieldPts;
+  if (nl <= 2 * (int64_t)std::max(c.num_sms, 1)) need = std::max({need, (f.imax + 1) * f.d0, (f.jmax + 1) * f.d1});
+  if (need <= 32) launch(fem2d_xy_fields_kernel<32>, 32);
+  else if (need <= 64) launch(fem2d_xy_fields_kernel<64>, 64);
   else launch(fem2d_xy_fields_kernel<kFieldMaxThreads>, kFieldMaxThreads);
   FEM2D_CUDA(cudaGetLastError());
   c.launches++;
