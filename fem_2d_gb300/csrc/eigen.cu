@@ -1193,7 +1193,7 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
     ProfScope ps(c, "spmm_slice", 2.0 * (8.0 * h.nnz_full + 16.0 * h.nnz_full), 0.0);
     if (!plan.tcs) {
       plan.tcs = std::make_unique<TcSpmm>();
-      plan.tcs->build(c, n, d.grp_h, h.row_ptr);
+      plan.tcs->build(c, n, d.grp_h, h.row_ptr, true);
     }
     TcSpmm& tcs = *plan.tcs;
     slice_release.t = &tcs;
@@ -1780,7 +1780,7 @@ void gep_spmm_tensor(Ctx& c, const HostGEP& h, const DeviceGEP& d, int which, do
   if (which != 0 && which != 1) fail(FEM2D_E_INVALID_ARG, "which must be 0 (A) or 1 (B)");
   if (nb < 1 || nb > 32) fail(FEM2D_E_INVALID_ARG, "1..32 columns");
   TcSpmm tcs;
-  tcs.build(c, h.n, d.grp_h, h.row_ptr);
+  tcs.build(c, h.n, d.grp_h, h.row_ptr, false);
   tcs.slice(c, 0, d.grp.p, d.row_ptr.p, which == 0 ? d.a.p : nullptr, which == 1 ? d.b.p : nullptr,
             which == 0 ? 1.0 : 0.0, which == 1 ? 1.0 : 0.0);
   Dev D{c, h, d, d.a.p, d.b.p};

@@ -1287,7 +1287,8 @@ void ozaki_gemm(Ctx& c, int64_t n, const BlockSets& s, int a, const double* C, i
   c.launches++;
 }
 
-void TcSpmm::build(Ctx& c, int64_t n, const std::vector<int32_t>& grp_h, const std::vector<int64_t>& row_ptr) {
+void TcSpmm::build(Ctx& c, int64_t n, const std::vector<int32_t>& grp_h, const std::vector<int64_t>& row_ptr,
+                   bool kept) {
   std::vector<int4> it;
   std::vector<int64_t> po, eo;
   std::vector<int32_t> run_first;   // first item of each run
@@ -1316,39 +1317,21 @@ void TcSpmm::build(Ctx& c, int64_t n, const std::vector<int32_t>& grp_h, const s
   plane_units = pcur;
   exp_count = ecur;
   nzero = (int)zr.size();
-  // The product kernel's order (two CTAs per SM): runs by falling cost, each to the CTA with the least
-  // work so far, every CTA's runs then in pattern order (neighbouring runs gather the same rows of X).
+  // The product kernel's order (two CTAs per SM), in a kept plan: runs by falling cost, each to the CTA with the
+  // least work so far, every CTA's runs then in pattern order (neighbouring runs gather the same rows of X).
   // An item costs about the same whatever its rows, since the gather, the MMAs and the waits are per item,
   // so its weight grows slowly with R. Dealing the runs out in turn instead left the busiest CTA with
-  // 53 items against a mean of 36 at 83k DoFs, and that CTA sets the kernel's time.
+  // 53 items against a mean of 36 at 83k DoFs, and that CTA sets the kernel's time. The dealing itself takes the
+  // host longer than one product gains, so a plan for a single product takes the runs in turn, and its buffers
+  // from the stream's pool: a cudaMalloc beside a GEP's one allocation starts a new block of device memory (12k DoFs:
+  // a product with its plan and slicing 370 us by cost and cudaMalloc, 300 in turn, 170 in turn from the pool).
   grid = std::max(1, std::min(std::max(nruns, 1), 2 * c.num_sms));
-  auto cost = [&](int g) {
-    return (int64_t)(run_first[g + 1] - run_first[g]) * (64 + grp_h[g + 1] - grp_h[g]);
-  };
-  std::vector<int32_t> by_cost(nruns), owner(nruns, 0);
-  std::iota(by_cost.begin(), by_cost.end(), 0);
-  std::stable_sort(by_cost.begin(), by_cost.end(), [&](int32_t x, int32_t y) { return cost(x) > cost(y); });
-  {
-    typedef std::pair<int64_t, int> Load;   // work so far, CTA
-    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
-    for (int b = 0; b < grid; b++) least.push({0, b});
-    for (int32_t g : by_cost) {
-      Load l = least.top();
-      least.pop();
-      owner[g] = l.second;
-      l.first += cost(g);
-      least.push(l);
-    }
-  }
   std::vector<TcSpmmItem> ci(it.size());
   std::vector<int32_t> cp(grid + 1, 0);
-  for (int g = 0; g < nruns; g++) cp[owner[g] + 1] += run_first[g + 1] - run_first[g];
-  for (int b = 0; b < grid; b++) cp[b + 1] += cp[b];
-  std::vector<int32_t> fill(cp.begin(), cp.end() - 1);
-  for (int g = 0; g < nruns; g++)
+  auto place = [&](int32_t& at, int g) {   // run g's items from position `at` on
     for (int q = run_first[g]; q < run_first[g + 1]; q++) {
       const int4 w = it[q];
-      TcSpmmItem m;
+      TcSpmmItem& m = ci[at++];
       m.cbase = row_ptr[grp_h[g]] + w.y;
       m.poff = po[q];
       m.eoff = (int32_t)eo[q];
@@ -1356,14 +1339,45 @@ void TcSpmm::build(Ctx& c, int64_t n, const std::vector<int32_t>& grp_h, const s
       m.R = (int16_t)w.z;
       m.Lc = (int16_t)w.w;
       m.last = q + 1 == run_first[g + 1] ? 1 : 0;
-      ci[fill[owner[g]]++] = m;
     }
-  items.upload(it, c.stream);
-  poff.upload(po, c.stream);
-  eoff.upload(eo, c.stream);
-  citems.upload(ci, c.stream);
-  cta_ptr.upload(cp, c.stream);
-  zruns.upload(zr.empty() ? std::vector<int2>{make_int2(0, 0)} : zr, c.stream);
+  };
+  if (kept) {
+    auto cost = [&](int g) {
+      return (int64_t)(run_first[g + 1] - run_first[g]) * (64 + grp_h[g + 1] - grp_h[g]);
+    };
+    std::vector<int32_t> order(nruns), owner(nruns, 0);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return cost(x) > cost(y); });
+    typedef std::pair<int64_t, int> Load;   // work so far, CTA
+    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
+    for (int b = 0; b < grid; b++) least.push({0, b});
+    for (int32_t g : order) {
+      Load l = least.top();
+      least.pop();
+      owner[g] = l.second;
+      l.first += cost(g);
+      least.push(l);
+    }
+    for (int g = 0; g < nruns; g++) cp[owner[g] + 1] += run_first[g + 1] - run_first[g];
+    for (int b = 0; b < grid; b++) cp[b + 1] += cp[b];
+    std::vector<int32_t> fill(cp.begin(), cp.end() - 1);
+    for (int g = 0; g < nruns; g++) place(fill[owner[g]], g);
+  } else {
+    for (int b = 0; b < grid; b++) {
+      cp[b + 1] = cp[b];
+      for (int g = b; g < nruns; g += grid) place(cp[b + 1], g);
+    }
+  }
+  auto up = [&](auto& buf, const auto& v) {
+    if (kept) buf.upload(v, c.stream);
+    else buf.upload_on(v, c.stream);
+  };
+  up(items, it);
+  up(poff, po);
+  up(eoff, eo);
+  up(citems, ci);
+  up(cta_ptr, cp);
+  up(zruns, zr.empty() ? std::vector<int2>{make_int2(0, 0)} : zr);
   (void)n;
 }
 

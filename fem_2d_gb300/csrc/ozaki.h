@@ -93,7 +93,8 @@ struct TcSpmm {
     DBuf<uint4> planes;
     DBuf<int> exps;
   } slot[kSlots];
-  void build(Ctx& c, int64_t n, const std::vector<int32_t>& grp, const std::vector<int64_t>& row_ptr);
+  // kept: for many products, also after c's stream is gone; else for one call on it
+  void build(Ctx& c, int64_t n, const std::vector<int32_t>& grp, const std::vector<int64_t>& row_ptr, bool kept);
   // slot k holds ca va + cb vb (vb may be null when cb = 0)
   void slice(Ctx& c, int k, const int32_t* grp, const int64_t* rp, const double* va, const double* vb, double ca,
              double cb);
