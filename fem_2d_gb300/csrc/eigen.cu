@@ -113,74 +113,85 @@ __global__ void __launch_bounds__(256) spmm_kernel(int64_t n, const int64_t* __r
 // the launch) with FP64 atomics. X is gathered once per run instead of once per row. Up to 64 rows x
 // 32 columns = 8 outputs per thread. One CTA per item, taken as CTAs finish: items differ tenfold in work, and
 // dealing them out over six CTAs per SM in turn left SMs idle (18.4M entries x 20 columns, both matrices:
-// 1.15 ms, now 0.81, against 0.70 ms for the products at the FP64 pipe's rate).
+// 1.15 ms, now 0.72, against 0.70 ms for the products at the FP64 pipe's rate). Items of less than kGrpSmall entries
+// on average (order 1) are dealt out in turn: there a CTA's start costs more than its item (3,322 DoFs of
+// order 1, 20 columns: 18.5 us with a CTA per item, 16.5 so).
 constexpr int kGrpChunk = 48;
 constexpr int kGrpRows = 64;
 constexpr int kGrpSeg = 256;
+constexpr int64_t kGrpSmall = 16;
 __global__ void zero_block_kernel(int64_t n, int nb, double* __restrict__ Y, int64_t ldy) {
   const int64_t total = n * nb;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x)
     Y[(t / nb) * ldy + t % nb] = 0.0;
 }
 
-__global__ void __launch_bounds__(256) spmm_group_kernel(const int2* __restrict__ work,
+// The combined values c1 v1 + c2 v2 by the matrices and coefficients in use: none (both zero), one matrix, two. A
+// coefficient of one, the usual case, costs no FP64 operation per entry, and no branch stands between an entry's
+// loads (with the coefficients tested per entry, 0.7 A + 1.3 B took up to 24% longer than here).
+enum SpmmValues { kSpmmNone, kSpmmOne, kSpmmOneScaled, kSpmmTwo, kSpmmTwoScaled };
+
+template <int VALUES, bool ONE_ITEM>
+__global__ void __launch_bounds__(256) spmm_group_kernel(int nwork, const int2* __restrict__ work,
                                                          const int32_t* __restrict__ grp,
                                                          const int64_t* __restrict__ rp,
                                                          const int32_t* __restrict__ col,
-                                                         const double* __restrict__ va, const double* __restrict__ vb,
-                                                         double ca, double cb, const double* __restrict__ X,
+                                                         const double* __restrict__ v1, const double* __restrict__ v2,
+                                                         double c1, double c2, const double* __restrict__ X,
                                                          int64_t ldx, int nb, double* __restrict__ Y, int64_t ldy) {
   __shared__ double xs[kGrpChunk * 32];
   __shared__ double vs[kGrpRows * (kGrpChunk + 1)];
-  const int2 it = work[blockIdx.x];
-  const int r0 = grp[it.x], R = grp[it.x + 1] - r0;
-  const int64_t c0 = rp[r0];
-  const int cend = min((int)(rp[r0 + 1] - c0), it.y + kGrpSeg);
-  const int32_t* cols = col + c0;
-  double acc[8];
+  int w = blockIdx.x;
+  do {
+    const int2 it = work[w];
+    const int r0 = grp[it.x], R = grp[it.x + 1] - r0;
+    const int64_t c0 = rp[r0];
+    const int cend = min((int)(rp[r0 + 1] - c0), it.y + kGrpSeg);
+    const int32_t* cols = col + c0;
+    double acc[8];
 #pragma unroll
-  for (int o = 0; o < 8; o++) acc[o] = 0.0;
-  for (int q0 = it.y; q0 < cend; q0 += kGrpChunk) {
-    const int qn = min(kGrpChunk, cend - q0);
-    __syncthreads();
-    for (int t = threadIdx.x; t < qn * nb; t += blockDim.x) {
-      const int q = t / nb, j = t - q * nb;
-      xs[q * 32 + j] = __ldg(X + (int64_t)__ldg(cols + q0 + q) * ldx + j);
-    }
-    for (int t = threadIdx.x; t < R * kGrpChunk; t += blockDim.x) {
-      const int r = t / kGrpChunk, q = t - r * kGrpChunk;
-      double v = 0.0;
-      if (q < qn) {
-        const int64_t k = rp[r0 + r] + q0 + q;
-        // (a coefficient of one, the usual case, costs no FP64 operation per entry)
-        if (ca == 1.0) v = __ldg(va + k);
-        else if (ca != 0.0) v = ca * __ldg(va + k);
-        if (cb != 0.0) v += cb * __ldg(vb + k);
+    for (int o = 0; o < 8; o++) acc[o] = 0.0;
+    for (int q0 = it.y; q0 < cend; q0 += kGrpChunk) {
+      const int qn = min(kGrpChunk, cend - q0);
+      __syncthreads();
+      for (int t = threadIdx.x; t < qn * nb; t += blockDim.x) {
+        const int q = t / nb, j = t - q * nb;
+        xs[q * 32 + j] = __ldg(X + (int64_t)__ldg(cols + q0 + q) * ldx + j);
       }
-      vs[r * (kGrpChunk + 1) + q] = v;
+      for (int t = threadIdx.x; t < R * kGrpChunk; t += blockDim.x) {
+        const int r = t / kGrpChunk, q = t - r * kGrpChunk;
+        double v = 0.0;
+        if (q < qn && VALUES != kSpmmNone) {
+          const int64_t k = rp[r0 + r] + q0 + q;
+          v = __ldg(v1 + k);
+          if (VALUES == kSpmmOneScaled || VALUES == kSpmmTwoScaled) v = __dmul_rn(c1, v);
+          if (VALUES == kSpmmTwo || VALUES == kSpmmTwoScaled) v = fma(c2, __ldg(v2 + k), v);
+        }
+        vs[r * (kGrpChunk + 1) + q] = v;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int o = 0; o < 8; o++) {
+        const int t = threadIdx.x + o * 256;
+        if (t < R * nb) {
+          const int r = t / nb, j = t - r * nb;
+          const double* vr = vs + r * (kGrpChunk + 1);
+          double s = acc[o];
+#pragma unroll 8
+          for (int q = 0; q < qn; q++) s += vr[q] * xs[q * 32 + j];
+          acc[o] = s;
+        }
+      }
     }
-    __syncthreads();
 #pragma unroll
     for (int o = 0; o < 8; o++) {
       const int t = threadIdx.x + o * 256;
       if (t < R * nb) {
         const int r = t / nb, j = t - r * nb;
-        const double* vr = vs + r * (kGrpChunk + 1);
-        double s = acc[o];
-#pragma unroll 8
-        for (int q = 0; q < qn; q++) s += vr[q] * xs[q * 32 + j];
-        acc[o] = s;
+        atomicAdd(Y + (int64_t)(r0 + r) * ldy + j, acc[o]);
       }
     }
-  }
-#pragma unroll
-  for (int o = 0; o < 8; o++) {
-    const int t = threadIdx.x + o * 256;
-    if (t < R * nb) {
-      const int r = t / nb, j = t - r * nb;
-      atomicAdd(Y + (int64_t)(r0 + r) * ldy + j, acc[o]);
-    }
-  }
+  } while (!ONE_ITEM && (w += gridDim.x) < nwork);
 }
 
 // Gram products in FP64 MMAs (mma.sync m8n8k4): the same rate as FP64 FMAs, but operands come straight from
@@ -609,8 +620,18 @@ struct Dev {
     if (d.nwork > 0 && nb <= 32) {
       const int64_t zb = std::min<int64_t>((h.n * nb + 255) / 256, (int64_t)c.num_sms * 8);
       zero_block_kernel<<<(int)std::max<int64_t>(zb, 1), 256, 0, c.stream>>>(h.n, nb, Y, ldy);
-            spmm_group_kernel<<<d.nwork, 256, 0, c.stream>>>(d.gwork.p, d.grp.p, d.row_ptr.p, d.col.p, va, vb, ca,
-                                                    cb, X, ldx, nb, Y, ldy);
+      const int grid = h.nnz_full >= kGrpSmall * d.nwork ? d.nwork : std::min(d.nwork, 6 * c.num_sms);
+      auto launch = [&](auto one, auto many, const double* v1, const double* v2, double c1, double c2) {
+        (grid == d.nwork ? one : many)<<<grid, 256, 0, c.stream>>>(d.nwork, d.gwork.p, d.grp.p, d.row_ptr.p, d.col.p, v1,
+                                                                   v2, c1, c2, X, ldx, nb, Y, ldy);
+      };
+#define FEM2D_SPMM(VALUES) spmm_group_kernel<VALUES, true>, spmm_group_kernel<VALUES, false>
+      if (nv == 0.0) launch(FEM2D_SPMM(kSpmmNone), nullptr, nullptr, 0.0, 0.0);
+      else if (nv == 1.0 && ca + cb == 1.0) launch(FEM2D_SPMM(kSpmmOne), ca != 0.0 ? va : vb, nullptr, 1.0, 0.0);
+      else if (nv == 1.0) launch(FEM2D_SPMM(kSpmmOneScaled), ca != 0.0 ? va : vb, nullptr, ca + cb, 0.0);
+      else if (ca == 1.0) launch(FEM2D_SPMM(kSpmmTwo), va, vb, 1.0, cb);
+      else launch(FEM2D_SPMM(kSpmmTwoScaled), va, vb, ca, cb);
+#undef FEM2D_SPMM
       c.launches += 2;
       return;
     }

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 import fem_2d_gb300 as fg
+from fem_2d_gb300 import configs
 
 pytestmark = pytest.mark.gpu
 
@@ -169,3 +170,30 @@ def test_block_gram_shapes(ctx, n, a, b):
         fg.block_gram_device(ctx, method, n, xd.data_ptr(), a + 3, a, yd.data_ptr(), b + 5, b, c.data_ptr())
         bound = 2.0 ** -53 * ((n + 8) * mag if method == fg.GRAM_FP64 else 2 * (n + 8) * mag + 2 * n * top)
         assert np.all(np.abs(c.cpu().numpy() - ref) <= 2 * bound), method
+
+
+@pytest.mark.parametrize("mesh", [(4, 3, 1, 12), (40, 30, 1, 1)])
+@pytest.mark.parametrize("nb", [1, 20, 32])
+def test_spmm_coefficients(ctx, mesh, nb):
+    """Operator products with no, one and two matrices and with unit and other coefficients, on a pencil with
+    long runs and on one of orders 1 (several thousand items of a few entries, several to a CTA): each sum of a
+    row's k products within 2 k + 4 roundings of the sum of magnitudes."""
+    import torch
+
+    nx, ny, p0, p1 = mesh
+    dom = fg.Domain.from_mesh(configs.build_mesh(configs.full_scale(seed=1, nx=nx, ny=ny, rounds=1, fraction=0.3, pmin=p0,
+                                                                    pmax=p1)))
+    gep = fg.galerkin_sample_gep_hcurl(fg.KOLeg, fg.CurlCurl, fg.L2Inner, dom, [14, 14], ctx=ctx)
+    A, B = gep.scipy()
+    x = np.random.default_rng(nb).standard_normal((gep.dimension, nb + 3))
+    xd = torch.from_numpy(x).cuda()
+    y = torch.empty((gep.dimension, nb + 1), dtype=torch.float64, device="cuda")
+    k = np.diff(A.indptr)[:, None]
+    for ca, cb in ((0.0, 0.0), (1.0, 0.0), (0.0, 1.0), (0.3, 0.0), (0.0, -2.5), (1.0, -10.0), (0.7, 1.3), (-1.0, 1.0)):
+        y.fill_(float("nan"))
+        torch.cuda.synchronize()
+        gep.spmm_device(ca, cb, xd.data_ptr(), nb + 3, nb, y.data_ptr(), nb + 1)
+        ctx.synchronize()
+        ref = (ca * A + cb * B) @ x[:, :nb]
+        mag = (abs(ca) * abs(A) + abs(cb) * abs(B)) @ np.abs(x[:, :nb])
+        assert np.all(np.abs(y[:, :nb].cpu().numpy() - ref) <= 2.0 ** -53 * 2 * (2 * k + 4) * mag), (ca, cb)
