@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(256) spmm_group_kernel(int nwork, const int2* 
 // partial C = X^T Y: CTA (x, y, z): a slice of the rows, 8 NTL columns of Y, up to 128 columns of X. Its
 // eight warps own 32 columns of X each; with fewer than 128 columns, the warps left split the rows again.
 constexpr int kGramMT = 4;   // 8-column tiles of X per warp
+constexpr size_t kGramOnePerSM = 116 * 1024;   // more than half of an SM's shared memory
 template <int NTL>
 __global__ void __launch_bounds__(256) dgram_kernel(int64_t n, const double* __restrict__ X, int64_t ldx, int a,
                                                     const double* __restrict__ Y, int64_t ldy, int b, int64_t rows,
@@ -255,6 +256,43 @@ __global__ void __launch_bounds__(256) dgram_kernel(int64_t n, const double* __r
     double s = 0.0;
     for (int q = 0; q < slices; q++) s += sm[((q * groups + (i >> 5)) * 32 + (i & 31)) * W + j];
     out[(int64_t)(a0 + i) * b + b0 + j] = s;
+  }
+}
+
+// The same with one FMA per product and no padding, eight entries of C per thread from entry e0 on: for many rows
+// of blocks whose 8 x 8 tiles are padded so far that the FP64 pipe mostly multiplies zeros (17 x 17 at 300k rows:
+// 267 us, 360 with MMAs; 5 x 60: 366 and 470; 40 x 33 at 80k: 243 and 332). It pays from 16,000 rows' worth of
+// products with zeros, but not with up to 8 columns of Y or below 45k rows.
+__global__ void __launch_bounds__(256) fgram_kernel(int64_t n, const double* __restrict__ X, int64_t ldx, int a,
+                                                    const double* __restrict__ Y, int64_t ldy, int b, int64_t rows, int e0,
+                                                    double* __restrict__ P) {
+  extern __shared__ double sm[];
+  double *xs = sm, *ys = sm + 32 * a;   // 32 rows of X and of Y
+  const int64_t r0 = blockIdx.x * rows, r1 = min(n, r0 + rows);
+  const int ab = a * b;
+  double acc[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) acc[q] = 0.0;
+  for (int64_t rt = r0; rt < r1; rt += 32) {
+    const int nr = (int)min((int64_t)32, r1 - rt);
+    __syncthreads();
+    for (int t = threadIdx.x; t < nr * a; t += 256) xs[t] = X[(rt + t / a) * ldx + t % a];
+    for (int t = threadIdx.x; t < nr * b; t += 256) ys[t] = Y[(rt + t / b) * ldy + t % b];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int e = e0 + threadIdx.x + 256 * q;
+      if (e >= ab) break;
+      const double *x = xs + e / b, *y = ys + e % b;
+      double s = acc[q];
+      for (int r = 0; r < nr; r++) s += x[r * a] * y[r * b];
+      acc[q] = s;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const int e = e0 + threadIdx.x + 256 * q;
+    if (e < ab) P[(int64_t)blockIdx.x * ab + e] = acc[q];
   }
 }
 
@@ -649,23 +687,39 @@ struct Dev {
   // C (device, a x b) = X^T Y on the FP64 pipe
   void fp64_gram(const double* X, int64_t ldx, int a, const double* Y, int64_t ldy, int b, double* Cd) {
     ProfScope ps(c, "dense_block", 8.0 * h.n * (a + b), 2.0 * h.n * a * b);
-    const int ab = a * b, ntl = std::min(4, (b + 7) / 8);
-    const int ny = (b + 8 * ntl - 1) / (8 * ntl), nz = (a + 127) / 128;
-    // rows per CTA: all SMs busy, but at least one MMA step of four rows for each of its row slices
-    const int groups = std::min(4, (a + 31) / 32), step = 4 * (8 / groups);
-    const int64_t want = std::max<int64_t>(1, 2 * c.num_sms / (ny * nz));
-    const int64_t rows = std::max<int64_t>(step, ((h.n + want - 1) / want + step - 1) / step * step);
-    const int nblk = (int)std::max<int64_t>(1, (h.n + rows - 1) / rows);
-    if (part.n < (size_t)nblk * ab) part.alloc_on((size_t)nblk * ab, c.stream);
-    const dim3 grid(nblk, ny, nz);
-    const size_t smem = sizeof(double) * 8 * 32 * 8 * ntl;
-    auto launch = [&](auto k) { k<<<grid, 256, smem, c.stream>>>(h.n, X, ldx, a, Y, ldy, b, rows, part.p); };
-    if (ntl == 1) launch(dgram_kernel<1>);
-    else if (ntl == 2) launch(dgram_kernel<2>);
-    else if (ntl == 3) launch(dgram_kernel<3>);
-    else launch(dgram_kernel<4>);
+    const int ab = a * b, ta = (a + 7) / 8, tb = (b + 7) / 8;
+    const int ny = (tb + 3) / 4, ntl = (tb + ny - 1) / ny, nz = (ta + 15) / 16;
+    int nblk;
+    const int64_t padding = 64 * ta * ny * ntl - ab;   // products with zeros per row
+    if (h.n >= 45000 && b > 8 && h.n * padding >= 16000 * (int64_t)ab && a + b <= 384) {
+      const int64_t rows = std::max<int64_t>(32, (h.n + 2 * c.num_sms - 1) / (2 * c.num_sms));
+      nblk = (int)((h.n + rows - 1) / rows);
+      if (part.n < (size_t)nblk * ab) part.alloc_on((size_t)nblk * ab, c.stream);
+      for (int e0 = 0; e0 < ab; e0 += 8 * 256)
+        fgram_kernel<<<nblk, 256, 32 * (a + b) * sizeof(double), c.stream>>>(h.n, X, ldx, a, Y, ldy, b, rows, e0, part.p);
+      c.launches += (ab + 8 * 256 - 1) / (8 * 256);
+    } else {
+      // Rows per CTA: all SMs busy, but at least one MMA step of four rows for each of its row slices. One layer of 128
+      // columns of X: two CTAs per SM. Several: one, held to that by the shared memory asked for, so that each
+      // layer's CTAs go one to an SM; the CTAs of a full layer otherwise may land in pairs on half of the SMs
+      // and those of a short one on the others (80k rows, 129 x 24: FP64 pipes busy for 52% on average and 96% at
+      // most, 924 us; 549 so).
+      const int step = 4 * (8 / std::min(4, (a + 31) / 32));
+      const int64_t want = std::max<int64_t>(1, (nz > 1 ? 1 : 2) * c.num_sms / ny);
+      const int64_t rows = std::max<int64_t>(step, ((h.n + want - 1) / want + step - 1) / step * step);
+      nblk = (int)std::max<int64_t>(1, (h.n + rows - 1) / rows);
+      if (part.n < (size_t)nblk * ab) part.alloc_on((size_t)nblk * ab, c.stream);
+      const dim3 grid(nblk, ny, nz);
+      const size_t smem = nz > 1 ? kGramOnePerSM : sizeof(double) * 8 * 32 * 8 * ntl;
+      auto launch = [&](auto k) { k<<<grid, 256, smem, c.stream>>>(h.n, X, ldx, a, Y, ldy, b, rows, part.p); };
+      if (ntl == 1) launch(dgram_kernel<1>);
+      else if (ntl == 2) launch(dgram_kernel<2>);
+      else if (ntl == 3) launch(dgram_kernel<3>);
+      else launch(dgram_kernel<4>);
+      c.launches++;
+    }
     reduce_partials_kernel<<<(ab + 31) / 32, 256, 0, c.stream>>>(part.p, nblk, ab, Cd);
-    c.launches += 2;
+    c.launches++;
   }
   // C (a x b, host row-major) = X^T Y
   void gram(const double* X, int64_t ldx, int a, const double* Y, int64_t ldy, int b, std::vector<double>& C) {
@@ -750,9 +804,12 @@ void setup_gemm_smem(int device) {
   auto allow = [](auto k, size_t bytes) {
     FEM2D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   };
-  allow(dgram_kernel<3>, 8 * 32 * 24 * sizeof(double));
-  allow(dgram_kernel<4>, 8 * 32 * 32 * sizeof(double));
+  allow(dgram_kernel<1>, kGramOnePerSM);
+  allow(dgram_kernel<2>, kGramOnePerSM);
+  allow(dgram_kernel<3>, kGramOnePerSM);
+  allow(dgram_kernel<4>, kGramOnePerSM);
   allow(gemm_nn_kernel, 96 * 1024);
+  allow(fgram_kernel, 96 * 1024);
   done[device] = true;
 }
 

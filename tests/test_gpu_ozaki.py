@@ -197,3 +197,22 @@ def test_spmm_coefficients(ctx, mesh, nb):
         ref = (ca * A + cb * B) @ x[:, :nb]
         mag = (abs(ca) * abs(A) + abs(cb) * abs(B)) @ np.abs(x[:, :nb])
         assert np.all(np.abs(y[:, :nb].cpu().numpy() - ref) <= 2.0 ** -53 * 2 * (2 * k + 4) * mag), (ca, cb)
+
+
+@pytest.mark.parametrize("n,a,b", [(45000, 17, 17), (45007, 33, 9), (60001, 5, 60), (50000, 9, 32), (44999, 17, 17),
+                                   (12160, 129, 24), (48640, 136, 40), (50011, 300, 33), (45000, 300, 90)])
+def test_block_gram_many_rows(ctx, n, a, b):
+    """FP64 Gram products of many rows: blocks whose tiles would be mostly padding (one FMA per product), more
+    columns of X than one layer of CTAs takes, and columns of Y that fill their tiles unevenly: each sum of n
+    products within n + 8 roundings of the sum of magnitudes."""
+    import torch
+
+    rng = np.random.default_rng(n + a + b)
+    x, y = rng.standard_normal((n, a + 1)), rng.standard_normal((n, b + 2))
+    xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    c = torch.full((a, b), float("nan"), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    fg.block_gram_device(ctx, fg.GRAM_FP64, n, xd.data_ptr(), a + 1, a, yd.data_ptr(), b + 2, b, c.data_ptr())
+    ref = x[:, :a].T @ y[:, :b]
+    mag = np.abs(x[:, :a]).T @ np.abs(y[:, :b])
+    assert np.all(np.abs(c.cpu().numpy() - ref) <= 2 * 2.0 ** -53 * (n + 8) * mag)
