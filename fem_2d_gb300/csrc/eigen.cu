@@ -848,7 +848,7 @@ void random_block_device(Ctx& c, int64_t n, int b, uint64_t seed, double* out, i
 
 }  // namespace
 
-MFDevice& mf_plan(MFPlan& p, Ctx& c, const Domain& dom, const HostGEP& h, std::unique_ptr<MFSymbolic> pre) {
+MFDevice& mf_plan(MFPlan& p, Ctx& c, const Domain& dom, const HostGEP& h, bool pairs, std::unique_ptr<MFSymbolic> pre) {
   if (!p.ready || p.device != c.device) {
     p.ready = false;
     p.mf.reset();
@@ -860,7 +860,7 @@ MFDevice& mf_plan(MFPlan& p, Ctx& c, const Domain& dom, const HostGEP& h, std::u
       else mf_symbolic(dom, h, *p.sym, p.lift.empty() ? nullptr : &p.lift);
     }
     p.mf.reset(new MFDevice);
-    p.mf->setup(c, *p.sym, 32);
+    p.mf->setup(c, *p.sym, 32, pairs && !p.dense);
     p.device = c.device;
     p.ready = true;
   }
@@ -873,7 +873,7 @@ MFDevice& mf_plan_dense(MFPlan& p, Ctx& c, const HostGEP& h) {
   p.sym.reset(new MFSymbolic);
   mf_symbolic_dense(h, *p.sym);
   p.mf.reset(new MFDevice);
-  p.mf->setup(c, *p.sym, 32);
+  p.mf->setup(c, *p.sym, 32, false);   // (inverted whole: no workspace in use)
   p.device = c.device;
   p.dense = true;
   p.ready = true;
@@ -980,7 +980,7 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
   }
   if (o.precond == 2 && !net) fail(FEM2D_E_INVALID_ARG, "precond 2 (learned) needs a trained network");
   if (o.precond < 0 || o.precond > 2) fail(FEM2D_E_INVALID_ARG, "precond must be 0, 1 or 2");
-  MFDevice* M = iterative ? nullptr : &mf_plan(plan, c, dom, h, sym_job.valid() ? sym_job.get() : nullptr);
+  MFDevice* M = iterative ? nullptr : &mf_plan(plan, c, dom, h, sigma > 0.0, sym_job.valid() ? sym_job.get() : nullptr);
   MFFactor fm, fp;
   // A + c B (c > 0) is SPD: factored without pivoting. c = |sigma| by default from kLargeN DoFs: the null
   // space of the curl-curl operator, smeared by rounding to |lambda| <~ eps ||A|| / lambda_min(B) (which
@@ -1002,7 +1002,7 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
         if (plan.lift[x] < 255) plan.lift[x]++;
       delayed += (int)fm.weak.size();
       plan.ready = false;
-      M = &mf_plan(plan, c, dom, h);
+      M = &mf_plan(plan, c, dom, h, sigma > 0.0);
       M->factor(c, sa.p, sb.p, 1.0, -sigma, false, fm);
     }
     M->factor(c, sa.p, sb.p, 1.0, cshift, true, fp);
@@ -1684,7 +1684,7 @@ void dense_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& d
                  double* value, double* vector) {
   const int64_t n = h.n;
   if (n > 1000) fail(FEM2D_E_TOO_LARGE, "Matrices Exceeded Maximum Size (1000x1000); Cannot Solve!");
-  MFDevice& mf = mf_plan(plan, c, dom, h);
+  MFDevice& mf = mf_plan(plan, c, dom, h, false);
   DBuf<double> Ad, Z;
   Ad.alloc_on((size_t)n * n, c.stream);
   Z.alloc_on((size_t)n * n, c.stream);
@@ -1774,7 +1774,7 @@ void shifted_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP&
     return rel;
   };
   for (int attempt = 0; attempt < 2; attempt++) {
-    MFDevice& mf = attempt == 0 ? mf_plan(plan, c, dom, h) : mf_plan_dense(plan, c, h);
+    MFDevice& mf = attempt == 0 ? mf_plan(plan, c, dom, h, false) : mf_plan_dense(plan, c, h);
     MFFactor fac;
     mf.factor(c, d.a.p, d.b.p, ca, cb, spd, fac);
     if (spd && (fac.flags & 2)) fail(FEM2D_E_B_NOT_SPD, "the shifted matrix is not positive definite");

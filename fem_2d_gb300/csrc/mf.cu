@@ -1517,7 +1517,7 @@ __global__ void gjp_unscramble_kernel(int n, const int32_t* __restrict__ piv, do
 
 }  // namespace
 
-void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
+void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max, bool pairs) {
   cudaStream_t st = c.stream;
   nf = s.nfronts;
   nlevels = s.nlevels;
@@ -1709,7 +1709,7 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max) {
   arena.add(woff, woff_h);
   piv_total = po;
   arena.reserve(work, std::max<int64_t>(wo, 1));
-  arena.reserve(work2, std::max<int64_t>(wo, 1));
+  if (pairs) arena.reserve(work2, std::max<int64_t>(wo, 1));
   arena.reserve(flags, 1);
   arena.reserve(weak_list, std::max<int64_t>(s.n, 1));
   arena.reserve(weak_count, 1);
@@ -1937,6 +1937,7 @@ void MFDevice::solve_pair(Ctx& c, const MFFactor& f1, const MFFactor& f2, const 
     return;
   }
   if (nb > nb_cap) fail(FEM2D_E_INVALID_ARG, "solve block wider than the workspace");
+  if (work2.n < work.n) work2.alloc(work.n);
   solve_sets(c, 2, &f1, &f2, B, ldb, X1, ldx1, X2, ldx2, nb);
 }
 

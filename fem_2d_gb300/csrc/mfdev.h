@@ -37,7 +37,7 @@ struct MFDevice {
   DBuf<uint8_t> desc;
   DBuf<int32_t> lfronts, dofs, ea_map;
   DBuf<int64_t> asm_pos, asm_csr, piv_off, woff;
-  DBuf<double> work, work2;   // a workspace per factorization of a pair of solves
+  DBuf<double> work, work2;   // workspaces; the second for pairs of solves, where the plan makes them
   DBuf<int> flags;
   DBuf<int32_t> weak_list;   // capacity n: weak-pivot DoFs recorded by the panel kernel
   DBuf<int> weak_count;
@@ -66,7 +66,8 @@ struct MFDevice {
   DBuf<double> sq;
   int ninv = 0, ninv_items = 0, max_inv_p = 0, npinv = 0;
 
-  void setup(Ctx& c, const MFSymbolic& s, int nb_max);
+  // pairs: solve_pair will be called (else its first call gets the second workspace, as large as the first)
+  void setup(Ctx& c, const MFSymbolic& s, int nb_max, bool pairs);
   // factor c_a*A + c_b*B (values in full-CSR order); Cholesky mode skips pivoting (SPD shifts)
   void factor(Ctx& c, const double* va, const double* vb, double ca, double cb, bool cholesky, MFFactor& out);
   // X = K^-1 B for an n x nb row-major block (nb <= nb_cap); B and X must not alias
@@ -107,7 +108,8 @@ struct MFPlan {
 
 // the plan's MFDevice, building the plan on first use (or after a device change); `pre`, when given, is
 // the sparse symbolic analysis already computed for this GEP
-MFDevice& mf_plan(MFPlan& p, Ctx& c, const Domain& dom, const HostGEP& h, std::unique_ptr<MFSymbolic> pre = nullptr);
+MFDevice& mf_plan(MFPlan& p, Ctx& c, const Domain& dom, const HostGEP& h, bool pairs,
+                  std::unique_ptr<MFSymbolic> pre = nullptr);
 // replace the plan by the dense single-front plan
 MFDevice& mf_plan_dense(MFPlan& p, Ctx& c, const HostGEP& h);
 

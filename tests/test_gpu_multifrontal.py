@@ -116,3 +116,18 @@ def test_factor_front_sizes(ctx, orders, copies):
         knorm = np.max(np.asarray(abs(K).sum(axis=1)).ravel())
         bwd = np.max(np.abs(K @ X - R), axis=0) / (knorm * np.max(np.abs(X), axis=0) + np.max(np.abs(R), axis=0))
         assert np.max(bwd) < 1e-13, bwd
+
+
+def test_eigensolve_after_shifted_solve(ctx):
+    """A plan made by a shifted solve has one workspace; an eigensolve on it, which solves with two matrices at
+    once, gives the eigenvalues of an eigensolve on a plan of its own."""
+    w = configs.full_scale(seed=5, nx=9, ny=5, rounds=2, fraction=0.4, pmin=2, pmax=6)
+    w.mesh_json = configs.grid_mesh_json(9, 5, 0.0, 1.87, 0.0, 1.0)
+    dom = fg.Domain.from_mesh(configs.build_mesh(w))
+    geps = [fg.galerkin_sample_gep_hcurl(fg.KOLeg, fg.CurlCurl, fg.L2Inner, dom, [10, 10], ctx=ctx) for _ in range(2)]
+    geps[0].shifted_solve(1.0, -10.0, np.ones(dom.num_dofs))
+    a, b = (fg.gpu_solve_gep_n(g, 10.0, 4).values for g in geps)
+    assert np.max(np.abs(a - b) / b) < 1e-11
+    x = geps[0].shifted_solve(1.0, -10.0, np.ones(dom.num_dofs))
+    A, B = geps[0].scipy()
+    assert np.linalg.norm((A - 10.0 * B) @ x - 1.0) <= 1e-9 * np.sqrt(dom.num_dofs)
