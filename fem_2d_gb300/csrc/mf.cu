@@ -2034,10 +2034,12 @@ void MFDevice::solve_sets(Ctx& c, int sets, const MFFactor* f1, const MFFactor* 
 // 1e-17, and the sign of its eigenvector follows the signs of that noise through the Householder reflectors: one
 // ulp in four of the 55 entries of a 10-DoF problem turns the vector round. The order of the sums is part
 // of that result, so it does not follow the tuned kernels (with them 37 of 120 small problems changed sign): LU in panels of 32 columns without pivoting, a
-// column's sums in plain loops, inverted squares, and on the levels whose fronts the chip could take row by row
-// (`parted`) the partitioned inverse. At most 1,000 DoFs: one CTA per front, then one per front and 32
-// columns; bound by the latency of a level (123 DoFs: 2.25 ms a solve with the tuned kernels, 2.27 with these).
-constexpr int kOrderedPanel = 32, kOrderedMaxP = 768;
+// column's sums in plain loops, inverted squares, and on levels of few or large fronts (`parted`: by the tree alone,
+// so that the order is the same on every chip) the partitioned inverse. At most 1,000 DoFs: one CTA per front, then one per front and 32
+// columns; bound by the latency of a level (123 DoFs: 2.25 ms a solve with the tuned kernels, 2.27 with these; 370 to
+// 984 DoFs: 0.6 to 5.6 ms of the 36 to 630 ms that the whole solve takes, most of it on the host; with the tuned
+// kernels 0.8 to 4.4).
+constexpr int kOrderedPanel = 32, kOrderedMaxP = 768, kOrderedParted = 38;
 
 __global__ void __launch_bounds__(256) mf_ordered_factor_kernel(const int32_t* __restrict__ lf,
                                                                 const FrontDesc* __restrict__ fd,
@@ -2234,13 +2236,12 @@ __global__ void __launch_bounds__(256) mf_ordered_backward_kernel(const int32_t*
 }
 
 bool MFDevice::solve_ordered(Ctx& c, const double* vals, int64_t n, const double* B, double* X, int* flags_out) {
-  // parted: the levels of few or large fronts, row by row over the chip
   std::vector<int> parted(nlevels, 0);
   for (int l = 0; l < nlevels; l++) {
     const int count = level_ptr[l + 1] - level_ptr[l];
     if (level_max_p[l] > kOrderedMaxP) return false;
     const bool large = level_max_p[l] > kSmallP || level_max_f[l] > kSmallF;
-    parted[l] = large || count * CL <= 2 * c.num_sms;
+    parted[l] = large || count <= kOrderedParted;
   }
   const cudaStream_t st = c.stream;
   const FrontDesc* fd = reinterpret_cast<const FrontDesc*>(desc.p);
