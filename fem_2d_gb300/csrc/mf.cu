@@ -1266,7 +1266,7 @@ constexpr int kTileRows = 8;
 constexpr int kChunkK = 128;
 constexpr int kTiledMaxP = 768;   // the wide inversion keeps one column per thread in shared memory
 constexpr int kTileThreads = 128;
-constexpr int kTiledLeaves = 304;
+constexpr int kTiledLeaves = 2;   // per SM
 constexpr int kTileSteps = kChunkK / 16;   // MMA steps (4 columns of the front) per warp and chunk
 
 struct TiledArgs {
@@ -1582,7 +1582,7 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max, bool pairs) {
     x.eptr = s.ea_ptr[f];
   }
   for (FrontDesc& x : fdh) x.prow = x.aux = 0;
-  // Tiled levels: every level above the leaves, and leaf levels of at most kTiledLeaves fronts (or with a
+  // Tiled levels: every level above the leaves, and leaf levels of at most kTiledLeaves fronts per SM (or with a
   // front too large for one CTA), if all their fronts have p <= kTiledMaxP. Their fronts get pull records
   // (for each front row, the children's update rows that add into it) and factor-time work items. Upper
   // levels gain at every width, since one CTA per front leaves its threads idle on the few pivots that
@@ -1612,7 +1612,7 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max, bool pairs) {
       else nl++;
       if (s.p[fr] > kTiledMaxP) fits = false;
     }
-    if (single_dense || !fits || !(nl > 0 || l > 0 || ns <= kTiledLeaves)) continue;
+    if (single_dense || !fits || !(nl > 0 || l > 0 || ns <= kTiledLeaves * c.num_sms)) continue;
     level_tiled[l] = 1;
     for (int k = s.level_ptr[l]; k < s.level_ptr[l + 1]; k++) {
       const int fr = s.level_fronts[k];
@@ -2037,8 +2037,8 @@ void MFDevice::solve_sets(Ctx& c, int sets, const MFFactor* f1, const MFFactor* 
 // column's sums in plain loops, inverted squares, and on levels of few or large fronts (`parted`: by the tree alone,
 // so that the order is the same on every chip) the partitioned inverse. At most 1,000 DoFs: one CTA per front, then one per front and 32
 // columns; bound by the latency of a level (123 DoFs: 2.25 ms a solve with the tuned kernels, 2.27 with these; 370 to
-// 984 DoFs: 0.6 to 5.6 ms of the 36 to 630 ms that the whole solve takes, most of it on the host; with the tuned
-// kernels 0.8 to 4.4).
+// 984 DoFs: 0.6 to 5.6 ms of the 36 to 630 ms that the whole solve takes, most of it on the host;
+// the kernels whose order they keep took 1.5 to 4.8).
 constexpr int kOrderedPanel = 32, kOrderedMaxP = 768, kOrderedParted = 38;
 
 __global__ void __launch_bounds__(256) mf_ordered_factor_kernel(const int32_t* __restrict__ lf,
