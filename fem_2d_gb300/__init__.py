@@ -146,6 +146,9 @@ def lib():
         "fem2d_ctx_fp64_peak": (ctypes.c_int, [P, dp]),
         "fem2d_ctx_mma_ns": (ctypes.c_int, [P, ctypes.c_int, dp]),
         "fem2d_dense_solve_gep": (ctypes.c_int, [P, P, d, dp, dp]),
+        "fem2d_gep_factor_solve": (ctypes.c_int, [P, P, dp, dp, ctypes.POINTER(ctypes.c_int), ctypes.c_int, dp, dp, dp]),
+        "fem2d_fronts_solve": (ctypes.c_int, [P, ctypes.c_int, dp, ctypes.c_int, ctypes.POINTER(ctypes.c_int),
+                                              ctypes.c_int, ctypes.c_int, dp, dp]),
         "fem2d_gep_shifted_solve": (ctypes.c_int, [P, P, d, d, ctypes.c_int, ctypes.c_int, dp, dp]),
         "fem2d_gpu_solve_gep": (ctypes.c_int, [P, P, d, ctypes.c_int, ctypes.POINTER(_fem2d_solve_opts), dp, dp, dp,
                                                 ctypes.POINTER(_fem2d_solve_stats)]),
@@ -583,6 +586,19 @@ class GEP:
                                              r2.shape[1], _ptr(r2, ctypes.c_double), _ptr(x, ctypes.c_double)))
         return x[:, 0] if one else x
 
+    def factor_solve(self, shifts, rhs):
+        """The unrefined solves of the eigensolver's search operator, for checking: for one or two shifts
+        (c_a, c_b, spd) the solutions of (c_a A + c_b B) X = rhs (n x k), two of them in one pass."""
+        r = np.ascontiguousarray(rhs, dtype=np.float64)
+        ca, cb = (np.array([float(s[q]) for s in shifts]) for q in (0, 1))
+        spd = np.array([1 if s[2] else 0 for s in shifts], dtype=np.int32)
+        x = [np.zeros_like(r) for _ in shifts]
+        _check(lib().fem2d_gep_factor_solve(self.ctx._h, self._h, _ptr(ca, ctypes.c_double), _ptr(cb, ctypes.c_double),
+                                            _ptr(spd, ctypes.c_int), r.shape[1], _ptr(r, ctypes.c_double),
+                                            _ptr(x[0], ctypes.c_double),
+                                            _ptr(x[1], ctypes.c_double) if len(x) > 1 else None))
+        return x
+
     def spmm_device(self, c_a, c_b, d_x, ldx, nb, d_y, ldy, ctx=None):
         """Y = c_a A X + c_b B X on the device (raw device pointers, row-major n x nb blocks)."""
         ctx = ctx or self.ctx
@@ -814,6 +830,17 @@ def block_gemm_device(ctx, method, n, d_x, ldx, a, d_c, b, alpha, beta, d_z, ldz
     _check(lib().fem2d_block_gemm_device(ctx._h, int(method), int(n), ctypes.c_void_p(d_x), int(ldx), int(a),
                                          ctypes.c_void_p(d_c), int(b), float(alpha), float(beta), ctypes.c_void_p(d_z),
                                          int(ldz)))
+
+
+def fronts_solve(ctx, k, pivots, rhs, spd=False):
+    """K X = rhs for a dense matrix eliminated in fronts of the given pivot counts (fem2d_fronts_solve), for checking."""
+    k = np.ascontiguousarray(k, dtype=np.float64)
+    r = np.ascontiguousarray(rhs, dtype=np.float64)
+    p = np.ascontiguousarray(pivots, dtype=np.int32)
+    x = np.zeros_like(r)
+    _check(lib().fem2d_fronts_solve(ctx._h, len(k), _ptr(k, ctypes.c_double), len(p), _ptr(p, ctypes.c_int),
+                                    1 if spd else 0, r.shape[1], _ptr(r, ctypes.c_double), _ptr(x, ctypes.c_double)))
+    return x
 
 
 def gpu_solve_gep_n(gep, target_eigenvalue, n_pairs, precond=0, tol=0.0, max_outer=0,

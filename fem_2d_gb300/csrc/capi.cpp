@@ -808,6 +808,31 @@ int fem2d_gep_shifted_solve(fem2d_ctx* c, const fem2d_gep* g, double c_a, double
   API_END
 }
 
+int fem2d_gep_factor_solve(fem2d_ctx* c, const fem2d_gep* g, const double* c_a, const double* c_b, const int* spd, int nrhs,
+                           const double* rhs, double* x1, double* x2) {
+  API_BEGIN
+  if (!c || !g || !c_a || !c_b || !spd || !rhs || !x1 || nrhs <= 0) fail(FEM2D_E_INVALID_ARG, "invalid argument");
+  FEM2D_CUDA(cudaSetDevice(c->c.device));
+  std::lock_guard<std::mutex> lk(g->plan.mu);
+  factor_solve(c->c, g->dom, g->h, g->d, g->plan, c_a, c_b, spd, nrhs, rhs, x1, x2);
+  API_END
+}
+
+int fem2d_fronts_solve(fem2d_ctx* c, int n, const double* k, int nfronts, const int* pivots, int spd, int nrhs,
+                       const double* rhs, double* x) {
+  API_BEGIN
+  if (!c || !k || !pivots || !rhs || !x || n <= 0 || nfronts <= 0 || nrhs <= 0) fail(FEM2D_E_INVALID_ARG, "invalid argument");
+  int64_t sum = 0;
+  for (int q = 0; q < nfronts; q++) {
+    if (pivots[q] <= 0) fail(FEM2D_E_INVALID_ARG, "a front without pivots");
+    sum += pivots[q];
+  }
+  if (sum != n || n > 8192) fail(FEM2D_E_INVALID_ARG, "the pivots must sum to n, at most 8,192");
+  FEM2D_CUDA(cudaSetDevice(c->c.device));
+  fronts_solve(c->c, n, k, nfronts, pivots, spd != 0, nrhs, rhs, x);
+  API_END
+}
+
 int fem2d_gep_spmm_device(fem2d_ctx* c, const fem2d_gep* g, double c_a, double c_b, const double* d_x, int64_t ldx,
                           int nb, double* d_y, int64_t ldy) {
   API_BEGIN

@@ -1812,6 +1812,90 @@ void shifted_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP&
 
 namespace fem2d {
 
+// host blocks of up to 32 columns of rhs through `solve(R, X1, X2, w)` on n x 32 device blocks, into x1 and x2 (or null)
+template <class F>
+static void by_column_blocks(Ctx& c, int64_t n, int nrhs, const double* rhs, double* x1, double* x2, const F& solve) {
+  DBuf<double> R, X1, X2;
+  R.alloc_on((size_t)n * 32, c.stream);
+  X1.alloc_on((size_t)n * 32, c.stream);
+  X2.alloc_on((size_t)n * 32, c.stream);
+  const size_t pitch = 32 * sizeof(double), host = (size_t)nrhs * sizeof(double);
+  for (int c0 = 0; c0 < nrhs; c0 += 32) {
+    const int w = std::min(32, nrhs - c0);
+    FEM2D_CUDA(cudaMemcpy2DAsync(R.p, pitch, rhs + c0, host, w * sizeof(double), n, cudaMemcpyHostToDevice, c.stream));
+    solve(R.p, X1.p, X2.p, w);
+    FEM2D_CUDA(cudaMemcpy2DAsync(x1 + c0, host, X1.p, pitch, w * sizeof(double), n, cudaMemcpyDeviceToHost, c.stream));
+    if (x2)
+      FEM2D_CUDA(cudaMemcpy2DAsync(x2 + c0, host, X2.p, pitch, w * sizeof(double), n, cudaMemcpyDeviceToHost, c.stream));
+    FEM2D_CUDA(cudaStreamSynchronize(c.stream));
+  }
+}
+
+void factor_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& d, MFPlan& plan, const double* ca,
+                  const double* cb, const int* spd, int nrhs, const double* rhs, double* x1, double* x2) {
+  MFDevice& mf = mf_plan(plan, c, dom, h, x2 != nullptr);
+  MFFactor fac[2];
+  for (int q = 0; q < (x2 ? 2 : 1); q++) {
+    mf.factor(c, d.a.p, d.b.p, ca[q], cb[q], spd[q] != 0, fac[q]);
+    if (spd[q] && (fac[q].flags & 2)) fail(FEM2D_E_B_NOT_SPD, "the shifted matrix is not positive definite");
+  }
+  by_column_blocks(c, h.n, nrhs, rhs, x1, x2, [&](const double* R, double* X1, double* X2, int w) {
+    if (x2) mf.solve_pair(c, fac[0], fac[1], R, 32, X1, 32, X2, 32, w);
+    else mf.solve(c, fac[0], R, 32, X1, 32, w);
+  });
+}
+
+void fronts_solve(Ctx& c, int n, const double* K, int nfronts, const int* pivots, bool spd, int nrhs, const double* rhs,
+                  double* x) {
+  MFSymbolic s;
+  s.n = n;
+  s.nfronts = s.nlevels = nfronts;
+  s.dof_ptr = s.asm_ptr = s.mat_off = {0};
+  s.level_ptr = {0};
+  s.ea_ptr = {0};
+  int first = 0;
+  for (int q = 0; q < nfronts; q++) {
+    const int P = pivots[q], F = n - first;
+    s.parent.push_back(q + 1 < nfronts ? q + 1 : -1);
+    s.level.push_back(q);
+    s.f.push_back(F);
+    s.p.push_back(P);
+    for (int i = 0; i < F; i++) s.dofs.push_back(first + i);
+    for (int i = 0; i < F; i++)
+      for (int j = 0; j < F; j++)
+        if (i < P || j < P) {
+          s.asm_pos.push_back((int64_t)i * F + j);
+          s.asm_csr.push_back((int64_t)(first + i) * n + first + j);
+        }
+    if (q + 1 < nfronts)
+      for (int i = 0; i < F - P; i++) s.ea_map.push_back(i);
+    s.dof_ptr.push_back((int64_t)s.dofs.size());
+    s.asm_ptr.push_back((int64_t)s.asm_pos.size());
+    s.mat_off.push_back(s.mat_off.back() + (int64_t)F * F);
+    s.ea_ptr.push_back((int64_t)s.ea_map.size());
+    s.level_ptr.push_back(q + 1);
+    s.level_fronts.push_back(q);
+    s.max_f = std::max(s.max_f, F);
+    s.max_p = std::max(s.max_p, P);
+    first += P;
+  }
+  s.mat_total = s.mat_off.back();
+  DBuf<double> Kd;
+  Kd.alloc_on((size_t)n * n, c.stream);
+  FEM2D_CUDA(cudaMemcpyAsync(Kd.p, K, (size_t)n * n * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+  MFDevice mf;
+  mf.setup(c, s, 32, false);
+  MFFactor fac;
+  mf.factor(c, Kd.p, Kd.p, 1.0, 0.0, spd, fac);
+  if (spd && (fac.flags & 2)) fail(FEM2D_E_B_NOT_SPD, "the matrix is not positive definite");
+  by_column_blocks(c, n, nrhs, rhs, x, nullptr,
+                   [&](const double* R, double* X1, double*, int w) { mf.solve(c, fac, R, 32, X1, 32, w); });
+}
+
+}  // namespace fem2d
+
+namespace fem2d {
+
 // C (device, row-major a x b) = X^T Y with the FP64 CUDA-core kernels (method 1) or the tensor-core
 // emulation (method 0); synchronises
 void block_gram(Ctx& c, int method, int64_t n, const double* X, int64_t ldx, int a, const double* Y, int64_t ldy,

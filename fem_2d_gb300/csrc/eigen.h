@@ -23,6 +23,13 @@ void gep_spmm_values(Ctx& c, const HostGEP& h, const DeviceGEP& d, const double*
 void shifted_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& d, MFPlan& plan, double ca,
                    double cb, bool spd,
                    int nrhs, const double* rhs, double* x);
+// the plan's solves as the search operator uses them, without refinement or fallback: x1 (and with x2 a pair of
+// solves) for the matrices ca[q] A + cb[q] B
+void factor_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& d, MFPlan& plan, const double* ca,
+                  const double* cb, const int* spd, int nrhs, const double* rhs, double* x1, double* x2);
+// the same for a dense n x n matrix (host, row-major) eliminated by a chain of fronts with the given pivot counts
+void fronts_solve(Ctx& c, int n, const double* K, int nfronts, const int* pivots, bool spd, int nrhs, const double* rhs,
+                  double* x);
 // C (device, row-major a x b) = X^T Y: method 0 on the tensor cores (ozaki.cu), 1 on the FP64 CUDA cores
 // Z = beta Z + alpha X C (device, C row-major a x b): method 0 tensor cores, 1 FP64 CUDA cores
 void block_gemm(Ctx& c, int method, int64_t n, const double* X, int64_t ldx, int a, const double* Cd, int b,

@@ -229,6 +229,17 @@ int fem2d_dense_solve_gep(fem2d_ctx* c, const fem2d_gep* g, double target, doubl
  * Returns FEM2D_E_B_NOT_SPD if spd != 0 and a non-positive pivot appears. */
 int fem2d_gep_shifted_solve(fem2d_ctx* c, const fem2d_gep* g, double c_a, double c_b, int spd, int nrhs,
                             const double* rhs, double* x);
+/* The factorizations and solves that gpu_solve_gep's search operator is made of, exposed for checking (no counterpart in
+ * the reference): x1 = (c_a[0] A + c_b[0] B)^-1 rhs and, with x2 != NULL, x2 = (c_a[1] A + c_b[1] B)^-1 rhs in one
+ * pass over the fronts, without the refinement and the fallback of fem2d_gep_shifted_solve. Host blocks, row-major
+ * n x nrhs; spd as there, one per matrix. */
+int fem2d_gep_factor_solve(fem2d_ctx* c, const fem2d_gep* g, const double* c_a, const double* c_b, const int* spd, int nrhs,
+                           const double* rhs, double* x1, double* x2);
+/* The same for K X = R with a dense matrix K (host, row-major n x n, n <= 8,192) eliminated front by front: front q
+ * holds all rows from its first pivot on and eliminates pivots[q] > 0 of them (they sum to n). Exposed for checking
+ * fronts of sizes that take a very large mesh. */
+int fem2d_fronts_solve(fem2d_ctx* c, int n, const double* k, int nfronts, const int* pivots, int spd, int nrhs,
+                       const double* rhs, double* x);
 
 /* Y = c_a A X + c_b B X with the GEP's device-resident A and B: the operator products an external
  * eigensolver applies to the GEP (MatMult in the PETSc hand-off of slepc_solve.rs:14-68). d_x and

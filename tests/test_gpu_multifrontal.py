@@ -131,3 +131,58 @@ def test_eigensolve_after_shifted_solve(ctx):
     x = geps[0].shifted_solve(1.0, -10.0, np.ones(dom.num_dofs))
     A, B = geps[0].scipy()
     assert np.linalg.norm((A - 10.0 * B) @ x - 1.0) <= 1e-9 * np.sqrt(dom.num_dofs)
+
+
+def _backward_error(K, X, R):
+    """Per column ||K X - R|| / (||K|| ||X|| + ||R||) in the infinity norm."""
+    knorm = np.max(np.asarray(abs(K).sum(axis=1)).ravel())
+    return np.max(np.abs(K @ X - R), axis=0) / (knorm * np.max(np.abs(X), axis=0) + np.max(np.abs(R), axis=0))
+
+
+@pytest.mark.parametrize("spd", [False, True])
+@pytest.mark.parametrize("pivots", [[9], [1, 7, 8, 9, 45], [160, 161, 199], [96, 200, 728], [101, 924], [768, 532],
+                                    [769, 531], [103, 700, 700, 545], [96, 801, 1152], [801, 763, 736]],
+                         ids=lambda p: "f%d_p%d" % (sum(p), p[0]))
+def test_fronts_of_every_size(ctx, pivots, spd):
+    """Unrefined solves with a dense matrix in chains of fronts: one front inverted whole, fronts in shared
+    memory, fronts of up to 256, 1,024, 2,048 and more rows (a kernel each), pivot counts on both sides of 160 and
+    768 (one CTA, tiled and cluster solves) that are and are not multiples of 8. Without spd the large entries
+    stand off the diagonal of their front's pivot square, so that every column is pivoted. Normwise backward
+    errors below n roundings."""
+    n = sum(pivots)
+    rng = np.random.default_rng(n + len(pivots))
+    G = rng.standard_normal((n, n))
+    if spd:
+        K = G @ G.T / n + 0.1 * np.eye(n)
+    else:
+        K, first = G, 0
+        for p in pivots:
+            K[first + rng.permutation(p), first + np.arange(p)] += 4.0 * np.sqrt(n)
+            first += p
+    R = rng.standard_normal((n, 33))
+    X = fg.fronts_solve(ctx, K, pivots, R, spd=spd)
+    assert np.max(_backward_error(K, X, R)) <= n * 2.0 ** -53
+
+
+@pytest.mark.parametrize("orders", [(1, 2), (3, 3), (5, 4), (8, 7), (9, 9), (12, 10)])
+@pytest.mark.parametrize("copies", [1, 90])
+def test_unrefined_solves(ctx, orders, copies):
+    """The eigensolver's solves as it uses them, without refinement or a dense fallback, singly and in pairs, on the
+    meshes of test_factor_front_sizes: the backward errors stay below the 1e-11 at which the eigensolver turns to
+    another scaling or plan, and a pair of solves gives the two single ones bit for bit."""
+    nx, ny = (3, 2) if copies == 1 else (16, 12)
+    if copies > 1 and orders[0] * orders[1] > 60:
+        nx, ny = 13, 12
+    pm = configs.build_mesh(configs.full_scale(seed=3, nx=nx, ny=ny, rounds=1, fraction=0.15, pmin=1, pmax=1))
+    leaves = [int(e) for e in np.nonzero(pm.elem_info()[:, 0] == 1)[0]]
+    pm.set_expansion_on_elems(leaves[::2], fg.Orders(*orders))
+    pm.set_expansion_on_elems(leaves[1::2], fg.Orders(orders[0], max(1, orders[1] - 1)))
+    gep = fg.galerkin_sample_gep_hcurl(fg.KOLeg, fg.CurlCurl, fg.L2Inner, fg.Domain.from_mesh(pm), [14, 14], ctx=ctx)
+    A, B = gep.scipy()
+    R = np.random.default_rng(7).standard_normal((gep.dimension, 35))
+    shifts = [(1.0, -10.0, False), (1.0, 10.0, True)]
+    single = [gep.factor_solve([s], R)[0] for s in shifts]
+    for (ca, cb, _), X in zip(shifts, single):
+        assert np.max(_backward_error((ca * A + cb * B).tocsr(), X, R)) < 1e-11
+    for X, Y in zip(single, gep.factor_solve(shifts, R)):
+        assert np.array_equal(X, Y)
