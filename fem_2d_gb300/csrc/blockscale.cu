@@ -260,13 +260,16 @@ void BlockScale::build(Ctx& c, const HostGEP& h, const DeviceGEP& d, double* sa,
       attr[c.device] = true;
     }
   }
-  if (nshort > 0)
+  if (nshort > 0) {
     run_cholinv_kernel<kSmallRun><<<nshort, 4 * kSmallRun, 2 * kSmallRun * kSmallRun * sizeof(double), c.stream>>>(
         list.p, grp_d.p, d.row_ptr.p, d.col.p, d.b.p, soff.p, S.p, flag.p);
-  if (ngrp > nshort)
+    c.launches++;
+  }
+  if (ngrp > nshort) {
     run_cholinv_kernel<kRun><<<ngrp - nshort, 4 * kRun, 2 * kRun * kRun * sizeof(double), c.stream>>>(
         list.p + nshort, grp_d.p, d.row_ptr.p, d.col.p, d.b.p, soff.p, S.p, flag.p);
-  c.launches += 2;
+    c.launches++;
+  }
   run_transform_kernel<<<dim3(ngrp, 2), kTransformThreads, kTransformSmem, c.stream>>>(
       grp_d.p, d.row_ptr.p, seg_ptr.p, seg.p, soff.p, S.p, d.a.p, d.b.p, sa, sb);
   c.launches++;
