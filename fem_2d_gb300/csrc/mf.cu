@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(256) mf_extend_add_kernel(const int32_t* __res
 constexpr int kFusedF = 164;
 constexpr int kFusedNarrowF = 64;   // on levels of at most one front per SM
 constexpr int kFusedSmallF = 64;   // fronts up to here: 128 threads
+constexpr size_t kFusedStatic = 4096, kSmemPerSM = 227 * 1024;   // static shared memory of a CTA (at most), an SM's
 
 // fronts that the solves may give one CTA (see there)
 constexpr int kSmallP = 160;
@@ -1670,12 +1671,23 @@ void MFDevice::setup(Ctx& c, const MFSymbolic& s, int nb_max, bool pairs) {
         for (int t0 = 0; t0 < F - P; t0 += 8) pi_h.insert(pi_h.end(), {fr, 0, t0, 0, fr, 1, t0, 0});
     }
     std::stable_sort(q.begin(), q.end(), [&](int32_t x, int32_t y) { return s.f[x] > s.f[y]; });
-    const int classes[] = {kFusedF, 116, 95, 82, kFusedSmallF, 48, 32};   // 1, 2, 3, 4, 6, ... CTAs per SM
-    const int ncl = (int)q.size() <= 2 * c.num_sms ? 1 : 7;
+    // The launches of one stream follow each other, so a group ends at a size class only once its fronts fill the
+    // chip; fewer join the next class (305 leaves at 12k DoFs, 98 of them in the first four classes: 1,501 us of
+    // launches after one another, 640 so).
+    const int classes[] = {116, 95, 82, kFusedSmallF, 48, 32};   // above: 1, 2, 3, 4, 6, ... CTAs per SM
+    const auto fills = [&](int f, size_t count) {
+      const int nt = f <= kFusedSmallF ? 128 : 256;
+      const size_t per = std::min<size_t>(768 / nt, kSmemPerSM / (fused_smem(f, nt) + kFusedStatic));
+      return count >= per * c.num_sms;
+    };
     size_t k0 = 0;
-    for (int cl = 0; cl < ncl && k0 < q.size(); cl++) {
-      size_t k1 = k0;
-      while (k1 < q.size() && (cl + 1 == ncl || s.f[q[k1]] > classes[cl + 1])) k1++;
+    for (int cl = 0; k0 < q.size(); cl++) {
+      size_t k1 = q.size();
+      if (cl < 6 && (int)q.size() > 2 * c.num_sms) {
+        k1 = k0;
+        while (k1 < q.size() && s.f[q[k1]] > classes[cl]) k1++;
+        if (k1 < q.size() && !fills(s.f[q[k0]], k1 - k0)) continue;
+      }
       if (k1 == k0) continue;
       fused_groups.push_back({l, (int)fused_h.size(), (int)(k1 - k0), s.f[q[k0]]});
       fused_h.insert(fused_h.end(), q.begin() + k0, q.begin() + k1);
