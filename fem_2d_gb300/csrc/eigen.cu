@@ -1157,7 +1157,7 @@ void sparse_solve(Ctx& c, const Domain& dom, const HostGEP& h, const DeviceGEP& 
   // take 3 to 4, and HierPoly pencils at 1M DoFs on which the product form ran out of cycles converge. A
   // target below zero keeps the product form: c + sigma may vanish there.
   const bool fractions = !iterative && sigma > 0.0;
-  // Out (ld lo) = T x for the nb columns x with B x given (BIn, ld lb); BIn and Out may not alias W1..W3
+  // Out (ld lo) = T x for the nb columns x with B x given (BIn, ld lb); neither may alias W2, W3 or the other
   auto apply_T = [&](const double* BIn, int64_t lb, double* Out, int64_t lo, int nb) {
     if (fractions) {
       if (nref_p == 0 && nref_m == 0) {

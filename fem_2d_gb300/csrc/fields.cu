@@ -27,7 +27,8 @@ constexpr int kSpecChunk = 256;     // specs staged per shared-memory pass
 constexpr size_t kFieldSmemMax = 200 * 1024;   // tables and staged specs
 
 template <int kFieldThreads>
-__global__ void __launch_bounds__(kFieldThreads) fem2d_xy_fields_kernel(const FieldItem* __restrict__ items, const int32_t* __restrict__ item_ptr,
+__global__ void __launch_bounds__(kFieldThreads)
+fem2d_xy_fields_kernel(const FieldItem* __restrict__ items, const int32_t* __restrict__ item_ptr,
                        const int32_t* __restrict__ order,
                        const uint32_t* __restrict__ codes, const int32_t* __restrict__ dofs,
                        const double* __restrict__ sol, int basis, int d0, int d1, int imax, int jmax,

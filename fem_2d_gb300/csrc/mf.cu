@@ -1,12 +1,13 @@
 // Numeric multifrontal factorization and block solves on the device (plan: mf.h, mf_symbolic.cpp).
 //
-// Fronts are dense, column-major, processed level by level (all fronts of a level in one launch per
-// step). Per level: assemble from the CSR values of c_a*A + c_b*B, extend-add the children's Schur
-// complements (one launch per child slot, so no two threads add to one entry), then a blocked
-// right-looking LU of the first p columns with partial pivoting restricted to the fully-summed rows
-// (or no pivoting in Cholesky mode for SPD shifts): panel (one CTA per front), unit-lower TRSM for
-// the U12 rows, FP64 GEMM update of the trailing block. The trailing (f-p)x(f-p) block left in place
-// is the update matrix for the parent.
+// Fronts are dense and column-major, processed level by level. A front that fits one CTA's shared memory is
+// assembled there from the CSR values of c_a*A + c_b*B and its children's Schur complements, its first p columns
+// are eliminated by a blocked LU with partial pivoting restricted to the fully-summed rows (or without
+// pivoting for SPD shifts), and it is written back once with its pivot square inverted (mf_front_kernel).
+// Larger fronts stay in global memory: assembly, extend-add of the children one after the other, then eight
+// columns per launch, a CTA per 8-column strip (mf_strip_kernel), and the inverses by strips
+// (mf_inverse_kernel, mf_partinv_kernel). The trailing (f-p)x(f-p) block left in place is the update matrix
+// for the parent.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(256) mf_extend_add_kernel(const int32_t* __res
 // one or two barriers, and pivots are compared as integers (a double comparison takes a slot of the FP64
 // pipe). Passing each front through global memory seven times per 32 columns (assembly, extend-adds, panel,
 // triangular solve, update, inverse, with 20 to 400 us per panel whatever its size) took 0.59 ms per
-// factorization at 832 DoFs, 3.7 at 29k, 7.0 at 83k and 59 at 1M; now 0.24, 2.6, 4.7 and 37.
+// factorization at 832 DoFs, 3.7 at 29k, 7.0 at 83k and 59 at 1M; now 0.24, 2.5, 4.1 and 33.
 // Larger fronts, and those above kFusedNarrowF rows of levels that would leave SMs idle, stay in global
 // memory and are factored by many CTAs each (mf_strip_kernel): a front of 160 rows keeps one SM's FP64 pipe
 // busy for half a millisecond. (Lines at 32 to 128 rows were within 10% of each other at 5k to 83k DoFs;
@@ -648,7 +649,8 @@ __global__ void __launch_bounds__(NT, 768 / NT) mf_front_kernel(const int32_t* _
 // update of the rows below -- and the CTA of strip s then factors that strip, the next micro-panel, while the
 // other strips are still being updated. A strip of f rows costs a few microseconds, so a narrow level of
 // large fronts is spread over the chip instead of being bound by one SM's FP64 rate per front; 32-column
-// panels by one CTA, whose own update is nearly all of it on one SM's FP64 pipe, took 85 to 170 us each at 1M DoFs, a strip step 20 to 80.
+// panels by one CTA, whose own update is nearly all of it on one SM's FP64 pipe, took 85 to 170 us each at 1M DoFs,
+// a strip step 20 to 80.
 // RPT: rows of the strip per thread in the micro-panel; 0: the front has more rows than fit, the strip stays
 // in global memory.
 template <int NT, int RPT>
@@ -897,8 +899,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256)
 // ------------------------------------------------------------------ small-front solves
 // Fronts with p <= kSmallP and f <= kSmallF (every front of an Elem-level elimination tree at the
 // orders this library meets in practice) are solved by one CTA each, with no sequential triangular
-// substitution: after the factorization, mf_invdiag_kernel overwrites each such front's p x p
-// diagonal LU square by (unit lower L11^-1, upper U11^-1), so both solve directions become dense,
+// substitution: the factorization leaves (unit lower L11^-1, upper U11^-1) in each such front's p x p
+// diagonal square (invert_square, or mf_inverse_kernel), so both solve directions become dense,
 // fully parallel products:
 //   forward:  y = L11^-1 P b_p,  b_s -= L21 y          (b_s goes to the parent)
 //   backward: x_p = U11^-1 (y - U12 x_s)
@@ -1086,7 +1088,8 @@ __device__ __forceinline__ void pair_dot(const double* __restrict__ A, const dou
   r1 = n1 < n ? r1 : acc;
 }
 
-// One factorization of the plan and what a solve with it writes. A launch serves one or two of them: the solves of one right-hand side with both shifted matrices go level by level together.
+// One factorization of the plan and what a solve with it writes. A launch serves one or two of them: the solves of
+// one right-hand side with both shifted matrices go level by level together.
 struct SolveSet {
   const int32_t *perm, *iperm;
   const double* F;
@@ -1248,8 +1251,8 @@ __global__ void __launch_bounds__(NT) mf_backward_small_kernel(const int32_t* __
 // FP64 rate per SM (under two FMA per clock) makes any solve confined to a few SMs the bottleneck. After
 // the factorization, every front of such a level is turned into its partitioned
 // inverse:
-//   diagonal square: unit lower L11^-1 and upper U11^-1      (mf_invdiag_kernel / _wide_kernel)
-//   L21 -> L21' = -L21 L11^-1,  U12 -> U12' = -U11^-1 U12    (mf_partinv_kernel)
+//   diagonal square: unit lower L11^-1 and upper U11^-1      (invert_square / mf_inverse_kernel)
+//   L21 -> L21' = -L21 L11^-1,  U12 -> U12' = -U11^-1 U12    (partinv_shared / mf_partinv_kernel)
 // so that each solve direction is one dense product with no dependency between rows:
 //   forward:  out[r] = v[r] + sum_{k < min(r, p)} F(r, k) v[k]            every row r < f
 //   backward: x[r]   = sum_{k = r}^{f - 1} F(r, k) z[k],  z = [y; x_s]    every pivot row r < p
@@ -1265,7 +1268,7 @@ __global__ void __launch_bounds__(NT) mf_backward_small_kernel(const int32_t* __
 // (24 right-hand sides), a level of 54 to 213 fronts on one CTA per front 27 to 35 us; now 8 to 14 us.
 constexpr int kTileRows = 8;
 constexpr int kChunkK = 128;
-constexpr int kTiledMaxP = 768;   // the wide inversion keeps one column per thread in shared memory
+constexpr int kTiledMaxP = 768;   // an inverse's strip and its diagonal blocks fit 98 KB of shared memory: two CTAs per SM
 constexpr int kTileThreads = 128;
 constexpr int kTiledLeaves = 2;   // per SM
 constexpr int kTileSteps = kChunkK / 16;   // MMA steps (4 columns of the front) per warp and chunk
@@ -2045,10 +2048,10 @@ void MFDevice::solve_sets(Ctx& c, int sets, const MFFactor* f1, const MFFactor* 
 // The dense eigensolve reads the lower triangle of B^-1 A, whose structurally zero entries are rounding noise of
 // 1e-17, and the sign of its eigenvector follows the signs of that noise through the Householder reflectors: one
 // ulp in four of the 55 entries of a 10-DoF problem turns the vector round. The order of the sums is part
-// of that result, so it does not follow the tuned kernels (with them 37 of 120 small problems changed sign): LU in panels of 32 columns without pivoting, a
-// column's sums in plain loops, inverted squares, and on levels of few or large fronts (`parted`: by the tree alone,
-// so that the order is the same on every chip) the partitioned inverse. At most 1,000 DoFs: one CTA per front, then one per front and 32
-// columns; bound by the latency of a level (123 DoFs: 2.25 ms a solve with the tuned kernels, 2.27 with these; 370 to
+// of that result, so it does not follow the tuned kernels (with them 37 of 120 small problems changed sign): LU in
+// panels of 32 columns without pivoting, a column's sums in plain loops, inverted squares, and on levels of few or
+// large fronts (`parted`: by the tree alone, so that the order is the same on every chip) the partitioned inverse.
+// At most 1,000 DoFs: one CTA per front, then one per front and 32 columns; bound by the latency of a level (123 DoFs: 2.25 ms a solve with the tuned kernels, 2.27 with these; 370 to
 // 984 DoFs: 0.6 to 5.6 ms of the 36 to 630 ms that the whole solve takes, most of it on the host;
 // the kernels whose order they keep took 1.5 to 4.8).
 constexpr int kOrderedPanel = 32, kOrderedMaxP = 768, kOrderedParted = 38;

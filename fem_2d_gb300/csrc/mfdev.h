@@ -39,7 +39,7 @@ struct MFDevice {
   DBuf<int64_t> asm_pos, asm_csr, piv_off, woff;
   DBuf<double> work, work2;   // workspaces; the second for pairs of solves, where the plan makes them
   DBuf<int> flags;
-  DBuf<int32_t> weak_list;   // capacity n: weak-pivot DoFs recorded by the panel kernel
+  DBuf<int32_t> weak_list;   // capacity n: weak-pivot DoFs recorded by the factorization
   DBuf<int> weak_count;
   // per level, the fronts solved by one CTA each (inverted diagonal blocks) and the rest (clusters)
   std::vector<int32_t> small_ptr, large_ptr;   // nlevels + 1 offsets into lsmall / llarge

@@ -122,8 +122,8 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 
 // The eight digits of va and vb relative to E, the biased exponent of the largest magnitude of their column
 // (or row), packed as BF16 pairs with va's in the low half: digit s is bits 49 - 7 s .. 55 - 7 s of the
-// mantissa shifted to E, with the value's sign. The kernels are bound by this integer work, so a pair of digits goes through each
-// step at once: a 28-bit half of the mantissa holds two 14-bit fields, one byte permute lays the same field of
+// mantissa shifted to E, with the value's sign. The kernels are bound by this integer work, so a pair of digits
+// goes through each step at once: a 28-bit half of the mantissa holds two 14-bit fields, one byte permute lays the same field of
 // both values side by side, and the BF16 number 128 + d is the bit pattern 0x4300 | d, from which one packed
 // FMA, (128 + d) sign - 128 sign, makes the signed digit. Some 26 instructions a value instead of 40.
 __device__ __forceinline__ uint32_t signed_digits(uint32_t d, uint32_t sign, uint32_t off) {
@@ -356,7 +356,6 @@ __global__ void __launch_bounds__(kGramThreads, 2)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (tid == 0) {
         const uint32_t aBase = smem_addr(sA), bBase = smem_addr(sB);
-#pragma unroll 1
         // digit s2 of X against Y's digit planes 0 .. 7 - s2 stacked along N, written at TMEM column
         // 32 s2: the pair (s2, t) lands in accumulator g = s2 + t (one MMA per digit of X; an MMA costs
         // about the same for every N up to 64, so wide N pays)
@@ -433,7 +432,6 @@ __global__ void __launch_bounds__(kGramThreads, 2)
   for (int j = 0; j < kHalf; j++) out[j] = acc[j];
 }
 
-// C[i * b + j] (row-major a x b) = sum over the CTAs of row range of the partial tiles
 // C = the sum of the partial tiles over the CTA row ranges, in a fixed order: 32 entries of one row of a tile
 // per CTA, eight threads each (one thread per entry took 42 us for 304 row ranges)
 __global__ void __launch_bounds__(256) ozaki_reduce_kernel(const double* __restrict__ P, int nrb, int ny, int a, int b,
@@ -723,7 +721,6 @@ __global__ void __launch_bounds__(GemmShape<PARTS>::threads, PARTS == 4 ? 1 : 2)
       if (stages == 1 && more) gemm_stage<PARTS>(sets, n, a, nt, ntiles, nk, sX);
       const bool first = (k0 % kChunk) == 0;   // the accumulators restart every 128 columns of K
       if (tid == 0) {
-#pragma unroll 1
         // digit s2 of X against C's digit planes 0 .. 7 - s2 stacked along N, written at TMEM column
         // 32 s2: the pair (s2, t) lands in accumulator g = s2 + t
 #pragma unroll 1
@@ -808,9 +805,9 @@ __global__ void __launch_bounds__(GemmShape<PARTS>::threads, PARTS == 4 ? 1 : 2)
 // s + t = g -- at most 8 pairs x 64 columns x 127^2 < 2^24, exact in FP32 -- and each TMEM lane holds
 // one or two such sums per run row. With nb <= 16 the eight groups x 16 columns fill one 128-row
 // operand (8 MMAs per plane step); with nb <= 32, groups 0..3 and 4..7 x 32 columns fill two (4 and 8
-// MMAs). Sums are joined exactly in int64 by their output's owner, fused into one integer and converted once per item and output to FP64 (one conversion and one FMA) and summed per run in
-// registers; every run is owned by one CTA, which writes
-// its rows of Y once (no atomics, no zero fill, deterministic). Pairs with s + t >= 8 are dropped: below
+// MMAs). Sums are joined exactly in int64 by their output's owner, fused into one integer, converted once per item
+// and output to FP64 (one conversion and one FMA) and summed per run in registers; every run is owned by one CTA,
+// which writes its rows of Y once (no atomics, no zero fill, deterministic). Pairs with s + t >= 8 are dropped: below
 // 2^-52 of max|m| max|x| of the item per term, FP64 rounding level in the normwise sense.
 //
 // Pipeline: two CTAs per SM, one shared-memory stage each, so one CTA's slicing overlaps the other's MMAs and
